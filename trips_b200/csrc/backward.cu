@@ -5,9 +5,9 @@
 //   * a warp per 8x4 pixel tile; the reference's O(K^2) inner loop (RenderBackward.cu:284-301) becomes a reverse
 //     running sum over the pixel's kept fragments;
 //   * fragments add image-space sums to a 32-byte row of their entry (one row per visible point and view, in screen
-//     order); the chain to position / size / pose is applied once per entry (entry_grad_finish_kernel), which adds to
-//     a 32-byte row per point (stored by spatial rank); one pass then writes the reference's layouts
-//     (unpack_point_kernel);
+//     order); one thread per point then gathers the rows of the point's entries (the binning pass noted which entry a
+//     point has in every view), applies the chain to position / size once per entry and writes the reference's
+//     layouts (point_grad_kernel); the camera sums are a pass of their own over the entries (entry_cam_grad_kernel);
 //   * pixels are enumerated with the ceil-halved layer sizes of the forward pass (the reference halves with
 //     floor here, RenderBackward.cu:112-130, and thereby skips rows of odd-sized layers).
 #include "common.cuh"
@@ -374,7 +374,7 @@ __global__ __launch_bounds__(kBwdThreads, (C <= 4 ? kBwdMinBlocks : 1)) void ble
                 const float lf  = pr.use_layer_point_size ? layer_factor<true>(ps, layer_s, g.L, &lf_grad) : 1.f;
                 const float gbs = conf * lf * ga;  // dLoss / d(bilinear weight) (RenderBackward.cu:385)
                 // image-space sums of the entry: the chain to position / size / pose is linear in them and is applied
-                // once per entry by entry_grad_finish_kernel
+                // once per entry by point_grad_kernel
                 const float4 h0 = make_float4(J0 * gbs, J1 * gbs, bf * conf * lf_grad * ga, bf * lf * ga);
                 float gt[(C + 3) & ~3];
 #pragma unroll
@@ -463,30 +463,176 @@ cudaError_t launch_blend_backward(const ScenePtrs& sc, const CamConst* cams, con
 }
 
 // ------------------------------------------------------------------------------------------------------------
-// per-entry gradient rows -> per-point sums (one set of atomics per visible point and view instead of one per
-// fragment), then the reference's output layouts (PointRenderer.cu:1423-1426)
+// per-entry gradient rows -> per-point gradients in the reference's output layouts (PointRenderer.cu:1423-1426)
 // ------------------------------------------------------------------------------------------------------------
-// Applies, once per entry, the chain from the accumulated image-space sums to the point: crop rotation, crop
-// transform, pinhole, division by z and the rotation (ProjectPointPinholeBackward, PointRendererHelper.h:434-494,
-// zero distortion), the softplus derivative for the size, and adds the entry's gradients to its point
-// (one set of atomics per visible point and view instead of one per fragment).  Pose and intrinsics gradients
-// are summed per view in double (RenderBackward.cu:453-466,587-611).
-// DIST: lens distortion between the division by z and the pinhole matrix (TripsRenderParams.distortion): the
-// view-space position then comes from the entry's world position (the stored projection cannot be undistorted in
-// closed form), the chain goes through J_p_dis^T and the eight coefficients receive J_dis_dis^T
-// (PointRendererHelper.h:468-491).  A separate instantiation: the plain pinhole carries none of it.
-template <int C, bool CAM_GRADS, bool DIST>
-__global__ __launch_bounds__(256) void entry_grad_finish_kernel(FwdBuffers fb, BwdBuffers bb, const CamConst* __restrict__ cams, int B)
+// View-space gradient of one entry from its image-space sums (sx, sy): crop rotation, crop transform, pinhole, lens
+// distortion (DIST), division by z (ProjectPointPinholeBackward, PointRendererHelper.h:434-494).
+struct ViewGrad
+{
+    float gv0, gv1, gv2;  // gradient of the view-space position
+    float gk0, gk1;       // gradient of the image-plane position before the crop transform
+    float kx, ky;         // the normalised coordinates the pinhole matrix sees
+    float gn0, gn1;       // gradient of the (distorted) normalised coordinates
+};
+
+template <bool DIST>
+__device__ __forceinline__ ViewGrad view_gradient(const CamConst& cam, float vx, float vy, float vz, float sx, float sy, float* Jk)
+{
+    ViewGrad r;
+    const float iz  = 1.f / vz;
+    const float gr0 = cam.r00 * sx + cam.r10 * sy;
+    const float gr1 = cam.r01 * sx + cam.r11 * sy;
+    r.gk0           = cam.cfx * gr0;
+    r.gk1           = cam.cs * gr0 + cam.cfy * gr1;
+    r.gn0           = cam.fx * r.gk0;
+    r.gn1           = cam.s * r.gk0 + cam.fy * r.gk1;
+    r.kx = vx * iz, r.ky = vy * iz;
+    float gn0 = r.gn0, gn1 = r.gn1;
+    if constexpr (DIST)
+    {
+        float xd, yd, Jd[4];
+        distort_point(cam, r.kx, r.ky, xd, yd, Jd, Jk);
+        gn0  = Jd[0] * r.gn0 + Jd[2] * r.gn1;
+        gn1  = Jd[1] * r.gn0 + Jd[3] * r.gn1;
+        r.kx = xd, r.ky = yd;
+    }
+    r.gv0 = iz * gn0;
+    r.gv1 = iz * gn1;
+    r.gv2 = (-vx * iz * iz) * gn0 + (-vy * iz * iz) * gn1;
+    return r;
+}
+
+// One thread per point: reads the point's entry index in every view, gathers the gradient rows of those entries, applies
+// the chain to the position and the softplus derivative to the size, sums over the views in view order (the same result
+// every time) and writes the output layouts once.
+//
+// Why a gather: the rows are read once each (32 bytes of a 64-byte DRAM piece), next to 4 B of entry index per point and
+// view and 20 B of point data.  Adding the rows to per-point accumulators entry by entry, which this replaces, read the
+// entry heads as well, needed 36 B per point cleared, updated by atomics, and read again in another order, and a spatial
+// sort of the points to keep those updates in L2.
+// Measured, the whole gradient bookkeeping (clearing, this kernel, camera sums), per-point accumulators / gather:
+// 6 M points x 8 views 1.05 / 0.73 ms, x 1 view 0.44 / 0.30 ms, 20 M x 2 views 1.54 / 0.85 ms, 2 M x 4 views 0.22 / 0.16 ms.
+// Random 32-byte reads: latency and loads in flight bound it (resident blocks of 256 threads at 3 / 4 / 5: 0.77 / 0.73 / 0.93 ms
+// on 6 M x 8, 0.99 / 0.85 / 1.04 ms on 20 M x 2; 5 spill).
+// With a texture index the descriptor / confidence gradients of all points sharing a column are added (atomics into
+// zeroed outputs); with the identity index they are plain stores.
+constexpr int kGradViews = 4;   // views whose rows a thread requests before it waits for any of them
+constexpr int kGradCams  = 32;  // cameras held in shared memory; further ones are read from global memory (uniform addresses)
+template <int C, bool DIST>
+__global__ __launch_bounds__(256, (C <= 4 ? 4 : 1)) void point_grad_kernel(ScenePtrs sc, FwdBuffers fb, BwdBuffers bb, const CamConst* __restrict__ cams, int B,
+                                                         TripsGrads out, const float* __restrict__ raw_texture,
+                                                         const float* __restrict__ raw_confidence, float confidence_scale)
 {
     constexpr int GS = egrad_stride(C);
-    constexpr int PS = egrad_stride(C);  // per-point row: xyz + size | descriptor row
-    constexpr int NA = CAM_GRADS ? (DIST ? 19 : 11) : 1;  // 6 pose + 5 pinhole (+ 8 distortion) sums per view
+    constexpr int C4 = (C + 3) & ~3;
+    __shared__ CamConst s_cam[kGradCams];
+    for (int k = threadIdx.x; k < min(B, kGradCams) * (int)(sizeof(CamConst) / 4); k += 256) ((int*)s_cam)[k] = ((const int*)cams)[k];
+    __syncthreads();
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < (size_t)sc.N; i += (size_t)gridDim.x * blockDim.x)
+    {
+        const float4 p  = __ldg(sc.position + i);
+        const float raw = __ldg(sc.point_size + i);
+        float gp0 = 0.f, gp1 = 0.f, gp2 = 0.f, gl = 0.f, gc = 0.f;
+        float gt[C4];
+#pragma unroll
+        for (int c = 0; c < C4; ++c) gt[c] = 0.f;
+        for (int vb = 0; vb < B; vb += kGradViews)
+        {
+            uint32_t ent[kGradViews];
+            float4 s4[kGradViews], row[kGradViews][C4 / 4];
+#pragma unroll
+            for (int j = 0; j < kGradViews; ++j) ent[j] = vb + j < B ? __ldg(fb.point_entry + (size_t)(vb + j) * sc.N + i) : kNoEntry;
+#pragma unroll
+            for (int j = 0; j < kGradViews; ++j)
+                if (ent[j] != kNoEntry)
+                {
+                    const float* eg = bb.egrad + (fb.entry_base[vb + j] + ent[j]) * GS;
+                    s4[j]           = *reinterpret_cast<const float4*>(eg);  // sum J0 gbs, sum J1 gbs, sum bf conf lf' ga, sum bf lf ga
+#pragma unroll
+                    for (int c = 0; c < C4; c += 4) row[j][c / 4] = *reinterpret_cast<const float4*>(eg + 4 + c);
+                }
+#pragma unroll
+            for (int j = 0; j < kGradViews; ++j)
+            {
+                if (ent[j] == kNoEntry) continue;
+                const int v         = vb + j;
+                const CamConst& cam = v < kGradCams ? s_cam[v] : cams[v];
+                float vx, vy, vz;
+                transform_point(cam, p.x, p.y, p.z, vx, vy, vz);
+                if (vz > 0.f && (s4[j].x != 0.f || s4[j].y != 0.f || s4[j].z != 0.f))
+                {
+                    const ViewGrad r = view_gradient<DIST>(cam, vx, vy, vz, s4[j].x, s4[j].y, nullptr);
+                    gp0 += cam.R[0] * r.gv0 + cam.R[3] * r.gv1 + cam.R[6] * r.gv2;
+                    gp1 += cam.R[1] * r.gv0 + cam.R[4] * r.gv1 + cam.R[7] * r.gv2;
+                    gp2 += cam.R[2] * r.gv0 + cam.R[5] * r.gv1 + cam.R[8] * r.gv2;
+                    gl += (cam.fx * cam.cfx / vz) * s4[j].z;
+                }
+                gc += s4[j].w;
+#pragma unroll
+                for (int c = 0; c < C4; c += 4)
+                {
+                    const float4 t4 = row[j][c / 4];
+                    gt[c] += t4.x, gt[c + 1] += t4.y, gt[c + 2] += t4.z, gt[c + 3] += t4.w;
+                }
+            }
+        }
+        if (out.points) reinterpret_cast<float4*>(out.points)[i] = make_float4(gp0, gp1, gp2, 0.f);
+        if (out.point_size) out.point_size[i] = gl == 0.f ? 0.f : tm_softplus_grad(raw) * gl;
+        // fused texture preparation: chain through sigmoid(scale * raw) and |raw| (raw_* are null when the caller passes
+        // activated tensors)
+        const int col = sc.index ? __ldg(sc.index + i) : (int)i;
+        if ((unsigned)col < (unsigned)sc.n_tex)
+        {
+            if (raw_confidence)
+            {
+                const float sg = tm_sigmoid(confidence_scale * raw_confidence[col]);
+                gc             = gc * (confidence_scale * (sg * (1.f - sg)));
+            }
+            if (raw_texture)
+            {
+#pragma unroll
+                for (int c = 0; c < C; ++c)
+                {
+                    const float w = raw_texture[(size_t)c * sc.n_tex + col];
+                    gt[c]         = w > 0.f ? gt[c] : (w < 0.f ? -gt[c] : 0.f);
+                }
+            }
+        }
+        if (!sc.index)
+        {
+            if (out.texture)
+            {
+#pragma unroll
+                for (int c = 0; c < C; ++c) out.texture[(size_t)c * sc.n_tex + i] = gt[c];
+            }
+            if (out.confidence) out.confidence[i] = gc;
+        }
+        else if ((unsigned)col < (unsigned)sc.n_tex)
+        {
+            if (out.texture)
+            {
+#pragma unroll
+                for (int c = 0; c < C; ++c)
+                    if (gt[c] != 0.f) atomicAdd(out.texture + (size_t)c * sc.n_tex + col, gt[c]);
+            }
+            if (out.confidence && gc != 0.f) atomicAdd(out.confidence + col, gc);
+        }
+    }
+}
+
+// Pose and intrinsics gradients, summed per view in double over the entries of the view (RenderBackward.cu:453-466,587-611).
+// DIST: the view-space position comes from the entry's world position (the stored projection cannot be undistorted in
+// closed form) and the eight coefficients receive J_dis_dis^T (PointRendererHelper.h:468-491).
+template <int C, bool DIST>
+__global__ __launch_bounds__(256) void entry_cam_grad_kernel(FwdBuffers fb, BwdBuffers bb, const CamConst* __restrict__ cams, int B)
+{
+    constexpr int GS = egrad_stride(C);
+    constexpr int NA = DIST ? 19 : 11;  // 6 pose + 5 pinhole (+ 8 distortion) sums per view
     __shared__ CamConst cam;
     __shared__ double s_acc[8][NA];
     const int b = blockIdx.y;
     if (threadIdx.x < sizeof(CamConst) / 4) ((int*)&cam)[threadIdx.x] = ((const int*)&cams[b])[threadIdx.x];
     __syncthreads();
-    const float fxc = cam.fx * cam.cfx;
     const unsigned long long first = fb.entry_base[b], n = fb.entry_base[b + 1] - first;
     const float4* head   = fb.ent_head + first * 2;
     const float* egrad   = bb.egrad + first * GS;
@@ -496,17 +642,11 @@ __global__ __launch_bounds__(256) void entry_grad_finish_kernel(FwdBuffers fb, B
     for (unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += (unsigned long long)gridDim.x * blockDim.x)
     {
-        const float* eg = egrad + i * GS;
-        const float4 s4 = *reinterpret_cast<const float4*>(eg);      // sum J0 gbs, sum J1 gbs, sum bf conf lf' ga, sum bf lf ga
-        const float4 e1 = head[2 * i + 1];  // pid z raw nl|rank
+        const float4 s4 = *reinterpret_cast<const float4*>(egrad + i * GS);
+        const float4 e1 = head[2 * i + 1];  // pid z raw nl
         const float4 e0 = head[2 * i];      // u v ps conf
-        const int pid   = __float_as_int(e1.x);
-        // row of the point: by spatial rank when the forward pass stored one (rows of a screen bin then share L2 lines)
-        const size_t row = fb.point_rank ? (size_t)(__float_as_uint(e1.w) >> kRankShift) : (size_t)pid;
         // View-space position from the stored projection: (u, v) back through crop rotation, crop transform and the
-        // pinhole matrix gives the normalised coordinates, the stored depth scales them.  This spares the read of the
-        // entry's world position (a third of the kernel's DRAM traffic); the round trip costs a few 1e-7 relative,
-        // far inside the gradient tolerance.
+        // pinhole matrix gives the normalised coordinates, the stored depth scales them.
         float vz = e1.y;
         float vx, vy;
         if constexpr (DIST)
@@ -529,214 +669,91 @@ __global__ __launch_bounds__(256) void entry_grad_finish_kernel(FwdBuffers fb, B
         }
         if (vz > 0.f && (s4.x != 0.f || s4.y != 0.f || s4.z != 0.f))
         {
-            const float iz  = 1.f / vz;
-            const float gr0 = cam.r00 * s4.x + cam.r10 * s4.y;
-            const float gr1 = cam.r01 * s4.x + cam.r11 * s4.y;
-            const float gk0 = cam.cfx * gr0;
-            const float gk1 = cam.cs * gr0 + cam.cfy * gr1;
-            float gn0 = cam.fx * gk0;
-            float gn1 = cam.s * gk0 + cam.fy * gk1;
-            float kx = vx * iz, ky = vy * iz;  // the normalised coordinates the pinhole matrix sees
+            float Jk[16];
+            const ViewGrad r = view_gradient<DIST>(cam, vx, vy, vz, s4.x, s4.y, DIST ? Jk : nullptr);
             if constexpr (DIST)
             {
-                float xd, yd, Jd[4], Jk[16];
-                distort_point(cam, kx, ky, xd, yd, Jd, CAM_GRADS ? Jk : nullptr);
-                if constexpr (CAM_GRADS)
-                {
 #pragma unroll
-                    for (int k = 0; k < 8; ++k) acc[11 + k] += (double)(Jk[k] * gn0 + Jk[8 + k] * gn1);
-                }
-                const float g0 = Jd[0] * gn0 + Jd[2] * gn1;
-                const float g1 = Jd[1] * gn0 + Jd[3] * gn1;
-                gn0 = g0, gn1 = g1;
-                kx = xd, ky = yd;
+                for (int k = 0; k < 8; ++k) acc[11 + k] += (double)(Jk[k] * r.gn0 + Jk[8 + k] * r.gn1);
             }
-            const float gv0 = iz * gn0;
-            const float gv1 = iz * gn1;
-            const float gv2 = (-vx * iz * iz) * gn0 + (-vy * iz * iz) * gn1;
-            const float gp0 = cam.R[0] * gv0 + cam.R[3] * gv1 + cam.R[6] * gv2;
-            const float gp1 = cam.R[1] * gv0 + cam.R[4] * gv1 + cam.R[7] * gv2;
-            const float gp2 = cam.R[2] * gv0 + cam.R[5] * gv1 + cam.R[8] * gv2;
-            const float gl  = tm_softplus_grad(e1.z) * (fxc / vz) * s4.z;
-            atomicAdd(reinterpret_cast<float4*>(bb.g_point + row * PS), make_float4(gp0, gp1, gp2, gl));
-            if constexpr (CAM_GRADS)
-            {
-                const float nx = kx, ny = ky;
-                acc[0] += (double)gv0;
-                acc[1] += (double)gv1;
-                acc[2] += (double)gv2;
-                acc[3] += (double)(vy * gv2 - vz * gv1);
-                acc[4] += (double)(vz * gv0 - vx * gv2);
-                acc[5] += (double)(vx * gv1 - vy * gv0);
-                acc[6] += (double)(nx * gk0);
-                acc[7] += (double)(ny * gk1);
-                acc[8] += (double)gk0;
-                acc[9] += (double)gk1;
-                acc[10] += (double)(ny * gk0);
-            }
+            acc[0] += (double)r.gv0;
+            acc[1] += (double)r.gv1;
+            acc[2] += (double)r.gv2;
+            acc[3] += (double)(vy * r.gv2 - vz * r.gv1);
+            acc[4] += (double)(vz * r.gv0 - vx * r.gv2);
+            acc[5] += (double)(vx * r.gv1 - vy * r.gv0);
+            acc[6] += (double)(r.kx * r.gk0);
+            acc[7] += (double)(r.ky * r.gk1);
+            acc[8] += (double)r.gk0;
+            acc[9] += (double)r.gk1;
+            acc[10] += (double)(r.ky * r.gk0);
         }
-        // (an entry whose texture index is out of range was drawn with alpha 0: its sums are zero, and the unpack pass
-        // skips its column anyway)
-        if (s4.w != 0.f) atomicAdd(bb.g_conf_pt + row, s4.w);
-        float gt[(C + 3) & ~3];
-        bool any = false;
-#pragma unroll
-        for (int c = 0; c < ((C + 3) & ~3); c += 4)
-        {
-            const float4 v4 = *reinterpret_cast<const float4*>(eg + 4 + c);
-            gt[c] = v4.x, gt[c + 1] = v4.y, gt[c + 2] = v4.z, gt[c + 3] = v4.w;
-            any |= (v4.x != 0.f || v4.y != 0.f || v4.z != 0.f || v4.w != 0.f);
-        }
-        // descriptor gradients share the point's row with the position gradient: both atomics hit one 32-byte sector
-        if (any) atomic_add_row<((C + 3) & ~3)>(bb.g_point + row * PS + 4, gt);
     }
-    if constexpr (CAM_GRADS)
-    {
-        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-        for (int k = 0; k < NA; ++k)
+    for (int k = 0; k < NA; ++k)
+    {
+        const double v = warp_sum_d(acc[k]);
+        if (lane == 0) s_acc[warp][k] = v;
+    }
+    __syncthreads();
+    if (threadIdx.x < NA)
+    {
+        double v = 0.0;
+        for (int w = 0; w < 8; ++w) v += s_acc[w][threadIdx.x];
+        if (v != 0.0)
         {
-            const double v = warp_sum_d(acc[k]);
-            if (lane == 0) s_acc[warp][k] = v;
-        }
-        __syncthreads();
-        if (threadIdx.x < NA)
-        {
-            double v = 0.0;
-            for (int w = 0; w < 8; ++w) v += s_acc[w][threadIdx.x];
-            if (v != 0.0)
-            {
-                if (threadIdx.x < 6)
-                    atomicAdd(bb.g_pose + (size_t)b * 6 + threadIdx.x, v);
-                else if (threadIdx.x < 11)
-                    atomicAdd(bb.g_k + (size_t)b * 5 + (threadIdx.x - 6), v);
-                else
-                    atomicAdd(bb.g_dis + (size_t)b * 8 + (threadIdx.x - 11), v);
-            }
+            if (threadIdx.x < 6)
+                atomicAdd(bb.g_pose + (size_t)b * 6 + threadIdx.x, v);
+            else if (threadIdx.x < 11)
+                atomicAdd(bb.g_k + (size_t)b * 5 + (threadIdx.x - 6), v);
+            else
+                atomicAdd(bb.g_dis + (size_t)b * 8 + (threadIdx.x - 11), v);
         }
     }
 }
 
-// per-point rows (keyed by point id) -> the reference's output layouts (PointRenderer.cu:1423-1426).  With a
-// texture index the descriptor / confidence gradients of all points sharing a column are added (atomics into
-// zeroed outputs); with the identity index they are plain stores.
-template <int C>
-__global__ __launch_bounds__(256) void unpack_point_kernel(const float* __restrict__ g_point, const float* __restrict__ g_conf_pt,
-                                                           const uint32_t* __restrict__ rank, const int32_t* __restrict__ index, int N, int n_tex,
-                                                           float4* __restrict__ g_points, float* __restrict__ g_size,
-                                                           float* __restrict__ g_texture, float* __restrict__ g_confidence,
-                                                           const float* __restrict__ raw_texture, const float* __restrict__ raw_confidence,
-                                                           float confidence_scale)
+// One block; a thread per component (the views of a call may share an image / camera index, so every component adds its
+// views in order).  One thread for everything took 12 us longer with 4 views: 76 dependent read-modify-writes.
+__global__ __launch_bounds__(64) void unpack_small_kernel(int C, int B, const CamConst* __restrict__ cams, const double* __restrict__ g_bg,
+                                                          const double* __restrict__ g_pose, const double* __restrict__ g_k,
+                                                          const double* __restrict__ g_dis, float* out_bg, double* out_pose, float* out_intr)
 {
-    constexpr int PS = egrad_stride(C);
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < (size_t)N; i += (size_t)gridDim.x * blockDim.x)
+    const int t = threadIdx.x;
+    if (out_bg && t < C) out_bg[t] = (float)g_bg[t];
+    if (out_pose && t < 6)
+        for (int b = 0; b < B; ++b) out_pose[(size_t)cams[b].image_index * 6 + t] += g_pose[b * 6 + t];
+    if (out_intr && t >= 32 && t < 45)
     {
-        const size_t r = rank ? (size_t)rank[i] : i;  // where the point's row lives
-        const float4 v = *reinterpret_cast<const float4*>(g_point + r * PS);
-        if (g_points) g_points[i] = make_float4(v.x, v.y, v.z, 0.f);
-        if (g_size) g_size[i] = v.w;
-        float gt[(C + 3) & ~3];
-#pragma unroll
-        for (int c = 0; c < ((C + 3) & ~3); c += 4)
-        {
-            const float4 t4 = *reinterpret_cast<const float4*>(g_point + r * PS + 4 + c);
-            gt[c] = t4.x, gt[c + 1] = t4.y, gt[c + 2] = t4.z, gt[c + 3] = t4.w;
-        }
-        float gc = g_conf_pt[r];
-        // fused texture preparation: chain through sigmoid(scale * raw) and |raw| (raw_* are null when the caller passes
-        // activated tensors)
-        const int col = index ? index[i] : (int)i;
-        if ((unsigned)col < (unsigned)n_tex)
-        {
-            if (raw_confidence)
-            {
-                const float sg = tm_sigmoid(confidence_scale * raw_confidence[col]);
-                gc             = gc * (confidence_scale * (sg * (1.f - sg)));
-            }
-            if (raw_texture)
-            {
-#pragma unroll
-                for (int c = 0; c < C; ++c)
-                {
-                    const float w = raw_texture[(size_t)c * n_tex + col];
-                    gt[c]         = w > 0.f ? gt[c] : (w < 0.f ? -gt[c] : 0.f);
-                }
-            }
-        }
-        if (!index)
-        {
-            if (g_texture)
-            {
-#pragma unroll
-                for (int c = 0; c < C; ++c) g_texture[(size_t)c * n_tex + i] = gt[c];
-            }
-            if (g_confidence) g_confidence[i] = gc;
-        }
-        else
-        {
-            const int tex = index[i];
-            if ((unsigned)tex >= (unsigned)n_tex) continue;
-            if (g_texture)
-            {
-#pragma unroll
-                for (int c = 0; c < C; ++c)
-                    if (gt[c] != 0.f) atomicAdd(g_texture + (size_t)c * n_tex + tex, gt[c]);
-            }
-            if (g_confidence && gc != 0.f) atomicAdd(g_confidence + tex, gc);
-        }
-    }
-}
-
-__global__ void unpack_small_kernel(int C, int B, const CamConst* __restrict__ cams, const double* g_bg, const double* g_pose,
-                                    const double* g_k, const double* g_dis, float* out_bg, double* out_pose, float* out_intr)
-{
-    // launched with one thread: B and C are tiny, and several views may share an image / camera index
-    if (out_bg)
-        for (int c = 0; c < C; ++c) out_bg[c] = (float)g_bg[c];
-    for (int b = 0; b < B; ++b)
-    {
-        if (out_pose)
-            for (int k = 0; k < 6; ++k) out_pose[(size_t)cams[b].image_index * 6 + k] += g_pose[b * 6 + k];
-        if (out_intr)
-        {
-            for (int k = 0; k < 5; ++k) out_intr[(size_t)cams[b].camera_index * 13 + k] += (float)g_k[b * 5 + k];
-            for (int k = 0; k < 8; ++k) out_intr[(size_t)cams[b].camera_index * 13 + 5 + k] += (float)g_dis[b * 8 + k];  // zero without distortion
-        }
+        const int k = t - 32;  // 5 pinhole values, then 8 distortion coefficients (zero without distortion)
+        for (int b = 0; b < B; ++b) out_intr[(size_t)cams[b].camera_index * 13 + k] += (float)(k < 5 ? g_k[b * 5 + k] : g_dis[b * 8 + k - 5]);
     }
 }
 
 cudaError_t launch_unpack_grads(const ScenePtrs& sc, const CamConst* cams, int B, const FwdBuffers& fb, const BwdBuffers& bb,
                                 const TripsGrads& out, const TripsRenderParams& pr, int sm_count, cudaStream_t st)
 {
-    // the entry counts live on the device: the grid covers a fixed share of the worst case and threads stride
+    if (sc.N > 0 && (out.pose_tangent || out.intrinsics))
     {
-        const bool cam_grads = out.pose_tangent || out.intrinsics;
-        int bx = max(1, min(sm_count * 8 / max(1, min(B, 8)) + 1, (sc.N + 255) / 256));
-        dim3 grid(bx, B);
-#define TRIPS_FIN_CASE(CC)                                                                                      \
-    case CC:                                                                                                    \
-        if (cam_grads && pr.distortion)                                                                         \
-            entry_grad_finish_kernel<CC, true, true><<<grid, 256, 0, st>>>(fb, bb, cams, B);                    \
-        else if (cam_grads)                                                                                     \
-            entry_grad_finish_kernel<CC, true, false><<<grid, 256, 0, st>>>(fb, bb, cams, B);                   \
-        else if (pr.distortion)                                                                                 \
-            entry_grad_finish_kernel<CC, false, true><<<grid, 256, 0, st>>>(fb, bb, cams, B);                   \
-        else                                                                                                    \
-            entry_grad_finish_kernel<CC, false, false><<<grid, 256, 0, st>>>(fb, bb, cams, B);                  \
+        // the entry counts live on the device: the grid covers a fixed share of the worst case and threads stride
+        const dim3 grid(max(1, min(sm_count * 8 / max(1, min(B, 8)) + 1, (sc.N + 255) / 256)), B);
+#define TRIPS_CAM_CASE(CC)                                                              \
+    case CC:                                                                            \
+        if (pr.distortion)                                                              \
+            entry_cam_grad_kernel<CC, true><<<grid, 256, 0, st>>>(fb, bb, cams, B);     \
+        else                                                                            \
+            entry_cam_grad_kernel<CC, false><<<grid, 256, 0, st>>>(fb, bb, cams, B);    \
         break;
-        if (sc.N > 0)
+        switch (sc.C)
         {
-            switch (sc.C)
-            {
-                TRIPS_FIN_CASE(3)
-                TRIPS_FIN_CASE(4)
-                TRIPS_FIN_CASE(6)
-                TRIPS_FIN_CASE(8)
-                TRIPS_FIN_CASE(16)
-                default: return cudaErrorInvalidValue;
-            }
+            TRIPS_CAM_CASE(3)
+            TRIPS_CAM_CASE(4)
+            TRIPS_CAM_CASE(6)
+            TRIPS_CAM_CASE(8)
+            TRIPS_CAM_CASE(16)
+            default: return cudaErrorInvalidValue;
         }
-#undef TRIPS_FIN_CASE
+#undef TRIPS_CAM_CASE
     }
     if (sc.N > 0 && (out.texture || out.confidence || out.points || out.point_size))
     {
@@ -754,26 +771,28 @@ cudaError_t launch_unpack_grads(const ScenePtrs& sc, const CamConst* cams, int B
                 if (e != cudaSuccess) return e;
             }
         }
-        int blocks = max(1, (int)min((size_t)sm_count * 16, ((size_t)sc.N + 255) / 256));
-#define TRIPS_UNPACK_CASE(CC)                                                                                           \
-    case CC:                                                                                                            \
-        unpack_point_kernel<CC><<<blocks, 256, 0, st>>>(bb.g_point, bb.g_conf_pt, fb.point_rank, sc.index, sc.N, sc.n_tex,   \
-                                                        (float4*)out.points, out.point_size, out.texture, out.confidence, \
-                                                        pr.texture_abs ? sc.texture : nullptr,                          \
-                                                        pr.confidence_is_raw ? sc.confidence : nullptr, pr.confidence_scale); \
+        const int blocks      = max(1, (int)min((size_t)sm_count * 16, ((size_t)sc.N + 255) / 256));
+        const float* raw_tex  = pr.texture_abs ? sc.texture : nullptr;
+        const float* raw_conf = pr.confidence_is_raw ? sc.confidence : nullptr;
+#define TRIPS_POINT_CASE(CC)                                                                                                              \
+    case CC:                                                                                                                              \
+        if (pr.distortion)                                                                                                                \
+            point_grad_kernel<CC, true><<<blocks, 256, 0, st>>>(sc, fb, bb, cams, B, out, raw_tex, raw_conf, pr.confidence_scale);        \
+        else                                                                                                                              \
+            point_grad_kernel<CC, false><<<blocks, 256, 0, st>>>(sc, fb, bb, cams, B, out, raw_tex, raw_conf, pr.confidence_scale);       \
         break;
         switch (sc.C)
         {
-            TRIPS_UNPACK_CASE(3)
-            TRIPS_UNPACK_CASE(4)
-            TRIPS_UNPACK_CASE(6)
-            TRIPS_UNPACK_CASE(8)
-            TRIPS_UNPACK_CASE(16)
+            TRIPS_POINT_CASE(3)
+            TRIPS_POINT_CASE(4)
+            TRIPS_POINT_CASE(6)
+            TRIPS_POINT_CASE(8)
+            TRIPS_POINT_CASE(16)
             default: return cudaErrorInvalidValue;
         }
-#undef TRIPS_UNPACK_CASE
+#undef TRIPS_POINT_CASE
     }
-    unpack_small_kernel<<<1, 1, 0, st>>>(sc.C, B, cams, bb.g_bg, bb.g_pose, bb.g_k, bb.g_dis, out.background, out.pose_tangent,
+    unpack_small_kernel<<<1, 64, 0, st>>>(sc.C, B, cams, bb.g_bg, bb.g_pose, bb.g_k, bb.g_dis, out.background, out.pose_tangent,
                                          out.intrinsics);
     return cudaGetLastError();
 }

@@ -120,9 +120,9 @@ struct TripsContext
     int sm_count = 148;
     std::string error;
     // forward scratch
-    DevBuf heavy, views, cams, bin_count, bin_base, view_total, bin_cursor, entry_base, entries, counts, offsets, partial, view_base, frags, rec_n, records, stats, ticket, rank, rank_scratch, rank_temp, resize_scratch, block_box, block_skip;
+    DevBuf heavy, views, cams, bin_count, bin_base, view_total, bin_cursor, entry_base, entries, counts, offsets, partial, view_base, frags, rec_n, records, stats, ticket, point_entry, resize_scratch, block_box, block_skip;
     // backward scratch
-    DevBuf egrad, g_point, g_conf_pt, g_small;
+    DevBuf egrad, g_small;
     // adam
     DevBuf adam_tab;
     // pinned host mirror of DevStats and the event behind which it becomes valid when a call did not wait for it
@@ -141,8 +141,6 @@ struct TripsContext
     TripsRenderParams params{};
     int B = 0, N = 0, n_tex = 0, C = 0;
     int nchunks = 0;
-    int rank_points = -1;                  // number of points the spatial ranks were computed for (-1: none yet)
-    int rank_age    = 0;                   // training forward passes since then
     size_t entry_cap = 0;                  // entries the two entry arrays (head | tail, in this order) are laid out for
     TripsStats host_stats{};
 };
@@ -220,7 +218,7 @@ static FwdBuffers fwd_buffers(TripsContext* c)
     fb.records    = (uint2*)c->records.p;
     fb.stats      = (DevStats*)c->stats.p;
     fb.ticket     = (unsigned int*)c->ticket.p;
-    fb.point_rank = c->rank_points >= 0 ? (const uint32_t*)c->rank.p : nullptr;
+    fb.point_entry = c->params.train ? (uint32_t*)c->point_entry.p : nullptr;
     fb.block_box  = (const float*)c->block_box.p;
     fb.block_skip = (const uint8_t*)c->block_skip.p;
     fb.heavy      = (uint2*)c->heavy.p;
@@ -288,8 +286,8 @@ void trips_context_destroy(TripsContext* c)
 {
     if (!c) return;
     DevBuf* all[] = {&c->heavy, &c->views, &c->cams, &c->bin_count, &c->bin_base, &c->view_total, &c->bin_cursor, &c->entry_base, &c->entries, &c->counts, &c->offsets,
-                     &c->partial, &c->view_base, &c->frags, &c->rec_n, &c->records, &c->stats, &c->ticket, &c->egrad, &c->g_point,
-                     &c->g_conf_pt, &c->g_small, &c->adam_tab, &c->rank, &c->rank_scratch, &c->rank_temp, &c->resize_scratch, &c->block_box, &c->block_skip};
+                     &c->partial, &c->view_base, &c->frags, &c->rec_n, &c->records, &c->stats, &c->ticket, &c->egrad,
+                     &c->point_entry, &c->g_small, &c->adam_tab, &c->resize_scratch, &c->block_box, &c->block_skip};
     for (DevBuf* b : all) free_buf(*b);
     c->timers.destroy();
     if (c->h_pinned) cudaFreeHost(c->h_pinned);
@@ -418,6 +416,7 @@ static int forward_views(TripsContext* ctx, const TripsScene* scene, const Trips
     {
         CU_CHECK(ctx, ensure(ctx->rec_n, P * B));
         CU_CHECK(ctx, ensure(ctx->records, sizeof(uint2) * 16 * P * B));
+        CU_CHECK(ctx, ensure(ctx->point_entry, sizeof(uint32_t) * N * B));
     }
     if (ctx->frags.bytes == 0) CU_CHECK(ctx, ensure(ctx->frags, 16 * 1024 * 1024));
     if (!ctx->entries.p || ctx->entry_C != C) CU_CHECK(ctx, ensure_entries(ctx, 1024, C, 1.0));
@@ -430,27 +429,6 @@ static int forward_views(TripsContext* ctx, const TripsScene* scene, const Trips
 
     ScenePtrs sp = scene_ptrs(scene);
     sp.dropout   = dropout;
-    // Spatial ranks of the points (where their gradient rows live, rank.cu): training only; refreshed when the number
-    // of points changes and every kRankRefresh forward passes, since points move slowly and a stale rank is still a
-    // valid permutation.  Entries carry the rank, so the backward pass of this forward pass sees the same ranks.
-    constexpr int kRankRefresh = 512;
-    if (params->train && N > 0 && N < (size_t)kMaxRankedPoints)
-    {
-        if (ctx->rank_points != (int)N || ctx->rank_age >= kRankRefresh)
-        {
-            const size_t tb = rank_temp_bytes((int)N);
-            CU_CHECK(ctx, ensure(ctx->rank, sizeof(uint32_t) * N));
-            CU_CHECK(ctx, ensure(ctx->rank_scratch, sizeof(uint32_t) * (4 * N + 8)));
-            CU_CHECK(ctx, ensure(ctx->rank_temp, tb));
-            CU_CHECK(ctx, launch_point_rank((const float4*)scene->position, (int)N, (unsigned*)ctx->rank_scratch.p, ctx->rank_temp.p, tb,
-                                            (unsigned*)ctx->rank.p, ctx->sm_count, st));
-            ctx->rank_points = (int)N;
-            ctx->rank_age    = 0;
-        }
-        ++ctx->rank_age;
-    }
-    else
-        ctx->rank_points = -1;
     FwdBuffers fb = fwd_buffers(ctx);
     // the counters start from zero; the status word keeps the bits raised by earlier calls until trips_last_status reads them
     CU_CHECK(ctx, clear_counters(ctx, st));
@@ -621,14 +599,10 @@ int trips_backward(TripsContext* ctx, const TripsScene* scene, const float* cons
 
     const size_t GS = (size_t)egrad_stride(C);
     CU_CHECK(ctx, ensure(ctx->egrad, sizeof(float) * GS * ctx->entry_cap + 16));  // one row per entry the arrays can hold
-    CU_CHECK(ctx, ensure(ctx->g_point, sizeof(float) * GS * N + 16));
-    CU_CHECK(ctx, ensure(ctx->g_conf_pt, sizeof(float) * N + 16));
     const size_t small_bytes = sizeof(double) * (TRIPS_MAX_CHANNELS + (size_t)B * 19);  // background | per view: 6 pose, 5 pinhole, 8 distortion
     CU_CHECK(ctx, ensure(ctx->g_small, small_bytes));
     BwdBuffers bb;
     bb.egrad        = (float*)ctx->egrad.p;
-    bb.g_point      = (float*)ctx->g_point.p;
-    bb.g_conf_pt    = (float*)ctx->g_conf_pt.p;
     bb.g_bg         = (double*)ctx->g_small.p;
     bb.g_pose       = bb.g_bg + TRIPS_MAX_CHANNELS;
     bb.g_k          = bb.g_pose + (size_t)B * 6;
@@ -638,9 +612,7 @@ int trips_backward(TripsContext* ctx, const TripsScene* scene, const float* cons
     // all accumulators start from zero (timed with the gradient bookkeeping of the unpack stage)
     auto clear_accumulators = [&]() -> cudaError_t {
         cudaError_t e = cudaSuccess;
-        if (N > 0 && e == cudaSuccess) e = cudaMemsetAsync(ctx->g_point.p, 0, sizeof(float) * GS * N, st);
-        if (N > 0 && e == cudaSuccess) e = cudaMemsetAsync(ctx->g_conf_pt.p, 0, sizeof(float) * N, st);
-        if (e == cudaSuccess) e = cudaMemsetAsync(ctx->g_small.p, 0, small_bytes, st);
+        e = cudaMemsetAsync(ctx->g_small.p, 0, small_bytes, st);
         if (grads->pose_tangent && e == cudaSuccess) e = cudaMemsetAsync(grads->pose_tangent, 0, sizeof(double) * 6 * scene->n_images, st);
         if (grads->intrinsics && e == cudaSuccess) e = cudaMemsetAsync(grads->intrinsics, 0, sizeof(float) * 13 * scene->n_cameras, st);
         if (N > 0 && e == cudaSuccess) e = launch_zero_entry_rows(C, B, fb, bb, ctx->sm_count, st);
@@ -652,7 +624,7 @@ int trips_backward(TripsContext* ctx, const TripsScene* scene, const float* cons
     const bool cam_grads = grads->pose_tangent || grads->intrinsics;
     STAGE(ctx, TRIPS_STAGE_BACKWARD, 1, st,
           launch_blend_backward(sp, (const CamConst*)ctx->cams.p, g, ctx->params, B, fb, bb, gin, cam_grads, ctx->sm_count, st));
-    const int n_unpack = (N > 0 ? 2 : 0) + 1;
+    const int n_unpack = (N > 0 ? 1 + (cam_grads ? 1 : 0) : 0) + 1;
     STAGE(ctx, TRIPS_STAGE_UNPACK, n_unpack, st,
           launch_unpack_grads(sp, (const CamConst*)ctx->cams.p, B, fb, bb, *grads, ctx->params, ctx->sm_count, st));
     return TRIPS_OK;
@@ -870,7 +842,6 @@ int trips_debug_points(TripsContext* ctx, int view, float* depth, int32_t* nlaye
         int32_t pid, nl;
         memcpy(&pid, en + 4, 4);
         memcpy(&nl, en + 7, 4);
-        nl &= (1 << kRankShift) - 1;  // the spatial rank shares the word
         if (pid < 0 || (size_t)pid >= N) continue;
         if (depth) depth[pid] = en[5];
         if (nlayers) nlayers[pid] = nl;

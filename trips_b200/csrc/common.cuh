@@ -13,8 +13,7 @@ constexpr unsigned kFull  = 0xffffffffu;
 constexpr int kBinShift   = 5;   // visible points are bucketed by 32x32-pixel screen bins of layer 0
 constexpr int kTileW      = 8;   // one warp renders / differentiates an 8x4 pixel tile
 constexpr int kTileH      = 4;
-constexpr int kRankShift  = 4;   // entry head: number of layers in the low 4 bits, spatial rank above
-constexpr int kMaxRankedPoints = 1 << 28;
+constexpr uint32_t kNoEntry = 0xffffffffu;  // a point that is not visible in a view
 constexpr int kHeavyList  = 512;      // lists longer than this get their 16 nearest fragments moved to the front by a block of their own
 constexpr int kHeavyCap   = 1 << 16;  // such lists per call the pre-selection handles; beyond that the blend walks them itself
 
@@ -82,8 +81,7 @@ struct DevStats
 // the stage that reads them, so that a stage's gathers touch fewer bytes it does not use (DRAM is read in 64-byte
 // pieces), while the binning pass still writes whole 32-byte sectors:
 //   head [2 x float4]     u, v (layer-0 image position), size in pixels, confidence (all the backward pass reads) |
-//                         point id (bits), view-space depth, raw point size, number of layers written (bits 0-3) and
-//                         spatial rank of the point (bits 4-31, see rank.cu; 0 when ranks are not in use)
+//                         point id (bits), view-space depth, raw point size, number of layers written (bits)
 //   tail [1 + C4/4 float4] world position x, y, z, texture index (bits) | descriptor row (C floats, padded to 4)
 __host__ __device__ constexpr int tail_stride(int C) { return 4 + ((C + 3) & ~3); }
 __host__ __device__ constexpr int entry_stride(int C) { return 8 + tail_stride(C); }  // floats per entry over both arrays
@@ -110,7 +108,7 @@ struct FwdBuffers
     uint2* records;                   // [B,P,16] (entry index within the view, alpha bits)
     DevStats* stats;
     unsigned int* ticket;
-    const uint32_t* point_rank;       // [N] spatial rank of every point, or nullptr: gradient rows are keyed by point id
+    uint32_t* point_entry;            // training: [B,N] entry (within the view) of every point, kNoEntry where it is not visible
     const float* block_box;           // [ceil(N / 8192), 6] bounding boxes (min xyz, max xyz) of blocks of consecutive points
     const uint8_t* block_skip;        // [B, ceil(N / 8192)] 1 = the block cannot hold a point visible in that view
     uint2* heavy;                     // [kHeavyCap] (view, pixel) of the lists longer than kHeavyList
@@ -131,8 +129,6 @@ struct ScenePtrs
 struct BwdBuffers
 {
     float* egrad;         // [sum V_b, egrad_stride] per-entry gradient accumulators
-    float* g_point;       // [N, egrad_stride] per-point sums keyed by point id: xyz + raw size | descriptor row
-    float* g_conf_pt;     // [N] confidence gradient keyed by point id
     double* g_bg;         // [C]
     double* g_pose;       // [B,6]
     double* g_k;          // [B,5]
@@ -325,9 +321,6 @@ int bin_scatter_launches(int N, int B);
 size_t resize_scratch_bytes(int64_t n_points);
 cudaError_t launch_resize_points(const int64_t* remove, int64_t n_remove, int64_t n_points, int64_t n_new, const TripsPointTensor* tensors,
                                  int n_tensors, void* scratch, DevStats* stats, int sm_count, cudaStream_t st);
-size_t rank_temp_bytes(int N);
-cudaError_t launch_point_rank(const float4* position, int N, unsigned* scratch, void* temp, size_t temp_bytes, unsigned* rank,
-                              int sm_count, cudaStream_t st);
 cudaError_t launch_scan(const Geom& g, int B, int k_keep, const FwdBuffers& fb, int nchunks, cudaStream_t st);
 // strict: an entry's layers start at the layer below log2(size) instead of layer 0 (strict_layers above)
 // entries_hint: the number of entries of the call as far as the host knows it (selects the size of the work tickets)

@@ -88,7 +88,7 @@ cudaError_t launch_setup_cams(const TripsView* d_views, int B, const double* pos
 // CountAndCollectTiled (RenderForward.cu:168-366); the list lengths are counted afterwards from the entries
 // (window_kernel<false>).  Both passes read every point ONCE per call and loop over the views with the point in
 // registers (the camera constants of up to kViewGroup views sit in shared memory): position, size and, in the scatter
-// pass, confidence, descriptor row and rank cost N reads per call instead of N x B, and softplus(size) is evaluated
+// pass, confidence and descriptor row cost N reads per call instead of N x B, and softplus(size) is evaluated
 // once per point.  Projecting twice avoids writing and re-reading a per-point record for all N x B point-views.
 // ------------------------------------------------------------------------------------------------------------
 struct Projected
@@ -411,7 +411,6 @@ struct PointRow
     bool fetched = false, tex_ok = false;
     int tex      = 0;
     float conf   = 0.f;
-    uint32_t rk  = 0u;
     float row[C4];
 };
 
@@ -434,7 +433,6 @@ __device__ __forceinline__ void fetch_point_row(const ScenePtrs& sc, const Trips
 #pragma unroll
         for (int c = 0; c < PointRow<C>::C4; ++c) d.row[c] = fabsf(d.row[c]);
     }
-    d.rk = fb.point_rank ? __ldg(fb.point_rank + i) : 0u;
 }
 
 // Writes entry `at` (index into the entry arrays) of point i as projected by `r`.
@@ -467,7 +465,7 @@ __device__ __forceinline__ void write_entry(const FwdBuffers& fb, const Geom& g,
         if (pr.drop_out_points_by_radius && (second ? rad : (float)(int)rad) < pr.drop_out_radius_threshold) break;
     }
     store_entry_head(fb.ent_head + at * 2, make_float4(r.u, r.v, r.ps, d.conf),
-                     make_float4(__int_as_float(i), r.z, raw, __uint_as_float((uint32_t)(layer - first) | (d.rk << kRankShift))));
+                     make_float4(__int_as_float(i), r.z, raw, __int_as_float(layer - first)));
     float4* e = reinterpret_cast<float4*>(fb.ent_tail + at * TS);
     if constexpr (C4 == 4)
         store_entry_head(e, make_float4(p.x, p.y, p.z, __int_as_float(d.tex_ok ? d.tex : -1)), make_float4(d.row[0], d.row[1], d.row[2], d.row[3]));
@@ -502,7 +500,12 @@ __global__ __launch_bounds__(kBinThreads, kScatterMinBlocks) void bin_scatter_ke
             PointRow<C> d;
             d.tex    = sc.index ? __ldg(sc.index + i) : i;
             d.tex_ok = (unsigned)d.tex < (unsigned)sc.n_tex;
-            if (discarded_for_confidence<ACT>(sc, pr, d.tex)) continue;
+            if (discarded_for_confidence<ACT>(sc, pr, d.tex))
+            {
+                if (fb.point_entry)
+                    for (int v = 0; v < nv; ++v) fb.point_entry[(size_t)(v0 + v) * sc.N + i] = kNoEntry;
+                continue;
+            }
             const float4 p  = __ldg(sc.position + i);
             const float raw = __ldg(sc.point_size + i);
             float sp        = -1.f;
@@ -518,7 +521,7 @@ __global__ __launch_bounds__(kBinThreads, kScatterMinBlocks) void bin_scatter_ke
                 for (int j = 0; j < kSweep; ++j)
                 {
                     const int v = vb + j;
-                    slot[j]     = 0;
+                    slot[j]     = kNoEntry;
                     if (v >= nv || ((skip >> v) & 1u)) continue;  // uniform
                     if (use_dropout && __ldg(sc.dropout + (size_t)(v0 + v) * sc.N + i) == 1.f) continue;
                     const Projected r = project_visible(s_cam[v], g, pr, p, raw, sp);
@@ -526,8 +529,12 @@ __global__ __launch_bounds__(kBinThreads, kScatterMinBlocks) void bin_scatter_ke
                     vis |= 1u << j;
                     slot[j] = atomicAdd(fb.bin_base + ((size_t)(v0 + v) * g.n_bins << kSubShift) + bin_key(g, r.u, r.v), 1u);
                 }
+                if (vis) fetch_point_row<C, ACT>(sc, pr, fb, i, d);  // travels with the slots
+                if (fb.point_entry)
+#pragma unroll
+                    for (int j = 0; j < kSweep; ++j)
+                        if (vb + j < nv) fb.point_entry[(size_t)(v0 + vb + j) * sc.N + i] = slot[j];
                 if (!vis) continue;
-                fetch_point_row<C, ACT>(sc, pr, fb, i, d);
 #pragma unroll
                 for (int j = 0; j < kSweep; ++j)
                 {
@@ -693,20 +700,32 @@ __global__ __launch_bounds__(kBinThreads) void bin_scatter_hot_kernel(ScenePtrs 
             PointRow<C> d;
             d.tex    = sc.index ? __ldg(sc.index + i) : i;
             d.tex_ok = (unsigned)d.tex < (unsigned)sc.n_tex;
-            if (discarded_for_confidence<ACT>(sc, pr, d.tex)) continue;
+            if (discarded_for_confidence<ACT>(sc, pr, d.tex))
+            {
+                if (fb.point_entry)
+                    for (int v = 0; v < nv; ++v) fb.point_entry[(size_t)(v0 + v) * sc.N + i] = kNoEntry;
+                continue;
+            }
             const float4 p  = __ldg(sc.position + i);
             const float raw = __ldg(sc.point_size + i);
             float sp        = -1.f;
             for (int v = 0; v < nv; ++v)
             {
-                if ((no_room >> v) & 1u) continue;  // uniform
-                if (use_dropout && __ldg(sc.dropout + (size_t)(v0 + v) * sc.N + i) == 1.f) continue;
-                const Projected r = project_visible(s_cam[v], g, pr, p, raw, sp);
-                if (!r.ok) continue;
-                fetch_point_row<C, ACT>(sc, pr, fb, i, d);
-                const uint32_t key  = (uint32_t)v * n_keys + (uint32_t)bin_key(g, r.u, r.v);
-                const int s         = hot_find(s_tag, key);
-                const uint32_t slot = s >= 0 ? s_base[s] + atomicAdd(s_cnt + s, 1u) : atomicAdd(cursors + key, 1u);
+                uint32_t slot = kNoEntry;
+                Projected r;
+                if (!((no_room >> v) & 1u) && !(use_dropout && __ldg(sc.dropout + (size_t)(v0 + v) * sc.N + i) == 1.f))
+                {
+                    r = project_visible(s_cam[v], g, pr, p, raw, sp);
+                    if (r.ok)
+                    {
+                        fetch_point_row<C, ACT>(sc, pr, fb, i, d);
+                        const uint32_t key = (uint32_t)v * n_keys + (uint32_t)bin_key(g, r.u, r.v);
+                        const int s        = hot_find(s_tag, key);
+                        slot               = s >= 0 ? s_base[s] + atomicAdd(s_cnt + s, 1u) : atomicAdd(cursors + key, 1u);
+                    }
+                }
+                if (fb.point_entry) fb.point_entry[(size_t)(v0 + v) * sc.N + i] = slot;
+                if (slot == kNoEntry) continue;
                 write_entry<C>(fb, g, pr, s_ebase[v] + slot, i, p, raw, r, d);
             }
         }
@@ -1057,13 +1076,13 @@ __device__ __forceinline__ void for_each_footprint(const float4* __restrict__ he
     if (base + lane < hi)
     {
         e0n = head[2 * (size_t)(base + lane)];      // u v ps conf
-        e1n = head[2 * (size_t)(base + lane) + 1];  // pid z raw nl|rank
+        e1n = head[2 * (size_t)(base + lane) + 1];  // pid z raw nl
     }
     for (; base < hi; base += kWinThreads)
     {
         const uint32_t ei = base + lane;
         const float4 e0 = e0n, e1 = e1n;
-        const int nl = ei < hi ? (__float_as_int(e1.w) & ((1 << kRankShift) - 1)) : 0;
+        const int nl = ei < hi ? __float_as_int(e1.w) : 0;
         if (base + kWinThreads + lane < hi)  // the next round's entry travels while this one is processed
         {
             e0n = head[2 * (size_t)(ei + kWinThreads)];
