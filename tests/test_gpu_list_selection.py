@@ -1,0 +1,40 @@
+"""Selection of the nearest fragments where the per-pixel sort can go wrong: list lengths around its chunks of 16 (and the
+shorter network for 8), many fragments of the same depth inside and across the end of the selection, and lists around
+the length at which a block of its own pre-selects them.  Kept points, their order and the pyramid must be the oracle's:
+ids bit for bit, alphas and colours to 1e-5 (16 products in 32 bits, 16 x 6e-8)."""
+import numpy as np
+import pytest
+
+from trips_b200 import scenes
+from util import gpu_render, oracle_frames, rel_err
+
+pytestmark = pytest.mark.gpu
+
+
+def _stack(n, copies, k_keep, seed):
+    """`n` distinct points, `copies` of each (ids i, i + n, ...): every copy has the same depth on the same pixels."""
+    s = scenes.tiny(seed=seed, n_points=n * copies, width=72, height=40, num_layers=3, k_keep=k_keep, n_views=2)
+    for c in range(1, copies):
+        s.position[c * n:(c + 1) * n] = s.position[:n]
+        s.point_size[c * n:(c + 1) * n] = s.point_size[:n]
+    s.confidence[:] = np.minimum(s.confidence, 0.1)  # the transmittance stays above the cut-off for all kept fragments
+    return s
+
+
+@pytest.mark.parametrize("k_keep", [1, 8, 16])
+@pytest.mark.parametrize("n,copies", [(40, 1), (12, 8), (12, 9), (12, 16), (12, 17), (200, 15), (12, 33), (300, 20), (3, 512), (3, 513), (2, 700)])
+def test_kept_fragments(oracle_lib, cuda_lib, n, copies, k_keep):
+    s = _stack(n, copies, k_keep, seed=200 + copies)
+    sa, op, frames = oracle_frames(s, train=True)
+    ns, info, blend = gpu_render(s, train=True)
+    outs = blend(info)
+    assert info.cache.last_status() == 0
+    for b, f in enumerate(frames):
+        nrec, pid, alpha = info.cache.debug_records(b, f.P)
+        onrec, opid, oalpha = f.records()
+        assert np.array_equal(nrec, onrec)
+        assert np.array_equal(pid, opid)
+        assert rel_err(alpha, oalpha, floor=1e-6) <= 1e-5
+        for l, ref in enumerate(f.pyramid()):
+            got = outs[l][b].detach().cpu().numpy()
+            assert np.max(np.abs(got - ref) / np.maximum(np.abs(ref), 1e-3)) <= 1e-5

@@ -1326,22 +1326,29 @@ cudaError_t launch_collect(const ScenePtrs& sc, const Geom& g, int B, const FwdB
 // ------------------------------------------------------------------------------------------------------------
 // per-pixel top-K selection + front-to-back blend
 //
-// One warp renders an 8x4 pixel tile of one view.
-//   phase A (lane = fragment, lanes densely packed over the tile's fragments): every fragment finds its pixel by a
-//     binary search over the tile's list lengths and its rank in the pixel's list by counting the smaller 64-bit
-//     keys; ranks below K go to shared memory in sorted order together with the descriptor row of their entry (and,
-//     when training, to the backward records).  Lists longer than kRankMax take the streaming path instead: a
-//     half-warp keeps the 16 nearest fragments in registers and merges the list in chunks of 16 with bitonic
-//     compare-exchange steps over warp shuffles.
-//   phase B (lane = pixel): the sequential transmittance recurrence and the colour sum over the kept fragments.
+// One warp renders an 8x4 pixel tile of one view, lane = pixel.
+//   staging: (depth, alpha, entry) of up to 16 fragments of every pixel go to shared memory with asynchronous copies, 8
+//     lanes on consecutive fragments of one list; loads by lane = pixel would touch 32 lines each.
+//   selection: every lane sorts its own list by depth in registers, 16 fragments at a time, with a fixed comparator
+//     network (Batcher's odd-even merge sort); further chunks are merged into the 16 nearest (bitonic half-cleaner +
+//     merge).  A comparator serves 32 pixels at once, so a chunk costs a few hundred instructions per WARP, whatever
+//     the lists look like.  Fragments of equal depth are put into point-id order afterwards; that is the rare path.
+//   blend: the sequential transmittance recurrence and the colour sum over the kept fragments.
 // Replaces FastSortFusedNew (RenderForward.cu:474-1059).
+//
+// What bounds it (ncu, one 1080p view of 6 M points): half of the issue slots and half of the load/store unit's wavefront
+// rate in use at 20 warps per SM, the rest are waits for the gathers of list heads and descriptor rows; DRAM at 27 %.
+// 190 M instructions, against 323 M when the fragments of a tile were ranked against each other with shuffles (lists of at
+// most 32) or sorted by half-warps, which this replaces: sort_blend stage 0.42 -> 0.31 ms on that view, 32.1 -> 22.9 ms on
+// 64 views of 10 M points (longer lists), 1.41 -> 0.87 ms on 2 1440p views of 20 M, 0.206 -> 0.070 ms on a 640x480 view of
+// 200 k points (lists up to 379, K = 8).
+// Loops stay rolled where they can: with the blend unrolled over 16 fragments and every network instantiated twice the
+// warps spent 8.6 of 20 cycles per instruction waiting for instruction fetches, and the kernel lost to its predecessor.
 // ------------------------------------------------------------------------------------------------------------
 typedef unsigned long long u64;
 constexpr u64 kInfKey    = 0xffffffffffffffffull;
-constexpr int kSbRing    = 2;    // descriptor rows requested ahead of their use in the blend loop (C <= 4)
-constexpr int kRankMax   = 32;   // longest list ranked by counting; longer lists use the streaming path (measured: 16 3.12 ms, 24 3.03, 32 3.02, 48 3.08, 64 3.15)
-constexpr int kSortedPad = 17;   // row pitch (entries) of the per-pixel sorted lists in shared memory
-constexpr int kSbStageMaxC = 0;  // widest descriptor whose rows are staged in shared memory by phase A (0: none; staging cost more L1 than it saved)
+constexpr int kSbPitch   = 17;   // row pitch (entries) of the per-pixel arrays in shared memory
+constexpr uint32_t kNoDepth = 0xffffffffu;  // sorts behind every depth
 constexpr int kSbThreads = 128;
 constexpr int kSbWarps   = kSbThreads / 32;
 
@@ -1499,49 +1506,62 @@ cudaError_t launch_heavy_topk(const Geom& g, int B, const FwdBuffers& fb, int sm
     return cudaGetLastError();
 }
 
-// A sorted entry in shared memory is (alpha, descriptor row[C]) when the row fits the shared-memory budget (C <= 4:
-// the gather happens in phase A where lanes are densely packed); for wider descriptors it is (entry index, alpha)
-// and phase B gathers.
-template <int C>
-struct SbEntry
+// 4 / 8 bytes global -> shared, asynchronous; the wait covers all of the thread's copies
+__device__ __forceinline__ void copy_async_4(void* dst_shared, const void* src_global)
 {
-    static constexpr bool kStaged = (C <= kSbStageMaxC);
-    static constexpr int kFloats  = kStaged ? (1 + C) : 2;
-};
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(dst_shared)), "l"(src_global) : "memory");
+}
+__device__ __forceinline__ void copy_async_8(void* dst_shared, const void* src_global)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(dst_shared)), "l"(src_global) : "memory");
+}
+__device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-template <int C>
-__device__ __forceinline__ void sb_store_entry(float* dst, const float* entries, unsigned eidx, unsigned alpha_bits)
+// ---- per-lane sorting in registers: depth bits as the key, position in the list as the payload ----
+__device__ __forceinline__ void order_pair(uint32_t& ka, uint32_t& kb, uint32_t& ia, uint32_t& ib)
 {
-    if constexpr (SbEntry<C>::kStaged)
+    const bool swap   = kb < ka;
+    const uint32_t k0 = swap ? kb : ka, k1 = swap ? ka : kb;
+    const uint32_t i0 = swap ? ib : ia, i1 = swap ? ia : ib;
+    ka = k0, kb = k1, ia = i0, ib = i1;
+}
+
+// Batcher's odd-even merge sort of the first N of 16 elements (ascending): 19 comparators for N = 8, 63 for 16.
+template <int N>
+__device__ __forceinline__ void sort_network(uint32_t (&key)[16], uint32_t (&idx)[16])
+{
+#pragma unroll
+    for (int p = 1; p < N; p *= 2)
     {
-        const float4 v4 = *reinterpret_cast<const float4*>(entries + (size_t)eidx * tail_stride(C) + 4);
-        dst[0]          = __uint_as_float(alpha_bits);
-        dst[1]          = v4.x;
-        if (C > 1) dst[2] = v4.y;
-        if (C > 2) dst[3] = v4.z;
-        if (C > 3) dst[4] = v4.w;
-    }
-    else
-    {
-        dst[0] = __uint_as_float(eidx);
-        dst[1] = __uint_as_float(alpha_bits);
+#pragma unroll
+        for (int k = p; k >= 1; k /= 2)
+        {
+#pragma unroll
+            for (int i = 0; i + k < N; ++i)
+            {
+                // element i is the lower partner of a comparator of distance k when it lies in the lower half of its block of
+                // 2k (counted from k mod p) and both partners lie in the same block of 2p
+                const int j0 = k % p;
+                if (i >= j0 && ((i - j0) % (2 * k)) < k && (i / (2 * p)) == ((i + k) / (2 * p))) order_pair(key[i], key[i + k], idx[i], idx[i + k]);
+            }
+        }
     }
 }
 
-// measured: 7 resident blocks (72 registers) 3.18 ms, 6 blocks (80) 3.46 ms, 5 blocks 3.83 ms, 8 blocks (64, spills) 3.76 ms
-constexpr int kSbMinBlocks = 7;
+// resident blocks, up to 4 channels / up to 8; measured: 4 / 5 / 6 blocks 2.84 / 2.82 / 3.35 ms (6 M points, 8 views, 4
+// channels, records still by pixel; 6 spills inside the networks), and 0.142 ms at 4 against 0.176 ms at 5 with 8 channels
+constexpr int kSbMinBlocks = 5, kSbMinBlocksWide = 4;
 template <int C>
-__global__ __launch_bounds__(kSbThreads, (C <= 8 ? kSbMinBlocks : 1)) void sort_blend_kernel(ScenePtrs sc, const __grid_constant__ Geom g, TripsRenderParams pr,
+__global__ __launch_bounds__(kSbThreads, (C <= 4 ? kSbMinBlocks : (C <= 8 ? kSbMinBlocksWide : 1))) void sort_blend_kernel(ScenePtrs sc, const __grid_constant__ Geom g, TripsRenderParams pr,
                                                                 int B, FwdBuffers fb, const __grid_constant__ LayerPtrs out,
                                                                 unsigned n_tiles_total)
 {
-    constexpr int E  = SbEntry<C>::kFloats;
     constexpr int ES = tail_stride(C);
-    __shared__ float s_sorted[kSbWarps][32 * kSortedPad * E];  // per warp: 32 pixels x K entries, nearest first
+    __shared__ uint32_t s_key[kSbWarps][32 * kSbPitch];  // depths of a chunk of 16 fragments per pixel; later the sorted list positions, [rank][lane]
+    __shared__ uint2 s_az[kSbWarps][32 * kSbPitch];      // (alpha bits, entry index) of the chunk
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     const int K    = pr.k_keep;
-    float* sorted  = s_sorted[warp];
     float bg[C];
 #pragma unroll
     for (int c = 0; c < C; ++c) bg[c] = __ldg(sc.background + c);
@@ -1563,293 +1583,211 @@ __global__ __launch_bounds__(kSbThreads, (C <= 8 ? kSbMinBlocks : 1)) void sort_
         const uint32_t n_entry = (uint32_t)(fb.entry_base[b + 1] - fb.entry_base[b]);
         int layer, gx, gy, p;
         tile_pixel(g, tile, lane, layer, gx, gy, p);  // lane i owns one pixel of the tile
-        uint32_t cnt_all = 0, start = 0;
+        uint32_t cnt = 0, start = 0;
         if (p >= 0 && fb.view_base[b + 1] != fb.view_base[b])  // (a view that did not fit the list buffer renders as background)
         {
-            cnt_all = fb.counts[bP + p];
-            start   = fb.offsets[bP + p] - cnt_all;  // offsets hold list ends after the collect pass
+            cnt   = fb.counts[bP + p];
+            start = fb.offsets[bP + p] - cnt;  // offsets hold list ends after the collect pass
+            // of a pre-selected list (heavy_topk_kernel) only the front matters: its 16 nearest fragments in depth order
+            if (preselected && cnt > (uint32_t)kHeavyList) cnt = 16u;
         }
-        // of a pre-selected list (heavy_topk_kernel) only the front matters: its 16 nearest fragments in depth order
-        const uint32_t cnt = (preselected && cnt_all > (uint32_t)kHeavyList) ? 16u : cnt_all;
-        uint32_t incl = cnt;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1)
-        {
-            uint32_t t = __shfl_up_sync(kFull, incl, o);
-            if (lane >= o) incl += t;
-        }
-        const uint32_t rel_start  = incl - cnt;
-        const uint32_t tile_total = __shfl_sync(kFull, incl, 31);
-        uint32_t max_cnt          = cnt;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) max_cnt = max(max_cnt, __shfl_xor_sync(kFull, max_cnt, o));
+        const uint32_t max_cnt = __reduce_max_sync(kFull, cnt);
+        const uint4* list      = frags + start;
 
-        if (max_cnt <= (uint32_t)kRankMax)
-        {
-            // ---- phase A, counting path: lane = fragment.  The fragment of the next round is fetched before the
-            //      ranking loop of the current one, so that its DRAM latency hides behind the loop ----
-            struct Loc
-            {
-                uint32_t seg_start, seg_cnt, idx;
-                int seg, seg_p;
-            };
-            auto locate = [&](uint32_t t) {
-                Loc L;
-                // pixel of this fragment: the last lane whose list starts at or before t
-                int seg = 0;
+        // ---- selection: the 16 nearest fragments of the lane's list, nearest first.  The network for 8, 12 or 16 goes by the
+        //      longest list of the tile (half of the tiles of a 720p view stay at 8; 12 instead of 16: 42 against 63 comparators) ----
+        uint32_t key[16], idx[16];
+        uint32_t dropped = kNoDepth;  // smallest depth among the fragments that are not kept
 #pragma unroll
-                for (int step = 16; step > 0; step >>= 1)
-                {
-                    const int probe       = seg + step;
-                    const uint32_t pstart = __shfl_sync(kFull, rel_start, probe & 31);
-                    if (probe < 32 && pstart <= t) seg = probe;
-                }
-                L.seg       = seg;
-                L.idx       = t - __shfl_sync(kFull, rel_start, seg);
-                L.seg_start = __shfl_sync(kFull, start, seg);
-                L.seg_cnt   = __shfl_sync(kFull, cnt, seg);
-                L.seg_p     = __shfl_sync(kFull, p, seg);
-                return L;
-            };
-            // Rounds of whole lists: a round takes the lists of consecutive pixels as long as they fit 32 lanes (every
-            // list has at most kRankMax = 32 fragments here), so the fragments of one pixel always sit in neighbouring
-            // lanes of one round and a fragment finds its rank by reading the keys of its list from those lanes with
-            // shuffles.  Reading the keys from the list in memory instead cost one gather over several 128-byte lines
-            // per key and lane, and it was the load/store unit's line rate that bounded this kernel.
-            static_assert(kRankMax <= 32, "a list ranked by shuffles must fit one round of 32 lanes");
-            struct Round
-            {
-                uint32_t base, total;  // fragments of the tile before this round, fragments in it
-                int end_px;            // first pixel (lane) of the next round
-            };
-            auto plan = [&](int first_px) {
-                Round r;
-                r.base              = __shfl_sync(kFull, rel_start, first_px & 31);
-                const unsigned fits = __ballot_sync(kFull, lane >= first_px && incl - r.base <= 32u);  // a run of lanes from first_px on
-                r.end_px            = first_px + __popc(fits);
-                r.total             = __shfl_sync(kFull, incl, (r.end_px - 1) & 31) - r.base;
-                return r;
-            };
-            Round rn     = plan(0);
-            Loc nxt      = locate(rn.base + lane);
-            uint4 f_next = make_uint4(kFull, kFull, 0u, 0u);
-            if ((uint32_t)lane < rn.total) f_next = frags[nxt.seg_start + nxt.idx];
-            for (;;)
-            {
-                const Round rc   = rn;
-                const Loc cur    = nxt;
-                const uint4 f    = f_next;
-                const bool valid = (uint32_t)lane < rc.total;
-                const bool more  = rc.end_px < 32 && rc.base + rc.total < tile_total;  // uniform
-                if (more)
-                {
-                    rn     = plan(rc.end_px);
-                    nxt    = locate(rn.base + lane);
-                    f_next = make_uint4(kFull, kFull, 0u, 0u);
-                    if ((uint32_t)lane < rn.total) f_next = frags[nxt.seg_start + nxt.idx];
-                }
-                const int lane0   = (int)(rc.base + lane - cur.idx - rc.base);  // lane of the first fragment of this fragment's list
-                const int longest = __reduce_max_sync(kFull, valid ? (int)cur.seg_cnt : 0);
-                const u64 mine    = ((u64)f.y << 32) | f.x;
-                int rank          = 0;
-                for (int i = 0; i < longest; ++i)
-                {
-                    const int src     = max(0, min(lane0 + i, 31));
-                    const uint32_t oy = __shfl_sync(kFull, f.y, src), ox = __shfl_sync(kFull, f.x, src);
-                    if (i < (int)cur.seg_cnt) rank += ((((u64)oy << 32) | ox) < mine) ? 1 : 0;
-                }
-                if (valid)
-                {
-                    if (f.w >= n_entry)
-                        atomicOr(&fb.stats->status, TRIPS_DEV_BAD_FRAGMENT);  // corrupted list: skip instead of gathering out of bounds
-                    else if (rank < K)
-                    {
-                        sb_store_entry<C>(sorted + (cur.seg * kSortedPad + rank) * E, entries, f.w, f.z);
-                        if (pr.train) fb.records[(bP + cur.seg_p) * 16 + rank] = make_uint2(f.w, f.z);
-                    }
-                }
-                if (!more) break;
-            }
-        }
-        else
+        for (int i = 0; i < 16; ++i) key[i] = kNoDepth, idx[i] = 0u;
+#pragma unroll 1
+        for (uint32_t c0 = 0; c0 < max_cnt; c0 += 16)
         {
-            // ---- phase A, streaming path: a half-warp per pixel keeps the 16 nearest fragments in registers ----
-            const int j     = lane & 15;
-            const int hbase = lane & 16;
-            for (int it = 0; it < 16; ++it)
+            // 8 lanes copy 8 (16) consecutive fragments of one pixel, 4 pixels per step: the lane = pixel pattern would touch
+            // 32 lines with every load
+            const uint32_t left = max_cnt - c0;
+            const int i8        = lane & 7;
+#pragma unroll 4
+            for (int q = 0; q < 8; ++q)
             {
-                const int src        = it * 2 + (hbase >> 4);
-                const uint32_t cnt_s = __shfl_sync(kFull, cnt, src);
-                const uint32_t beg_s = __shfl_sync(kFull, start, src);
-                const int p_s        = __shfl_sync(kFull, p, src);
-                const uint32_t cnt_o = __shfl_xor_sync(kFull, cnt_s, 16);
-                KeyVal v;
-                v.key   = kInfKey;
-                v.alpha = 0u;
-                v.eidx  = 0u;
-                if (j < (int)cnt_s)
+                const int src          = q * 4 + (lane >> 3);
+                const uint32_t n_src   = __shfl_sync(kFull, cnt, src);
+                const uint32_t beg_src = __shfl_sync(kFull, start, src);
+                const uint32_t i       = c0 + i8;
+                const uint4* f         = frags + beg_src + i;
+                uint32_t* dk           = s_key[warp] + src * kSbPitch + i8;
+                uint2* da              = s_az[warp] + src * kSbPitch + i8;
+                if (i < n_src) copy_async_4(dk, &f->y), copy_async_8(da, &f->z);
+                if (left > 8 && i + 8 < n_src) copy_async_4(dk + 8, &f[8].y), copy_async_8(da + 8, &f[8].z);
+            }
+            copy_async_wait();
+            __syncwarp();
+            uint32_t k2[16], i2[16];
+            uint32_t nearest = kNoDepth;
+#pragma unroll
+            for (int i = 0; i < 16; ++i)
+            {
+                k2[i]   = (i < 8 || left > 8) && c0 + i < cnt ? s_key[warp][lane * kSbPitch + i] : kNoDepth;
+                i2[i]   = c0 + i;
+                nearest = min(nearest, k2[i]);
+            }
+            __syncwarp();  // the next chunk may overwrite the staged depths
+            if (!__any_sync(kFull, nearest < key[15]))  // nothing nearer in any of the 32 lists
+            {
+                dropped = min(dropped, nearest);
+                continue;
+            }
+            if (left <= 8)
+                sort_network<8>(k2, i2);
+            else if (left <= 12)
+                sort_network<12>(k2, i2);
+            else
+                sort_network<16>(k2, i2);
+            if (c0 == 0)
+            {
+#pragma unroll
+                for (int i = 0; i < 16; ++i) key[i] = k2[i], idx[i] = i2[i];
+                continue;
+            }
+#pragma unroll
+            for (int i = 0; i < 16; ++i)
+            {
+                const bool take = k2[15 - i] < key[i];
+                dropped         = min(dropped, take ? key[i] : k2[15 - i]);
+                if (take) key[i] = k2[15 - i], idx[i] = i2[15 - i];
+            }
+#pragma unroll
+            for (int st = 8; st > 0; st >>= 1)
+#pragma unroll
+                for (int i = 0; i < 16; ++i)
+                    if ((i & st) == 0) order_pair(key[i], key[i + st], idx[i], idx[i + st]);
+        }
+        bool tie = false;
+#pragma unroll
+        for (int j = 0; j < 15; ++j) tie |= key[j] == key[j + 1] && key[j] != kNoDepth;
+        const bool tie_end = dropped == key[15] && dropped != kNoDepth;
+        const int n        = min((int)cnt, K);
+        const int n_max    = min((int)max_cnt, K);
+        uint32_t* order    = s_key[warp] + lane;  // list position of the fragment of rank j at order[32 * j]
+#pragma unroll
+        for (int j = 0; j < 16; ++j)
+            if (j < 8 || max_cnt > 8) order[32 * j] = idx[j];
+        // equal depths go by point id (the total order of the lists); rare, so the lists are read in place
+        if (__any_sync(kFull, tie || tie_end))
+        {
+            if (tie_end)  // a tie across the end of the selection: of the fragments at the last kept depth those with the smallest ids stay
+            {
+                int j = 15;
+                while (j > 0 && list[order[32 * (j - 1)]].y == dropped) --j;
+                uint32_t last = 0;
+                for (bool first = true; j < 16; ++j, first = false)
                 {
-                    const uint4 f = frags[beg_s + j];
-                    v.key         = ((u64)f.y << 32) | f.x;
-                    v.alpha       = f.z;
-                    v.eidx        = f.w;
-                }
-                v = bitonic_sort16(v, j);
-                const uint32_t cnt_max = max(cnt_s, cnt_o);
-                for (uint32_t ch = 16; ch < cnt_max; ch += 16)
-                {
-                    KeyVal nk;
-                    nk.key   = kInfKey;
-                    nk.alpha = 0u;
-                    nk.eidx  = 0u;
-                    if (ch + j < cnt_s)
+                    uint32_t best = 0xffffffffu, at = order[32 * j];
+                    for (uint32_t i = 0; i < cnt; ++i)
                     {
-                        const uint4 f = frags[beg_s + ch + j];
-                        nk.key        = ((u64)f.y << 32) | f.x;
-                        nk.alpha      = f.z;
-                        nk.eidx       = f.w;
+                        const uint2 f = *reinterpret_cast<const uint2*>(list + i);
+                        if (f.y == dropped && (first || f.x > last) && f.x <= best) best = f.x, at = i;
                     }
-                    topk_merge16(v, nk, j, hbase);
-                }
-                if (j < min((int)cnt_s, K))
-                {
-                    if (v.eidx >= n_entry)
-                    {
-                        atomicOr(&fb.stats->status, TRIPS_DEV_BAD_FRAGMENT);
-                        v.eidx  = 0;
-                        v.alpha = 0;
-                    }
-                    sb_store_entry<C>(sorted + (src * kSortedPad + j) * E, entries, v.eidx, v.alpha);
-                    if (pr.train && p_s >= 0) fb.records[(bP + p_s) * 16 + j] = make_uint2(v.eidx, v.alpha);
+                    order[32 * j] = at, last = best;
                 }
             }
+            const int n16 = min((int)cnt, 16);
+            while (tie)  // at most 15 sweeps of a bubble sort over equal neighbours
+            {
+                tie = false;
+                for (int j = 0; j + 1 < n16; ++j)
+                {
+                    const uint32_t ia = order[32 * j], ib = order[32 * (j + 1)];
+                    const uint2 fa = *reinterpret_cast<const uint2*>(list + ia), fb2 = *reinterpret_cast<const uint2*>(list + ib);
+                    if (fa.y == fb2.y && fb2.x < fa.x) order[32 * j] = ib, order[32 * (j + 1)] = ia, tie = true;
+                }
+            }
+            __syncwarp();
         }
-        __syncwarp();
 
-        // ---- phase B: lane = pixel.  T_j = T_{j-1} * (1 - a_{j-1}), colour summed in the order of a 16-leaf
-        //      butterfly (RenderForward.cu:940-994) so that results do not depend on how lanes are assigned ----
-        const int n = min((int)cnt, K);
-        int n_max   = n;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) n_max = max(n_max, __shfl_xor_sync(kFull, n_max, o));
+        // ---- blend.  T_j = T_{j-1} * (1 - a_{j-1}), colour summed in the order of a 16-leaf butterfly
+        //      (RenderForward.cu:940-994) so that results do not depend on how lanes are assigned: four leaves per turn ----
         float run = 1.f, t_last = 1.f, tn_last = 1.f;
         int m      = 0;
         bool alive = true;
-        float s0[C], s1[C], s2[C], s3[C];
+        const bool one_chunk = max_cnt <= 16;  // (alpha, entry) of all fragments are staged
+        float half0[C], half1[C];              // sums of leaves 0..7 and 8..15
 #pragma unroll
-        for (int c = 0; c < C; ++c) s0[c] = s1[c] = s2[c] = s3[c] = 0.f;
-        const float* my_sorted = sorted + lane * kSortedPad * E;
-        // descriptor rows are requested kRing entries ahead of their use (the gathers are independent of the recurrence)
+        for (int c = 0; c < C; ++c) half0[c] = half1[c] = 0.f;
         constexpr int kRows = (C + 3) / 4;
-        constexpr int kRing = SbEntry<C>::kStaged ? 1 : (C <= 4 ? kSbRing : (C <= 8 ? 2 : 1));
-        float4 ring[kRing][kRows];
-        auto fetch_row = [&](int j, float4 (&dst)[kRows]) {
-            if (!SbEntry<C>::kStaged && j < n)
-            {
-                unsigned eidx = __float_as_uint(my_sorted[j * E]);
-                if (eidx >= n_entry) eidx = 0;  // only after a corrupted list was flagged in phase A: read in bounds
-                const float* rp = entries + (size_t)eidx * ES + 4;
-#pragma unroll
-                for (int r = 0; r < kRows; ++r) dst[r] = *reinterpret_cast<const float4*>(rp + 4 * r);
-            }
-        };
-#pragma unroll
-        for (int d = 0; d < kRing; ++d) fetch_row(d, ring[d]);
-#pragma unroll
-        for (int j = 0; j < 16; ++j)
+        float4 row[4][kRows];                   // descriptor rows of this turn's fragments
+        uint2 rec[4];                           // (entry index, alpha bits)
+#pragma unroll 1
+        for (int j0 = 0; j0 < n_max; j0 += 4)
         {
-            if (j >= n_max) break;
-            float leaf[C];
 #pragma unroll
-            for (int c = 0; c < C; ++c) leaf[c] = 0.f;
-            if (j < n)
+            for (int u = 0; u < 4; ++u)
+                if (j0 + u < n)
+                {
+                    const uint32_t at = order[32 * (j0 + u)];
+                    const uint2 az    = one_chunk ? s_az[warp][lane * kSbPitch + at] : *reinterpret_cast<const uint2*>(&list[at].z);
+                    const bool bad    = az.y >= n_entry;  // corrupted list: draws nothing, reads in bounds
+                    if (bad) atomicOr(&fb.stats->status, TRIPS_DEV_BAD_FRAGMENT);
+                    rec[u]          = make_uint2(bad ? 0u : az.y, bad ? 0u : az.x);
+                    const float* rp = entries + (size_t)rec[u].x * ES + 4;
+#pragma unroll
+                    for (int r = 0; r < kRows; ++r) row[u][r] = *reinterpret_cast<const float4*>(rp + 4 * r);
+                }
+            float pair[C], quad[C];
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
             {
-                const float* e = my_sorted + j * E;
-                float a;
-                float row[C];
-                if constexpr (SbEntry<C>::kStaged)
-                {
-                    a = e[0];
+                float leaf[C];
 #pragma unroll
-                    for (int c = 0; c < C; ++c) row[c] = e[1 + c];
-                }
-                else
+                for (int c = 0; c < C; ++c) leaf[c] = 0.f;
+                const int j = j0 + u;
+                if (j < n)
                 {
-                    a = (__float_as_uint(e[0]) < n_entry) ? e[1] : 0.f;  // a corrupted entry draws nothing
+                    const float a     = __uint_as_float(rec[u].y);
+                    const float T_out = (j == 0 || run >= kAlphaCut) ? run : 0.f;
+                    const float w     = T_out * a;
 #pragma unroll
-                    for (int c = 0; c < C; c += 4)
+                    for (int c = 0; c < C; ++c)
                     {
-                        const float4 v4 = ring[j % kRing][c / 4];
-                        row[c] = v4.x;
-                        if (c + 1 < C) row[c + 1] = v4.y;
-                        if (c + 2 < C) row[c + 2] = v4.z;
-                        if (c + 3 < C) row[c + 3] = v4.w;
+                        const float4 v4 = row[u][c / 4];
+                        leaf[c]         = w * ((c & 3) == 0 ? v4.x : ((c & 3) == 1 ? v4.y : ((c & 3) == 2 ? v4.z : v4.w)));
                     }
+                    if (alive && T_out >= kAlphaCut)
+                    {
+                        m = j + 1;
+                        if (pr.train) fb.records[(bP + p) * 16 + j] = rec[u];
+                    }
+                    else
+                        alive = false;
+                    if (j == n - 1)
+                    {
+                        t_last  = T_out;
+                        tn_last = run * (1.f - a);
+                    }
+                    run = run * (1.f - a);
                 }
-                const float T_out = (j == 0 || run >= kAlphaCut) ? run : 0.f;
-                const float w     = T_out * a;
 #pragma unroll
-                for (int c = 0; c < C; ++c) leaf[c] = w * row[c];
-                if (alive && T_out >= kAlphaCut)
-                    m = j + 1;
-                else
-                    alive = false;
-                if (j == n - 1)
+                for (int c = 0; c < C; ++c)
                 {
-                    t_last  = T_out;
-                    tn_last = run * (1.f - a);
+                    if (u == 0 || u == 2)
+                        pair[c] = leaf[c];
+                    else if (u == 1)
+                        quad[c] = pair[c] + leaf[c];
+                    else
+                        quad[c] = quad[c] + (pair[c] + leaf[c]);
                 }
-                run = run * (1.f - a);
             }
-            if (j + kRing < 16) fetch_row(j + kRing, ring[j % kRing]);
-            // binary-counter accumulation = pairwise tree over leaves 0..15
 #pragma unroll
             for (int c = 0; c < C; ++c)
             {
-                if ((j & 1) == 0)
-                    s0[c] = leaf[c];
+                if (j0 < 8)
+                    half0[c] = j0 == 0 ? quad[c] : half0[c] + quad[c];
                 else
-                {
-                    float p1 = s0[c] + leaf[c];
-                    if ((j & 2) == 0)
-                        s1[c] = p1;
-                    else
-                    {
-                        float p2 = s1[c] + p1;
-                        if ((j & 4) == 0)
-                            s2[c] = p2;
-                        else
-                        {
-                            float p3 = s2[c] + p2;
-                            if ((j & 8) == 0)
-                                s3[c] = p3;
-                            else
-                                s3[c] = s3[c] + p3;  // j == 15: the root
-                        }
-                    }
-                }
+                    half1[c] = j0 == 8 ? quad[c] : half1[c] + quad[c];
             }
         }
         if (p >= 0)
         {
-            // pending partial sums of an incomplete tree: the missing leaves are zeros, which add exactly
-            float col[C];
-            const int jm = n_max;
-#pragma unroll
-            for (int c = 0; c < C; ++c)
-            {
-                float t = 0.f;
-                if (jm >= 16)
-                    t = s3[c];
-                else
-                {
-                    if (jm & 1) t = s0[c];
-                    if (jm & 2) t = s1[c] + t;
-                    if (jm & 4) t = s2[c] + t;
-                    if (jm & 8) t = s3[c] + t;
-                }
-                col[c] = t;
-            }
             float wb;
             if (n == 0)
                 wb = 1.f;  // the reference reads a neighbouring lane here (RenderForward.cu:1002-1003): defined as pure background
@@ -1862,7 +1800,7 @@ __global__ __launch_bounds__(kSbThreads, (C <= 8 ? kSbMinBlocks : 1)) void sort_
 #pragma unroll
             for (int c = 0; c < C; ++c)
             {
-                float v = col[c];
+                float v = half0[c] + half1[c];
                 if (wb >= kAlphaCut) v += bg[c] * (wb * 1.f);
                 o[(size_t)c * Hl * Wl] = v;
             }
