@@ -103,7 +103,6 @@ __global__ __launch_bounds__(kBwdThreads, (C <= 4 ? kBwdMinBlocks : 1)) void ble
         if (lane == 0) next_tile = atomicAdd(fb.ticket, 1u);
         const int b          = ticket / (unsigned)g.n_tiles;
         const unsigned tile  = ticket - b * (unsigned)g.n_tiles;
-        const size_t bP      = (size_t)b * g.P;
         const float* desc    = fb.ent_tail + fb.entry_base[b] * DS + 4;  // descriptor row of entry e at desc + e * DS
         const float4* head   = fb.ent_head + fb.entry_base[b] * 2;
         float* egrad         = bb.egrad + fb.entry_base[b] * GS;
@@ -117,7 +116,7 @@ __global__ __launch_bounds__(kBwdThreads, (C <= 4 ? kBwdMinBlocks : 1)) void ble
         for (int c = 0; c < C; ++c) gin[c] = 0.f;
         if (p >= 0)
         {
-            m            = fb.rec_n[bP + p];
+            m            = fb.rec_n[(size_t)ticket * 32 + lane];  // tickets run over the tiles of all views
             const int Wl = g.W[layer], Hl = g.H[layer];
             const float* gi = grad_in.p[layer] + ((size_t)b * C * Hl + gy) * Wl + gx;
 #pragma unroll
@@ -138,23 +137,16 @@ __global__ __launch_bounds__(kBwdThreads, (C <= 4 ? kBwdMinBlocks : 1)) void ble
         }
         const int rel     = incl - m;
         const int n_entry = __shfl_sync(kFull, incl, 31);
-        // the tile's records (entry index, alpha) -> shared memory.  The 16 records of a pixel are one 128-byte line: eight
-        // lanes read the eight 16-byte pieces of one pixel's line, so a load instruction touches 4 lines instead of 32
-        // (the load/store unit handles one line per cycle); pieces beyond the pixel's record count are not read.
-#pragma unroll
-        for (int it = 0; it < 8; ++it)
+        // the tile's records (entry index, alpha) -> shared memory: lane = pixel, 256 consecutive bytes per rank
         {
-            const int q   = it * 4 + (lane >> 3);  // pixel of the tile
-            const int k   = lane & 7;              // piece: records 2k, 2k+1
-            const int m_q = __shfl_sync(kFull, m, q);
-            const int p_q = __shfl_sync(kFull, p, q);
-            if (2 * k < m_q)
-            {
-                const uint4 v = *(reinterpret_cast<const uint4*>(fb.records + (bP + p_q) * 16) + k);
-                uint2* dst    = s_rec[warp] + q * kPad + 2 * k;
-                dst[0]        = make_uint2(v.x < n_ent ? v.x : 0u, v.x < n_ent ? v.y : 0u);  // a corrupted record contributes nothing
-                dst[1]        = make_uint2(v.z < n_ent ? v.z : 0u, v.z < n_ent ? v.w : 0u);
-            }
+            const uint2* rec = fb.records + (size_t)ticket * (16 * 32) + lane;
+#pragma unroll 8
+            for (int j = 0; j < m_max; ++j)
+                if (j < m)
+                {
+                    const uint2 v = rec[j * 32];
+                    my_rec[j]     = make_uint2(v.x < n_ent ? v.x : 0u, v.x < n_ent ? v.y : 0u);  // a corrupted record contributes nothing
+                }
         }
         __syncwarp();
         // (pixel, slot in the padded per-pixel arrays) of the e-th kept fragment of the tile: a table written by the

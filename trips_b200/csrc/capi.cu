@@ -414,8 +414,8 @@ static int forward_views(TripsContext* ctx, const TripsScene* scene, const Trips
     CU_CHECK(ctx, ensure(ctx->ticket, sizeof(unsigned) * (size_t)(B > 64 ? B : 64)));
     if (params->train)
     {
-        CU_CHECK(ctx, ensure(ctx->rec_n, P * B));
-        CU_CHECK(ctx, ensure(ctx->records, sizeof(uint2) * 16 * P * B));
+        CU_CHECK(ctx, ensure(ctx->rec_n, (size_t)g.n_tiles * 32 * B));
+        CU_CHECK(ctx, ensure(ctx->records, sizeof(uint2) * 16 * 32 * (size_t)g.n_tiles * B));
         CU_CHECK(ctx, ensure(ctx->point_entry, sizeof(uint32_t) * N * B));
     }
     if (ctx->frags.bytes == 0) CU_CHECK(ctx, ensure(ctx->frags, 16 * 1024 * 1024));
@@ -893,43 +893,45 @@ int trips_debug_records(TripsContext* ctx, int view, int32_t* nrec, int32_t* rec
     if (!ctx->have_forward || !ctx->params.train) return fail(ctx, TRIPS_ERR_NO_FORWARD, "no training forward pass");
     if (view < 0 || view >= ctx->B) return fail(ctx, TRIPS_ERR_INVALID_ARG, "view out of range");
     cudaStream_t st = (cudaStream_t)stream;
-    const size_t P = (size_t)ctx->geom.P, off = (size_t)view * P;
-    std::vector<uint8_t> n(P);
-    std::vector<uint2> r(P * 16);
+    const Geom& g = ctx->geom;
+    const size_t T = (size_t)g.n_tiles;
+    std::vector<uint8_t> n(T * 32);
+    std::vector<uint2> r(T * 16 * 32);
     const size_t ES = 8;  // the two float4 of an entry's head
     unsigned long long eb[2];
     CU_CHECK(ctx, cudaMemcpyAsync(eb, (unsigned long long*)ctx->entry_base.p + view, sizeof(eb), cudaMemcpyDeviceToHost, st));
-    CU_CHECK(ctx, cudaMemcpyAsync(n.data(), (uint8_t*)ctx->rec_n.p + off, P, cudaMemcpyDeviceToHost, st));
-    CU_CHECK(ctx, cudaMemcpyAsync(r.data(), (uint2*)ctx->records.p + off * 16, sizeof(uint2) * 16 * P, cudaMemcpyDeviceToHost, st));
+    CU_CHECK(ctx, cudaMemcpyAsync(n.data(), (uint8_t*)ctx->rec_n.p + (size_t)view * T * 32, n.size(), cudaMemcpyDeviceToHost, st));
+    CU_CHECK(ctx, cudaMemcpyAsync(r.data(), (uint2*)ctx->records.p + (size_t)view * T * 16 * 32, sizeof(uint2) * r.size(), cudaMemcpyDeviceToHost, st));
     CU_CHECK(ctx, cudaStreamSynchronize(st));
     const size_t n_e = (size_t)(eb[1] - eb[0]);
     std::vector<float> e(n_e * ES);
     if (n_e) CU_CHECK(ctx, cudaMemcpyAsync(e.data(), (float*)ctx->entries.p + eb[0] * ES, sizeof(float) * n_e * ES, cudaMemcpyDeviceToHost, st));
     CU_CHECK(ctx, cudaStreamSynchronize(st));
-    // records hold the entry index of the fragment's point; report the point id
-    for (size_t p = 0; p < P; ++p)
-        for (int j = 0; j < n[p]; ++j)
-        {
-            const uint32_t ei = r[p * 16 + j].x;
-            uint32_t pid      = 0xffffffffu;
-            if (ei < n_e) memcpy(&pid, e.data() + (size_t)ei * ES + 4, 4);
-            r[p * 16 + j].x = pid;
-        }
-    for (size_t p = 0; p < P; ++p)
-    {
-        if (nrec) nrec[p] = n[p];
-        for (int j = 0; j < 16; ++j)
-        {
-            const bool present = j < n[p];
-            if (rec_pid) rec_pid[p * 16 + j] = present ? (int32_t)r[p * 16 + j].x : -1;
-            if (rec_alpha)
+    // the device holds the records by tile, rank and lane and with the entry index of the fragment's point; report them
+    // per pixel and with the point id
+    for (int l = 0; l < g.L; ++l)
+        for (int y = 0; y < g.H[l]; ++y)
+            for (int x = 0; x < g.W[l]; ++x)
             {
-                float a;
-                memcpy(&a, &r[p * 16 + j].y, 4);
-                rec_alpha[p * 16 + j] = present ? a : -1.f;
+                int tile, lane;
+                pixel_tile(g, l, x, y, tile, lane);
+                const size_t p = (size_t)g.base[l] + (size_t)y * g.W[l] + x;
+                const int m    = n[(size_t)tile * 32 + lane];
+                if (nrec) nrec[p] = m;
+                for (int j = 0; j < 16; ++j)
+                {
+                    const uint2 q   = r[((size_t)tile * 16 + j) * 32 + lane];
+                    int32_t pid     = -1;
+                    float a         = -1.f;
+                    if (j < m)
+                    {
+                        if (q.x < n_e) memcpy(&pid, e.data() + (size_t)q.x * ES + 4, 4);
+                        memcpy(&a, &q.y, 4);
+                    }
+                    if (rec_pid) rec_pid[p * 16 + j] = pid;
+                    if (rec_alpha) rec_alpha[p * 16 + j] = a;
+                }
             }
-        }
-    }
     return TRIPS_OK;
 }
 

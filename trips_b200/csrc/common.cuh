@@ -104,8 +104,9 @@ struct FwdBuffers
     unsigned long long* view_base;    // [B+1] first fragment of each view in `frags`
     uint4* frags;                     // [frag_cap] x = point id, y = depth bits (y:x = 64-bit sort key), z = alpha bits, w = entry index within the view
     unsigned long long frag_cap;
-    uint8_t* rec_n;                   // [B,P] records kept for backward
-    uint2* records;                   // [B,P,16] (entry index within the view, alpha bits)
+    uint8_t* rec_n;                   // [B,n_tiles,32] records kept for backward, by tile and lane (pixel of the tile)
+    uint2* records;                   // [B,n_tiles,16,32] (entry index within the view, alpha bits), by tile, rank and lane: a warp's
+                                      // access to one rank of its tile is 256 consecutive bytes
     DevStats* stats;
     unsigned int* ticket;
     uint32_t* point_entry;            // training: [B,N] entry (within the view) of every point, kNoEntry where it is not visible
@@ -306,6 +307,21 @@ __device__ __forceinline__ void tile_pixel(const Geom& g, int tile, int lane, in
     gx           = tx * kTileW + (lane & (kTileW - 1));
     gy           = ty * kTileH + (lane >> 3);
     p            = (gx < g.W[l] && gy < g.H[l]) ? g.base[l] + gy * g.W[l] + gx : -1;
+}
+
+// The inverse: tile of a view and lane that own pixel (gx, gy) of a layer.
+__host__ __device__ __forceinline__ void pixel_tile(const Geom& g, int layer, int gx, int gy, int& tile, int& lane)
+{
+    lane = ((gy & (kTileH - 1)) << 3) | (gx & (kTileW - 1));
+    if (layer < g.reg_layers)
+    {
+        const int rx = gx >> (6 - layer), ry = gy >> (6 - layer);  // regions are 64 >> layer pixels wide and high
+        const int tx = (gx >> 3) - rx * (8 >> layer), ty = (gy >> 2) - ry * (16 >> layer);
+        const int first = layer == 0 ? 0 : (layer == 1 ? 128 : (layer == 2 ? 160 : 168));
+        tile            = (ry * g.reg_x + rx) * g.reg_tiles + first + (ty << (3 - layer)) + tx;
+    }
+    else
+        tile = g.tile_base[layer] + (gy >> 2) * g.tiles_x[layer] + (gx >> 3);
 }
 
 // ---- launchers (forward.cu / backward.cu / adam.cu) ----

@@ -1717,6 +1717,7 @@ __global__ __launch_bounds__(kSbThreads, (C <= 4 ? kSbMinBlocks : (C <= 8 ? kSbM
         constexpr int kRows = (C + 3) / 4;
         float4 row[4][kRows];                   // descriptor rows of this turn's fragments
         uint2 rec[4];                           // (entry index, alpha bits)
+        uint2* records = fb.records + (size_t)ticket * (16 * 32);  // tickets run over the tiles of all views
 #pragma unroll 1
         for (int j0 = 0; j0 < n_max; j0 += 4)
         {
@@ -1755,7 +1756,7 @@ __global__ __launch_bounds__(kSbThreads, (C <= 4 ? kSbMinBlocks : (C <= 8 ? kSbM
                     if (alive && T_out >= kAlphaCut)
                     {
                         m = j + 1;
-                        if (pr.train) fb.records[(bP + p) * 16 + j] = rec[u];
+                        if (pr.train) records[j * 32 + lane] = rec[u];
                     }
                     else
                         alive = false;
@@ -1804,8 +1805,8 @@ __global__ __launch_bounds__(kSbThreads, (C <= 4 ? kSbMinBlocks : (C <= 8 ? kSbM
                 if (wb >= kAlphaCut) v += bg[c] * (wb * 1.f);
                 o[(size_t)c * Hl * Wl] = v;
             }
-            if (pr.train) fb.rec_n[bP + p] = (uint8_t)m;
         }
+        if (pr.train) fb.rec_n[(size_t)ticket * 32 + lane] = (uint8_t)m;
         __syncwarp();
     }
 }

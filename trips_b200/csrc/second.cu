@@ -146,13 +146,16 @@ __global__ __launch_bounds__(128) void second_blend_kernel(ScenePtrs sc, const _
         // ---- records for the backward pass: the leading fragments whose weight is above the cut-off ----
         if (pr.train)
         {
+            int tile, lane;
+            pixel_tile(g, layer, gx, gy, tile, lane);
+            const size_t bt = (size_t)b * g.n_tiles + tile;
             int m = 0;
             while (m < n && w[m] >= kAlphaCut)
             {
-                fb.records[(bP + p) * 16 + m] = make_uint2(ent[m], __float_as_uint(al[m]));
+                fb.records[(bt * 16 + m) * 32 + lane] = make_uint2(ent[m], __float_as_uint(al[m]));
                 ++m;
             }
-            fb.rec_n[bP + p] = (uint8_t)m;
+            fb.rec_n[bt * 32 + lane] = (uint8_t)m;
         }
     }
 }
