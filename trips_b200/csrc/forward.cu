@@ -121,7 +121,7 @@ __device__ __forceinline__ Projected project_visible(const CamConst& cam, const 
 
 constexpr int kBinThreads     = 256;
 constexpr int kBinBlocksPerSM = 8;
-constexpr int kScatterMinBlocks = 3;   // measured on config 3: 1.46 ms unbounded (95 registers), 1.34 ms at 3 resident blocks (85), 1.36 ms at 4 (64)
+constexpr int kScatterMinBlocks = 4, kScatterMinBlocksWide = 3;  // up to 4 channels / more; measured at 3 / 4: 6 M points 1.26 / 1.23 ms (8 views), 0.346 / 0.313 ms (1 view); 8 channels 0.116 / 0.127 ms
 constexpr int kBinChunk       = 8192;  // points per bounding box
 constexpr int kBinTicket      = 1024;
 constexpr int kSweep          = 4;      // views whose entry slots a thread requests before it waits for any of them  // points per work ticket of the binning kernels; a ticket lies inside one box
@@ -235,15 +235,18 @@ __global__ __launch_bounds__(128) void block_visibility_kernel(const CamConst* _
 
 // Work distribution of the binning kernels: tickets of kBinTicket consecutive points from one counter, so that every SM
 // is busy until the last ticket whatever the number of resident blocks is (a static split left a partial last wave).
-// Returns false when the cloud is exhausted; `skip` gets one bit per view of the group whose bounding-box test rules the
+// Thread 0 holds the following ticket in `ahead`, requested while the current one is worked on (`ahead` starts from
+// first_point_ticket).  Returns false when the cloud is exhausted; `skip` gets one bit per view of the group whose bounding-box test rules the
 // ticket's points out.
-__device__ __forceinline__ bool next_point_ticket(unsigned* ticket, int N, unsigned* s_ticket, const uint8_t* __restrict__ block_skip, int v0,
-                                                  int nv, int& first, int& last, unsigned& skip)
+__device__ __forceinline__ unsigned first_point_ticket(unsigned* ticket) { return threadIdx.x == 0 ? atomicAdd(ticket, 1u) : 0u; }
+__device__ __forceinline__ bool next_point_ticket(unsigned* ticket, unsigned& ahead, int N, unsigned* s_ticket,
+                                                  const uint8_t* __restrict__ block_skip, int v0, int nv, int& first, int& last, unsigned& skip)
 {
     __syncthreads();
-    if (threadIdx.x == 0) *s_ticket = atomicAdd(ticket, 1u);
+    if (threadIdx.x == 0) *s_ticket = ahead;
     __syncthreads();
     const unsigned t = *s_ticket;
+    if (threadIdx.x == 0) ahead = atomicAdd(ticket, 1u);
     if (t >= ((unsigned)N + kBinTicket - 1) / kBinTicket) return false;
     first = (int)(t * kBinTicket);
     last  = min(N, first + kBinTicket);
@@ -277,6 +280,21 @@ __device__ __forceinline__ bool discarded_for_confidence(const ScenePtrs& sc, co
     return c < pr.stability_cutoff_value;
 }
 
+// What both binning passes read of a point; requested one point ahead.
+struct PointHead
+{
+    float4 p;
+    float raw;
+    int tex;
+    __device__ __forceinline__ void fetch(const ScenePtrs& sc, int i, int last)
+    {
+        if (i >= last) return;
+        tex = sc.index ? __ldg(sc.index + i) : i;
+        p   = __ldg(sc.position + i);
+        raw = __ldg(sc.point_size + i);
+    }
+};
+
 // ACT: the scene tensors may be raw parameters (fused texture preparation); compiled separately so that the common case
 // carries none of its code.  One launch handles the views [v0, v0 + nv).
 template <bool ACT>
@@ -288,15 +306,18 @@ __global__ __launch_bounds__(kBinThreads) void bin_count_kernel(ScenePtrs sc, co
     for (int k = threadIdx.x; k < nv * (int)(sizeof(CamConst) / 4); k += kBinThreads) ((int*)s_cam)[k] = ((const int*)(cams + v0))[k];
     const bool use_dropout = pr.train && sc.dropout;  // the mask applies with and without viewer_only (RenderForward.cu:224-240)
     int first, last;
-    unsigned skip;
-    while (next_point_ticket(ticket, sc.N, &s_ticket, fb.block_skip, v0, nv, first, last, skip))
+    unsigned skip, ahead = first_point_ticket(ticket);
+    while (next_point_ticket(ticket, ahead, sc.N, &s_ticket, fb.block_skip, v0, nv, first, last, skip))
     {
+        PointHead nx;
+        nx.fetch(sc, first + threadIdx.x, last);
         for (int i = first + threadIdx.x; i < last; i += kBinThreads)
         {
-            const int tex = sc.index ? __ldg(sc.index + i) : i;
-            if (discarded_for_confidence<ACT>(sc, pr, tex)) continue;
-            const float4 p  = __ldg(sc.position + i);
-            const float raw = __ldg(sc.point_size + i);
+            const PointHead h = nx;
+            nx.fetch(sc, i + kBinThreads, last);
+            if (discarded_for_confidence<ACT>(sc, pr, h.tex)) continue;
+            const float4 p  = h.p;
+            const float raw = h.raw;
             float sp        = -1.f;
             for (int v = 0; v < nv; ++v)
             {
@@ -478,7 +499,7 @@ __device__ __forceinline__ void write_entry(const FwdBuffers& fb, const Geom& g,
 }
 
 template <int C, bool ACT>
-__global__ __launch_bounds__(kBinThreads, kScatterMinBlocks) void bin_scatter_kernel(ScenePtrs sc, const CamConst* __restrict__ cams, const __grid_constant__ Geom g,
+__global__ __launch_bounds__(kBinThreads, (C <= 4 ? kScatterMinBlocks : kScatterMinBlocksWide)) void bin_scatter_kernel(ScenePtrs sc, const CamConst* __restrict__ cams, const __grid_constant__ Geom g,
                                                                   TripsRenderParams pr, FwdBuffers fb, int v0, int nv, unsigned* ticket)
 {
     __shared__ CamConst s_cam[kViewGroup];
@@ -491,14 +512,18 @@ __global__ __launch_bounds__(kBinThreads, kScatterMinBlocks) void bin_scatter_ke
     for (int v = 0; v < nv; ++v) no_room |= (s_ebase[v + 1] == s_ebase[v] ? 1u : 0u) << v;
     const bool use_dropout = pr.train && sc.dropout;
     int first, last;
-    unsigned skip;
-    while (next_point_ticket(ticket, sc.N, &s_ticket, fb.block_skip, v0, nv, first, last, skip))
+    unsigned skip, ahead = first_point_ticket(ticket);
+    while (next_point_ticket(ticket, ahead, sc.N, &s_ticket, fb.block_skip, v0, nv, first, last, skip))
     {
         skip |= no_room;
+        PointHead nx;
+        nx.fetch(sc, first + threadIdx.x, last);
         for (int i = first + threadIdx.x; i < last; i += kBinThreads)
         {
+            const PointHead h = nx;
+            nx.fetch(sc, i + kBinThreads, last);
             PointRow<C> d;
-            d.tex    = sc.index ? __ldg(sc.index + i) : i;
+            d.tex    = h.tex;
             d.tex_ok = (unsigned)d.tex < (unsigned)sc.n_tex;
             if (discarded_for_confidence<ACT>(sc, pr, d.tex))
             {
@@ -506,8 +531,8 @@ __global__ __launch_bounds__(kBinThreads, kScatterMinBlocks) void bin_scatter_ke
                     for (int v = 0; v < nv; ++v) fb.point_entry[(size_t)(v0 + v) * sc.N + i] = kNoEntry;
                 continue;
             }
-            const float4 p  = __ldg(sc.position + i);
-            const float raw = __ldg(sc.point_size + i);
+            const float4 p  = h.p;
+            const float raw = h.raw;
             float sp        = -1.f;
             // Views are handled kSweep at a time in two sweeps: the first projects and takes the entry slots (up to kSweep
             // returning atomics in flight per thread instead of one), the second projects again (the same arithmetic,
