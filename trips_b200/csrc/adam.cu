@@ -39,8 +39,7 @@ __device__ __forceinline__ void adam_element(const TripsAdamTensor& t, float& w,
     w = nw;
 }
 
-__global__ __launch_bounds__(256) void adam_kernel(const TripsAdamTensor* __restrict__ tensors,
-                                                   const int64_t* __restrict__ block_start, int n_tensors)
+__device__ __forceinline__ void adam_block(const TripsAdamTensor* tensors, const int64_t* block_start, int n_tensors)
 {
     __shared__ TripsAdamTensor t;
     __shared__ int64_t first_block;
@@ -99,6 +98,34 @@ __global__ __launch_bounds__(256) void adam_kernel(const TripsAdamTensor* __rest
             t.weights[i] = w, t.first_moments[i] = m, t.second_moments[i] = v, t.steps[i] = s;
         }
     }
+}
+
+__global__ __launch_bounds__(256) void adam_kernel(const TripsAdamTensor* __restrict__ tensors,
+                                                   const int64_t* __restrict__ block_start, int n_tensors)
+{
+    adam_block(tensors, block_start, n_tensors);
+}
+
+// The same with the table as a kernel argument (up to kAdamTable tensors): no copies ahead of the launch.
+struct AdamTable
+{
+    TripsAdamTensor tensors[kAdamTable];
+    int64_t block_start[kAdamTable + 1];
+};
+__global__ __launch_bounds__(256) void adam_by_value_kernel(const __grid_constant__ AdamTable table, int n_tensors)
+{
+    adam_block(table.tensors, table.block_start, n_tensors);
+}
+
+cudaError_t launch_adam_by_value(const TripsAdamTensor* h_tensors, const int64_t* h_block_start, int n_tensors, cudaStream_t st)
+{
+    if (n_tensors < 1 || n_tensors > kAdamTable) return cudaErrorInvalidValue;
+    if (h_block_start[n_tensors] <= 0) return cudaSuccess;
+    AdamTable t{};
+    for (int i = 0; i < n_tensors; ++i) t.tensors[i] = h_tensors[i];
+    for (int i = 0; i <= n_tensors; ++i) t.block_start[i] = h_block_start[i];
+    adam_by_value_kernel<<<(unsigned)h_block_start[n_tensors], 256, 0, st>>>(t, n_tensors);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_adam(const TripsAdamTensor* d_tensors, const int64_t* d_block_start, int n_tensors, int64_t total_blocks,

@@ -94,13 +94,13 @@ __global__ __launch_bounds__(kBwdThreads, (C <= 4 ? kBwdMinBlocks : 1)) void ble
     // records in flight belong to one view
     const unsigned n_total = (unsigned)g.n_tiles * (unsigned)B;
     unsigned next_tile = 0;
-    if (lane == 0) next_tile = atomicAdd(fb.ticket, 1u);
+    if (lane == 0) next_tile = atomicAdd(bb.ticket, 1u);
     for (;;)
     {
         // the ticket of the following tile is requested now, a whole tile ahead of its use
         const unsigned ticket = __shfl_sync(kFull, next_tile, 0);
         if (ticket >= n_total) break;
-        if (lane == 0) next_tile = atomicAdd(fb.ticket, 1u);
+        if (lane == 0) next_tile = atomicAdd(bb.ticket, 1u);
         const int b          = ticket / (unsigned)g.n_tiles;
         const unsigned tile  = ticket - b * (unsigned)g.n_tiles;
         const float* desc    = fb.ent_tail + fb.entry_base[b] * DS + 4;  // descriptor row of entry e at desc + e * DS
@@ -431,8 +431,6 @@ cudaError_t launch_blend_backward(const ScenePtrs& sc, const CamConst* cams, con
                                   int B, const FwdBuffers& fb, const BwdBuffers& bb, const ConstLayerPtrs& grad_in,
                                   bool want_cam_grads, int sm_count, cudaStream_t st)
 {
-    cudaError_t e = cudaMemsetAsync(fb.ticket, 0, sizeof(unsigned), st);
-    if (e != cudaSuccess) return e;
     const int grid = (int)max(1u, min((unsigned)(sm_count * kBwdBlocksPerSM), ((unsigned)g.n_tiles * (unsigned)B + kBwdWarps - 1) / kBwdWarps));
 #define TRIPS_BWD_CASE(CC)                                                                                         \
     case CC:                                                                                                       \

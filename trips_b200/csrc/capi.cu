@@ -120,7 +120,8 @@ struct TripsContext
     int sm_count = 148;
     std::string error;
     // forward scratch
-    DevBuf heavy, views, cams, bin_count, bin_base, view_total, bin_cursor, entry_base, entries, counts, offsets, partial, view_base, frags, rec_n, records, stats, ticket, point_entry, resize_scratch, block_box, block_skip;
+    DevBuf heavy, cams, zeroed, bin_base, view_total, bin_cursor, entry_base, entries, offsets, partial, view_base, frags, rec_n, records, stats, point_entry, resize_scratch, block_box, block_skip;
+    size_t zero_bins = 0, zero_counts = 0;  // where bin_count and counts start inside `zeroed` (behind the work counters)
     // backward scratch
     DevBuf egrad, g_small;
     // adam
@@ -198,17 +199,20 @@ static ScenePtrs scene_ptrs(const TripsScene* s)
     return sp;
 }
 
-static FwdBuffers fwd_buffers(TripsContext* c)
+// work counters of the binning passes: one per pass and group of views
+static size_t ticket_groups(int B) { return 2 * (((size_t)B + kViewGroup - 1) / kViewGroup); }
+
+static FwdBuffers fwd_buffers(TripsContext* c, int B)
 {
     FwdBuffers fb;
-    fb.bin_count  = (uint32_t*)c->bin_count.p;
+    fb.bin_count  = (uint32_t*)((char*)c->zeroed.p + c->zero_bins);
     fb.bin_base   = (uint32_t*)c->bin_base.p;
     fb.view_total = (uint32_t*)c->view_total.p;
     fb.bin_cursor = (uint32_t*)c->bin_cursor.p;
     fb.entry_base = (unsigned long long*)c->entry_base.p;
     fb.ent_head   = (float4*)c->entries.p;
     fb.ent_tail   = (float*)c->entries.p + 8 * c->entry_cap;
-    fb.counts     = (uint32_t*)c->counts.p;
+    fb.counts     = (uint32_t*)((char*)c->zeroed.p + c->zero_counts);
     fb.offsets    = (uint32_t*)c->offsets.p;
     fb.partial    = (uint32_t*)c->partial.p;
     fb.view_base  = (unsigned long long*)c->view_base.p;
@@ -217,7 +221,10 @@ static FwdBuffers fwd_buffers(TripsContext* c)
     fb.rec_n      = (uint8_t*)c->rec_n.p;
     fb.records    = (uint2*)c->records.p;
     fb.stats      = (DevStats*)c->stats.p;
-    fb.ticket     = (unsigned int*)c->ticket.p;
+    fb.ticket         = (unsigned int*)c->zeroed.p;
+    fb.ticket_count   = fb.ticket + ticket_groups(B);
+    fb.ticket_collect = fb.ticket_count + B;
+    fb.ticket_blend   = fb.ticket_collect + B;
     fb.point_entry = c->params.train ? (uint32_t*)c->point_entry.p : nullptr;
     fb.block_box  = (const float*)c->block_box.p;
     fb.block_skip = (const uint8_t*)c->block_skip.p;
@@ -225,21 +232,13 @@ static FwdBuffers fwd_buffers(TripsContext* c)
     return fb;
 }
 
-// DevStats is allocated once and zeroed then; afterwards only its counters are cleared per call.
+// DevStats is allocated once and zeroed then; afterwards setup_cams_kernel clears its counters per call.
 static cudaError_t ensure_stats(TripsContext* c, cudaStream_t st)
 {
     if (c->stats.p) return cudaSuccess;
     cudaError_t e = ensure(c->stats, sizeof(DevStats));
     if (e != cudaSuccess) return e;
     return cudaMemsetAsync(c->stats.p, 0, sizeof(DevStats), st);
-}
-
-static cudaError_t clear_counters(TripsContext* c, cudaStream_t st)
-{
-    static_assert(offsetof(DevStats, status) + sizeof(unsigned) == offsetof(DevStats, culled_blocks), "the counters lie on either side of the status word");
-    cudaError_t e = cudaMemsetAsync(c->stats.p, 0, offsetof(DevStats, status), st);
-    if (e != cudaSuccess) return e;
-    return cudaMemsetAsync((char*)c->stats.p + offsetof(DevStats, culled_blocks), 0, sizeof(unsigned int), st);
 }
 
 static bool valid_channels(int c) { return c == 3 || c == 4 || c == 6 || c == 8 || c == 16; }
@@ -285,8 +284,8 @@ int trips_context_create(TripsContext** out, int device)
 void trips_context_destroy(TripsContext* c)
 {
     if (!c) return;
-    DevBuf* all[] = {&c->heavy, &c->views, &c->cams, &c->bin_count, &c->bin_base, &c->view_total, &c->bin_cursor, &c->entry_base, &c->entries, &c->counts, &c->offsets,
-                     &c->partial, &c->view_base, &c->frags, &c->rec_n, &c->records, &c->stats, &c->ticket, &c->egrad,
+    DevBuf* all[] = {&c->heavy, &c->cams, &c->zeroed, &c->bin_base, &c->view_total, &c->bin_cursor, &c->entry_base, &c->entries, &c->offsets,
+                     &c->partial, &c->view_base, &c->frags, &c->rec_n, &c->records, &c->stats, &c->egrad,
                      &c->point_entry, &c->g_small, &c->adam_tab, &c->resize_scratch, &c->block_box, &c->block_skip};
     for (DevBuf* b : all) free_buf(*b);
     c->timers.destroy();
@@ -396,9 +395,13 @@ static int forward_views(TripsContext* ctx, const TripsScene* scene, const Trips
     const int nchunks = (int)((P + kScanChunk - 1) / kScanChunk);
     const size_t n_box = (N + 8191) / 8192 + 1;
 
-    CU_CHECK(ctx, ensure(ctx->views, sizeof(TripsView) * B));
     CU_CHECK(ctx, ensure(ctx->cams, sizeof(CamConst) * B));
-    CU_CHECK(ctx, ensure(ctx->bin_count, sizeof(uint32_t) * (size_t)g.n_bins * 32 * B));  // one counter per (bin, 8x4 tile of the bin)
+    // everything a pass wants zeroed, in one buffer and one clear: work counters | visible points per (bin, 8x4 tile of the bin) | list lengths
+    auto aligned      = [](size_t n) { return (n + 255) & ~(size_t)255; };
+    ctx->zero_bins    = aligned(sizeof(unsigned) * (ticket_groups(B) + 2 * (size_t)B + 1));
+    ctx->zero_counts  = ctx->zero_bins + aligned(sizeof(uint32_t) * (size_t)g.n_bins * 32 * B);
+    const size_t zero_bytes = ctx->zero_counts + sizeof(uint32_t) * P * B;
+    CU_CHECK(ctx, ensure(ctx->zeroed, zero_bytes));
     CU_CHECK(ctx, ensure(ctx->bin_base, sizeof(uint32_t) * (size_t)g.n_bins * 32 * B));
     CU_CHECK(ctx, ensure(ctx->view_total, sizeof(uint32_t) * B));
     CU_CHECK(ctx, ensure(ctx->bin_cursor, sizeof(uint32_t) * (size_t)g.n_bins * B));
@@ -406,12 +409,10 @@ static int forward_views(TripsContext* ctx, const TripsScene* scene, const Trips
     CU_CHECK(ctx, ensure(ctx->block_box, sizeof(float) * 6 * n_box));
     CU_CHECK(ctx, ensure(ctx->block_skip, (size_t)B * n_box));
     CU_CHECK(ctx, ensure(ctx->heavy, sizeof(uint2) * (size_t)kHeavyCap));
-    CU_CHECK(ctx, ensure(ctx->counts, sizeof(uint32_t) * P * B));
     CU_CHECK(ctx, ensure(ctx->offsets, sizeof(uint32_t) * P * B));
     CU_CHECK(ctx, ensure(ctx->partial, sizeof(uint32_t) * (size_t)nchunks * B));
     CU_CHECK(ctx, ensure(ctx->view_base, sizeof(unsigned long long) * (B + 1)));
     CU_CHECK(ctx, ensure_stats(ctx, st));
-    CU_CHECK(ctx, ensure(ctx->ticket, sizeof(unsigned) * (size_t)(B > 64 ? B : 64)));
     if (params->train)
     {
         CU_CHECK(ctx, ensure(ctx->rec_n, (size_t)g.n_tiles * 32 * B));
@@ -429,15 +430,11 @@ static int forward_views(TripsContext* ctx, const TripsScene* scene, const Trips
 
     ScenePtrs sp = scene_ptrs(scene);
     sp.dropout   = dropout;
-    FwdBuffers fb = fwd_buffers(ctx);
-    // the counters start from zero; the status word keeps the bits raised by earlier calls until trips_last_status reads them
-    CU_CHECK(ctx, clear_counters(ctx, st));
-    CU_CHECK(ctx, cudaMemsetAsync(ctx->counts.p, 0, sizeof(uint32_t) * P * B, st));
-    // the view table comes from pageable host memory: the copy is staged before the call returns
-    CU_CHECK(ctx, cudaMemcpyAsync(ctx->views.p, views, sizeof(TripsView) * B, cudaMemcpyHostToDevice, st));
-    STAGE(ctx, TRIPS_STAGE_SETUP, 1, st,
-          launch_setup_cams((const TripsView*)ctx->views.p, B, scene->poses, scene->n_images, scene->intrinsics,
-                            scene->n_cameras, params->distortion, params->dist_cutoff, (CamConst*)ctx->cams.p, fb.stats, st));
+    FwdBuffers fb = fwd_buffers(ctx, B);
+    CU_CHECK(ctx, cudaMemsetAsync(ctx->zeroed.p, 0, zero_bytes, st));
+    STAGE(ctx, TRIPS_STAGE_SETUP, (B + kViewTable - 1) / kViewTable, st,
+          launch_setup_cams(views, B, scene->poses, scene->n_images, scene->intrinsics, scene->n_cameras, params->distortion,
+                            params->dist_cutoff, (CamConst*)ctx->cams.p, fb.stats, st));
     const CamConst* cams = (const CamConst*)ctx->cams.p;
     // crowded: the last call that reported back saw more than kHotKey visible points in one (view, bin, tile) group
     STAGE(ctx, TRIPS_STAGE_BIN_POINTS, bin_count_launches((int)N, B), st,
@@ -448,7 +445,7 @@ static int forward_views(TripsContext* ctx, const TripsScene* scene, const Trips
         CU_CHECK(ctx, cudaStreamSynchronize(st));
         CU_CHECK(ctx, ensure_entries(ctx, (size_t)h_stats->visible, C, kGrowth));
         ctx->crowded = h_stats->max_key >= kHotKey;  // this call's own count pass already knows
-        fb           = fwd_buffers(ctx);
+        fb           = fwd_buffers(ctx, B);
     }
     STAGE(ctx, TRIPS_STAGE_BIN_POINTS, bin_scatter_launches((int)N, B), st, launch_bin_scatter(sp, cams, g, *params, B, fb, ctx->crowded, ctx->sm_count, st));
     if (N > 0) STAGE(ctx, TRIPS_STAGE_COUNT, 1, st, launch_count(sp, g, B, fb, strict_layers(*params), wait_for_sizes ? (unsigned long long)h_stats->visible : ctx->need_entries, ctx->sm_count, st));
@@ -464,7 +461,7 @@ static int forward_views(TripsContext* ctx, const TripsScene* scene, const Trips
         if ((size_t)h_stats->frag_need * sizeof(uint4) > ctx->frags.bytes)
         {
             CU_CHECK(ctx, ensure(ctx->frags, (size_t)h_stats->frag_need * sizeof(uint4), kGrowth));
-            fb = fwd_buffers(ctx);
+            fb = fwd_buffers(ctx, B);
         }
         ctx->need_entries = h_stats->visible;
         ctx->need_frags   = h_stats->frag_need;
@@ -599,7 +596,7 @@ int trips_backward(TripsContext* ctx, const TripsScene* scene, const float* cons
 
     const size_t GS = (size_t)egrad_stride(C);
     CU_CHECK(ctx, ensure(ctx->egrad, sizeof(float) * GS * ctx->entry_cap + 16));  // one row per entry the arrays can hold
-    const size_t small_bytes = sizeof(double) * (TRIPS_MAX_CHANNELS + (size_t)B * 19);  // background | per view: 6 pose, 5 pinhole, 8 distortion
+    const size_t small_bytes = sizeof(double) * (TRIPS_MAX_CHANNELS + (size_t)B * 19 + 1);  // background | per view: 6 pose, 5 pinhole, 8 distortion | work counter
     CU_CHECK(ctx, ensure(ctx->g_small, small_bytes));
     BwdBuffers bb;
     bb.egrad        = (float*)ctx->egrad.p;
@@ -607,8 +604,9 @@ int trips_backward(TripsContext* ctx, const TripsScene* scene, const float* cons
     bb.g_pose       = bb.g_bg + TRIPS_MAX_CHANNELS;
     bb.g_k          = bb.g_pose + (size_t)B * 6;
     bb.g_dis        = bb.g_k + (size_t)B * 5;
+    bb.ticket       = (unsigned int*)(bb.g_dis + (size_t)B * 8);
     ScenePtrs sp  = scene_ptrs(scene);
-    FwdBuffers fb = fwd_buffers(ctx);
+    FwdBuffers fb = fwd_buffers(ctx, B);
     // all accumulators start from zero (timed with the gradient bookkeeping of the unpack stage)
     auto clear_accumulators = [&]() -> cudaError_t {
         cudaError_t e = cudaSuccess;
@@ -670,6 +668,11 @@ int trips_adam_step(TripsContext* ctx, const TripsAdamTensor* tensors, int n_ten
         start[i + 1] = start[i] + (t.n + kAdamPerBlock - 1) / kAdamPerBlock;
     }
     if (start[n_tensors] >= (1ll << 31)) return fail(ctx, TRIPS_ERR_TOO_LARGE, "too many elements for one Adam launch");
+    if (n_tensors <= kAdamTable)
+    {
+        STAGE(ctx, TRIPS_STAGE_ADAM, 1, st, launch_adam_by_value(tensors, start.data(), n_tensors, st));
+        return TRIPS_OK;
+    }
     const size_t tab_bytes   = sizeof(TripsAdamTensor) * n_tensors;
     const size_t tab_aligned = (tab_bytes + 15) & ~(size_t)15;
     CU_CHECK(ctx, ensure(ctx->adam_tab, tab_aligned + sizeof(int64_t) * (n_tensors + 1)));
@@ -867,7 +870,7 @@ int trips_debug_lists(TripsContext* ctx, int view, int32_t* counts, int64_t* off
     unsigned long long vb[2];
     CU_CHECK(ctx, cudaMemcpyAsync(vb, (unsigned long long*)ctx->view_base.p + view, sizeof(vb), cudaMemcpyDeviceToHost, st));
     std::vector<uint32_t> c(P), e(P);
-    CU_CHECK(ctx, cudaMemcpyAsync(c.data(), (uint32_t*)ctx->counts.p + off, sizeof(uint32_t) * P, cudaMemcpyDeviceToHost, st));
+    CU_CHECK(ctx, cudaMemcpyAsync(c.data(), (const uint32_t*)((const char*)ctx->zeroed.p + ctx->zero_counts) + off, sizeof(uint32_t) * P, cudaMemcpyDeviceToHost, st));
     CU_CHECK(ctx, cudaMemcpyAsync(e.data(), (uint32_t*)ctx->offsets.p + off, sizeof(uint32_t) * P, cudaMemcpyDeviceToHost, st));
     CU_CHECK(ctx, cudaStreamSynchronize(st));
     const unsigned long long nf = vb[1] - vb[0];

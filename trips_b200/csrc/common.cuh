@@ -14,6 +14,7 @@ constexpr int kBinShift   = 5;   // visible points are bucketed by 32x32-pixel s
 constexpr int kTileW      = 8;   // one warp renders / differentiates an 8x4 pixel tile
 constexpr int kTileH      = 4;
 constexpr uint32_t kNoEntry = 0xffffffffu;  // a point that is not visible in a view
+constexpr int kViewGroup  = 16;  // views whose camera constants are in shared memory at a time in the binning passes (one launch per group)
 constexpr int kHeavyList  = 512;      // lists longer than this get their 16 nearest fragments moved to the front by a block of their own
 constexpr int kHeavyCap   = 1 << 16;  // such lists per call the pre-selection handles; beyond that the blend walks them itself
 
@@ -108,7 +109,11 @@ struct FwdBuffers
     uint2* records;                   // [B,n_tiles,16,32] (entry index within the view, alpha bits), by tile, rank and lane: a warp's
                                       // access to one rank of its tile is 256 consecutive bytes
     DevStats* stats;
-    unsigned int* ticket;
+    // work counters of the persistent kernels, zeroed with bin_count and counts by one clear per forward pass
+    unsigned int* ticket;             // binning passes: one per pass and group of views
+    unsigned int* ticket_count;       // [B] count pass
+    unsigned int* ticket_collect;     // [B] collect pass
+    unsigned int* ticket_blend;
     uint32_t* point_entry;            // training: [B,N] entry (within the view) of every point, kNoEntry where it is not visible
     const float* block_box;           // [ceil(N / 8192), 6] bounding boxes (min xyz, max xyz) of blocks of consecutive points
     const uint8_t* block_skip;        // [B, ceil(N / 8192)] 1 = the block cannot hold a point visible in that view
@@ -130,6 +135,7 @@ struct ScenePtrs
 struct BwdBuffers
 {
     float* egrad;         // [sum V_b, egrad_stride] per-entry gradient accumulators
+    unsigned int* ticket; // work counter of the tile kernel
     double* g_bg;         // [C]
     double* g_pose;       // [B,6]
     double* g_k;          // [B,5]
@@ -325,8 +331,9 @@ __host__ __device__ __forceinline__ void pixel_tile(const Geom& g, int layer, in
 }
 
 // ---- launchers (forward.cu / backward.cu / adam.cu) ----
-cudaError_t launch_setup_cams(const TripsView* d_views, int B, const double* poses, int n_images, const float* intrinsics,
+cudaError_t launch_setup_cams(const TripsView* h_views, int B, const double* poses, int n_images, const float* intrinsics,
                               int n_cameras, int distortion, float dist_cutoff, CamConst* cams, DevStats* stats, cudaStream_t st);
+constexpr int kViewTable = 32;  // views passed to one launch of setup_cams_kernel as an argument;
 cudaError_t launch_bin_count(const ScenePtrs& sc, const CamConst* cams, const Geom& g, const TripsRenderParams& pr, int B,
                              const FwdBuffers& fb, unsigned long long entry_cap, bool hot, int sm_count, cudaStream_t st);
 cudaError_t launch_bin_scatter(const ScenePtrs& sc, const CamConst* cams, const Geom& g, const TripsRenderParams& pr, int B,
@@ -357,6 +364,8 @@ cudaError_t launch_unpack_grads(const ScenePtrs& sc, const CamConst* cams, int B
                                 const TripsGrads& out, const TripsRenderParams& pr, int sm_count, cudaStream_t st);
 cudaError_t launch_adam(const TripsAdamTensor* d_tensors, const int64_t* d_block_start, int n_tensors, int64_t total_blocks,
                         cudaStream_t st);
+constexpr int kAdamTable = 16;  // tensors whose table travels as a kernel argument
+cudaError_t launch_adam_by_value(const TripsAdamTensor* h_tensors, const int64_t* h_block_start, int n_tensors, cudaStream_t st);
 cudaError_t launch_fused_reduce_adam(const float* const* grad_ptrs, float* const* param_ptrs, int world, int rank,
                                      const TripsAdamSegment* segs, int n_seg, int64_t lo, int64_t hi, float* m_state,
                                      float* v_state, int32_t* steps, int sm_count, cudaStream_t st);

@@ -13,13 +13,26 @@ namespace trips
 // ------------------------------------------------------------------------------------------------------------
 // per-view camera constants
 // ------------------------------------------------------------------------------------------------------------
-__global__ void setup_cams_kernel(const TripsView* __restrict__ views, int B, const double* __restrict__ poses, int n_images,
+// The view table travels as a kernel argument: a copy from pageable host memory costs a staging copy on the host and a
+// transfer of its own on the stream.
+struct ViewTable
+{
+    TripsView v[kViewTable];
+};
+__global__ void setup_cams_kernel(const __grid_constant__ ViewTable views, int b0, int B, const double* __restrict__ poses, int n_images,
                                   const float* __restrict__ intrinsics, int n_cameras, int distortion, float dist_cutoff,
                                   CamConst* __restrict__ cams, DevStats* stats)
 {
-    int b = blockIdx.x * blockDim.x + threadIdx.x;
+    const int b = b0 + (int)threadIdx.x;
+    if (b == 0)
+    {
+        // the counters of the call start from zero; the status word keeps the bits raised by earlier calls until
+        // trips_last_status reads them
+        stats->visible = stats->kept = stats->frag_need = 0ull;
+        stats->max_len = stats->n_heavy = stats->max_key = stats->pad0 = stats->culled_blocks = 0u;
+    }
     if (b >= B) return;
-    const TripsView v = views[b];
+    const TripsView& v = views.v[threadIdx.x];
     CamConst c;
     const double* p = poses + (size_t)min(max(v.image_index, 0), n_images - 1) * 8;
     // DeviceRenderParams::Pose: SE3d cast to float (RenderConstants.h:85-88)
@@ -72,10 +85,17 @@ __global__ void setup_cams_kernel(const TripsView* __restrict__ views, int B, co
     cams[b]        = c;
 }
 
-cudaError_t launch_setup_cams(const TripsView* d_views, int B, const double* poses, int n_images, const float* intrinsics,
+cudaError_t launch_setup_cams(const TripsView* h_views, int B, const double* poses, int n_images, const float* intrinsics,
                               int n_cameras, int distortion, float dist_cutoff, CamConst* cams, DevStats* stats, cudaStream_t st)
 {
-    setup_cams_kernel<<<(B + 63) / 64, 64, 0, st>>>(d_views, B, poses, n_images, intrinsics, n_cameras, distortion, dist_cutoff, cams, stats);
+    for (int b0 = 0; b0 < B; b0 += kViewTable)
+    {
+        ViewTable t;
+        const int n = min(kViewTable, B - b0);
+        for (int k = 0; k < n; ++k) t.v[k] = h_views[b0 + k];
+        for (int k = n; k < kViewTable; ++k) t.v[k] = h_views[b0];
+        setup_cams_kernel<<<1, kViewTable, 0, st>>>(t, b0, B, poses, n_images, intrinsics, n_cameras, distortion, dist_cutoff, cams, stats);
+    }
     return cudaGetLastError();
 }
 
@@ -125,7 +145,6 @@ constexpr int kScatterMinBlocks = 4, kScatterMinBlocksWide = 3;  // up to 4 chan
 constexpr int kBinChunk       = 8192;  // points per bounding box
 constexpr int kBinTicket      = 1024;
 constexpr int kSweep          = 4;      // views whose entry slots a thread requests before it waits for any of them  // points per work ticket of the binning kernels; a ticket lies inside one box
-constexpr int kViewGroup      = 16;    // views whose camera constants are in shared memory at a time (one launch per group)
 static_assert(kBinChunk % kBinTicket == 0, "a ticket must not straddle two bounding boxes");
 
 // Bounding boxes of blocks of consecutive points and the conservative frustum test on them: the reference computes
@@ -769,10 +788,6 @@ cudaError_t launch_bin_count(const ScenePtrs& sc, const CamConst* cams, const Ge
     const int n_keys   = g.n_bins << kSubShift;
     const int grid     = sm_count * kBinBlocksPerSM;
     const int n_groups = (B + kViewGroup - 1) / kViewGroup;
-    cudaError_t e      = cudaMemsetAsync(fb.bin_count, 0, sizeof(uint32_t) * (size_t)B * n_keys, st);
-    if (e != cudaSuccess) return e;
-    e = cudaMemsetAsync(fb.ticket, 0, 2 * n_groups * sizeof(unsigned), st);  // one counter per pass and view group
-    if (e != cudaSuccess) return e;
     if (sc.N > 0 && fb.block_box && fb.block_skip)
     {
         const int nbk = (sc.N + kBinChunk - 1) / kBinChunk;
@@ -1073,13 +1088,13 @@ __device__ __forceinline__ int window_pixel(const Geom& g, const Window& w, int 
 }
 
 // the chunk [c0, c1) of the view's entries and the first bin it touches; false when the view has no more chunks
-__device__ __forceinline__ bool next_chunk(const FwdBuffers& fb, const Geom& g, int b, uint32_t n_entry, uint32_t* s_tmp, int kWinChunk,
+__device__ __forceinline__ bool next_chunk(const FwdBuffers& fb, const Geom& g, int b, unsigned* ticket, uint32_t n_entry, uint32_t* s_tmp, int kWinChunk,
                                            uint32_t& c0, uint32_t& c1, int& first_bin)
 {
     __syncthreads();
     if (threadIdx.x == 0)
     {
-        const uint32_t t = atomicAdd(fb.ticket + b, 1u);
+        const uint32_t t = atomicAdd(ticket + b, 1u);
         uint32_t lo      = (uint32_t)min((unsigned long long)t * kWinChunk, (unsigned long long)n_entry);
         s_tmp[0]         = lo;
         // last bin whose first entry is <= lo (empty bins share their first entry with the next non-empty one)
@@ -1258,7 +1273,7 @@ __global__ __launch_bounds__(kWinThreads, kWinMinBlocks) void window_kernel(cons
     const uint32_t* bfirst = fb.bin_cursor + (size_t)b * g.n_bins;
     uint32_t c0, c1;
     int bin;
-    while (next_chunk(fb, g, b, n_entry, s_tmp, chunk, c0, c1, bin))
+    while (next_chunk(fb, g, b, COLLECT ? fb.ticket_collect : fb.ticket_count, n_entry, s_tmp, chunk, c0, c1, bin))
     {
         for (; bin < g.n_bins && bfirst[bin] < c1; ++bin)
         {
@@ -1343,8 +1358,6 @@ __global__ __launch_bounds__(kWinThreads, kWinMinBlocks) void window_kernel(cons
 cudaError_t launch_count(const ScenePtrs& sc, const Geom& g, int B, const FwdBuffers& fb, bool strict, unsigned long long entries_hint, int sm_count,
                          cudaStream_t st)
 {
-    cudaError_t e = cudaMemsetAsync(fb.ticket, 0, sizeof(unsigned) * B, st);
-    if (e != cudaSuccess) return e;
     // entries_hint: the number of entries of the call as far as the host knows it (the previous call's, or this call's own count)
     const bool few  = entries_hint / kWinChunkCount < (unsigned long long)kWinTicketsPerBlock * sm_count * kWinMinBlocks;
     const int chunk = few ? kWinChunkCountFew : kWinChunkCount;
@@ -1357,8 +1370,6 @@ cudaError_t launch_count(const ScenePtrs& sc, const Geom& g, int B, const FwdBuf
 
 cudaError_t launch_collect(const ScenePtrs& sc, const Geom& g, int B, const FwdBuffers& fb, bool strict, int sm_count, cudaStream_t st)
 {
-    cudaError_t e = cudaMemsetAsync(fb.ticket, 0, sizeof(unsigned) * B, st);
-    if (e != cudaSuccess) return e;
     if (strict)
         window_kernel<true, true><<<sm_count * kWinBlocksPerSM, kWinThreads, 0, st>>>(g, fb, B, kWinChunkCollect);
     else
@@ -1611,13 +1622,13 @@ __global__ __launch_bounds__(kSbThreads, (C <= 4 ? kSbMinBlocks : (C <= 8 ? kSbM
 
     const bool preselected = fb.stats->n_heavy <= (unsigned)kHeavyCap;  // heavy_topk_kernel handled every long list
     unsigned next_ticket = 0;
-    if (lane == 0) next_ticket = atomicAdd(fb.ticket, 1u);
+    if (lane == 0) next_ticket = atomicAdd(fb.ticket_blend, 1u);
     for (;;)
     {
         // the ticket of the following tile is requested now, a whole tile ahead of its use
         const unsigned ticket = __shfl_sync(kFull, next_ticket, 0);
         if (ticket >= n_tiles_total) break;
-        if (lane == 0) next_ticket = atomicAdd(fb.ticket, 1u);
+        if (lane == 0) next_ticket = atomicAdd(fb.ticket_blend, 1u);
         const int b          = ticket / (unsigned)g.n_tiles;
         const int tile       = ticket - b * (unsigned)g.n_tiles;
         const size_t bP      = (size_t)b * g.P;
@@ -1858,9 +1869,7 @@ cudaError_t launch_sort_blend(const ScenePtrs& sc, const Geom& g, const TripsRen
                               const LayerPtrs& out, int sm_count, cudaStream_t st)
 {
     const unsigned n_tiles = (unsigned)g.n_tiles * (unsigned)B;
-    cudaError_t e          = cudaMemsetAsync(fb.ticket, 0, sizeof(unsigned), st);
-    if (e != cudaSuccess) return e;
-    int blocks = (int)min((unsigned)(sm_count * 16), (n_tiles + kSbWarps - 1) / kSbWarps);
+    int blocks             = (int)min((unsigned)(sm_count * 16), (n_tiles + kSbWarps - 1) / kSbWarps);
     blocks     = max(blocks, 1);
     switch (sc.C)
     {
