@@ -1041,9 +1041,12 @@ constexpr int kWinChunkCountFew = 1024;  // the same when the call has too few e
 constexpr int kWinTicketsPerBlock = 6;   // measured count pass, tickets of 4096 / 1024: config 4 (2 views, 16 M entries) 0.58 / 0.25 ms, config 2
                                          // (4 M) 0.093 / 0.09 ms; config 3 (27 M) 0.31 / 0.52 ms, config 5 (39 M) 0.40 / 0.53 ms
 constexpr int kWinChunkCollect = 1024;  // and collecting pass: the lists a chunk writes to must stay in L2 until complete (measured with tile-ordered entries: 256 1.80 ms, 512 1.46 ms, 1024 1.35 ms, 2048 1.47 ms)
-constexpr int kWinThreads    = 256;
-constexpr int kWinBlocksPerSM = 8;  // grid size of the window kernels, in blocks per SM
-constexpr int kWinMinBlocks  = 5;  // resident blocks the register allocation leaves room for
+constexpr int kWinChunkCollectFew = 512;  // calls with few entries, by blocks of 128 threads: 2 views, 16 M entries (uneven density) 0.91 -> 0.69 ms; on 40 M entries 1024 entries by 256 threads is better (1.87 against 1.92 ms)
+// Threads of a block.  Half as many per barrier suits the counting pass (40 M entries 0.405 -> 0.380 ms, crowded clouds 0.145 ->
+// 0.122 ms); the collecting pass at 1024 entries per chunk wants 256 (1.25 against 1.45 ms with 128).
+constexpr int kWinThreadsCount = 128, kWinThreadsCollect = 256, kWinThreadsCollectFew = 128;
+constexpr int kWinWarpsPerSM   = 64;  // grid size of the window kernels, in warps per SM
+constexpr int kWinMinWarps     = 40;  // resident warps the register allocation leaves room for
 constexpr int kWinMax     = 34 * 34 + 18 * 18 + 10 * 10 + 6 * 6 + 4 * 4 + 3 * 3 * 3;  // 1659 window pixels over 8 layers
 
 // Window of a bin: on layer l it starts at ((32 bx) >> l, (32 by) >> l) and is win_w(l) pixels wide; the counters of
@@ -1125,7 +1128,7 @@ __device__ __forceinline__ bool next_chunk(const FwdBuffers& fb, const Geom& g, 
 // First layer of an entry written by the strict two-layer rule: the layer below log2(size), as write_entry computed it.
 __device__ __forceinline__ int strict_first_layer(float ps, int L) { return ps > 1.f ? min(tm_floor_log2(ps), L - 1) : 0; }
 
-template <bool WITH_E1, bool STRICT, class Body>
+template <int THREADS, bool WITH_E1, bool STRICT, class Body>
 __device__ __forceinline__ void for_each_footprint(const float4* __restrict__ head, uint32_t lo, uint32_t hi, uint8_t* queue, int L, Body&& body)
 {
     const int lane = threadIdx.x & 31;
@@ -1136,15 +1139,15 @@ __device__ __forceinline__ void for_each_footprint(const float4* __restrict__ he
         e0n = head[2 * (size_t)(base + lane)];      // u v ps conf
         e1n = head[2 * (size_t)(base + lane) + 1];  // pid z raw nl
     }
-    for (; base < hi; base += kWinThreads)
+    for (; base < hi; base += THREADS)
     {
         const uint32_t ei = base + lane;
         const float4 e0 = e0n, e1 = e1n;
         const int nl = ei < hi ? __float_as_int(e1.w) : 0;
-        if (base + kWinThreads + lane < hi)  // the next round's entry travels while this one is processed
+        if (base + THREADS + lane < hi)  // the next round's entry travels while this one is processed
         {
-            e0n = head[2 * (size_t)(ei + kWinThreads)];
-            e1n = head[2 * (size_t)(ei + kWinThreads) + 1];
+            e0n = head[2 * (size_t)(ei + THREADS)];
+            e1n = head[2 * (size_t)(ei + THREADS) + 1];
         }
         int first = 0;
         if constexpr (STRICT)
@@ -1212,11 +1215,11 @@ __device__ __forceinline__ uint64_t evict_last_policy()
 // and flushing a window of shared-memory counters with three block barriers: its footprints go straight to the pixels'
 // global counters.  (On a 2560x1440 view of 20 M points with half of the bins nearly empty, the blocks that drew the
 // sparse tickets ran 12 times longer than the others.)  Not inlined: the dense path keeps its registers.
-template <bool COLLECT, bool STRICT>
+template <int THREADS, bool COLLECT, bool STRICT>
 __device__ __noinline__ void sparse_bin_footprints(const Geom& g, const float4* __restrict__ head, uint32_t lo, uint32_t hi, uint8_t* queue,
                                                    uint32_t* pixel_ctr, uint4* frags, uint64_t keep)
 {
-    for_each_footprint<COLLECT, STRICT>(head, lo, hi, queue, g.L, [&](const float4& e0, const float4& e1, float x, float y, int layer, uint32_t ei) {
+    for_each_footprint<THREADS, COLLECT, STRICT>(head, lo, hi, queue, g.L, [&](const float4& e0, const float4& e1, float x, float y, int layer, uint32_t ei) {
         const int px = __float2int_rd(x), py = __float2int_rd(y);
         const int Wl = g.W[layer];
         uint32_t* c  = pixel_ctr + g.base[layer] + py * Wl + px;
@@ -1253,14 +1256,14 @@ __device__ __noinline__ void sparse_bin_footprints(const Geom& g, const float4* 
     });
 }
 
-template <bool COLLECT, bool STRICT>
-__global__ __launch_bounds__(kWinThreads, kWinMinBlocks) void window_kernel(const __grid_constant__ Geom g, FwdBuffers fb, int B, int chunk)
+template <int THREADS, bool COLLECT, bool STRICT>
+__global__ __launch_bounds__(THREADS, kWinMinWarps * 32 / THREADS) void window_kernel(const __grid_constant__ Geom g, FwdBuffers fb, int B, int chunk)
 {
     __shared__ uint32_t s_cnt[kWinMax];
     __shared__ uint32_t s_base[COLLECT ? kWinMax : 1];
     __shared__ uint32_t s_tmp[2];
     const uint64_t keep = evict_last_policy();
-    __shared__ uint8_t s_queue[kWinThreads / 32][32 * (TRIPS_MAX_LAYERS - 1)];
+    __shared__ uint8_t s_queue[THREADS / 32][32 * (TRIPS_MAX_LAYERS - 1)];
     // all blocks walk the views in the same order: the lists, counters and entries in flight belong to one view (or two,
     // where blocks cross over), which keeps the partially written list sectors of a view in L2 until they are complete
     for (int b = 0; b < B; ++b)
@@ -1282,15 +1285,15 @@ __global__ __launch_bounds__(kWinThreads, kWinMinBlocks) void window_kernel(cons
             if (lo >= hi) continue;  // uniform: all threads read the same values
             if (bin_end - bfirst[bin] <= (uint32_t)kWinSparse)  // the whole bin is sparse (a short piece of a dense bin still pays off in the window)
             {
-                sparse_bin_footprints<COLLECT, STRICT>(g, head, lo, hi, s_queue[threadIdx.x >> 5], pixel_ctr, frags, keep);
+                sparse_bin_footprints<THREADS, COLLECT, STRICT>(g, head, lo, hi, s_queue[threadIdx.x >> 5], pixel_ctr, frags, keep);
                 continue;
             }
             const Window w = make_window(g, bin);
             const int n_win = win_off(g.L);
-            for (int i = threadIdx.x; i < n_win; i += kWinThreads) s_cnt[i] = 0;
+            for (int i = threadIdx.x; i < n_win; i += THREADS) s_cnt[i] = 0;
             __syncthreads();
             // ---- fragments per window pixel ----
-            for_each_footprint<false, STRICT>(head, lo, hi, s_queue[threadIdx.x >> 5], g.L,
+            for_each_footprint<THREADS, false, STRICT>(head, lo, hi, s_queue[threadIdx.x >> 5], g.L,
                                       [&](const float4&, const float4&, float x, float y, int layer, uint32_t) {
                                           const int ww = win_w(layer);
                                           uint32_t* c  = s_cnt + win_off(layer) + (__float2int_rd(y) - w.y0(layer)) * ww + (__float2int_rd(x) - w.x0(layer));
@@ -1301,7 +1304,7 @@ __global__ __launch_bounds__(kWinThreads, kWinMinBlocks) void window_kernel(cons
                                       });
             __syncthreads();
             // ---- one global atomic per touched pixel ----
-            for (int i = threadIdx.x; i < n_win; i += kWinThreads)
+            for (int i = threadIdx.x; i < n_win; i += THREADS)
             {
                 const uint32_t c = s_cnt[i];
                 if (c)
@@ -1320,7 +1323,7 @@ __global__ __launch_bounds__(kWinThreads, kWinMinBlocks) void window_kernel(cons
             if (COLLECT)
             {
                 // ---- slots inside the reserved ranges; alpha and the fragment itself ----
-                for_each_footprint<true, STRICT>(head, lo, hi, s_queue[threadIdx.x >> 5], g.L,
+                for_each_footprint<THREADS, true, STRICT>(head, lo, hi, s_queue[threadIdx.x >> 5], g.L,
                                          [&](const float4& e0, const float4& e1, float x, float y, int layer, uint32_t ei) {
                                              // x, y equal (u, v) * 2^-layer exactly (power-of-two scaling)
                                              const float conf   = e0.w;
@@ -1355,25 +1358,38 @@ __global__ __launch_bounds__(kWinThreads, kWinMinBlocks) void window_kernel(cons
     }
 }
 
+// Too few entries for kWinTicketsPerBlock tickets of kWinChunkCount per 8 resident warps?  entries_hint: the number of
+// entries of the call as far as the host knows it (the previous call's, or this call's own count)
+static bool few_entries(unsigned long long entries_hint, int sm_count)
+{
+    return entries_hint / kWinChunkCount < (unsigned long long)kWinTicketsPerBlock * sm_count * (kWinMinWarps / 8);
+}
+
+template <int THREADS, bool COLLECT>
+static void run_window(const Geom& g, int B, const FwdBuffers& fb, bool strict, int chunk, int sm_count, cudaStream_t st)
+{
+    const int grid = sm_count * (kWinWarpsPerSM * 32 / THREADS);
+    if (strict)
+        window_kernel<THREADS, COLLECT, true><<<grid, THREADS, 0, st>>>(g, fb, B, chunk);
+    else
+        window_kernel<THREADS, COLLECT, false><<<grid, THREADS, 0, st>>>(g, fb, B, chunk);
+}
+
 cudaError_t launch_count(const ScenePtrs& sc, const Geom& g, int B, const FwdBuffers& fb, bool strict, unsigned long long entries_hint, int sm_count,
                          cudaStream_t st)
 {
-    // entries_hint: the number of entries of the call as far as the host knows it (the previous call's, or this call's own count)
-    const bool few  = entries_hint / kWinChunkCount < (unsigned long long)kWinTicketsPerBlock * sm_count * kWinMinBlocks;
-    const int chunk = few ? kWinChunkCountFew : kWinChunkCount;
-    if (strict)
-        window_kernel<false, true><<<sm_count * kWinBlocksPerSM, kWinThreads, 0, st>>>(g, fb, B, chunk);
-    else
-        window_kernel<false, false><<<sm_count * kWinBlocksPerSM, kWinThreads, 0, st>>>(g, fb, B, chunk);
+    run_window<kWinThreadsCount, false>(g, B, fb, strict, few_entries(entries_hint, sm_count) ? kWinChunkCountFew : kWinChunkCount, sm_count, st);
     return cudaGetLastError();
 }
 
-cudaError_t launch_collect(const ScenePtrs& sc, const Geom& g, int B, const FwdBuffers& fb, bool strict, int sm_count, cudaStream_t st)
+// crowded: the lists of a few bins take everything; small chunks then mean more atomics on the same pixels (0.44 against 0.49 ms)
+cudaError_t launch_collect(const ScenePtrs& sc, const Geom& g, int B, const FwdBuffers& fb, bool strict, bool crowded, unsigned long long entries_hint,
+                           int sm_count, cudaStream_t st)
 {
-    if (strict)
-        window_kernel<true, true><<<sm_count * kWinBlocksPerSM, kWinThreads, 0, st>>>(g, fb, B, kWinChunkCollect);
+    if (!crowded && few_entries(entries_hint, sm_count))
+        run_window<kWinThreadsCollectFew, true>(g, B, fb, strict, kWinChunkCollectFew, sm_count, st);
     else
-        window_kernel<true, false><<<sm_count * kWinBlocksPerSM, kWinThreads, 0, st>>>(g, fb, B, kWinChunkCollect);
+        run_window<kWinThreadsCollect, true>(g, B, fb, strict, kWinChunkCollect, sm_count, st);
     return cudaGetLastError();
 }
 
