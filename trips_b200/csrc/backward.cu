@@ -44,9 +44,9 @@ constexpr int kPad        = 17;   // row pitch (entries) of the per-pixel arrays
 constexpr int kBwdThreads = 128;  // 4 warps x (32 x 17 slots x 12 bytes + fragment table + gradient tile) = 32 KB of static shared memory
 constexpr int kBwdWarps   = kBwdThreads / 32;
 
-// One warp differentiates an 8x4 pixel tile; tiles come from one ticket counter over all views, in the order of
+// One warp differentiates an 8x4 pixel tile; tiles come from a few ticket counters over all views, in the order of
 // tile_pixel (region-major), so the entries and gradient rows a tile touches are a short, L2-resident range.
-//   staging: the tile's records go to shared memory (8 lanes per pixel row: 4 lines per load instruction).
+//   staging: the tile's records go to shared memory (lane = pixel: 256 consecutive bytes per rank).
 //   phase 0 (lane = kept fragment, lanes densely packed over the tile's fragments): gather the descriptor row of
 //     the fragment's entry, G_j = <col_j, g> and alpha_j go to shared memory.
 //   phase 1 (lane = pixel, shared memory only): the sequential recurrences over the pixel's kept fragments:
@@ -90,17 +90,15 @@ __global__ __launch_bounds__(kBwdThreads, (C <= 4 ? kBwdMinBlocks : 1)) void ble
 #pragma unroll
     for (int c = 0; c < C; ++c) acc_bg[c] = 0.0;
 
-    // one ticket counter over all views: the views are processed one after the other, so the entries, gradient rows and
+    // the tickets run over the tiles of all views: the views are processed one after the other, so the entries, gradient rows and
     // records in flight belong to one view
     const unsigned n_total = (unsigned)g.n_tiles * (unsigned)B;
-    unsigned next_tile = 0;
-    if (lane == 0) next_tile = atomicAdd(bb.ticket, 1u);
+    TileTickets tickets;
+    tickets.start(bb.ticket, n_total, blockIdx.x * kBwdWarps + warp, lane);
     for (;;)
     {
-        // the ticket of the following tile is requested now, a whole tile ahead of its use
-        const unsigned ticket = __shfl_sync(kFull, next_tile, 0);
+        const unsigned ticket = tickets.next(lane);
         if (ticket >= n_total) break;
-        if (lane == 0) next_tile = atomicAdd(bb.ticket, 1u);
         const int b          = ticket / (unsigned)g.n_tiles;
         const unsigned tile  = ticket - b * (unsigned)g.n_tiles;
         const float* desc    = fb.ent_tail + fb.entry_base[b] * DS + 4;  // descriptor row of entry e at desc + e * DS

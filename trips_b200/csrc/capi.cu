@@ -201,6 +201,8 @@ static ScenePtrs scene_ptrs(const TripsScene* s)
 
 // work counters of the binning passes: one per pass and group of views
 static size_t ticket_groups(int B) { return 2 * (((size_t)B + kViewGroup - 1) / kViewGroup); }
+// work counter of the blend: behind those of the binning, count and collect passes, on a line of its own
+static size_t blend_ticket_at(int B) { return (ticket_groups(B) + 2 * (size_t)B + 31) / 32 * 32; }
 
 static FwdBuffers fwd_buffers(TripsContext* c, int B)
 {
@@ -224,7 +226,7 @@ static FwdBuffers fwd_buffers(TripsContext* c, int B)
     fb.ticket         = (unsigned int*)c->zeroed.p;
     fb.ticket_count   = fb.ticket + ticket_groups(B);
     fb.ticket_collect = fb.ticket_count + B;
-    fb.ticket_blend   = fb.ticket_collect + B;
+    fb.ticket_blend   = fb.ticket + blend_ticket_at(B);
     fb.point_entry = c->params.train ? (uint32_t*)c->point_entry.p : nullptr;
     fb.block_box  = (const float*)c->block_box.p;
     fb.block_skip = (const uint8_t*)c->block_skip.p;
@@ -398,7 +400,7 @@ static int forward_views(TripsContext* ctx, const TripsScene* scene, const Trips
     CU_CHECK(ctx, ensure(ctx->cams, sizeof(CamConst) * B));
     // everything a pass wants zeroed, in one buffer and one clear: work counters | visible points per (bin, 8x4 tile of the bin) | list lengths
     auto aligned      = [](size_t n) { return (n + 255) & ~(size_t)255; };
-    ctx->zero_bins    = aligned(sizeof(unsigned) * (ticket_groups(B) + 2 * (size_t)B + 1));
+    ctx->zero_bins    = aligned(sizeof(unsigned) * (blend_ticket_at(B) + 1));
     ctx->zero_counts  = ctx->zero_bins + aligned(sizeof(uint32_t) * (size_t)g.n_bins * 32 * B);
     const size_t zero_bytes = ctx->zero_counts + sizeof(uint32_t) * P * B;
     CU_CHECK(ctx, ensure(ctx->zeroed, zero_bytes));
@@ -596,7 +598,7 @@ int trips_backward(TripsContext* ctx, const TripsScene* scene, const float* cons
 
     const size_t GS = (size_t)egrad_stride(C);
     CU_CHECK(ctx, ensure(ctx->egrad, sizeof(float) * GS * ctx->entry_cap + 16));  // one row per entry the arrays can hold
-    const size_t small_bytes = sizeof(double) * (TRIPS_MAX_CHANNELS + (size_t)B * 19 + 1);  // background | per view: 6 pose, 5 pinhole, 8 distortion | work counter
+    const size_t small_bytes = sizeof(double) * (TRIPS_MAX_CHANNELS + (size_t)B * 19) + sizeof(unsigned) * kTileCounters * kTileCounterPitch;  // background | per view: 6 pose, 5 pinhole, 8 distortion | work counters
     CU_CHECK(ctx, ensure(ctx->g_small, small_bytes));
     BwdBuffers bb;
     bb.egrad        = (float*)ctx->egrad.p;
