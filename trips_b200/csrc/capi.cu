@@ -478,7 +478,7 @@ static int forward_views(TripsContext* ctx, const TripsScene* scene, const Trips
         CU_CHECK(ctx, cudaEventRecord(ctx->totals_ev, st));
         ctx->pending = true;
     }
-    if (N > 0) STAGE(ctx, TRIPS_STAGE_COLLECT, 1, st, launch_collect(sp, g, B, fb, strict_layers(*params), ctx->crowded, wait_for_sizes ? (unsigned long long)h_stats->visible : ctx->need_entries, ctx->sm_count, st));
+    if (N > 0) STAGE(ctx, TRIPS_STAGE_COLLECT, 1, st, launch_collect(sp, g, B, fb, strict_layers(*params), wait_for_sizes ? (unsigned long long)h_stats->visible : ctx->need_entries, ctx->sm_count, st));
     LayerPtrs out{};
     for (int l = 0; l < g.L; ++l) out.p[l] = out_layers[l] + out_view_offset * (size_t)C * g.W[l] * g.H[l];
     if (second_pipeline(*params))

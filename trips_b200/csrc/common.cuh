@@ -388,7 +388,7 @@ cudaError_t launch_scan(const Geom& g, int B, int k_keep, const FwdBuffers& fb, 
 // entries_hint: the number of entries of the call as far as the host knows it (selects the size of the work tickets)
 cudaError_t launch_count(const ScenePtrs& sc, const Geom& g, int B, const FwdBuffers& fb, bool strict, unsigned long long entries_hint, int sm_count,
                          cudaStream_t st);
-cudaError_t launch_collect(const ScenePtrs& sc, const Geom& g, int B, const FwdBuffers& fb, bool strict, bool crowded, unsigned long long entries_hint, int sm_count, cudaStream_t st);
+cudaError_t launch_collect(const ScenePtrs& sc, const Geom& g, int B, const FwdBuffers& fb, bool strict, unsigned long long entries_hint, int sm_count, cudaStream_t st);
 // top-K + blend by the rules of the reference's second forward pipeline (one thread per pixel)
 cudaError_t launch_second_blend(const ScenePtrs& sc, const Geom& g, const TripsRenderParams& pr, int B, const FwdBuffers& fb,
                                 const LayerPtrs& out, int sm_count, cudaStream_t st);
