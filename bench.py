@@ -160,21 +160,21 @@ def stage_bytes(stage, N, P, C, B, F, Kf, V=0):
         return 36 * (N * (C + 1 + 4 + 1))
     if stage == "unpack_grads":
         # no term in the reference's formula (its backward kernel adds straight into the outputs); what the stage must move:
-        # per visible point and view one 32-byte gradient row cleared, read and its 32-byte entry head read, per point one row
-        # (4 + C4 + 1 floats) cleared, read and written out in the reference's layouts
+        # per visible point and view one 32-byte gradient row cleared and read, per point its entry index in every view, its
+        # position and size, and the outputs in the reference's layouts
         c4 = (C + 3) // 4 * 4
-        return 96 * V + (2 * 4 * (5 + c4) + 4 * (4 + 1 + C + 1)) * N
+        return 2 * 4 * (4 + c4) * V + (4 * B + 20 + 4 * (4 + 1 + C + 1)) * N
     return 0
 
 
-# DRAM bytes (read + write) per unit of work, from the ncu captures summarised under profiles/: the tile kernels, the
-# gradient finish / unpack kernels and Adam from one view of config 3 (rasterizer_kernels_c3_6Mpts_1view_ncu_sections.md:
-# same list density and the same N as the benchmark), the binning kernels, which read every point once for all views of a
-# call, from a quarter of the points with all 8 views (binning_adam_kernels_1.5Mpts_8views_ncu_sections.md).
-# Traffic grows in proportion to the unit count.  Units: F fragments, Kf kept fragments, NB points x views, V entries
-# (visible points over all views), N points.
-DRAM_BYTES_PER_UNIT = {"count": [(5.2, "F")], "collect": [(20.2, "F")], "sort_blend": [(35.4, "F")], "blend_backward": [(41.6, "Kf")],
-                       "bin_points": [(43.1, "NB")], "unpack_grads": [(23.4 + 126.5, "V"), (196.9, "N")], "adam": [(337.3, "N")]}
+# DRAM bytes (read + write) per unit of work, from the ncu captures summarised under profiles/: the tile kernels and Adam
+# from one view of config 3 (rasterizer_kernels_c3_6Mpts_1view_ncu_sections.md: same list density and the same N as the
+# benchmark), the binning kernels, which read every point once for all views of a call, from a quarter of the points with
+# all 8 views (binning_adam_kernels_1.5Mpts_8views_ncu_sections.md).  Traffic grows in proportion to the unit count.  The
+# gradient gather has no figure of its own yet and is left out of the sums.  Units: F fragments, Kf kept fragments, NB
+# points x views, N points.
+DRAM_BYTES_PER_UNIT = {"count": [(5.2, "F")], "collect": [(20.2, "F")], "sort_blend": [(35.6, "F")], "blend_backward": [(35.5, "Kf")],
+                       "bin_points": [(43.1, "NB")], "adam": [(337.3, "N")]}
 
 
 def stage_traffic(stage, N, B, F, Kf, V=0):
