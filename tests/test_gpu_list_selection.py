@@ -38,3 +38,31 @@ def test_kept_fragments(oracle_lib, cuda_lib, n, copies, k_keep):
         for l, ref in enumerate(f.pyramid()):
             got = outs[l][b].detach().cpu().numpy()
             assert np.max(np.abs(got - ref) / np.maximum(np.abs(ref), 1e-3)) <= 1e-5
+
+
+@pytest.mark.parametrize("order", ["random", "near_first", "far_first"])
+def test_long_lists_in_any_order(oracle_lib, cuda_lib, order):
+    """Lists far above the pre-selection length whose fragments come in random order, nearest first and farthest first (the
+    order of the points): the bound that the pre-selection starts from lets about 50, or more than fit its table, pass."""
+    s = scenes.tiny(seed=300, n_points=6000, width=32, height=24, num_layers=2, n_views=1)
+    s.position[:, 0:3:2] *= 0.02
+    s.position[:, 1] *= 0.02
+    pose = s.poses[0]
+    q, t = np.asarray(pose[:4], np.float64), np.asarray(pose[4:7], np.float64)
+    x, y, z, w = q
+    forward = np.array([2 * (x * z - w * y), 2 * (y * z + w * x), 1 - 2 * (x * x + y * y)])  # third row of the rotation
+    rng = np.random.default_rng(5)
+    along = rng.uniform(-0.5, 0.5, s.n_points)
+    along = {"random": along, "near_first": np.sort(along), "far_first": np.sort(along)[::-1]}[order]
+    s.position[:, :3] = (s.position[:, :3].astype(np.float64) + along[:, None] * forward).astype(np.float32)
+    sa, op, frames = oracle_frames(s, train=True)
+    ns, info, blend = gpu_render(s, train=True)
+    outs = blend(info)
+    assert info.cache.last_status() == 0 and info.cache.stats()["max_list_length"] > 600
+    f = frames[0]
+    nrec, pid, alpha = info.cache.debug_records(0, f.P)
+    onrec, opid, oalpha = f.records()
+    assert np.array_equal(nrec, onrec) and np.array_equal(pid, opid)
+    for l, ref in enumerate(f.pyramid()):
+        got = outs[l][0].detach().cpu().numpy()
+        assert np.max(np.abs(got - ref) / np.maximum(np.abs(ref), 1e-3)) <= 1e-5
