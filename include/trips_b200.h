@@ -150,7 +150,8 @@ int trips_forward(TripsContext* ctx, const TripsScene* scene, const TripsView* v
 
 /* Replaces BlendPointCloudBackward / BlendBackwardsBilinearFast
  * (src/lib/rendering/PointRenderer.cu:1232-1427, RenderBackward.cu:90-691).  Uses the records of the last
- * trips_forward on this context.  grad_layers: HOST array of num_layers device pointers, same shapes as out_layers. */
+ * trips_forward on this context: `position` and `point_size` of `scene` are not read, gradients are those of the points
+ * that were rendered.  grad_layers: HOST array of num_layers device pointers, same shapes as out_layers. */
 int trips_backward(TripsContext* ctx, const TripsScene* scene, const float* const* grad_layers, const TripsGrads* grads,
                    void* stream);
 

@@ -1,6 +1,7 @@
 """The gather of per-entry gradient rows into per-point gradients (point_grad_kernel) at the sizes where it can go wrong:
 view counts around the rows requested at a time (4) and above the cameras held in shared memory (32), clouds that take the
-aggregating binning kernels (they note the entry of a point in their own code), and a dropout mask.
+aggregating binning kernels (they note the entry of a point in their own code), a dropout mask, and points that change or
+are gone by the time of the backward pass (their gradients are those of the points that were rendered).
 
 Gradients are fp32 sums over fragments of both signs in another order than the oracle's: the bound of 1e-4 on elements
 above 1 % of the tensor's largest magnitude is the one of the parity tests (thousands of terms x 6e-8)."""
@@ -13,7 +14,7 @@ from util import gpu_render, oracle_frames, rel_err
 pytestmark = pytest.mark.gpu
 
 
-def _check(s, dropout=None, **kw):
+def _check(s, dropout=None, between=None, **kw):
     import torch
     sa, op, frames = oracle_frames(s, train=True, **kw) if dropout is None else (None, None, None)
     ns, info, blend = gpu_render(s, train=True, **kw)
@@ -31,6 +32,8 @@ def _check(s, dropout=None, **kw):
             g = np.stack([grads[b][s.channels * base:s.channels * (base + w * h)].reshape(s.channels, h, w) for b in range(s.n_views)])
             loss = loss + (outs[l] * torch.from_numpy(g).cuda()).sum()
             base += w * h
+        if between is not None:
+            between(info, ns.point_cloud_cuda)
         loss.backward()
         torch.cuda.synchronize()
         assert info.cache.last_status() == 0
@@ -52,7 +55,7 @@ def _check(s, dropout=None, **kw):
         r = f.backward(grads[b])
         for k in ref:
             ref[k] = ref[k] + r[k]
-    for call in range(2):  # a sized call, then one in the steady state
+    for call in range(2 if between is None else 1):  # a sized call, then one in the steady state
         got = backward()
         for k in ref:
             assert rel_err(got[k].reshape(ref[k].shape), ref[k]) <= 1e-4, f"{k}, call {call}"
@@ -73,3 +76,31 @@ def test_crowded_cloud(oracle_lib, cuda_lib, n_views):
 def test_dropout_mask(oracle_lib, cuda_lib):
     s = scenes.tiny(seed=90, n_points=3000, n_views=3)
     _check(s, dropout=(np.random.default_rng(1).random((3, 3000)) < 0.5).astype(np.float32))
+
+
+def _move(info, cloud):
+    import torch
+    with torch.no_grad():
+        cloud.t_position[:, :3] += 0.3 * torch.randn_like(cloud.t_position[:, :3])
+        cloud.t_point_size -= 1.0
+
+
+def _take_away(info, cloud):
+    with_points = info.cache._scene_struct
+
+    def without_points(*args):
+        scene = with_points(*args)
+        scene.position = scene.point_size = None
+        return scene
+
+    info.cache._scene_struct = without_points
+
+
+@pytest.mark.parametrize("between", [_move, _take_away])
+@pytest.mark.parametrize("crowded", [False, True])
+@pytest.mark.parametrize("n_views", [2, 17])
+def test_points_are_those_of_the_forward_pass(oracle_lib, cuda_lib, between, crowded, n_views):
+    s = scenes.tiny(seed=95, n_points=12000 if crowded else 1500, n_views=n_views, width=64, height=48, num_layers=3)
+    if crowded:
+        s.position[:, :3] *= 0.02
+    _check(s, between=between)

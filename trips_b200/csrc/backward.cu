@@ -492,14 +492,14 @@ __device__ __forceinline__ ViewGrad view_gradient(const CamConst& cam, float vx,
 
 // One thread per point: reads the point's entry index in every view, gathers the gradient rows of those entries, applies
 // the chain to the position and the softplus derivative to the size, sums over the views in view order (the same result
-// every time) and writes the output layouts once.
+// every time) and writes the output layouts once.  Position and raw size are those the forward pass saw (point_state, written
+// by the binning pass): the rows belong to that projection, whatever has become of the caller's tensors since.
 //
-// Why a gather: the rows are read once each (32 bytes of a 64-byte DRAM piece), next to 4 B of entry index per point and
-// view and 20 B of point data.  Adding the rows to per-point accumulators entry by entry, which this replaces, read the
+// Why a gather: the rows are read once each, next to 4 B of entry index per point and view and 16 B of point data.  Adding the rows to per-point accumulators entry by entry, which this replaces, read the
 // entry heads as well, needed 36 B per point cleared, updated by atomics, and read again in another order, and a spatial
 // sort of the points to keep those updates in L2.
 // Measured, the whole gradient bookkeeping (clearing, this kernel, camera sums), per-point accumulators / gather:
-// 6 M points x 8 views 1.05 / 0.73 ms, x 1 view 0.44 / 0.30 ms, 20 M x 2 views 1.54 / 0.85 ms, 2 M x 4 views 0.22 / 0.16 ms.
+// 6 M points x 8 views 1.05 / 0.73 ms, x 1 view 0.44 / 0.27 ms, 20 M x 2 views 1.54 / 0.75 ms, 2 M x 4 views 0.22 / 0.16 ms.
 // Random 32-byte reads: latency and loads in flight bound it (resident blocks of 256 threads at 3 / 4 / 5: 0.77 / 0.73 / 0.93 ms
 // on 6 M x 8, 0.99 / 0.85 / 1.04 ms on 20 M x 2; 5 spill).
 // With a texture index the descriptor / confidence gradients of all points sharing a column are added (atomics into
@@ -518,8 +518,7 @@ __global__ __launch_bounds__(256, (C <= 4 ? 4 : 1)) void point_grad_kernel(Scene
     __syncthreads();
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < (size_t)sc.N; i += (size_t)gridDim.x * blockDim.x)
     {
-        const float4 p  = __ldg(sc.position + i);
-        const float raw = __ldg(sc.point_size + i);
+        const float4 p = __ldg(fb.point_state + i);  // x y z raw size
         float gp0 = 0.f, gp1 = 0.f, gp2 = 0.f, gl = 0.f, gc = 0.f;
         float gt[C4];
 #pragma unroll
@@ -565,7 +564,7 @@ __global__ __launch_bounds__(256, (C <= 4 ? 4 : 1)) void point_grad_kernel(Scene
             }
         }
         if (out.points) reinterpret_cast<float4*>(out.points)[i] = make_float4(gp0, gp1, gp2, 0.f);
-        if (out.point_size) out.point_size[i] = gl == 0.f ? 0.f : tm_softplus_grad(raw) * gl;
+        if (out.point_size) out.point_size[i] = gl == 0.f ? 0.f : tm_softplus_grad(p.w) * gl;
         // fused texture preparation: chain through sigmoid(scale * raw) and |raw| (raw_* are null when the caller passes
         // activated tensors)
         const int col = sc.index ? __ldg(sc.index + i) : (int)i;

@@ -120,7 +120,7 @@ struct TripsContext
     int sm_count = 148;
     std::string error;
     // forward scratch
-    DevBuf heavy, cams, zeroed, bin_base, view_total, bin_cursor, entry_base, entries, offsets, partial, view_base, frags, rec_n, records, stats, point_entry, resize_scratch, block_box, block_skip;
+    DevBuf heavy, cams, zeroed, bin_base, view_total, bin_cursor, entry_base, entries, offsets, partial, view_base, frags, rec_n, records, stats, point_entry, point_state, resize_scratch, block_box, block_skip;
     size_t zero_bins = 0, zero_counts = 0;  // where bin_count and counts start inside `zeroed` (behind the work counters)
     // backward scratch
     DevBuf egrad, g_small;
@@ -228,6 +228,7 @@ static FwdBuffers fwd_buffers(TripsContext* c, int B)
     fb.ticket_collect = fb.ticket_count + B;
     fb.ticket_blend   = fb.ticket + blend_ticket_at(B);
     fb.point_entry = c->params.train ? (uint32_t*)c->point_entry.p : nullptr;
+    fb.point_state = c->params.train ? (float4*)c->point_state.p : nullptr;
     fb.block_box  = (const float*)c->block_box.p;
     fb.block_skip = (const uint8_t*)c->block_skip.p;
     fb.heavy      = (uint2*)c->heavy.p;
@@ -288,7 +289,7 @@ void trips_context_destroy(TripsContext* c)
     if (!c) return;
     DevBuf* all[] = {&c->heavy, &c->cams, &c->zeroed, &c->bin_base, &c->view_total, &c->bin_cursor, &c->entry_base, &c->entries, &c->offsets,
                      &c->partial, &c->view_base, &c->frags, &c->rec_n, &c->records, &c->stats, &c->egrad,
-                     &c->point_entry, &c->g_small, &c->adam_tab, &c->resize_scratch, &c->block_box, &c->block_skip};
+                     &c->point_entry, &c->point_state, &c->g_small, &c->adam_tab, &c->resize_scratch, &c->block_box, &c->block_skip};
     for (DevBuf* b : all) free_buf(*b);
     c->timers.destroy();
     if (c->h_pinned) cudaFreeHost(c->h_pinned);
@@ -420,6 +421,7 @@ static int forward_views(TripsContext* ctx, const TripsScene* scene, const Trips
         CU_CHECK(ctx, ensure(ctx->rec_n, (size_t)g.n_tiles * 32 * B));
         CU_CHECK(ctx, ensure(ctx->records, sizeof(uint2) * 16 * 32 * (size_t)g.n_tiles * B));
         CU_CHECK(ctx, ensure(ctx->point_entry, sizeof(uint32_t) * N * B));
+        CU_CHECK(ctx, ensure(ctx->point_state, sizeof(float4) * N));
     }
     if (ctx->frags.bytes == 0) CU_CHECK(ctx, ensure(ctx->frags, 16 * 1024 * 1024));
     if (!ctx->entries.p || ctx->entry_C != C) CU_CHECK(ctx, ensure_entries(ctx, 1024, C, 1.0));

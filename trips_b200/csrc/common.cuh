@@ -115,6 +115,7 @@ struct FwdBuffers
     unsigned int* ticket_collect;     // [B] collect pass
     unsigned int* ticket_blend;
     uint32_t* point_entry;            // training: [B,N] entry (within the view) of every point, kNoEntry where it is not visible
+    float4* point_state;              // training: [N] position and raw size of the points that were not discarded, as this pass saw them
     const float* block_box;           // [ceil(N / 8192), 6] bounding boxes (min xyz, max xyz) of blocks of consecutive points
     const uint8_t* block_skip;        // [B, ceil(N / 8192)] 1 = the block cannot hold a point visible in that view
     uint2* heavy;                     // [kHeavyCap] (view, pixel) of the lists longer than kHeavyList

@@ -556,6 +556,7 @@ __global__ __launch_bounds__(kBinThreads, (C <= 4 ? kScatterMinBlocks : kScatter
             }
             const float4 p  = h.p;
             const float raw = h.raw;
+            if (fb.point_state && v0 == 0) fb.point_state[i] = make_float4(p.x, p.y, p.z, raw);
             float sp        = -1.f;
             // Views are handled kSweep at a time in two sweeps: the first projects and takes the entry slots (up to kSweep
             // returning atomics in flight per thread instead of one), the second projects again (the same arithmetic,
@@ -722,6 +723,7 @@ __global__ __launch_bounds__(kBinThreads) void bin_scatter_hot_kernel(ScenePtrs 
             if (discarded_for_confidence<ACT>(sc, pr, tex)) continue;
             const float4 p  = __ldg(sc.position + i);
             const float raw = __ldg(sc.point_size + i);
+            if (fb.point_state && v0 == 0) fb.point_state[i] = make_float4(p.x, p.y, p.z, raw);
             float sp        = -1.f;
             for (int v = 0; v < nv; ++v)
             {
