@@ -299,6 +299,9 @@ int trips_debug_lists(TripsContext* ctx, int view, int32_t* counts, int64_t* off
 /* Backward records of view `view`: nrec [P] int32, point ids [P,16] int32 (-1 = absent), alphas [P,16] (-1 = absent).
  * RenderForward.cu:957-979. */
 int trips_debug_records(TripsContext* ctx, int view, int32_t* nrec, int32_t* rec_pid, float* rec_alpha, void* stream);
+/* The selection that is applied to very long lists, on n >= 16 distinct keys (HOST array): positions [16] of the 16 smallest in
+ * ascending order, and how many times it gathered them.  HOST output pointers.  No counterpart in the reference. */
+int trips_debug_nearest(TripsContext* ctx, const uint64_t* keys, int n, uint32_t* positions, int* gatherings, void* stream);
 
 #ifdef __cplusplus
 }

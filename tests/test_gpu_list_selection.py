@@ -2,6 +2,8 @@
 shorter network for 8), many fragments of the same depth inside and across the end of the selection, and lists around
 the length at which a block of its own pre-selects them.  Kept points, their order and the pyramid must be the oracle's:
 ids bit for bit, alphas and colours to 1e-5 (16 products in 32 bits, 16 x 6e-8)."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -9,6 +11,22 @@ from trips_b200 import scenes
 from util import gpu_render, oracle_frames, rel_err
 
 pytestmark = pytest.mark.gpu
+
+
+def _check(s, views=None, min_length=0):
+    sa, op, frames = oracle_frames(s, train=True, views=views)
+    ns, info, blend = gpu_render(s, train=True)
+    outs = blend(info)
+    assert info.cache.last_status() == 0 and info.cache.stats()["max_list_length"] >= min_length
+    for b, f in zip(range(s.n_views) if views is None else views, frames):
+        nrec, pid, alpha = info.cache.debug_records(b, f.P)
+        onrec, opid, oalpha = f.records()
+        assert np.array_equal(nrec, onrec)
+        assert np.array_equal(pid, opid)
+        assert rel_err(alpha, oalpha, floor=1e-6) <= 1e-5
+        for l, ref in enumerate(f.pyramid()):
+            got = outs[l][b].detach().cpu().numpy()
+            assert np.max(np.abs(got - ref) / np.maximum(np.abs(ref), 1e-3)) <= 1e-5
 
 
 def _stack(n, copies, k_keep, seed):
@@ -25,25 +43,13 @@ def _stack(n, copies, k_keep, seed):
 @pytest.mark.parametrize("n,copies", [(40, 1), (12, 8), (12, 9), (12, 16), (12, 17), (200, 15), (12, 33), (300, 20), (3, 512), (3, 513), (2, 700)])
 def test_kept_fragments(oracle_lib, cuda_lib, n, copies, k_keep):
     s = _stack(n, copies, k_keep, seed=200 + copies)
-    sa, op, frames = oracle_frames(s, train=True)
-    ns, info, blend = gpu_render(s, train=True)
-    outs = blend(info)
-    assert info.cache.last_status() == 0
-    for b, f in enumerate(frames):
-        nrec, pid, alpha = info.cache.debug_records(b, f.P)
-        onrec, opid, oalpha = f.records()
-        assert np.array_equal(nrec, onrec)
-        assert np.array_equal(pid, opid)
-        assert rel_err(alpha, oalpha, floor=1e-6) <= 1e-5
-        for l, ref in enumerate(f.pyramid()):
-            got = outs[l][b].detach().cpu().numpy()
-            assert np.max(np.abs(got - ref) / np.maximum(np.abs(ref), 1e-3)) <= 1e-5
+    _check(s)
 
 
 @pytest.mark.parametrize("order", ["random", "near_first", "far_first"])
 def test_long_lists_in_any_order(oracle_lib, cuda_lib, order):
-    """Lists far above the pre-selection length whose fragments come in random order, nearest first and farthest first (the
-    order of the points): the bound that the pre-selection starts from lets about 50, or more than fit its table, pass."""
+    """Lists far above the pre-selection length of points numbered at random, nearest first and farthest first.  (The order inside
+    a list is left to the passes that write it; test_selection_in_a_given_order fixes it.)"""
     s = scenes.tiny(seed=300, n_points=6000, width=32, height=24, num_layers=2, n_views=1)
     s.position[:, 0:3:2] *= 0.02
     s.position[:, 1] *= 0.02
@@ -55,14 +61,49 @@ def test_long_lists_in_any_order(oracle_lib, cuda_lib, order):
     along = rng.uniform(-0.5, 0.5, s.n_points)
     along = {"random": along, "near_first": np.sort(along), "far_first": np.sort(along)[::-1]}[order]
     s.position[:, :3] = (s.position[:, :3].astype(np.float64) + along[:, None] * forward).astype(np.float32)
-    sa, op, frames = oracle_frames(s, train=True)
-    ns, info, blend = gpu_render(s, train=True)
-    outs = blend(info)
-    assert info.cache.last_status() == 0 and info.cache.stats()["max_list_length"] > 600
-    f = frames[0]
-    nrec, pid, alpha = info.cache.debug_records(0, f.P)
-    onrec, opid, oalpha = f.records()
-    assert np.array_equal(nrec, onrec) and np.array_equal(pid, opid)
-    for l, ref in enumerate(f.pyramid()):
-        got = outs[l][0].detach().cpu().numpy()
-        assert np.max(np.abs(got - ref) / np.maximum(np.abs(ref), 1e-3)) <= 1e-5
+    _check(s, min_length=600)
+
+
+def _order(order, n, rng):
+    keys = (rng.choice(2 * n, n, replace=False).astype(np.uint64) << 32) | rng.permutation(n).astype(np.uint64)
+    if order in ("ascending", "descending"):
+        return np.sort(keys) if order == "ascending" else np.sort(keys)[::-1].copy()
+    if order == "one_depth":
+        return (np.uint64(0x41f00000) << np.uint64(32)) | rng.permutation(n).astype(np.uint64)
+    if order != "random":  # all near fragments in the shares of 15 of the 64 groups, so that the first bound is of no use
+        few = np.arange(n) % 256 < 60
+        keys[~few] += np.uint64(4 * n) << np.uint64(32)
+        keys[few] = np.sort(keys[few]) if order == "few_groups_ascending" else np.sort(keys[few])[::-1]
+    return keys
+
+
+@pytest.mark.parametrize("order", ["random", "ascending", "descending", "one_depth", "few_groups_ascending", "few_groups_descending"])
+def test_selection_in_a_given_order(cuda_lib, order):
+    """The pre-selection on keys in a given order: the 16 smallest, ascending, in few gatherings whatever the order."""
+    import torch
+    from trips_b200 import _lib
+    rng = np.random.default_rng(11)
+    ctx = C.c_void_p()
+    _lib.check(cuda_lib.trips_context_create(C.byref(ctx), torch.cuda.current_device()))
+    try:
+        for n in (16, 17, 32, 63, 255, 256, 257, 513, 2048, 8193, 300_007):
+            keys = _order(order, n, rng)
+            pos, walks = np.zeros(16, np.uint32), C.c_int()
+            _lib.check(cuda_lib.trips_debug_nearest(ctx, keys.ctypes.data, n, pos.ctypes.data, C.byref(walks), None), ctx)
+            assert np.array_equal(pos, np.argsort(keys)[:16]), n
+            assert walks.value <= 67
+            if not order.startswith("few_groups") and n >= 513:
+                assert walks.value == 1  # at most 64 keys within the first bound in order, more than 128 of a random order never
+            elif n >= 8193:
+                assert walks.value > 1
+    finally:
+        cuda_lib.trips_context_destroy(ctx)
+
+
+@pytest.mark.parametrize("n_points,n_views", [(8692, 1), (8693, 1), (40_000, 3), (400_000, 1)])
+def test_lists_shared_by_blocks(oracle_lib, cuda_lib, n_points, n_views):
+    """Lists around and far above the length from which several blocks share one, in the same call as short ones."""
+    s = scenes.tiny(seed=310, n_points=n_points, width=32, height=24, num_layers=2, n_views=n_views)
+    s.position[:-500, :3] *= 0.001
+    s.confidence[:] = np.minimum(s.confidence, 0.1)
+    _check(s, min_length=8192)

@@ -231,7 +231,9 @@ static FwdBuffers fwd_buffers(TripsContext* c, int B)
     fb.point_state = c->params.train ? (float4*)c->point_state.p : nullptr;
     fb.block_box  = (const float*)c->block_box.p;
     fb.block_skip = (const uint8_t*)c->block_skip.p;
-    fb.heavy      = (uint2*)c->heavy.p;
+    fb.heavy.item     = (uint4*)c->heavy.p;
+    fb.heavy.nearest  = (uint32_t*)(fb.heavy.item + kHeavyCap);
+    fb.heavy.finished = fb.heavy.nearest + 16 * (size_t)kHeavyShared;
     return fb;
 }
 
@@ -411,7 +413,7 @@ static int forward_views(TripsContext* ctx, const TripsScene* scene, const Trips
     CU_CHECK(ctx, ensure(ctx->entry_base, sizeof(unsigned long long) * (B + 1)));
     CU_CHECK(ctx, ensure(ctx->block_box, sizeof(float) * 6 * n_box));
     CU_CHECK(ctx, ensure(ctx->block_skip, (size_t)B * n_box));
-    CU_CHECK(ctx, ensure(ctx->heavy, sizeof(uint2) * (size_t)kHeavyCap));
+    CU_CHECK(ctx, ensure(ctx->heavy, kHeavyBytes));
     CU_CHECK(ctx, ensure(ctx->offsets, sizeof(uint32_t) * P * B));
     CU_CHECK(ctx, ensure(ctx->partial, sizeof(uint32_t) * (size_t)nchunks * B));
     CU_CHECK(ctx, ensure(ctx->view_base, sizeof(unsigned long long) * (B + 1)));
@@ -939,6 +941,31 @@ int trips_debug_records(TripsContext* ctx, int view, int32_t* nrec, int32_t* rec
                     if (rec_alpha) rec_alpha[p * 16 + j] = a;
                 }
             }
+    return TRIPS_OK;
+}
+
+int trips_debug_nearest(TripsContext* ctx, const uint64_t* keys, int n, uint32_t* positions, int* gatherings, void* stream)
+{
+    if (!ctx) return TRIPS_ERR_INVALID_ARG;
+    if (!keys || n < 16) return fail(ctx, TRIPS_ERR_INVALID_ARG, "at least 16 keys");
+    cudaStream_t st = (cudaStream_t)stream;
+    DevBuf buf;
+    const size_t key_bytes = sizeof(uint64_t) * (size_t)n;
+    uint32_t result[17]    = {};
+    auto run = [&]() -> cudaError_t {
+        cudaError_t e = ensure(buf, key_bytes + sizeof(result));
+        uint32_t* out = (uint32_t*)((char*)buf.p + key_bytes);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(buf.p, keys, key_bytes, cudaMemcpyHostToDevice, st);
+        if (e == cudaSuccess) e = launch_nearest_16((const unsigned long long*)buf.p, (uint32_t)n, out, st);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(result, out, sizeof(result), cudaMemcpyDeviceToHost, st);
+        const cudaError_t s = cudaStreamSynchronize(st);
+        return e != cudaSuccess ? e : s;
+    };
+    const cudaError_t e = run();
+    free_buf(buf);
+    CU_CHECK(ctx, e);
+    if (positions) memcpy(positions, result, sizeof(uint32_t) * 16);
+    if (gatherings) *gatherings = (int)result[16];
     return TRIPS_OK;
 }
 

@@ -16,7 +16,10 @@ constexpr int kTileH      = 4;
 constexpr uint32_t kNoEntry = 0xffffffffu;  // a point that is not visible in a view
 constexpr int kViewGroup  = 16;  // views whose camera constants are in shared memory at a time in the binning passes (one launch per group)
 constexpr int kHeavyList  = 512;      // lists longer than this get their 16 nearest fragments moved to the front by a block of their own
-constexpr int kHeavyCap   = 1 << 16;  // such lists per call the pre-selection handles; beyond that the blend walks them itself
+constexpr int kHeavyPart  = 8192;     // longer ones are shared by several blocks, each with a part of at most this many fragments ...
+constexpr int kHeavyParts = 256;      // ... or by this many blocks
+constexpr int kHeavyCap   = 1 << 17;  // such lists and parts per call the pre-selection handles; beyond that the blend walks the lists itself
+constexpr int kHeavyShared = 1 << 16; // parts of shared lists per call; beyond that a long list gets one block
 
 // Pyramid geometry shared by all views of a call.
 struct Geom
@@ -70,9 +73,9 @@ struct DevStats
     unsigned long long kept;
     unsigned long long frag_need;  // fragments over all views (needed list slots, whether or not they fitted)
     unsigned int max_len;
-    unsigned int n_heavy;          // pixels whose list is longer than kHeavyList (they are pre-selected before the blend)
+    unsigned int n_heavy;          // lists longer than kHeavyList (they are pre-selected before the blend); every part of a shared one counts
     unsigned int max_key;          // largest number of visible points in one (view, screen bin, tile) group
-    unsigned int pad0;
+    unsigned int n_shared;         // parts of shared lists among them
     unsigned int status;
     unsigned int culled_blocks;  // (view, block of consecutive points) pairs skipped by the bounding-box test, counted once per pass
 };
@@ -90,6 +93,15 @@ __host__ __device__ constexpr int entry_stride(int C) { return 8 + tail_stride(C
 __host__ __device__ constexpr int egrad_stride(int C) { return 4 + ((C + 3) & ~3); }
 
 // Everything the forward kernels need besides the scene (all device pointers into context scratch).
+// Lists longer than kHeavyList, found by the scan.  A list of several parts has one item per part.
+struct HeavyLists
+{
+    uint4* item;        // [kHeavyCap] view, pixel, part | parts << 16, where the list's parts start in `nearest` and `finished`
+    uint32_t* nearest;  // [kHeavyShared, 16] list positions of a part's nearest fragments
+    uint32_t* finished; // [kHeavyShared] parts of the list that are done, at the list's first part
+};
+constexpr size_t kHeavyBytes = sizeof(uint4) * kHeavyCap + sizeof(uint32_t) * 17 * (size_t)kHeavyShared;
+
 struct FwdBuffers
 {
     uint32_t* bin_count;              // [B,n_bins,32] visible points per (screen bin, 8x4 tile of the bin)
@@ -118,7 +130,7 @@ struct FwdBuffers
     float4* point_state;              // training: [N] position and raw size of the points that were not discarded, as this pass saw them
     const float* block_box;           // [ceil(N / 8192), 6] bounding boxes (min xyz, max xyz) of blocks of consecutive points
     const uint8_t* block_skip;        // [B, ceil(N / 8192)] 1 = the block cannot hold a point visible in that view
-    uint2* heavy;                     // [kHeavyCap] (view, pixel) of the lists longer than kHeavyList
+    HeavyLists heavy;
 };
 
 struct ScenePtrs
@@ -393,6 +405,7 @@ cudaError_t launch_collect(const ScenePtrs& sc, const Geom& g, int B, const FwdB
 // top-K + blend by the rules of the reference's second forward pipeline (one thread per pixel)
 cudaError_t launch_second_blend(const ScenePtrs& sc, const Geom& g, const TripsRenderParams& pr, int B, const FwdBuffers& fb,
                                 const LayerPtrs& out, int sm_count, cudaStream_t st);
+cudaError_t launch_nearest_16(const unsigned long long* d_keys, uint32_t n, uint32_t* d_result, cudaStream_t st);  // n >= 16; d_result [17]
 cudaError_t launch_heavy_topk(const Geom& g, int B, const FwdBuffers& fb, int sm_count, cudaStream_t st);
 cudaError_t launch_sort_blend(const ScenePtrs& sc, const Geom& g, const TripsRenderParams& pr, int B, const FwdBuffers& fb,
                               const LayerPtrs& out, int sm_count, cudaStream_t st);

@@ -29,7 +29,7 @@ __global__ void setup_cams_kernel(const __grid_constant__ ViewTable views, int b
         // the counters of the call start from zero; the status word keeps the bits raised by earlier calls until
         // trips_last_status reads them
         stats->visible = stats->kept = stats->frag_need = 0ull;
-        stats->max_len = stats->n_heavy = stats->max_key = stats->pad0 = stats->culled_blocks = 0u;
+        stats->max_len = stats->n_heavy = stats->max_key = stats->n_shared = stats->culled_blocks = 0u;
     }
     if (b >= B) return;
     const TripsView& v = views.v[threadIdx.x];
@@ -885,7 +885,7 @@ __device__ __forceinline__ uint32_t block_excl_scan_256(uint32_t v, uint32_t* sm
 }
 
 __global__ __launch_bounds__(256) void scan_reduce_kernel(const uint32_t* __restrict__ counts, int P, int nchunks, int k_keep,
-                                                          uint32_t* __restrict__ partial, DevStats* stats, uint2* __restrict__ heavy)
+                                                          uint32_t* __restrict__ partial, DevStats* stats, HeavyLists heavy)
 {
     __shared__ uint32_t sm[8];
     const int b           = blockIdx.y;
@@ -900,10 +900,19 @@ __global__ __launch_bounds__(256) void scan_reduce_kernel(const uint32_t* __rest
         sum += v;
         kept += min(v, (uint32_t)k_keep);
         mx = max(mx, v);
-        if (v > (uint32_t)kHeavyList)  // a list worth a block of its own (heavy_topk_kernel); rare
+        if (v > (uint32_t)kHeavyList)  // a list worth a block of its own, or several (heavy_topk_kernel); rare
         {
-            const unsigned slot = atomicAdd(&stats->n_heavy, 1u);
-            if (slot < (unsigned)kHeavyCap) heavy[slot] = make_uint2((unsigned)b, (unsigned)i);
+            unsigned parts = min((v - 1) / kHeavyPart + 1, (unsigned)kHeavyParts), shared = 0;
+            if (parts > 1)
+            {
+                shared = atomicAdd(&stats->n_shared, parts);
+                if (shared + parts > (unsigned)kHeavyShared)
+                    parts = 1;
+                else
+                    heavy.finished[shared] = 0;
+            }
+            const unsigned slot = atomicAdd(&stats->n_heavy, parts);
+            for (unsigned t = 0; t < parts && slot + t < (unsigned)kHeavyCap; ++t) heavy.item[slot + t] = make_uint4((unsigned)b, (unsigned)i, t | parts << 16, shared);
         }
     }
     uint32_t total;
@@ -1429,31 +1438,127 @@ constexpr int kSbWarps   = kSbThreads / 32;
 // would keep one warp of the blend kernel busy on its own while the rest of the machine idles.  Here a block of 256
 // threads takes one such list and moves its 16 nearest fragments to the front, in depth order, by swapping them with the
 // fragments that were there - the list stays the same set of fragments.  The blend kernel then reads only the first 16
-// entries of every list longer than kHeavyList.  Lists are found by the scan (scan_reduce_kernel); with more than
-// kHeavyCap of them nothing is done here and the blend kernel, which sees the same counter, walks them itself.
+// entries of every list longer than kHeavyList.  A list longer than kHeavyPart is shared by several blocks, each of which
+// selects the 16 nearest of its part; the last one to finish selects from those and swaps.  Lists and parts are found by the
+// scan (scan_reduce_kernel); with more than kHeavyCap of them nothing is done here and the blend kernel, which sees the same
+// counter, walks the lists itself.
 //
-// Selection: every half-warp finds the nearest fragment of its sixteenth of the list; the farthest of those 16 bounds the
-// 16th nearest of all.  What is not beyond that bound - 54 fragments expected of a list in random order, whatever its
-// length (16 x the 16th harmonic number) - is gathered in shared memory and ranked by counting.  If it is more than fits
-// (241 of a list in depth order), the 16th of what did fit is a closer bound, with at least kHeavyCand - 16 fragments fewer
-// inside it, and the gathering is repeated.  Two light passes over the keys, where sorting every 16 keys into the nearest ones took 14 exchange
-// steps of three shuffles per chunk: 62 M fragments in lists of about 3000 took 580 us, now about 250
-// us (sort_blend 0.88 -> 0.55 ms; 20 M points at 1440p, lists up to 1473, 0.87 -> 0.79 ms).
-constexpr int kHeavyCand = 128;
-static_assert(kHeavyList >= 256, "every half-warp must own at least one fragment");
-__global__ __launch_bounds__(256) void heavy_topk_kernel(const __grid_constant__ Geom g, FwdBuffers fb, int B)
+// What bounds it: on long lists the two walks over the keys (8 of 16 bytes used; the second comes from L2), on lists of about
+// 1000 the barriers of a list.  sort_blend stage, ms, half-warps with sorted streams and one block per list / a bound from 16
+// half-warps and one block per list / this: 2 M points in 2 pixels x 8 views 1.48 / 2.5 / 0.39, 700 k points in 4 pixels x 8
+// views 0.26 / 0.36 / 0.18, 3 M points in 64x64 pixels x 4 views 0.90 / 0.53 / 0.54, 20 M points at 1440p x 2 views (lists up
+// to 1473) 1.39 / 0.80 / 0.79.  Parts of 4096 / 8192 / 16384 fragments: within 3 % on the longest lists, 16384 leaves more of the
+// chip idle on single lists, 4096 costs 10 % on the crowded 8-view calls.
+constexpr int kHeavyCand   = 128;  // fragments within the bound that are ranked at a time
+constexpr int kHeavyGroups = 64;   // groups of 4 threads that each bring their nearest fragment
+// Keys a thread requests before it looks at any of them, and resident blocks: 4 keys and 6 blocks suit lists of about 1000,
+// 8 keys and 4 blocks the very long ones (2 M points in 2 pixels x 8 views 0.39 / 0.31 ms, 700 k points, lists up to 866, x 8
+// views 1.17 / 1.23 ms).
+constexpr int kHeavyBatch  = 4;
+constexpr int kHeavyBlocks = 6;
+struct HeavyShared
 {
-    __shared__ u64 s_min[16];
-    __shared__ u64 s_key[kHeavyCand];
-    __shared__ uint32_t s_pos[kHeavyCand];
-    __shared__ uint32_t s_win[16], s_vac[16];
-    __shared__ unsigned s_n;
+    u64 nearest[kHeavyGroups];
+    u64 key[kHeavyCand];
+    uint32_t pos[kHeavyCand];
+    uint32_t win[16];  // the result: indices of the 16 smallest keys, ascending
+    u64 bound;
+    unsigned found;
+};
+
+// The 16 smallest of n >= 16 distinct keys, by a block of 256 threads.  Every group of 4 threads brings the smallest key of
+// its share; the 16th smallest of those bounds the 16th smallest of all.  What is not beyond that bound - 18 keys expected in
+// random order whatever n is, at most 64 in ascending or descending order - is gathered and ranked by counting.  If it is more
+// than fits (the small keys are in the shares of fewer than 16 groups), the 16th of what did fit is a closer bound and
+// the gathering is repeated; from the third time on the bound is found by bisection, so that no order takes more than 66
+// repetitions.  Returns the number of times the keys were gathered.
+template <class KeyAt>
+__device__ int nearest_16(uint32_t n, KeyAt&& key_at, HeavyShared& sh)
+{
+    const uint32_t t = threadIdx.x;
+    u64 k[kHeavyBatch], nearest = kInfKey;
+    for (uint32_t i0 = t; i0 < n; i0 += 256 * kHeavyBatch)
+    {
+#pragma unroll
+        for (int u = 0; u < kHeavyBatch; ++u) k[u] = i0 + 256 * u < n ? key_at(i0 + 256 * u) : kInfKey;
+#pragma unroll
+        for (int u = 0; u < kHeavyBatch; ++u) nearest = min(nearest, k[u]);
+    }
+    nearest = min(nearest, __shfl_xor_sync(kFull, nearest, 1));
+    nearest = min(nearest, __shfl_xor_sync(kFull, nearest, 2));
+    if ((t & 3) == 0) sh.nearest[t >> 2] = nearest;
+    if (t < 16) sh.win[t] = t;
+    __syncthreads();
+    {
+        // rank of the group's key: each of its threads counts over a quarter of the others
+        unsigned r = 0;
+#pragma unroll 4
+        for (unsigned q0 = 0; q0 < kHeavyGroups / 4; ++q0)
+        {
+            const unsigned q = q0 * 4 + (t & 3);
+            const u64 other  = sh.nearest[q];
+            r += (other < nearest || (other == nearest && q < t >> 2)) ? 1u : 0u;
+        }
+        r += __shfl_xor_sync(kFull, r, 1);
+        r += __shfl_xor_sync(kFull, r, 2);
+        if (r == 15u && (t & 3) == 0) sh.bound = nearest;
+        if (t == 0) sh.found = 0;
+    }
+    __syncthreads();
+    u64 bound = sh.bound;
+    u64 low = 0, high = bound;  // fewer than 16 keys up to low, at least 16 up to high
+    const bool held = n <= 256 * kHeavyBatch;  // the threads still hold all keys
+    for (int walks = 1;; ++walks)
+    {
+        for (uint32_t i0 = t; i0 < n; i0 += 256 * kHeavyBatch)
+        {
+            if (!held)
+            {
+#pragma unroll
+                for (int u = 0; u < kHeavyBatch; ++u) k[u] = i0 + 256 * u < n ? key_at(i0 + 256 * u) : kInfKey;
+            }
+#pragma unroll
+            for (int u = 0; u < kHeavyBatch; ++u)
+                if (k[u] <= bound && i0 + 256 * u < n)
+                {
+                    const unsigned at = atomicAdd(&sh.found, 1u);
+                    if (at < (unsigned)kHeavyCand) sh.key[at] = k[u], sh.pos[at] = i0 + 256 * u;
+                }
+        }
+        __syncthreads();
+        const unsigned found = sh.found, m = min(found, (unsigned)kHeavyCand);
+        if (found >= 16u && t < m)
+        {
+            const u64 mine = sh.key[t];
+            unsigned r     = 0;
+            for (unsigned q = 0; q < m; ++q) r += sh.key[q] < mine ? 1u : 0u;
+            if (r < 16u) sh.win[r] = sh.pos[t];
+            if (r == 15u) sh.bound = mine;
+        }
+        __syncthreads();
+        // all of this is uniform; keys that are not distinct (there are none) end with low and high next to each other
+        if ((found >= 16u && found <= (unsigned)kHeavyCand) || (found > (unsigned)kHeavyCand && high - low <= 1)) return walks;
+        if (found < 16u)
+            low = bound;
+        else
+            high = min(bound, sh.bound);
+        bound = (walks <= 2 && found >= 16u) || high - low <= 1 ? high : low + (high - low) / 2;
+        if (t == 0) sh.found = 0;
+        __syncthreads();
+    }
+}
+
+__global__ __launch_bounds__(256, kHeavyBlocks) void heavy_topk_kernel(const __grid_constant__ Geom g, FwdBuffers fb, int B)
+{
+    __shared__ HeavyShared sh;
+    __shared__ uint32_t s_vac[16];
+    __shared__ unsigned s_last;
     const unsigned n_heavy = fb.stats->n_heavy;
     if (n_heavy == 0 || n_heavy > (unsigned)kHeavyCap) return;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, j = lane & 15, hw = threadIdx.x >> 4;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, j = lane & 15;
     for (unsigned h = blockIdx.x; h < n_heavy; h += gridDim.x)
     {
-        const uint2 e = fb.heavy[h];
+        const uint4 e = fb.heavy.item[h];
         const int b   = (int)e.x;
         if (b >= B || fb.view_base[b + 1] == fb.view_base[b]) continue;  // uniform: the view did not fit the list buffer
         const size_t bP    = (size_t)b * g.P;
@@ -1463,56 +1568,35 @@ __global__ __launch_bounds__(256) void heavy_topk_kernel(const __grid_constant__
             const uint2 k = *reinterpret_cast<const uint2*>(list + i);
             return ((u64)k.y << 32) | k.x;
         };
-        auto half_warp_min = [&](u64 v) {
-#pragma unroll
-            for (int o = 8; o > 0; o >>= 1) v = min(v, __shfl_xor_sync(kFull, v, o));
-            return v;
-        };
-        u64 nearest = kInfKey;
-#pragma unroll 4
-        for (uint32_t i = threadIdx.x; i < cnt; i += 256) nearest = min(nearest, key_at(i));
-        nearest = half_warp_min(nearest);
-        if (j == 0) s_min[hw] = nearest;
-        if (threadIdx.x == 0) s_n = 0;
-        if (threadIdx.x < 16) s_win[threadIdx.x] = s_vac[threadIdx.x] = threadIdx.x;
-        __syncthreads();
-        u64 bound = 0;
-#pragma unroll
-        for (int k = 0; k < 16; ++k) bound = max(bound, s_min[k]);
-        for (;;)
+        const uint32_t part = e.z & 0xffffu, parts = e.z >> 16;
+        const uint32_t first = (uint32_t)((u64)cnt * part / parts), last = (uint32_t)((u64)cnt * (part + 1) / parts);
+        if (threadIdx.x < 16) s_vac[threadIdx.x] = threadIdx.x;
+        nearest_16(last - first, [&](uint32_t i) { return key_at(first + i); }, sh);
+        if (parts > 1)  // uniform
         {
-#pragma unroll 4
-            for (uint32_t i = threadIdx.x; i < cnt; i += 256)
+            uint32_t* nearest = fb.heavy.nearest + 16 * (size_t)e.w;  // of all parts of this list
+            if (threadIdx.x < 16)
             {
-                const u64 k = key_at(i);
-                if (k <= bound)
-                {
-                    const unsigned at = atomicAdd(&s_n, 1u);
-                    if (at < (unsigned)kHeavyCand) s_key[at] = k, s_pos[at] = i;
-                }
+                nearest[16 * part + threadIdx.x] = first + sh.win[threadIdx.x];
+                __threadfence();
             }
             __syncthreads();
-            const unsigned found = s_n, n = min(found, (unsigned)kHeavyCand);  // at least 16: the nearest fragment of every half-warp
-            if (threadIdx.x < n)
+            if (threadIdx.x == 0)
             {
-                const u64 k = s_key[threadIdx.x];
-                unsigned r  = 0;
-                for (unsigned q = 0; q < n; ++q) r += s_key[q] < k ? 1u : 0u;
-                if (r < 16u) s_win[r] = s_pos[threadIdx.x];
-                if (r == 15u) s_min[0] = k;
+                s_last = atomicAdd(fb.heavy.finished + e.w, 1u) == parts - 1 ? 1u : 0u;
+                __threadfence();
             }
             __syncthreads();
-            if (found <= (unsigned)kHeavyCand) break;  // uniform
-            if (s_min[0] >= bound) break;  // uniform; not with distinct keys
-            bound = s_min[0];
-            if (threadIdx.x == 0) s_n = 0;
+            if (!s_last) continue;  // uniform
+            nearest_16(16 * parts, [&](uint32_t i) { return key_at(__ldcg(nearest + i)); }, sh);
+            if (threadIdx.x < 16) sh.win[threadIdx.x] = __ldcg(nearest + sh.win[threadIdx.x]);
             __syncthreads();
         }
         if (warp == 0)
         {
             // lanes 0..15 hold the 16 nearest fragments in depth order (cnt > kHeavyList >= 16: all present); swap them to the front
             const bool act    = lane < 16;
-            const uint32_t wp = s_win[j];
+            const uint32_t wp = sh.win[j];
             uint4 winner = make_uint4(0u, 0u, 0u, 0u), front = winner;
             if (act)
             {
@@ -1535,7 +1619,22 @@ __global__ __launch_bounds__(256) void heavy_topk_kernel(const __grid_constant__
 
 cudaError_t launch_heavy_topk(const Geom& g, int B, const FwdBuffers& fb, int sm_count, cudaStream_t st)
 {
-    heavy_topk_kernel<<<sm_count * 6, 256, 0, st>>>(g, fb, B);
+    heavy_topk_kernel<<<sm_count * kHeavyBlocks, 256, 0, st>>>(g, fb, B);
+    return cudaGetLastError();
+}
+
+// the selection alone, for inspection: result[0..15] the positions, result[16] the number of gatherings
+__global__ __launch_bounds__(256, kHeavyBlocks) void nearest_16_kernel(const u64* __restrict__ keys, uint32_t n, uint32_t* __restrict__ result)
+{
+    __shared__ HeavyShared sh;
+    const int walks = nearest_16(n, [&](uint32_t i) { return keys[i]; }, sh);
+    if (threadIdx.x < 16) result[threadIdx.x] = sh.win[threadIdx.x];
+    if (threadIdx.x == 16) result[16] = (uint32_t)walks;
+}
+
+cudaError_t launch_nearest_16(const unsigned long long* d_keys, uint32_t n, uint32_t* d_result, cudaStream_t st)
+{
+    nearest_16_kernel<<<1, 256, 0, st>>>(d_keys, n, d_result);
     return cudaGetLastError();
 }
 
