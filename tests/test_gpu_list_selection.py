@@ -64,6 +64,22 @@ def test_long_lists_in_any_order(oracle_lib, cuda_lib, order):
     _check(s, min_length=600)
 
 
+@pytest.mark.parametrize("k_keep", [5, 16])
+@pytest.mark.parametrize("n_points", [900, 9000, 60_000])
+def test_wall_facing_the_camera(oracle_lib, cuda_lib, n_points, k_keep):
+    """All fragments of all lists at one depth or at one of three: ids alone decide, within the selection and across its end."""
+    s = scenes.tiny(seed=320, n_points=n_points, width=72, height=40, num_layers=3, k_keep=k_keep, n_views=2)
+    s.poses[:] = 0.0
+    s.poses[:, 3] = 1.0  # no rotation: depth = z + 4, exactly
+    s.poses[:, 6] = 4.0
+    s.position[:, 2] = 0.0
+    s.position[::5, 2] = -0.25
+    s.position[::7, 2] = 0.25
+    s.position[: n_points // 2, 2] = 0.0
+    s.confidence[:] = np.minimum(s.confidence, 0.1)
+    _check(s, min_length=16 * (n_points // 3000))
+
+
 def _order(order, n, rng):
     keys = (rng.choice(2 * n, n, replace=False).astype(np.uint64) << 32) | rng.permutation(n).astype(np.uint64)
     if order in ("ascending", "descending"):

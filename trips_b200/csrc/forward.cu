@@ -1794,9 +1794,9 @@ __global__ __launch_bounds__(kSbThreads, (C <= 4 ? kSbMinBlocks : (C <= 8 ? kSbM
                 for (int i = 0; i < 16; ++i)
                     if ((i & st) == 0) order_pair(key[i], key[i + st], idx[i], idx[i + st]);
         }
-        bool tie = false;
+        uint32_t ties = 0;  // bit j: ranks j and j + 1 are equal
 #pragma unroll
-        for (int j = 0; j < 15; ++j) tie |= key[j] == key[j + 1] && key[j] != kNoDepth;
+        for (int j = 0; j < 15; ++j) ties |= key[j] == key[j + 1] && key[j] != kNoDepth ? 1u << j : 0u;
         const bool tie_end = dropped == key[15] && dropped != kNoDepth;
         const int n        = min((int)cnt, K);
         const int n_max    = min((int)max_cnt, K);
@@ -1804,35 +1804,49 @@ __global__ __launch_bounds__(kSbThreads, (C <= 4 ? kSbMinBlocks : (C <= 8 ? kSbM
 #pragma unroll
         for (int j = 0; j < 16; ++j)
             if (j < 8 || max_cnt > 8) order[32 * j] = idx[j];
-        // equal depths go by point id (the total order of the lists); rare, so the lists are read in place
-        if (__any_sync(kFull, tie || tie_end))
+        // Equal depths go by point id (the total order of the lists), the ids read from the lists in place.  Some percent of the
+        // tiles of a scene of surfaces have such a pair, so this goes from tie to tie and looks at nothing else: functions that
+        // gather all ids and sort them in registers cost 10 % there by their registers alone.  A wall that faces the camera, all of one
+        // depth: 2 M points in 640x480 (lists up to 45) 0.57 -> 0.23 ms, in 4 views of 1280x960 0.95 -> 0.76 ms, against sweeps
+        // over all ranks and one scan of the list per rank.
+        if (__any_sync(kFull, ties || tie_end))
         {
             if (tie_end)  // a tie across the end of the selection: of the fragments at the last kept depth those with the smallest ids stay
             {
-                int j = 15;
-                while (j > 0 && list[order[32 * (j - 1)]].y == dropped) --j;
-                uint32_t last = 0;
-                for (bool first = true; j < 16; ++j, first = false)
+                const int first = 15 - __clz(~(ties << 17));  // rank of the first of them; the ranks from there on are filled in order
+                ties &= (1u << first) - 1u;
+                uint2* kept = s_az[warp] + lane * kSbPitch;  // (id, list position) at kept[rank]; not in use, the list is longer than a chunk
+                int end     = first;
+                uint32_t worst = 0xffffffffu;
+#pragma unroll 4
+                for (uint32_t i = 0; i < cnt; ++i)
                 {
-                    uint32_t best = 0xffffffffu, at = order[32 * j];
-                    for (uint32_t i = 0; i < cnt; ++i)
+                    const uint2 f = *reinterpret_cast<const uint2*>(list + i);
+                    if (f.y != dropped || f.x >= worst) continue;
+                    int k = end < 16 ? end++ : 15;
+                    for (; k > first; --k)
                     {
-                        const uint2 f = *reinterpret_cast<const uint2*>(list + i);
-                        if (f.y == dropped && (first || f.x > last) && f.x <= best) best = f.x, at = i;
+                        const uint2 before = kept[k - 1];
+                        if (before.x < f.x) break;
+                        kept[k] = before;
                     }
-                    order[32 * j] = at, last = best;
+                    kept[k] = make_uint2(f.x, i);
+                    if (end == 16) worst = kept[15].x;
                 }
+                for (int k = first; k < 16; ++k) order[32 * k] = kept[k].y;
             }
-            const int n16 = min((int)cnt, 16);
-            while (tie)  // at most 15 sweeps of a bubble sort over equal neighbours
+            for (uint32_t left = ties; left; left &= left - 1)  // insertion of the higher rank of every pair, lowest pair first
             {
-                tie = false;
-                for (int j = 0; j + 1 < n16; ++j)
+                int k             = __ffs(left);
+                const uint32_t at = order[32 * k], id = list[at].x;
+                do
                 {
-                    const uint32_t ia = order[32 * j], ib = order[32 * (j + 1)];
-                    const uint2 fa = *reinterpret_cast<const uint2*>(list + ia), fb2 = *reinterpret_cast<const uint2*>(list + ib);
-                    if (fa.y == fb2.y && fb2.x < fa.x) order[32 * j] = ib, order[32 * (j + 1)] = ia, tie = true;
-                }
+                    const uint32_t before = order[32 * (k - 1)];
+                    if (list[before].x < id) break;
+                    order[32 * k] = before;
+                    --k;
+                } while (k > 0 && ((ties >> (k - 1)) & 1u));
+                order[32 * k] = at;
             }
             __syncwarp();
         }
