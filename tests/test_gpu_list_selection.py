@@ -1,5 +1,5 @@
-"""Selection of the nearest fragments where the per-pixel sort can go wrong: list lengths around its chunks of 16 (and the
-shorter network for 8), many fragments of the same depth inside and across the end of the selection, and lists around
+"""Selection of the nearest fragments where the per-pixel sort can go wrong: list lengths around its chunks of 16 (the
+shorter networks for 8 and 12, the comparators for up to 4), many fragments of the same depth inside and across the end of the selection, and lists around
 the length at which a block of its own pre-selects them.  Kept points, their order and the pyramid must be the oracle's:
 ids bit for bit, alphas and colours to 1e-5 (16 products in 32 bits, 16 x 6e-8)."""
 import ctypes as C
@@ -40,7 +40,7 @@ def _stack(n, copies, k_keep, seed):
 
 
 @pytest.mark.parametrize("k_keep", [1, 8, 16])
-@pytest.mark.parametrize("n,copies", [(40, 1), (12, 8), (12, 9), (12, 16), (12, 17), (200, 15), (12, 33), (300, 20), (3, 512), (3, 513), (2, 700)])
+@pytest.mark.parametrize("n,copies", [(40, 1), (12, 2), (12, 3), (12, 4), (12, 5), (12, 8), (12, 9), (12, 16), (12, 17), (200, 15), (12, 33), (300, 20), (3, 512), (3, 513), (2, 700)])
 def test_kept_fragments(oracle_lib, cuda_lib, n, copies, k_keep):
     s = _stack(n, copies, k_keep, seed=200 + copies)
     _check(s)

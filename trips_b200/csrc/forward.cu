@@ -1726,130 +1726,164 @@ __global__ __launch_bounds__(kSbThreads, (C <= 4 ? kSbMinBlocks : (C <= 8 ? kSbM
         const uint32_t max_cnt = __reduce_max_sync(kFull, cnt);
         const uint4* list      = frags + start;
 
-        // ---- selection: the 16 nearest fragments of the lane's list, nearest first.  The network for 8, 12 or 16 goes by the
-        //      longest list of the tile (half of the tiles of a 720p view stay at 8; 12 instead of 16: 42 against 63 comparators) ----
-        uint32_t key[16], idx[16];
-        uint32_t dropped = kNoDepth;  // smallest depth among the fragments that are not kept
-#pragma unroll
-        for (int i = 0; i < 16; ++i) key[i] = kNoDepth, idx[i] = 0u;
-#pragma unroll 1
-        for (uint32_t c0 = 0; c0 < max_cnt; c0 += 16)
+        if (max_cnt <= 4)
         {
-            // 8 lanes copy 8 (16) consecutive fragments of one pixel, 4 pixels per step: the lane = pixel pattern would touch
-            // 32 lines with every load
-            const uint32_t left = max_cnt - c0;
-            const int i8        = lane & 7;
+            // A tile of short lists: lane = pixel reads them in place, five comparators on depth and id sort them, and the blend
+            // finds alphas and entries where a staged chunk would be.  Staging, the networks and the search for ties cost such a tile
+            // more than all of the rest: 7 views of 1158x940 with 0.45 fragments per pixel 0.43 -> 0.34 ms (0.30 with the fragments of
+            // a tile ranked by shuffles), 11 of 835x489 with 8 channels 0.32 -> 0.28, and nothing where lists are longer.
+            // (Requesting lengths and ends of the next tile's lists ahead made this case 0.49: instructions bound it, not latency.)
+            uint32_t id[4], key[4], at[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+            {
+                key[j] = kNoDepth, id[j] = 0u, at[j] = j;
+                if (j < (int)cnt)
+                {
+                    const uint4 f = list[j];
+                    id[j] = f.x, key[j] = f.y;
+                    s_az[warp][lane * kSbPitch + j] = make_uint2(f.z, f.w);
+                }
+            }
+            auto sort_pair = [&](int a, int b) {
+                const bool swap = key[b] < key[a] || (key[b] == key[a] && id[b] < id[a]);
+                const uint32_t k0 = swap ? key[b] : key[a], k1 = swap ? key[a] : key[b];
+                const uint32_t d0 = swap ? id[b] : id[a], d1 = swap ? id[a] : id[b];
+                const uint32_t a0 = swap ? at[b] : at[a], a1 = swap ? at[a] : at[b];
+                key[a] = k0, key[b] = k1, id[a] = d0, id[b] = d1, at[a] = a0, at[b] = a1;
+            };
+            if (max_cnt > 1) sort_pair(0, 1), sort_pair(2, 3), sort_pair(0, 2), sort_pair(1, 3), sort_pair(1, 2);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) s_key[warp][32 * j + lane] = at[j];
+        }
+        else
+        {
+            // ---- selection: the 16 nearest fragments of the lane's list, nearest first.  The network for 8, 12 or 16 goes by the
+            //      longest list of the tile (half of the tiles of a 720p view stay at 8; 12 instead of 16: 42 against 63 comparators) ----
+            uint32_t key[16], idx[16];
+            uint32_t dropped = kNoDepth;  // smallest depth among the fragments that are not kept
+#pragma unroll
+            for (int i = 0; i < 16; ++i) key[i] = kNoDepth, idx[i] = 0u;
+#pragma unroll 1
+            for (uint32_t c0 = 0; c0 < max_cnt; c0 += 16)
+            {
+                // 8 lanes copy 8 (16) consecutive fragments of one pixel, 4 pixels per step: the lane = pixel pattern would touch
+                // 32 lines with every load
+                const uint32_t left = max_cnt - c0;
+                const int i8        = lane & 7;
 #pragma unroll 4
-            for (int q = 0; q < 8; ++q)
-            {
-                const int src          = q * 4 + (lane >> 3);
-                const uint32_t n_src   = __shfl_sync(kFull, cnt, src);
-                const uint32_t beg_src = __shfl_sync(kFull, start, src);
-                const uint32_t i       = c0 + i8;
-                const uint4* f         = frags + beg_src + i;
-                uint32_t* dk           = s_key[warp] + src * kSbPitch + i8;
-                uint2* da              = s_az[warp] + src * kSbPitch + i8;
-                if (i < n_src) copy_async_4(dk, &f->y), copy_async_8(da, &f->z);
-                if (left > 8 && i + 8 < n_src) copy_async_4(dk + 8, &f[8].y), copy_async_8(da + 8, &f[8].z);
-            }
-            copy_async_wait();
-            __syncwarp();
-            uint32_t k2[16], i2[16];
-            uint32_t nearest = kNoDepth;
-#pragma unroll
-            for (int i = 0; i < 16; ++i)
-            {
-                k2[i]   = (i < 8 || left > 8) && c0 + i < cnt ? s_key[warp][lane * kSbPitch + i] : kNoDepth;
-                i2[i]   = c0 + i;
-                nearest = min(nearest, k2[i]);
-            }
-            __syncwarp();  // the next chunk may overwrite the staged depths
-            if (!__any_sync(kFull, nearest < key[15]))  // nothing nearer in any of the 32 lists
-            {
-                dropped = min(dropped, nearest);
-                continue;
-            }
-            if (left <= 8)
-                sort_network<8>(k2, i2);
-            else if (left <= 12)
-                sort_network<12>(k2, i2);
-            else
-                sort_network<16>(k2, i2);
-            if (c0 == 0)
-            {
-#pragma unroll
-                for (int i = 0; i < 16; ++i) key[i] = k2[i], idx[i] = i2[i];
-                continue;
-            }
-#pragma unroll
-            for (int i = 0; i < 16; ++i)
-            {
-                const bool take = k2[15 - i] < key[i];
-                dropped         = min(dropped, take ? key[i] : k2[15 - i]);
-                if (take) key[i] = k2[15 - i], idx[i] = i2[15 - i];
-            }
-#pragma unroll
-            for (int st = 8; st > 0; st >>= 1)
+                for (int q = 0; q < 8; ++q)
+                {
+                    const int src          = q * 4 + (lane >> 3);
+                    const uint32_t n_src   = __shfl_sync(kFull, cnt, src);
+                    const uint32_t beg_src = __shfl_sync(kFull, start, src);
+                    const uint32_t i       = c0 + i8;
+                    const uint4* f         = frags + beg_src + i;
+                    uint32_t* dk           = s_key[warp] + src * kSbPitch + i8;
+                    uint2* da              = s_az[warp] + src * kSbPitch + i8;
+                    if (i < n_src) copy_async_4(dk, &f->y), copy_async_8(da, &f->z);
+                    if (left > 8 && i + 8 < n_src) copy_async_4(dk + 8, &f[8].y), copy_async_8(da + 8, &f[8].z);
+                }
+                copy_async_wait();
+                __syncwarp();
+                uint32_t k2[16], i2[16];
+                uint32_t nearest = kNoDepth;
 #pragma unroll
                 for (int i = 0; i < 16; ++i)
-                    if ((i & st) == 0) order_pair(key[i], key[i + st], idx[i], idx[i + st]);
-        }
-        uint32_t ties = 0;  // bit j: ranks j and j + 1 are equal
-#pragma unroll
-        for (int j = 0; j < 15; ++j) ties |= key[j] == key[j + 1] && key[j] != kNoDepth ? 1u << j : 0u;
-        const bool tie_end = dropped == key[15] && dropped != kNoDepth;
-        const int n        = min((int)cnt, K);
-        const int n_max    = min((int)max_cnt, K);
-        uint32_t* order    = s_key[warp] + lane;  // list position of the fragment of rank j at order[32 * j]
-#pragma unroll
-        for (int j = 0; j < 16; ++j)
-            if (j < 8 || max_cnt > 8) order[32 * j] = idx[j];
-        // Equal depths go by point id (the total order of the lists), the ids read from the lists in place.  Some percent of the
-        // tiles of a scene of surfaces have such a pair, so this goes from tie to tie and looks at nothing else: functions that
-        // gather all ids and sort them in registers cost 10 % there by their registers alone.  A wall that faces the camera, all of one
-        // depth: 2 M points in 640x480 (lists up to 45) 0.57 -> 0.23 ms, in 4 views of 1280x960 0.95 -> 0.76 ms, against sweeps
-        // over all ranks and one scan of the list per rank.
-        if (__any_sync(kFull, ties || tie_end))
-        {
-            if (tie_end)  // a tie across the end of the selection: of the fragments at the last kept depth those with the smallest ids stay
-            {
-                const int first = 15 - __clz(~(ties << 17));  // rank of the first of them; the ranks from there on are filled in order
-                ties &= (1u << first) - 1u;
-                uint2* kept = s_az[warp] + lane * kSbPitch;  // (id, list position) at kept[rank]; not in use, the list is longer than a chunk
-                int end     = first;
-                uint32_t worst = 0xffffffffu;
-#pragma unroll 4
-                for (uint32_t i = 0; i < cnt; ++i)
                 {
-                    const uint2 f = *reinterpret_cast<const uint2*>(list + i);
-                    if (f.y != dropped || f.x >= worst) continue;
-                    int k = end < 16 ? end++ : 15;
-                    for (; k > first; --k)
-                    {
-                        const uint2 before = kept[k - 1];
-                        if (before.x < f.x) break;
-                        kept[k] = before;
-                    }
-                    kept[k] = make_uint2(f.x, i);
-                    if (end == 16) worst = kept[15].x;
+                    k2[i]   = (i < 8 || left > 8) && c0 + i < cnt ? s_key[warp][lane * kSbPitch + i] : kNoDepth;
+                    i2[i]   = c0 + i;
+                    nearest = min(nearest, k2[i]);
                 }
-                for (int k = first; k < 16; ++k) order[32 * k] = kept[k].y;
-            }
-            for (uint32_t left = ties; left; left &= left - 1)  // insertion of the higher rank of every pair, lowest pair first
-            {
-                int k             = __ffs(left);
-                const uint32_t at = order[32 * k], id = list[at].x;
-                do
+                __syncwarp();  // the next chunk may overwrite the staged depths
+                if (!__any_sync(kFull, nearest < key[15]))  // nothing nearer in any of the 32 lists
                 {
-                    const uint32_t before = order[32 * (k - 1)];
-                    if (list[before].x < id) break;
-                    order[32 * k] = before;
-                    --k;
-                } while (k > 0 && ((ties >> (k - 1)) & 1u));
-                order[32 * k] = at;
+                    dropped = min(dropped, nearest);
+                    continue;
+                }
+                if (left <= 8)
+                    sort_network<8>(k2, i2);
+                else if (left <= 12)
+                    sort_network<12>(k2, i2);
+                else
+                    sort_network<16>(k2, i2);
+                if (c0 == 0)
+                {
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) key[i] = k2[i], idx[i] = i2[i];
+                    continue;
+                }
+#pragma unroll
+                for (int i = 0; i < 16; ++i)
+                {
+                    const bool take = k2[15 - i] < key[i];
+                    dropped         = min(dropped, take ? key[i] : k2[15 - i]);
+                    if (take) key[i] = k2[15 - i], idx[i] = i2[15 - i];
+                }
+#pragma unroll
+                for (int st = 8; st > 0; st >>= 1)
+#pragma unroll
+                    for (int i = 0; i < 16; ++i)
+                        if ((i & st) == 0) order_pair(key[i], key[i + st], idx[i], idx[i + st]);
             }
-            __syncwarp();
+            uint32_t ties = 0;  // bit j: ranks j and j + 1 are equal
+#pragma unroll
+            for (int j = 0; j < 15; ++j) ties |= key[j] == key[j + 1] && key[j] != kNoDepth ? 1u << j : 0u;
+            const bool tie_end = dropped == key[15] && dropped != kNoDepth;
+            uint32_t* order    = s_key[warp] + lane;  // list position of the fragment of rank j at order[32 * j]
+#pragma unroll
+            for (int j = 0; j < 16; ++j)
+                if (j < 8 || max_cnt > 8) order[32 * j] = idx[j];
+            // Equal depths go by point id (the total order of the lists), the ids read from the lists in place.  Some percent of the
+            // tiles of a scene of surfaces have such a pair, so this goes from tie to tie and looks at nothing else: functions that
+            // gather all ids and sort them in registers cost 10 % there by their registers alone.  A wall that faces the camera, all of one
+            // depth: 2 M points in 640x480 (lists up to 45) 0.57 -> 0.23 ms, in 4 views of 1280x960 0.95 -> 0.76 ms, against sweeps
+            // over all ranks and one scan of the list per rank.
+            if (__any_sync(kFull, ties || tie_end))
+            {
+                if (tie_end)  // a tie across the end of the selection: of the fragments at the last kept depth those with the smallest ids stay
+                {
+                    const int first = 15 - __clz(~(ties << 17));  // rank of the first of them; the ranks from there on are filled in order
+                    ties &= (1u << first) - 1u;
+                    uint2* kept = s_az[warp] + lane * kSbPitch;  // (id, list position) at kept[rank]; not in use, the list is longer than a chunk
+                    int end     = first;
+                    uint32_t worst = 0xffffffffu;
+#pragma unroll 4
+                    for (uint32_t i = 0; i < cnt; ++i)
+                    {
+                        const uint2 f = *reinterpret_cast<const uint2*>(list + i);
+                        if (f.y != dropped || f.x >= worst) continue;
+                        int k = end < 16 ? end++ : 15;
+                        for (; k > first; --k)
+                        {
+                            const uint2 before = kept[k - 1];
+                            if (before.x < f.x) break;
+                            kept[k] = before;
+                        }
+                        kept[k] = make_uint2(f.x, i);
+                        if (end == 16) worst = kept[15].x;
+                    }
+                    for (int k = first; k < 16; ++k) order[32 * k] = kept[k].y;
+                }
+                for (uint32_t left = ties; left; left &= left - 1)  // insertion of the higher rank of every pair, lowest pair first
+                {
+                    int k             = __ffs(left);
+                    const uint32_t at = order[32 * k], id = list[at].x;
+                    do
+                    {
+                        const uint32_t before = order[32 * (k - 1)];
+                        if (list[before].x < id) break;
+                        order[32 * k] = before;
+                        --k;
+                    } while (k > 0 && ((ties >> (k - 1)) & 1u));
+                    order[32 * k] = at;
+                }
+                __syncwarp();
+            }
         }
+        const int n           = min((int)cnt, K);
+        const int n_max       = min((int)max_cnt, K);
+        const uint32_t* order = s_key[warp] + lane;  // list position of the fragment of rank j at order[32 * j]
 
         // ---- blend.  T_j = T_{j-1} * (1 - a_{j-1}), colour summed in the order of a 16-leaf butterfly
         //      (RenderForward.cu:940-994) so that results do not depend on how lanes are assigned: four leaves per turn ----
