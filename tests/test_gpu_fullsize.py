@@ -151,3 +151,29 @@ def test_full_size_parity(name, oracle_lib, cuda_lib):
         assert rel_err(gintr[v, :5], ref["intrinsics"][b][:5]) <= TOL_GRAD, "intrinsics gradient"
     report["gradients"] = grads
     parity_report(name, report)
+
+
+@pytest.mark.parametrize("flags", [{}, dict(render_points_in_all_lower_resolutions=False)], ids=["first_pipeline", "strict_layers"])
+def test_large_calls_match_single_views(cuda_lib, flags):
+    """Above 18 M entries a call counts its fragments in tickets of 4096 entries instead of 1024, and above 0.8 M it collects them
+    in larger blocks: a call with all views must give every view the lists, records and pixels, bit for bit, that a call
+    of its own gives it (those are compared with the oracle above)."""
+    import torch
+    s = scenes.config3()
+    ns, info, blend = gpu_render(s, train=True, **flags)
+    outs = blend(info)
+    assert info.cache.last_status() == 0 and info.cache.stats()["visible_points"] > 19_000_000
+    P = scenes.num_pyramid_pixels(s.width, s.height, s.num_layers)
+    for v in range(0, s.n_views, 3):
+        _, single, _ = gpu_render(s, train=True, views=[v], **flags)
+        single.scene = ns
+        ref = blend(single)
+        assert single.cache.last_status() == 0 and single.cache.stats()["visible_points"] < 18_000_000
+        for l, o in enumerate(ref):
+            assert torch.equal(outs[l][v], o[0]), f"view {v}, layer {l}"
+        counts, offsets, frags = info.cache.debug_lists(v, P)
+        ref_counts, _, ref_frags = single.cache.debug_lists(0, P)
+        assert np.array_equal(counts, ref_counts)
+        assert np.array_equal(sort_lists(counts, offsets, frags), sort_lists(counts, offsets, ref_frags))
+        for got, want in zip(info.cache.debug_records(v, P), single.cache.debug_records(0, P)):
+            assert np.array_equal(got, want)

@@ -1052,7 +1052,10 @@ constexpr int kWinChunkCountFew = 1024;  // the same when the call has too few e
 constexpr int kWinTicketsPerBlock = 6;   // measured count pass, tickets of 4096 / 1024: config 4 (2 views, 16 M entries) 0.58 / 0.25 ms, config 2
                                          // (4 M) 0.093 / 0.09 ms; config 3 (27 M) 0.31 / 0.52 ms, config 5 (39 M) 0.40 / 0.53 ms
 constexpr int kWinChunkCollect = 1024;  // and collecting pass: the lists a chunk writes to must stay in L2 until complete (measured with tile-ordered entries: 256 1.80 ms, 512 1.46 ms, 1024 1.35 ms, 2048 1.47 ms)
-constexpr int kWinChunkCollectFew = 512;  // calls with few entries, by blocks of 128 threads: 2 views, 16 M entries (uneven density) 0.91 -> 0.69 ms; on 40 M entries 1024 entries by 256 threads is better (1.87 against 1.92 ms)
+// A call with fewer chunks of 1024 than resident blocks takes 512, by blocks of 128 threads: 0.5 M entries in 11 views 0.55 -> 0.50 ms,
+// 3 views of 2.4 k points at 1440p 0.55 -> 0.37.  Above that they lose, on crowded clouds most: 12 M entries in 64x64 pixels 0.440 ->
+// 0.478 ms, 10 M in 88x88 0.284 -> 0.296.
+constexpr int kWinChunkCollectFew = 512;
 // Threads of a block.  Half as many per barrier suits the counting pass (40 M entries 0.405 -> 0.380 ms, crowded clouds 0.145 ->
 // 0.122 ms); the collecting pass at 1024 entries per chunk wants 256 (1.25 against 1.45 ms with 128).
 constexpr int kWinThreadsCount = 128, kWinThreadsCollect = 256, kWinThreadsCollectFew = 128;
@@ -1139,11 +1142,12 @@ __device__ __forceinline__ bool next_chunk(const FwdBuffers& fb, const Geom& g, 
 // First layer of an entry written by the strict two-layer rule: the layer below log2(size), as write_entry computed it.
 __device__ __forceinline__ int strict_first_layer(float ps, int L) { return ps > 1.f ? min(tm_floor_log2(ps), L - 1) : 0; }
 
+// first_warp: the warp of the block that takes the first 32 entries
 template <int THREADS, bool WITH_E1, bool STRICT, class Body>
-__device__ __forceinline__ void for_each_footprint(const float4* __restrict__ head, uint32_t lo, uint32_t hi, uint8_t* queue, int L, Body&& body)
+__device__ __forceinline__ void for_each_footprint(const float4* __restrict__ head, uint32_t lo, uint32_t hi, uint8_t* queue, int L, Body&& body, unsigned first_warp = 0)
 {
     const int lane = threadIdx.x & 31;
-    uint32_t base  = lo + (threadIdx.x & ~31);
+    uint32_t base  = lo + ((threadIdx.x + 32 * first_warp) & (THREADS - 32));
     float4 e0n = make_float4(0.f, 0.f, 0.f, 0.f), e1n = e0n;
     if (base + lane < hi)
     {
@@ -1225,10 +1229,13 @@ __device__ __forceinline__ uint64_t evict_last_policy()
 // A bin with few entries inside a ticket (sky, far ground: a ticket can span hundreds of such bins) is not worth clearing
 // and flushing a window of shared-memory counters with three block barriers: its footprints go straight to the pixels'
 // global counters.  (On a 2560x1440 view of 20 M points with half of the bins nearly empty, the blocks that drew the
-// sparse tickets ran 12 times longer than the others.)  Not inlined: the dense path keeps its registers.
+// sparse tickets ran 12 times longer than the others.)  The bins take turns in which warp of the block gets their first 32
+// entries: most sparse bins have no more, and with warp 0 in charge of all of them the rest of the block idled through such
+// chunks (20 M points at 1440p: count 0.29 -> 0.17 ms, collect in chunks of 1024 0.91 -> 0.55; 4 k points in 11 views 0.67 -> 0.35
+// and 1.63 -> 0.50).  Not inlined: the dense path keeps its registers.
 template <int THREADS, bool COLLECT, bool STRICT>
 __device__ __noinline__ void sparse_bin_footprints(const Geom& g, const float4* __restrict__ head, uint32_t lo, uint32_t hi, uint8_t* queue,
-                                                   uint32_t* pixel_ctr, uint4* frags, uint64_t keep)
+                                                   uint32_t* pixel_ctr, uint4* frags, uint64_t keep, unsigned first_warp)
 {
     for_each_footprint<THREADS, COLLECT, STRICT>(head, lo, hi, queue, g.L, [&](const float4& e0, const float4& e1, float x, float y, int layer, uint32_t ei) {
         const int px = __float2int_rd(x), py = __float2int_rd(y);
@@ -1264,7 +1271,7 @@ __device__ __noinline__ void sparse_bin_footprints(const Geom& g, const float4* 
             store_frag(frags + s01, make_uint4(pid, zb, alpha(dx0, dy1), ei), keep);
             store_frag(frags + s11, make_uint4(pid, zb, alpha(dx1, dy1), ei), keep);
         }
-    });
+    }, first_warp);
 }
 
 template <int THREADS, bool COLLECT, bool STRICT>
@@ -1296,7 +1303,7 @@ __global__ __launch_bounds__(THREADS, kWinMinWarps * 32 / THREADS) void window_k
             if (lo >= hi) continue;  // uniform: all threads read the same values
             if (bin_end - bfirst[bin] <= (uint32_t)kWinSparse)  // the whole bin is sparse (a short piece of a dense bin still pays off in the window)
             {
-                sparse_bin_footprints<THREADS, COLLECT, STRICT>(g, head, lo, hi, s_queue[threadIdx.x >> 5], pixel_ctr, frags, keep);
+                sparse_bin_footprints<THREADS, COLLECT, STRICT>(g, head, lo, hi, s_queue[threadIdx.x >> 5], pixel_ctr, frags, keep, (unsigned)bin);
                 continue;
             }
             const Window w = make_window(g, bin);
@@ -1393,12 +1400,10 @@ cudaError_t launch_count(const ScenePtrs& sc, const Geom& g, int B, const FwdBuf
     return cudaGetLastError();
 }
 
-// (12 M entries in a few bins lose 0.05 ms of 0.44 with the small chunks: more atomics on the same pixels; uneven scenes of the
-// same size, which look alike to the host, gain 0.2 ms)
 cudaError_t launch_collect(const ScenePtrs& sc, const Geom& g, int B, const FwdBuffers& fb, bool strict, unsigned long long entries_hint, int sm_count,
                            cudaStream_t st)
 {
-    if (few_entries(entries_hint, sm_count))
+    if (entries_hint / kWinChunkCollect < (unsigned long long)sm_count * (kWinMinWarps * 32 / kWinThreadsCollect))
         run_window<kWinThreadsCollectFew, true>(g, B, fb, strict, kWinChunkCollectFew, sm_count, st);
     else
         run_window<kWinThreadsCollect, true>(g, B, fb, strict, kWinChunkCollect, sm_count, st);
