@@ -13,6 +13,10 @@ pytestmark = pytest.mark.gpu
 
 TOL_PYRAMID = 1e-5
 TOL_GRAD = 1e-4
+# Pose gradients are sums of terms of both signs over all points.  The terms of this variant's second view, each an fp32 sum of
+# the four or more fragments of a footprint, add up to 2.09 in magnitude and to 1e-4 as a sum, against a floor of 1.5e-3 (1 % of
+# the view's largest component): 4 x 2^-24 x 2.09 / 1.5e-3 = 3.3e-4.  Seen: 1.6e-4 in 900 runs.
+TOL_POSE = {"second_combine_three_views_long_lists": 3.3e-4}
 
 
 def _variants():
@@ -192,7 +196,7 @@ def test_forward_backward_parity(name, oracle_lib, cuda_lib):
     gpose = ns.poses.tangent_poses.grad.cpu().numpy()
     gintr = ns.intrinsics.intrinsics.grad.cpu().numpy()
     for b in range(len(frames)):
-        assert rel_err(gpose[b], ref["pose"][b]) <= TOL_GRAD, "pose gradient"
+        assert rel_err(gpose[b], ref["pose"][b]) <= TOL_POSE.get(name, TOL_GRAD), "pose gradient"
         assert rel_err(gintr[b, :5], ref["intrinsics"][b][:5]) <= TOL_GRAD, "intrinsics gradient"
         if kw.get("distortion"):
             assert np.all(ref["intrinsics"][b][5:] != 0)
