@@ -143,8 +143,8 @@ constexpr int kBinThreads     = 256;
 constexpr int kBinBlocksPerSM = 8;
 constexpr int kScatterMinBlocks = 4, kScatterMinBlocksWide = 3;  // up to 4 channels / more; measured at 3 / 4: 6 M points 1.26 / 1.23 ms (8 views), 0.346 / 0.313 ms (1 view); 8 channels 0.116 / 0.127 ms
 constexpr int kBinChunk       = 8192;  // points per bounding box
-constexpr int kBinTicket      = 1024;
-constexpr int kSweep          = 4;      // views whose entry slots a thread requests before it waits for any of them  // points per work ticket of the binning kernels; a ticket lies inside one box
+constexpr int kBinTicket      = 1024;  // points per work ticket of the binning kernels; a ticket lies inside one box
+constexpr int kSweep          = 4;     // views whose entry slots a thread requests before it waits for any of them
 static_assert(kBinChunk % kBinTicket == 0, "a ticket must not straddle two bounding boxes");
 
 // Bounding boxes of blocks of consecutive points and the conservative frustum test on them: the reference computes
@@ -254,18 +254,17 @@ __global__ __launch_bounds__(128) void block_visibility_kernel(const CamConst* _
 
 // Work distribution of the binning kernels: tickets of kBinTicket consecutive points from one counter, so that every SM
 // is busy until the last ticket whatever the number of resident blocks is (a static split left a partial last wave).
-// Thread 0 holds the following ticket in `ahead`, requested while the current one is worked on (`ahead` starts from
-// first_point_ticket).  Returns false when the cloud is exhausted; `skip` gets one bit per view of the group whose bounding-box test rules the
+// (A block does not ask for its next ticket before it is done: where there are fewer tickets than blocks, those that come
+// first would take two each - 130 k points in 11 views 0.23 instead of 0.17 ms - and elsewhere it gains nothing.)
+// Returns false when the cloud is exhausted; `skip` gets one bit per view of the group whose bounding-box test rules the
 // ticket's points out.
-__device__ __forceinline__ unsigned first_point_ticket(unsigned* ticket) { return threadIdx.x == 0 ? atomicAdd(ticket, 1u) : 0u; }
-__device__ __forceinline__ bool next_point_ticket(unsigned* ticket, unsigned& ahead, int N, unsigned* s_ticket,
-                                                  const uint8_t* __restrict__ block_skip, int v0, int nv, int& first, int& last, unsigned& skip)
+__device__ __forceinline__ bool next_point_ticket(unsigned* ticket, int N, unsigned* s_ticket, const uint8_t* __restrict__ block_skip, int v0,
+                                                  int nv, int& first, int& last, unsigned& skip)
 {
     __syncthreads();
-    if (threadIdx.x == 0) *s_ticket = ahead;
+    if (threadIdx.x == 0) *s_ticket = atomicAdd(ticket, 1u);
     __syncthreads();
     const unsigned t = *s_ticket;
-    if (threadIdx.x == 0) ahead = atomicAdd(ticket, 1u);
     if (t >= ((unsigned)N + kBinTicket - 1) / kBinTicket) return false;
     first = (int)(t * kBinTicket);
     last  = min(N, first + kBinTicket);
@@ -325,8 +324,8 @@ __global__ __launch_bounds__(kBinThreads) void bin_count_kernel(ScenePtrs sc, co
     for (int k = threadIdx.x; k < nv * (int)(sizeof(CamConst) / 4); k += kBinThreads) ((int*)s_cam)[k] = ((const int*)(cams + v0))[k];
     const bool use_dropout = pr.train && sc.dropout;  // the mask applies with and without viewer_only (RenderForward.cu:224-240)
     int first, last;
-    unsigned skip, ahead = first_point_ticket(ticket);
-    while (next_point_ticket(ticket, ahead, sc.N, &s_ticket, fb.block_skip, v0, nv, first, last, skip))
+    unsigned skip;
+    while (next_point_ticket(ticket, sc.N, &s_ticket, fb.block_skip, v0, nv, first, last, skip))
     {
         PointHead nx;
         nx.fetch(sc, first + threadIdx.x, last);
@@ -535,8 +534,8 @@ __global__ __launch_bounds__(kBinThreads, (C <= 4 ? kScatterMinBlocks : kScatter
     for (int v = 0; v < nv; ++v) no_room |= (s_ebase[v + 1] == s_ebase[v] ? 1u : 0u) << v;
     const bool use_dropout = pr.train && sc.dropout;
     int first, last;
-    unsigned skip, ahead = first_point_ticket(ticket);
-    while (next_point_ticket(ticket, ahead, sc.N, &s_ticket, fb.block_skip, v0, nv, first, last, skip))
+    unsigned skip;
+    while (next_point_ticket(ticket, sc.N, &s_ticket, fb.block_skip, v0, nv, first, last, skip))
     {
         skip |= no_room;
         PointHead nx;
@@ -579,11 +578,6 @@ __global__ __launch_bounds__(kBinThreads, (C <= 4 ? kScatterMinBlocks : kScatter
                     slot[j] = atomicAdd(fb.bin_base + ((size_t)(v0 + v) * g.n_bins << kSubShift) + bin_key(g, r.u, r.v), 1u);
                 }
                 if (vis) fetch_point_row<C, ACT>(sc, pr, fb, i, d);  // travels with the slots
-                if (fb.point_entry)
-#pragma unroll
-                    for (int j = 0; j < kSweep; ++j)
-                        if (vb + j < nv) fb.point_entry[(size_t)(v0 + vb + j) * sc.N + i] = slot[j];
-                if (!vis) continue;
 #pragma unroll
                 for (int j = 0; j < kSweep; ++j)
                 {
@@ -592,6 +586,10 @@ __global__ __launch_bounds__(kBinThreads, (C <= 4 ? kScatterMinBlocks : kScatter
                     const Projected r = project_visible(s_cam[v], g, pr, p, raw, sp);
                     write_entry<C>(fb, g, pr, s_ebase[v] + slot[j], i, p, raw, r, d);
                 }
+                if (fb.point_entry)  // behind the entries: the slots are on their way while the points are projected again
+#pragma unroll
+                    for (int j = 0; j < kSweep; ++j)
+                        if (vb + j < nv) fb.point_entry[(size_t)(v0 + vb + j) * sc.N + i] = slot[j];
             }
         }
     }
