@@ -96,7 +96,7 @@ __host__ __device__ constexpr int egrad_stride(int C) { return 4 + ((C + 3) & ~3
 // Lists longer than kHeavyList, found by the scan.  A list of several parts has one item per part.
 struct HeavyLists
 {
-    uint4* item;        // [kHeavyCap] view, pixel, part | parts << 16, where the list's parts start in `nearest` and `finished`
+    uint4* item;        // [kHeavyCap] view, pixel, part | parts << 16 (0: empty), where the list's parts start in `nearest` and `finished`
     uint32_t* nearest;  // [kHeavyShared, 16] list positions of a part's nearest fragments
     uint32_t* finished; // [kHeavyShared] parts of the list that are done, at the list's first part
 };

@@ -889,28 +889,51 @@ __global__ __launch_bounds__(256) void scan_reduce_kernel(const uint32_t* __rest
     const int b           = blockIdx.y;
     const uint32_t* c     = counts + (size_t)b * P;
     const int start       = blockIdx.x * kScanChunk + threadIdx.x;
-    uint32_t sum = 0, kept = 0, mx = 0;
+    uint32_t v[8], sum = 0, kept = 0, mx = 0;
 #pragma unroll
     for (int k = 0; k < 8; ++k)
     {
         const int i = start + k * 256;  // the order of a sum does not matter: neighbouring threads read neighbouring counts
-        uint32_t v = (i < P) ? c[i] : 0u;
-        sum += v;
-        kept += min(v, (uint32_t)k_keep);
-        mx = max(mx, v);
-        if (v > (uint32_t)kHeavyList)  // a list worth a block of its own, or several (heavy_topk_kernel); rare
+        v[k]        = (i < P) ? c[i] : 0u;
+        sum += v[k];
+        kept += min(v[k], (uint32_t)k_keep);
+        mx = max(mx, v[k]);
+    }
+    // lists worth a block of their own, or several (heavy_topk_kernel): a warp reserves the items of its lists together (one
+    // atomic per list queued up where most lists are long: 90 k long lists of 88x88 pixels in 11 views 0.041 -> 0.025 ms)
+    if (__any_sync(kFull, mx > (uint32_t)kHeavyList))
+    {
+        const int lane = threadIdx.x & 31;
+        auto parts_of  = [](uint32_t n) { return n > (uint32_t)kHeavyList ? min((n - 1) / kHeavyPart + 1, (uint32_t)kHeavyParts) : 0u; };
+        uint32_t items = 0, shared_items = 0;
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
         {
-            unsigned parts = min((v - 1) / kHeavyPart + 1, (unsigned)kHeavyParts), shared = 0;
-            if (parts > 1)
-            {
-                shared = atomicAdd(&stats->n_shared, parts);
-                if (shared + parts > (unsigned)kHeavyShared)
-                    parts = 1;
-                else
-                    heavy.finished[shared] = 0;
-            }
-            const unsigned slot = atomicAdd(&stats->n_heavy, parts);
-            for (unsigned t = 0; t < parts && slot + t < (unsigned)kHeavyCap; ++t) heavy.item[slot + t] = make_uint4((unsigned)b, (unsigned)i, t | parts << 16, shared);
+            const uint32_t parts = parts_of(v[k]);
+            items += parts;
+            shared_items += parts > 1 ? parts : 0u;
+        }
+        const uint32_t items_incl = warp_incl_scan(items, lane), shared_incl = warp_incl_scan(shared_items, lane);
+        uint32_t slot = 0, shared = 0;
+        if (lane == 31)
+        {
+            slot = atomicAdd(&stats->n_heavy, items_incl);
+            if (shared_incl) shared = atomicAdd(&stats->n_shared, shared_incl);
+        }
+        slot   = __shfl_sync(kFull, slot, 31) + items_incl - items;
+        shared = __shfl_sync(kFull, shared, 31) + shared_incl - shared_items;
+#pragma unroll 1
+        for (int k = 0; k < 8; ++k)
+        {
+            const uint32_t n     = c[min(start + k * 256, P - 1)];
+            const uint32_t parts = start + k * 256 < P ? parts_of(n) : 0u;
+            // no room for its parts: one block takes the whole list, the other items stay empty
+            const bool whole = parts > 1 && shared + parts > (uint32_t)kHeavyShared;
+            if (parts > 1 && !whole) heavy.finished[shared] = 0;
+            for (uint32_t t = 0; t < parts && slot + t < (uint32_t)kHeavyCap; ++t)
+                heavy.item[slot + t] = make_uint4((unsigned)b, (unsigned)(start + k * 256), whole ? (t == 0 ? 1u << 16 : 0u) : t | parts << 16, shared);
+            slot += parts;
+            shared += parts > 1 ? parts : 0u;
         }
     }
     uint32_t total;
@@ -1563,7 +1586,7 @@ __global__ __launch_bounds__(256, kHeavyBlocks) void heavy_topk_kernel(const __g
     {
         const uint4 e = fb.heavy.item[h];
         const int b   = (int)e.x;
-        if (b >= B || fb.view_base[b + 1] == fb.view_base[b]) continue;  // uniform: the view did not fit the list buffer
+        if (e.z == 0 || b >= B || fb.view_base[b + 1] == fb.view_base[b]) continue;  // uniform: an empty item, or the view did not fit the list buffer
         const size_t bP    = (size_t)b * g.P;
         const uint32_t cnt = fb.counts[bP + e.y];
         uint4* list        = fb.frags + fb.view_base[b] + (fb.offsets[bP + e.y] - cnt);  // offsets hold list ends after the collect pass
