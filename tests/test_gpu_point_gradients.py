@@ -8,6 +8,7 @@ above 1 % of the tensor's largest magnitude is the one of the parity tests (thou
 import numpy as np
 import pytest
 
+import oracle
 from trips_b200 import scenes
 from util import gpu_render, oracle_frames, rel_err
 
@@ -16,7 +17,12 @@ pytestmark = pytest.mark.gpu
 
 def _check(s, dropout=None, between=None, **kw):
     import torch
-    sa, op, frames = oracle_frames(s, train=True, **kw) if dropout is None else (None, None, None)
+    if dropout is None:
+        sa, op, frames = oracle_frames(s, train=True, **kw)
+    else:
+        op = oracle.make_params(s.num_layers, s.k_keep, True, **kw)
+        sa = [oracle.SceneArrays.from_scene(s, dropout=mask) for mask in dropout]
+        frames = [oracle.forward(a, oracle.make_view(s.width, s.height, s.poses[b], s.intrinsics[b]), op) for b, a in enumerate(sa)]
     ns, info, blend = gpu_render(s, train=True, **kw)
     params = dict(texture=ns.texture.texture_raw, confidence=ns.texture.confidence_raw, position=ns.point_cloud_cuda.t_position,
                   point_size=ns.point_cloud_cuda.t_point_size)
@@ -44,12 +50,6 @@ def _check(s, dropout=None, between=None, **kw):
 
     if dropout is not None:
         info.cache.dropout_points = torch.from_numpy(dropout).cuda()
-        got = backward()
-        hidden = dropout.all(axis=0)  # points dropped in every view receive nothing
-        assert hidden.any() and np.abs(got["position"][~hidden]).max() > 0
-        assert not got["position"][hidden].any() and not got["point_size"].reshape(-1)[hidden].any()
-        assert not got["texture"][:, hidden].any() and not got["confidence"].reshape(-1)[hidden].any()
-        return
     ref = {k: 0.0 for k in params}
     for b, f in enumerate(frames):
         r = f.backward(grads[b])
@@ -59,6 +59,7 @@ def _check(s, dropout=None, between=None, **kw):
         got = backward()
         for k in ref:
             assert rel_err(got[k].reshape(ref[k].shape), ref[k]) <= 1e-4, f"{k}, call {call}"
+    return got
 
 
 @pytest.mark.parametrize("n_views", [1, 3, 4, 5, 33])
@@ -73,9 +74,19 @@ def test_crowded_cloud(oracle_lib, cuda_lib, n_views):
     _check(s)
 
 
-def test_dropout_mask(oracle_lib, cuda_lib):
-    s = scenes.tiny(seed=90, n_points=3000, n_views=3)
-    _check(s, dropout=(np.random.default_rng(1).random((3, 3000)) < 0.5).astype(np.float32))
+@pytest.mark.parametrize("crowded", [False, True])
+def test_dropout_mask(oracle_lib, cuda_lib, crowded):
+    """Points dropped in some views, and 30 % of them in all: those receive nothing (the oracle's gradients are exactly 0)."""
+    n = 12000 if crowded else 3000
+    s = scenes.tiny(seed=90, n_points=n, n_views=3)
+    if crowded:
+        s.position[:, :3] *= 0.02
+    rng = np.random.default_rng(1)
+    mask = (rng.random((3, n)) < 0.5) | (rng.random(n) < 0.2)
+    got = _check(s, dropout=mask.astype(np.float32))
+    hidden = mask.all(axis=0)
+    assert not got["position"][hidden].any() and not got["point_size"].reshape(-1)[hidden].any()
+    assert not got["texture"][:, hidden].any() and not got["confidence"].reshape(-1)[hidden].any()
 
 
 def _move(info, cloud):
