@@ -27,6 +27,7 @@ def _check(s, views=None, min_length=0):
         for l, ref in enumerate(f.pyramid()):
             got = outs[l][b].detach().cpu().numpy()
             assert np.max(np.abs(got - ref) / np.maximum(np.abs(ref), 1e-3)) <= 1e-5
+    return info
 
 
 def _stack(n, copies, k_keep, seed):
@@ -123,3 +124,12 @@ def test_lists_shared_by_blocks(oracle_lib, cuda_lib, n_points, n_views):
     s.position[:-500, :3] *= 0.001
     s.confidence[:] = np.minimum(s.confidence, 0.1)
     _check(s, min_length=8192)
+
+
+def test_more_long_lists_than_the_preselection_takes(oracle_lib, cuda_lib):
+    """Above 131 072 long lists in a call nothing is pre-selected and the blend walks them itself."""
+    s = scenes.tiny(seed=330, n_points=1_500_000, width=96, height=80, num_layers=3, n_views=34, size_range=(1e-3, 2e-2))
+    s.confidence[:] = np.minimum(s.confidence, 0.1)
+    info = _check(s, views=[0, 13, 33], min_length=1000)
+    P = scenes.num_pyramid_pixels(s.width, s.height, s.num_layers)
+    assert sum(int((info.cache.debug_lists(v, P)[0] > 512).sum()) for v in range(s.n_views)) > 131_072
