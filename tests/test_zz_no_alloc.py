@@ -2,9 +2,9 @@
 
 Some users of this library run the optimizer step at a point where device memory cannot be allocated: the training
 framework's pool already owns every free byte, or the host application forbids cudaMalloc after start-up.  For them
-the library has a second Adam entry point whose tensor table sits in a fixed device array instead of allocated
-scratch.  It must produce exactly what the allocating entry point produces (the two run the same kernel on the same
-table, so the bar is bit equality), on a first call (which also resolves the array's address) and on a second call
+the library has a second Adam entry point whose tensor table sits in a fixed device array.  trips_adam_step passes the
+table of up to 16 tensors as a kernel argument and keeps larger ones in scratch that it allocates.  The fixed array must give
+exactly what either gives (the same arithmetic on the same table, so the bar is bit equality), on a first call (which also resolves the array's address) and on a second call
 that reuses the array; the second call must leave the amount of free device memory unchanged; and a call on a stream
 that is being captured must be refused before anything is enqueued (the table is uploaded from the call's stack frame).
 
@@ -38,11 +38,12 @@ def _table(_lib, params, grads, m, v, steps, lr):
     return (_lib.TripsAdamTensor * len(rows))(*rows)
 
 
-def test_static_adam_matches_allocating_adam_twice(cuda_lib):
+@pytest.mark.parametrize("n_tensors", [5, 16, 17, 64])
+def test_static_adam_matches_allocating_adam_twice(cuda_lib, n_tensors):
     import torch
     from trips_b200 import _lib
     L = cuda_lib
-    sizes = [4 * 5003, 5003, 20012, 7, 4096 * 3 + 1]
+    sizes = ([4 * 5003, 5003, 20012, 7, 4096 * 3 + 1] + [0, 1, 4095, 4096, 33] * 12)[:n_tensors]
     lr = 2e-3
     ref = _tensors(torch, _lib, np.random.default_rng(1), sizes, lr)
     new = [[t.clone() for t in group] for group in ref]

@@ -1,14 +1,15 @@
 // trips_adam_step_static: the fused Adam step for callers that must not allocate device memory.
 //
-// trips_adam_step keeps the table that tells the kernel where every parameter tensor lives (pointers, sizes,
-// hyper-parameters, and the first thread block of each tensor) in context scratch that it cudaMallocs on first use
-// and regrows when more tensors arrive.  Some callers cannot tolerate that: an optimizer step issued while the
-// framework above holds every free byte in its own caching pool, or a plugin whose host rules forbid cudaMalloc
-// after start-up.  This variant places the same table in a fixed device array that is part of the loaded library
-// image, so that a call does no cudaMalloc, no cudaFree and no allocating library call; it needs no TripsContext
-// either.  The table is uploaded from this function's stack frame with every call, so the call belongs on a stream
-// that executes it now: a stream that is being captured is refused (TRIPS_ERR_UNSUPPORTED) before anything is
-// enqueued, because a recorded copy would read the dead stack frame when the graph is replayed.
+// The table that tells the kernel where every parameter tensor lives (pointers, sizes, hyper-parameters, and the first
+// thread block of each tensor) travels as a kernel argument in trips_adam_step for up to 16 tensors; for more it lies in
+// context scratch that trips_adam_step cudaMallocs on first use and regrows when more tensors arrive.  Some callers
+// cannot tolerate that: an optimizer step issued while the framework above holds every free byte in its own caching
+// pool, or a plugin whose host rules forbid cudaMalloc after start-up.  This variant places the same table in a fixed
+// device array that is part of the loaded library image, so that a call does no cudaMalloc, no cudaFree and no
+// allocating library call; it needs no TripsContext either.  The table is uploaded from this function's stack frame
+// with every call, so the call belongs on a stream that executes it now: a stream that is being captured is refused
+// (TRIPS_ERR_UNSUPPORTED) before anything is enqueued, because a recorded copy would read the dead stack frame when
+// the graph is replayed.
 #include <mutex>
 
 #include "common.cuh"
