@@ -115,3 +115,37 @@ def test_points_are_those_of_the_forward_pass(oracle_lib, cuda_lib, between, cro
     if crowded:
         s.position[:, :3] *= 0.02
     _check(s, between=between)
+
+
+@pytest.mark.parametrize("indexed", [False, True])
+def test_entry_table_in_groups_of_views(cuda_lib, indexed):
+    """11 M points x 100 views: the table of a point's entries would exceed its limit of 4 GB and is filled for 97 views at a time.
+    The gradients are those of two calls with half of the views each, whose tables hold all of theirs."""
+    import torch
+    n, shown = 11_000_000, 4000
+    s = scenes.tiny(seed=96, n_points=n, n_views=100, width=61, height=43, num_layers=3)
+    s.position[shown // 2:n - shown // 2, 1] += 1000.0  # out of every view
+    index = np.random.default_rng(3).permutation(n).astype(np.int32) if indexed else None
+    ns, info, blend = gpu_render(s, train=True, index=index)
+    params = dict(texture=ns.texture.texture_raw, confidence=ns.texture.confidence_raw, position=ns.point_cloud_cuda.t_position,
+                  point_size=ns.point_cloud_cuda.t_point_size)
+    for t in params.values():
+        t.requires_grad_(True)
+    images, gen = info.images, torch.Generator(device="cuda")
+    gen.manual_seed(1)
+    targets = [torch.randn((100, s.channels, h, w), generator=gen, device="cuda") for w, h in scenes.layer_sizes(s.width, s.height, s.num_layers)]
+
+    def gradients(first, last):
+        info.images = images[first:last]
+        torch.autograd.backward(blend(info), [t[first:last] for t in targets])
+        assert info.cache.last_status() == 0
+        got = {k: t.grad.double() for k, t in params.items()}
+        for t in params.values():
+            t.grad = None
+        return got
+
+    whole, a, b = gradients(0, 100), gradients(0, 50), gradients(50, 100)
+    for k in params:
+        ref = a[k] + b[k]
+        scale = ref.abs().max()
+        assert scale > 0 and float(((whole[k] - ref).abs() / ref.abs().clamp(min=1e-2 * scale)).max()) <= 1e-4, k

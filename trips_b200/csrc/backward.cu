@@ -504,9 +504,11 @@ __device__ __forceinline__ ViewGrad view_gradient(const CamConst& cam, float vx,
 // on 6 M x 8, 0.99 / 0.85 / 1.04 ms on 20 M x 2; 5 spill).
 // With a texture index the descriptor / confidence gradients of all points sharing a column are added (atomics into
 // zeroed outputs); with the identity index they are plain stores.
+// ACC: adds to the outputs, for the views behind the first entry_views (identity index; with a texture index the descriptor and
+// confidence gradients are added anyway).
 constexpr int kGradViews = 4;   // views whose rows a thread requests before it waits for any of them
 constexpr int kGradCams  = 32;  // cameras held in shared memory; further ones are read from global memory (uniform addresses)
-template <int C, bool DIST>
+template <int C, bool DIST, bool ACC>
 __global__ __launch_bounds__(256, (C <= 4 ? 4 : 1)) void point_grad_kernel(ScenePtrs sc, FwdBuffers fb, BwdBuffers bb, const CamConst* __restrict__ cams, int B,
                                                          TripsGrads out, const float* __restrict__ raw_texture,
                                                          const float* __restrict__ raw_confidence, float confidence_scale)
@@ -563,8 +565,18 @@ __global__ __launch_bounds__(256, (C <= 4 ? 4 : 1)) void point_grad_kernel(Scene
                 }
             }
         }
-        if (out.points) reinterpret_cast<float4*>(out.points)[i] = make_float4(gp0, gp1, gp2, 0.f);
-        if (out.point_size) out.point_size[i] = gl == 0.f ? 0.f : tm_softplus_grad(p.w) * gl;
+        auto put = [](float* dst, float v) { *dst = ACC ? *dst + v : v; };
+        if (out.points)
+        {
+            float4* dst = reinterpret_cast<float4*>(out.points) + i;
+            if constexpr (ACC)
+            {
+                const float4 before = *dst;
+                gp0 += before.x, gp1 += before.y, gp2 += before.z;
+            }
+            *dst = make_float4(gp0, gp1, gp2, 0.f);
+        }
+        if (out.point_size) put(out.point_size + i, gl == 0.f ? 0.f : tm_softplus_grad(p.w) * gl);
         // fused texture preparation: chain through sigmoid(scale * raw) and |raw| (raw_* are null when the caller passes
         // activated tensors)
         const int col = sc.index ? __ldg(sc.index + i) : (int)i;
@@ -590,9 +602,9 @@ __global__ __launch_bounds__(256, (C <= 4 ? 4 : 1)) void point_grad_kernel(Scene
             if (out.texture)
             {
 #pragma unroll
-                for (int c = 0; c < C; ++c) out.texture[(size_t)c * sc.n_tex + i] = gt[c];
+                for (int c = 0; c < C; ++c) put(out.texture + (size_t)c * sc.n_tex + i, gt[c]);
             }
-            if (out.confidence) out.confidence[i] = gc;
+            if (out.confidence) put(out.confidence + i, gc);
         }
         else if ((unsigned)col < (unsigned)sc.n_tex)
         {
@@ -604,6 +616,19 @@ __global__ __launch_bounds__(256, (C <= 4 ? 4 : 1)) void point_grad_kernel(Scene
             }
             if (out.confidence && gc != 0.f) atomicAdd(out.confidence + col, gc);
         }
+    }
+}
+
+// Fills the point-to-entry table of a view group from the entries (view v0 + blockIdx.y); it holds kNoEntry before.
+__global__ __launch_bounds__(256) void note_entries_kernel(FwdBuffers fb, int v0, int N)
+{
+    const int v = v0 + blockIdx.y;
+    const unsigned long long first = fb.entry_base[v], n = fb.entry_base[v + 1] - first;
+    uint32_t* table = fb.point_entry + (size_t)blockIdx.y * N;
+    for (unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (unsigned long long)gridDim.x * blockDim.x)
+    {
+        const unsigned pid = __float_as_uint(fb.ent_head[(first + i) * 2 + 1].x);
+        if (pid < (unsigned)N) table[pid] = (uint32_t)i;
     }
 }
 
@@ -717,6 +742,8 @@ __global__ __launch_bounds__(64) void unpack_small_kernel(int C, int B, const Ca
     }
 }
 
+int unpack_launches(int B, int entry_views) { return entry_views < B ? 2 * ((B + entry_views - 1) / entry_views) : 1; }
+
 cudaError_t launch_unpack_grads(const ScenePtrs& sc, const CamConst* cams, int B, const FwdBuffers& fb, const BwdBuffers& bb,
                                 const TripsGrads& out, const TripsRenderParams& pr, int sm_count, cudaStream_t st)
 {
@@ -761,23 +788,38 @@ cudaError_t launch_unpack_grads(const ScenePtrs& sc, const CamConst* cams, int B
         const int blocks      = max(1, (int)min((size_t)sm_count * 16, ((size_t)sc.N + 255) / 256));
         const float* raw_tex  = pr.texture_abs ? sc.texture : nullptr;
         const float* raw_conf = pr.confidence_is_raw ? sc.confidence : nullptr;
-#define TRIPS_POINT_CASE(CC)                                                                                                              \
-    case CC:                                                                                                                              \
-        if (pr.distortion)                                                                                                                \
-            point_grad_kernel<CC, true><<<blocks, 256, 0, st>>>(sc, fb, bb, cams, B, out, raw_tex, raw_conf, pr.confidence_scale);        \
-        else                                                                                                                              \
-            point_grad_kernel<CC, false><<<blocks, 256, 0, st>>>(sc, fb, bb, cams, B, out, raw_tex, raw_conf, pr.confidence_scale);       \
-        break;
-        switch (sc.C)
+        for (int v0 = 0; v0 < B; v0 += fb.entry_views)
         {
-            TRIPS_POINT_CASE(3)
-            TRIPS_POINT_CASE(4)
-            TRIPS_POINT_CASE(6)
-            TRIPS_POINT_CASE(8)
-            TRIPS_POINT_CASE(16)
-            default: return cudaErrorInvalidValue;
-        }
+            const int nv   = min(fb.entry_views, B - v0);
+            FwdBuffers fbv = fb;
+            fbv.entry_base = fb.entry_base + v0;
+            if (fb.entry_views < B)
+            {
+                cudaError_t e = cudaMemsetAsync(fb.point_entry, 0xff, sizeof(uint32_t) * (size_t)sc.N * nv, st);  // kNoEntry
+                if (e != cudaSuccess) return e;
+                note_entries_kernel<<<dim3(max(1, sm_count * 8 / nv), nv), 256, 0, st>>>(fb, v0, sc.N);
+            }
+#define TRIPS_POINT_LAUNCH(CC, DIST, ACC) \
+    point_grad_kernel<CC, DIST, ACC><<<blocks, 256, 0, st>>>(sc, fbv, bb, cams + v0, nv, out, raw_tex, raw_conf, pr.confidence_scale)
+#define TRIPS_POINT_CASE(CC)                                                                              \
+    case CC:                                                                                              \
+        if (pr.distortion)                                                                                \
+            v0 ? TRIPS_POINT_LAUNCH(CC, true, true) : TRIPS_POINT_LAUNCH(CC, true, false);                \
+        else                                                                                              \
+            v0 ? TRIPS_POINT_LAUNCH(CC, false, true) : TRIPS_POINT_LAUNCH(CC, false, false);              \
+        break;
+            switch (sc.C)
+            {
+                TRIPS_POINT_CASE(3)
+                TRIPS_POINT_CASE(4)
+                TRIPS_POINT_CASE(6)
+                TRIPS_POINT_CASE(8)
+                TRIPS_POINT_CASE(16)
+                default: return cudaErrorInvalidValue;
+            }
 #undef TRIPS_POINT_CASE
+#undef TRIPS_POINT_LAUNCH
+        }
     }
     unpack_small_kernel<<<1, 64, 0, st>>>(sc.C, B, cams, bb.g_bg, bb.g_pose, bb.g_k, bb.g_dis, out.background, out.pose_tangent,
                                          out.intrinsics);

@@ -204,6 +204,12 @@ static size_t ticket_groups(int B) { return 2 * (((size_t)B + kViewGroup - 1) / 
 // work counter of the blend: behind those of the binning, count and collect passes, on a line of its own
 static size_t blend_ticket_at(int B) { return (ticket_groups(B) + 2 * (size_t)B + 31) / 32 * 32; }
 
+// views the point-to-entry table holds at a time
+static int entry_views(int B, int N)
+{
+    return (int)std::min<size_t>((size_t)B, std::max<size_t>(1, kEntryTableBytes / (sizeof(uint32_t) * (size_t)std::max(1, N))));
+}
+
 static FwdBuffers fwd_buffers(TripsContext* c, int B)
 {
     FwdBuffers fb;
@@ -228,6 +234,8 @@ static FwdBuffers fwd_buffers(TripsContext* c, int B)
     fb.ticket_collect = fb.ticket_count + B;
     fb.ticket_blend   = fb.ticket + blend_ticket_at(B);
     fb.point_entry = c->params.train ? (uint32_t*)c->point_entry.p : nullptr;
+    fb.entry_views = entry_views(B, c->N);
+    fb.note_entry  = fb.entry_views == B ? fb.point_entry : nullptr;
     fb.point_state = c->params.train ? (float4*)c->point_state.p : nullptr;
     fb.block_box  = (const float*)c->block_box.p;
     fb.block_skip = (const uint8_t*)c->block_skip.p;
@@ -422,7 +430,7 @@ static int forward_views(TripsContext* ctx, const TripsScene* scene, const Trips
     {
         CU_CHECK(ctx, ensure(ctx->rec_n, (size_t)g.n_tiles * 32 * B));
         CU_CHECK(ctx, ensure(ctx->records, sizeof(uint2) * 16 * 32 * (size_t)g.n_tiles * B));
-        CU_CHECK(ctx, ensure(ctx->point_entry, sizeof(uint32_t) * N * B));
+        CU_CHECK(ctx, ensure(ctx->point_entry, sizeof(uint32_t) * N * entry_views(B, (int)N)));
         CU_CHECK(ctx, ensure(ctx->point_state, sizeof(float4) * N));
     }
     if (ctx->frags.bytes == 0) CU_CHECK(ctx, ensure(ctx->frags, 16 * 1024 * 1024));
@@ -628,7 +636,7 @@ int trips_backward(TripsContext* ctx, const TripsScene* scene, const float* cons
     const bool cam_grads = grads->pose_tangent || grads->intrinsics;
     STAGE(ctx, TRIPS_STAGE_BACKWARD, 1, st,
           launch_blend_backward(sp, (const CamConst*)ctx->cams.p, g, ctx->params, B, fb, bb, gin, cam_grads, ctx->sm_count, st));
-    const int n_unpack = (N > 0 ? 1 + (cam_grads ? 1 : 0) : 0) + 1;
+    const int n_unpack = (N > 0 ? unpack_launches(B, fb.entry_views) + (cam_grads ? 1 : 0) : 0) + 1;
     STAGE(ctx, TRIPS_STAGE_UNPACK, n_unpack, st,
           launch_unpack_grads(sp, (const CamConst*)ctx->cams.p, B, fb, bb, *grads, ctx->params, ctx->sm_count, st));
     return TRIPS_OK;

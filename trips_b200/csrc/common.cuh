@@ -14,6 +14,9 @@ constexpr int kBinShift   = 5;   // visible points are bucketed by 32x32-pixel s
 constexpr int kTileW      = 8;   // one warp renders / differentiates an 8x4 pixel tile
 constexpr int kTileH      = 4;
 constexpr uint32_t kNoEntry = 0xffffffffu;  // a point that is not visible in a view
+// Point-to-entry table of a training call: at most this many bytes.  It has 4 bytes per point and view, also where most points
+// are visible in few of the views; a call of 20 M points reaches the limit with 53 views.
+constexpr size_t kEntryTableBytes = (size_t)4 << 30;
 constexpr int kViewGroup  = 16;  // views whose camera constants are in shared memory at a time in the binning passes (one launch per group)
 constexpr int kHeavyList  = 512;      // lists longer than this get their 16 nearest fragments moved to the front by a block of their own
 constexpr int kHeavyPart  = 8192;     // longer ones are shared by several blocks, each with a part of at most this many fragments ...
@@ -126,7 +129,10 @@ struct FwdBuffers
     unsigned int* ticket_count;       // [B] count pass
     unsigned int* ticket_collect;     // [B] collect pass
     unsigned int* ticket_blend;
-    uint32_t* point_entry;            // training: [B,N] entry (within the view) of every point, kNoEntry where it is not visible
+    uint32_t* point_entry;            // training: [entry_views,N] entry (within the view) of every point, kNoEntry where it is not visible
+    int entry_views;                  // B, or fewer where the table of all views would be larger than kEntryTableBytes: the backward
+                                      // pass then fills it for so many views at a time
+    uint32_t* note_entry;             // point_entry where the binning pass notes the entries of all views, else nullptr
     float4* point_state;              // training: [N] position and raw size of the points that were not discarded, as this pass saw them
     const float* block_box;           // [ceil(N / 8192), 6] bounding boxes (min xyz, max xyz) of blocks of consecutive points
     const uint8_t* block_skip;        // [B, ceil(N / 8192)] 1 = the block cannot hold a point visible in that view
@@ -413,6 +419,7 @@ cudaError_t launch_zero_entry_rows(int C, int B, const FwdBuffers& fb, const Bwd
 cudaError_t launch_blend_backward(const ScenePtrs& sc, const CamConst* cams, const Geom& g, const TripsRenderParams& pr,
                                   int B, const FwdBuffers& fb, const BwdBuffers& bb, const ConstLayerPtrs& grad_in,
                                   bool want_cam_grads, int sm_count, cudaStream_t st);
+int unpack_launches(int B, int entry_views);  // launches of the point gradients
 cudaError_t launch_unpack_grads(const ScenePtrs& sc, const CamConst* cams, int B, const FwdBuffers& fb, const BwdBuffers& bb,
                                 const TripsGrads& out, const TripsRenderParams& pr, int sm_count, cudaStream_t st);
 cudaError_t launch_adam(const TripsAdamTensor* d_tensors, const int64_t* d_block_start, int n_tensors, int64_t total_blocks,

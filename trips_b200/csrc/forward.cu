@@ -549,8 +549,8 @@ __global__ __launch_bounds__(kBinThreads, (C <= 4 ? kScatterMinBlocks : kScatter
             d.tex_ok = (unsigned)d.tex < (unsigned)sc.n_tex;
             if (discarded_for_confidence<ACT>(sc, pr, d.tex))
             {
-                if (fb.point_entry)
-                    for (int v = 0; v < nv; ++v) fb.point_entry[(size_t)(v0 + v) * sc.N + i] = kNoEntry;
+                if (fb.note_entry)
+                    for (int v = 0; v < nv; ++v) fb.note_entry[(size_t)(v0 + v) * sc.N + i] = kNoEntry;
                 continue;
             }
             const float4 p  = h.p;
@@ -586,10 +586,10 @@ __global__ __launch_bounds__(kBinThreads, (C <= 4 ? kScatterMinBlocks : kScatter
                     const Projected r = project_visible(s_cam[v], g, pr, p, raw, sp);
                     write_entry<C>(fb, g, pr, s_ebase[v] + slot[j], i, p, raw, r, d);
                 }
-                if (fb.point_entry)  // behind the entries: the slots are on their way while the points are projected again
+                if (fb.note_entry)  // behind the entries: the slots are on their way while the points are projected again
 #pragma unroll
                     for (int j = 0; j < kSweep; ++j)
-                        if (vb + j < nv) fb.point_entry[(size_t)(v0 + vb + j) * sc.N + i] = slot[j];
+                        if (vb + j < nv) fb.note_entry[(size_t)(v0 + vb + j) * sc.N + i] = slot[j];
             }
         }
     }
@@ -750,8 +750,8 @@ __global__ __launch_bounds__(kBinThreads) void bin_scatter_hot_kernel(ScenePtrs 
             d.tex_ok = (unsigned)d.tex < (unsigned)sc.n_tex;
             if (discarded_for_confidence<ACT>(sc, pr, d.tex))
             {
-                if (fb.point_entry)
-                    for (int v = 0; v < nv; ++v) fb.point_entry[(size_t)(v0 + v) * sc.N + i] = kNoEntry;
+                if (fb.note_entry)
+                    for (int v = 0; v < nv; ++v) fb.note_entry[(size_t)(v0 + v) * sc.N + i] = kNoEntry;
                 continue;
             }
             const float4 p  = __ldg(sc.position + i);
@@ -772,7 +772,7 @@ __global__ __launch_bounds__(kBinThreads) void bin_scatter_hot_kernel(ScenePtrs 
                         slot               = s >= 0 ? s_base[s] + atomicAdd(s_cnt + s, 1u) : atomicAdd(cursors + key, 1u);
                     }
                 }
-                if (fb.point_entry) fb.point_entry[(size_t)(v0 + v) * sc.N + i] = slot;
+                if (fb.note_entry) fb.note_entry[(size_t)(v0 + v) * sc.N + i] = slot;
                 if (slot == kNoEntry) continue;
                 write_entry<C>(fb, g, pr, s_ebase[v] + slot, i, p, raw, r, d);
             }
