@@ -60,7 +60,8 @@ constexpr int kBwdWarps   = kBwdThreads / 32;
 // at 16-20 resident warps per SM; DRAM is at 20-30 %.  Hence the care for lines per instruction (entries ordered by
 // tile, paired atomics, coalesced staging) and for instructions per fragment (fragment table, no shuffle searches).
 constexpr int kBwdBlocksPerSM = 12;  // grid size of the persistent kernel, in blocks per SM
-// measured: 5 resident blocks (96 registers) 3.59 ms, 4 blocks (108) 3.63 ms, 6 blocks (80) 3.76 ms
+// Resident blocks, 4 / 5 / 6 (register caps 128 / 96 / 80), grid 12 blocks per SM at 5 and as many as are resident otherwise: 6 M points
+// x 8 views 3.66 / 3.11 / 2.97 ms, 20 M x 2 views 0.81 / 0.70 / 0.77, 1.3 M points with long lists x 5 views 0.56 / 0.49 / 0.62.
 constexpr int kBwdMinBlocks = 5;
 // SAT: saturated_alpha_accumulation as the reference's backward pass has it (RenderBackward.cu:227-259); a separate
 // instantiation, so that the common case carries none of its code or registers.

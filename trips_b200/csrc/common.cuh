@@ -18,7 +18,11 @@ constexpr uint32_t kNoEntry = 0xffffffffu;  // a point that is not visible in a 
 // are visible in few of the views; a call of 20 M points reaches the limit with 53 views.
 constexpr size_t kEntryTableBytes = (size_t)4 << 30;
 constexpr int kViewGroup  = 16;  // views whose camera constants are in shared memory at a time in the binning passes (one launch per group)
-constexpr int kHeavyList  = 512;      // lists longer than this get their 16 nearest fragments moved to the front by a block of their own
+// Lists longer than kHeavyList get their 16 nearest fragments moved to the front by a block of their own.  sort_blend, ms, at 128 /
+// 256 / 512 / 1024 / 4096: 20 M points at 1440p x 2 views 1.17 / 0.89 / 0.75 / 0.80 / 0.79, 3 M points in 64x64 pixels x 4 views
+// 0.54 / 0.54 / 0.54 / 0.59 / 1.31, 1.6 M points in 53x28 pixels x 8 views 0.70 / 0.71 / 0.73 / 0.79 / 1.10; 64 views of 10 M points 23.5
+// at 128 and 22.9 from 256 on.
+constexpr int kHeavyList  = 512;
 constexpr int kHeavyPart  = 8192;     // longer ones are shared by several blocks, each with a part of at most this many fragments ...
 constexpr int kHeavyParts = 256;      // ... or by this many blocks
 constexpr int kHeavyCap   = 1 << 17;  // such lists and parts per call the pre-selection handles; beyond that the blend walks the lists itself

@@ -352,7 +352,7 @@ __global__ __launch_bounds__(kBinThreads) void bin_count_kernel(ScenePtrs sc, co
 // view_total[b] = visible points of the view.  A turn of the block covers 16384 keys, 16 consecutive ones per thread (64
 // bytes, vector loads and stores): the turns follow one another, and with one key per thread a 1080p view (65 k keys) took
 // 64 of them, each two dependent loads and three barriers long.
-// Measured on a 1080p view: 90 us with one key per thread and turn; sixteen take the whole binning stage from 0.347 to 0.292 ms.
+// Measured on a 1080p view: 90 us with one key per thread and turn; sixteen take the whole binning stage from 0.326 to 0.270 ms.
 constexpr int kScanKeys = 16;
 __global__ __launch_bounds__(1024) void bin_scan_kernel(const uint32_t* __restrict__ counts, uint32_t* __restrict__ key_first,
                                                         uint32_t* __restrict__ bin_first, int n_keys, uint32_t* __restrict__ view_total, DevStats* stats)
@@ -1405,9 +1405,14 @@ static bool few_entries(unsigned long long entries_hint, int sm_count)
 }
 
 template <int THREADS, bool COLLECT>
-static void run_window(const Geom& g, int B, const FwdBuffers& fb, bool strict, int chunk, int sm_count, cudaStream_t st)
+static void run_window(const Geom& g, int B, const FwdBuffers& fb, bool strict, int chunk, unsigned long long entries_hint, int sm_count, cudaStream_t st)
 {
-    const int grid = sm_count * (kWinWarpsPerSM * 32 / THREADS);
+    // No more blocks than the call has chunks: every block asks for a ticket in every view, and with twice as many blocks of half the
+    // size small calls spent longer on that than before (0.7 M entries in 11 views: count 0.063 -> 0.084 ms; 0.055 like this).  The
+    // hint may be an earlier call's: four blocks per SM take whatever there is.
+    const unsigned long long most = (unsigned long long)sm_count * (kWinWarpsPerSM * 32 / THREADS);
+    const unsigned long long want = entries_hint / chunk + B;
+    const int grid                = (int)min(most, max((unsigned long long)sm_count * 4, want));
     if (strict)
         window_kernel<THREADS, COLLECT, true><<<grid, THREADS, 0, st>>>(g, fb, B, chunk);
     else
@@ -1417,7 +1422,7 @@ static void run_window(const Geom& g, int B, const FwdBuffers& fb, bool strict, 
 cudaError_t launch_count(const ScenePtrs& sc, const Geom& g, int B, const FwdBuffers& fb, bool strict, unsigned long long entries_hint, int sm_count,
                          cudaStream_t st)
 {
-    run_window<kWinThreadsCount, false>(g, B, fb, strict, few_entries(entries_hint, sm_count) ? kWinChunkCountFew : kWinChunkCount, sm_count, st);
+    run_window<kWinThreadsCount, false>(g, B, fb, strict, few_entries(entries_hint, sm_count) ? kWinChunkCountFew : kWinChunkCount, entries_hint, sm_count, st);
     return cudaGetLastError();
 }
 
@@ -1425,9 +1430,9 @@ cudaError_t launch_collect(const ScenePtrs& sc, const Geom& g, int B, const FwdB
                            cudaStream_t st)
 {
     if (entries_hint / kWinChunkCollect < (unsigned long long)sm_count * (kWinMinWarps * 32 / kWinThreadsCollect))
-        run_window<kWinThreadsCollectFew, true>(g, B, fb, strict, kWinChunkCollectFew, sm_count, st);
+        run_window<kWinThreadsCollectFew, true>(g, B, fb, strict, kWinChunkCollectFew, entries_hint, sm_count, st);
     else
-        run_window<kWinThreadsCollect, true>(g, B, fb, strict, kWinChunkCollect, sm_count, st);
+        run_window<kWinThreadsCollect, true>(g, B, fb, strict, kWinChunkCollect, entries_hint, sm_count, st);
     return cudaGetLastError();
 }
 
