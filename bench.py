@@ -163,18 +163,21 @@ def stage_bytes(stage, N, P, C, B, F, Kf, V=0):
         # per visible point and view one 32-byte gradient row cleared and read, per point its entry index in every view, its
         # position and size, and the outputs in the reference's layouts
         c4 = (C + 3) // 4 * 4
-        return 2 * 4 * (4 + c4) * V + (4 * B + 20 + 4 * (4 + 1 + C + 1)) * N
+        return 2 * 4 * (4 + c4) * V + (4 * B + 16 + 4 * (4 + 1 + C + 1)) * N
     return 0
 
 
-# DRAM bytes (read + write) per unit of work, from the ncu captures summarised under profiles/: the tile kernels and Adam
-# from one view of config 3 (rasterizer_kernels_c3_6Mpts_1view_ncu_sections.md: same list density and the same N as the
-# benchmark), the binning kernels, which read every point once for all views of a call, from a quarter of the points with
-# all 8 views (binning_adam_kernels_1.5Mpts_8views_ncu_sections.md).  Traffic grows in proportion to the unit count.  The
-# gradient gather has no figure of its own yet and is left out of the sums.  Units: F fragments, Kf kept fragments, NB
-# points x views, N points.
-DRAM_BYTES_PER_UNIT = {"count": [(5.2, "F")], "collect": [(20.2, "F")], "sort_blend": [(35.6, "F")], "blend_backward": [(35.5, "Kf")],
-                       "bin_points": [(43.1, "NB")], "adam": [(337.3, "N")]}
+# DRAM bytes (read + write) per unit of work, from the ncu captures summarised under profiles/: the tile kernels, the gradient
+# gather and Adam from one view of config 3 (rasterizer_kernels_c3_6Mpts_1view_ncu_sections.md: same list density and the
+# same N as the benchmark), the binning kernels, which read every point once for all views of a call, from a quarter of the
+# points with all 8 views (binning_adam_kernels_1.5Mpts_8views_ncu_sections.md).  Traffic grows in proportion to the unit
+# count.  The scan has no capture and is left out of the sums.  Units: F fragments, Kf kept fragments, NB points x views, V
+# entries (visible points over all views), N points.
+# unpack_grads: 15.1 bytes per row cleared, 127.2 per row gathered (127 bytes of DRAM for a 32-byte row at a random address),
+# 4 per entry index, 16 of point state and 35 of gradients per point.
+DRAM_BYTES_PER_UNIT = {"count": [(5.2, "F")], "collect": [(20.2, "F")], "sort_blend": [(34.5, "F")], "blend_backward": [(36.0, "Kf")],
+                       "bin_points": [(48.8, "NB")], "unpack_grads": [(15.1 + 127.2, "V"), (4.0, "NB"), (16.0 + 35.0, "N")],
+                       "adam": [(337.3, "N")]}
 
 
 def stage_traffic(stage, N, B, F, Kf, V=0):
@@ -590,6 +593,7 @@ def run_ours(args, rank, world, local_rank):
                 # the whole step against the HBM roofline: algorithmic bytes of all stages / step time, and the same on measured DRAM bytes
                 "step_frac": total_alg / (ms_step * 1e-3) / 1e9 / peak,
                 "step_frac_dram": (total_traffic / (ms_step * 1e-3) / 1e9 / peak) if total_traffic else None,
+                "step_frac_dram_without": [k for k in per_stage if k in step_stages and stage_traffic(k, N, B, F, Kf, V) is None],
                 "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum per unit of work (profiles/rasterizer_kernels_c3_6Mpts_1view_ncu_sections.md, binning_adam_kernels_1.5Mpts_8views_ncu_sections.md) x units of this run",
                 "alg_bytes_per_launch": dom_bytes,
                 "step_alg_bytes": total_alg, "step_gbs": total_alg / (ms_step * 1e-3) / 1e9, "stages": per_stage}
