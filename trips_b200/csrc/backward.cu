@@ -501,8 +501,9 @@ __device__ __forceinline__ ViewGrad view_gradient(const CamConst& cam, float vx,
 // sort of the points to keep those updates in L2.
 // Measured, the whole gradient bookkeeping (clearing, this kernel, camera sums), per-point accumulators / gather:
 // 6 M points x 8 views 1.05 / 0.73 ms, x 1 view 0.44 / 0.27 ms, 20 M x 2 views 1.54 / 0.75 ms, 2 M x 4 views 0.22 / 0.16 ms.
-// Random 32-byte reads: latency and loads in flight bound it (resident blocks of 256 threads at 3 / 4 / 5: 0.77 / 0.73 / 0.93 ms
-// on 6 M x 8, 0.99 / 0.85 / 1.04 ms on 20 M x 2; 5 spill).
+// Random 32-byte reads: a row costs 127 bytes of DRAM on one view of 6 M points and 92 on 8 views of 1.5 M, and the kernel
+// moves 4.8-5.4 TB/s (resident blocks of 256 threads at 3 / 4 / 5: 0.77 / 0.73 / 0.93 ms on 6 M x 8, 0.99 / 0.85 / 1.04 ms on 20 M x 2;
+// 5 spill).
 // With a texture index the descriptor / confidence gradients of all points sharing a column are added (atomics into
 // zeroed outputs); with the identity index they are plain stores.
 // ACC: adds to the outputs, for the views behind the first entry_views (identity index; with a texture index the descriptor and

@@ -92,8 +92,10 @@ struct DevStats
 // the stage that reads them, so that a stage's gathers touch fewer bytes it does not use (DRAM is read in 64-byte
 // pieces), while the binning pass still writes whole 32-byte sectors:
 //   head [2 x float4]     u, v (layer-0 image position), size in pixels, confidence (all the backward pass reads) |
-//                         point id (bits), view-space depth, raw point size, number of layers written (bits)
-//   tail [1 + C4/4 float4] world position x, y, z, texture index (bits) | descriptor row (C floats, padded to 4)
+//                         point id (bits), view-space depth, raw point size (fills the sector: nothing reads it), number of layers
+//                         written (bits)
+//   tail [1 + C4/4 float4] world position x, y, z (read for the camera gradients with lens distortion only), texture index
+//                         (bits) | descriptor row (C floats, padded to 4)
 __host__ __device__ constexpr int tail_stride(int C) { return 4 + ((C + 3) & ~3); }
 __host__ __device__ constexpr int entry_stride(int C) { return 8 + tail_stride(C); }  // floats per entry over both arrays
 // Gradient accumulator of an entry: sums over its fragments of (J0 gbs, J1 gbs, bf conf lf' ga, bf lf ga) | descriptor row.

@@ -1445,15 +1445,15 @@ cudaError_t launch_collect(const ScenePtrs& sc, const Geom& g, int B, const FwdB
 //   selection: every lane sorts its own list by depth in registers, 16 fragments at a time, with a fixed comparator
 //     network (Batcher's odd-even merge sort); further chunks are merged into the 16 nearest (bitonic half-cleaner +
 //     merge).  A comparator serves 32 pixels at once, so a chunk costs a few hundred instructions per WARP, whatever
-//     the lists look like.  Fragments of equal depth are put into point-id order afterwards; that is the rare path.
+//     the lists look like.  Fragments of equal depth are put into point-id order afterwards.
 //   blend: the sequential transmittance recurrence and the colour sum over the kept fragments.
 // Replaces FastSortFusedNew (RenderForward.cu:474-1059).
 //
 // What bounds it (ncu, one 1080p view of 6 M points): half of the issue slots and half of the load/store unit's wavefront
 // rate in use at 20 warps per SM, the rest are waits for the gathers of list heads and descriptor rows; DRAM at 27 %.
-// 190 M instructions, against 323 M when the fragments of a tile were ranked against each other with shuffles (lists of at
+// 184 M instructions, against 323 M when the fragments of a tile were ranked against each other with shuffles (lists of at
 // most 32) or sorted by half-warps, which this replaces: sort_blend stage 0.42 -> 0.31 ms on that view, 32.1 -> 22.9 ms on
-// 64 views of 10 M points (longer lists), 1.41 -> 0.87 ms on 2 1440p views of 20 M, 0.206 -> 0.070 ms on a 640x480 view of
+// 64 views of 10 M points (longer lists), 1.41 -> 0.75 ms on 2 1440p views of 20 M, 0.206 -> 0.070 ms on a 640x480 view of
 // 200 k points (lists up to 379, K = 8).
 // Loops stay rolled where they can: with the blend unrolled over 16 fragments and every network instantiated twice the
 // warps spent 8.6 of 20 cycles per instruction waiting for instruction fetches, and the kernel lost to its predecessor.
