@@ -210,6 +210,21 @@ static int entry_views(int B, int N)
     return (int)std::min<size_t>((size_t)B, std::max<size_t>(1, kEntryTableBytes / (sizeof(uint32_t) * (size_t)std::max(1, N))));
 }
 
+// Room for what the pre-selection of a call can meet: a list has more than kHeavyList fragments, a part of a shared one at
+// least half of kHeavyPart, and a call at most 4 fragments per point, layer and view.
+static HeavyLists heavy_lists(int N, int L, int B, void* p)
+{
+    HeavyLists h;
+    const unsigned long long most = 4ull * N * L * B;
+    h.cap        = (unsigned)std::min<unsigned long long>(kHeavyCap, most / kHeavyList + 1);
+    h.shared_cap = (unsigned)std::min<unsigned long long>(kHeavyShared, most / (kHeavyPart / 2) + 1);
+    h.item       = (uint4*)p;
+    h.nearest    = (uint32_t*)(h.item + h.cap);
+    h.finished   = h.nearest + 16 * (size_t)h.shared_cap;
+    return h;
+}
+static size_t heavy_bytes(const HeavyLists& h) { return sizeof(uint4) * h.cap + sizeof(uint32_t) * 17 * (size_t)h.shared_cap; }
+
 static FwdBuffers fwd_buffers(TripsContext* c, int B)
 {
     FwdBuffers fb;
@@ -239,9 +254,7 @@ static FwdBuffers fwd_buffers(TripsContext* c, int B)
     fb.point_state = c->params.train ? (float4*)c->point_state.p : nullptr;
     fb.block_box  = (const float*)c->block_box.p;
     fb.block_skip = (const uint8_t*)c->block_skip.p;
-    fb.heavy.item     = (uint4*)c->heavy.p;
-    fb.heavy.nearest  = (uint32_t*)(fb.heavy.item + kHeavyCap);
-    fb.heavy.finished = fb.heavy.nearest + 16 * (size_t)kHeavyShared;
+    fb.heavy      = heavy_lists(c->N, c->geom.L, B, c->heavy.p);
     return fb;
 }
 
@@ -421,7 +434,7 @@ static int forward_views(TripsContext* ctx, const TripsScene* scene, const Trips
     CU_CHECK(ctx, ensure(ctx->entry_base, sizeof(unsigned long long) * (B + 1)));
     CU_CHECK(ctx, ensure(ctx->block_box, sizeof(float) * 6 * n_box));
     CU_CHECK(ctx, ensure(ctx->block_skip, (size_t)B * n_box));
-    CU_CHECK(ctx, ensure(ctx->heavy, kHeavyBytes));
+    CU_CHECK(ctx, ensure(ctx->heavy, heavy_bytes(heavy_lists((int)N, g.L, B, nullptr))));
     CU_CHECK(ctx, ensure(ctx->offsets, sizeof(uint32_t) * P * B));
     CU_CHECK(ctx, ensure(ctx->partial, sizeof(uint32_t) * (size_t)nchunks * B));
     CU_CHECK(ctx, ensure(ctx->view_base, sizeof(unsigned long long) * (B + 1)));

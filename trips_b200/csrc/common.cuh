@@ -25,8 +25,8 @@ constexpr int kViewGroup  = 16;  // views whose camera constants are in shared m
 constexpr int kHeavyList  = 512;
 constexpr int kHeavyPart  = 8192;     // longer ones are shared by several blocks, each with a part of at most this many fragments ...
 constexpr int kHeavyParts = 256;      // ... or by this many blocks
-constexpr int kHeavyCap   = 1 << 17;  // such lists and parts per call the pre-selection handles; beyond that the blend walks the lists itself
-constexpr int kHeavyShared = 1 << 16; // parts of shared lists per call; beyond that a long list gets one block
+constexpr int kHeavyCap   = 1 << 17;  // such lists and parts per call the pre-selection handles at most; beyond that the blend walks the lists itself
+constexpr int kHeavyShared = 1 << 16; // parts of shared lists per call at most; beyond that a long list gets one block
 
 // Pyramid geometry shared by all views of a call.
 struct Geom
@@ -105,11 +105,11 @@ __host__ __device__ constexpr int egrad_stride(int C) { return 4 + ((C + 3) & ~3
 // Lists longer than kHeavyList, found by the scan.  A list of several parts has one item per part.
 struct HeavyLists
 {
-    uint4* item;        // [kHeavyCap] view, pixel, part | parts << 16 (0: empty), where the list's parts start in `nearest` and `finished`
-    uint32_t* nearest;  // [kHeavyShared, 16] list positions of a part's nearest fragments
-    uint32_t* finished; // [kHeavyShared] parts of the list that are done, at the list's first part
+    uint4* item;        // [cap] view, pixel, part | parts << 16 (0: empty), where the list's parts start in `nearest` and `finished`
+    uint32_t* nearest;  // [shared_cap, 16] list positions of a part's nearest fragments
+    uint32_t* finished; // [shared_cap] parts of the list that are done, at the list's first part
+    unsigned cap, shared_cap;
 };
-constexpr size_t kHeavyBytes = sizeof(uint4) * kHeavyCap + sizeof(uint32_t) * 17 * (size_t)kHeavyShared;
 
 struct FwdBuffers
 {

@@ -928,9 +928,9 @@ __global__ __launch_bounds__(256) void scan_reduce_kernel(const uint32_t* __rest
             const uint32_t n     = c[min(start + k * 256, P - 1)];
             const uint32_t parts = start + k * 256 < P ? parts_of(n) : 0u;
             // no room for its parts: one block takes the whole list, the other items stay empty
-            const bool whole = parts > 1 && shared + parts > (uint32_t)kHeavyShared;
+            const bool whole = parts > 1 && shared + parts > heavy.shared_cap;
             if (parts > 1 && !whole) heavy.finished[shared] = 0;
-            for (uint32_t t = 0; t < parts && slot + t < (uint32_t)kHeavyCap; ++t)
+            for (uint32_t t = 0; t < parts && slot + t < heavy.cap; ++t)
                 heavy.item[slot + t] = make_uint4((unsigned)b, (unsigned)(start + k * 256), whole ? (t == 0 ? 1u << 16 : 0u) : t | parts << 16, shared);
             slot += parts;
             shared += parts > 1 ? parts : 0u;
@@ -1585,7 +1585,7 @@ __global__ __launch_bounds__(256, kHeavyBlocks) void heavy_topk_kernel(const __g
     __shared__ uint32_t s_vac[16];
     __shared__ unsigned s_last;
     const unsigned n_heavy = fb.stats->n_heavy;
-    if (n_heavy == 0 || n_heavy > (unsigned)kHeavyCap) return;
+    if (n_heavy == 0 || n_heavy > fb.heavy.cap) return;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, j = lane & 15;
     for (unsigned h = blockIdx.x; h < n_heavy; h += gridDim.x)
     {
@@ -1729,7 +1729,7 @@ __global__ __launch_bounds__(kSbThreads, (C <= 4 ? kSbMinBlocks : (C <= 8 ? kSbM
 #pragma unroll
     for (int c = 0; c < C; ++c) bg[c] = __ldg(sc.background + c);
 
-    const bool preselected = fb.stats->n_heavy <= (unsigned)kHeavyCap;  // heavy_topk_kernel handled every long list
+    const bool preselected = fb.stats->n_heavy <= fb.heavy.cap;  // heavy_topk_kernel handled every long list
     unsigned next_ticket = 0;
     if (lane == 0) next_ticket = atomicAdd(fb.ticket_blend, 1u);
     for (;;)
