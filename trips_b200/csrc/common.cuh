@@ -297,16 +297,11 @@ __device__ __forceinline__ float layer_factor(float ps, int layer, int L, float*
     }
     else
     {
-        float l_l = (float)(1 << lo);
-        float l_h = (float)(1 << hi);
-        f         = (ps - l_l) / (l_h - l_l);
+        // hi = lo + 1: the layers' sizes differ by 2^lo, and a division by it is a product with its exact reciprocal
+        const float l_l = (float)(1 << lo), inv = __int_as_float((127 - lo) << 23);
+        f               = (ps - l_l) * inv;
         if (layer == lo) f = 1.f - f;
-        if (grad)
-        {
-            float J = 1.f / (l_h - l_l);
-            if (layer == lo) J = -J;
-            *grad = J;
-        }
+        if (grad) *grad = layer == lo ? -inv : inv;
     }
     return f;
 }

@@ -1299,7 +1299,6 @@ template <int THREADS, bool COLLECT, bool STRICT>
 __global__ __launch_bounds__(THREADS, kWinMinWarps * 32 / THREADS) void window_kernel(const __grid_constant__ Geom g, FwdBuffers fb, int B, int chunk)
 {
     __shared__ uint32_t s_cnt[kWinMax];
-    __shared__ uint32_t s_base[COLLECT ? kWinMax : 1];
     __shared__ uint32_t s_tmp[2];
     const uint64_t keep = evict_last_policy();
     __shared__ uint8_t s_queue[THREADS / 32][32 * (TRIPS_MAX_LAYERS - 1)];
@@ -1350,10 +1349,7 @@ __global__ __launch_bounds__(THREADS, kWinMinWarps * 32 / THREADS) void window_k
                 {
                     const int pix = window_pixel(g, w, i);
                     if (COLLECT)
-                    {
-                        s_base[i] = (pix >= 0) ? atomicAdd(pixel_ctr + pix, c) : 0u;
-                        s_cnt[i]  = 0;
-                    }
+                        s_cnt[i] = pix >= 0 ? atomicAdd(pixel_ctr + pix, c) : 0u;  // from here on the pixel's next free slot
                     else if (pix >= 0)
                         atomicAdd(pixel_ctr + pix, c);
                 }
@@ -1381,16 +1377,16 @@ __global__ __launch_bounds__(THREADS, kWinMinWarps * 32 / THREADS) void window_k
                                                  return __float_as_uint(a);
                                              };
                                              // the four slots first, then the four stores: the shared-memory atomics do not wait for one another
-                                             const uint32_t s00 = s_base[li] + atomicAdd(s_cnt + li, 1u);
-                                             const uint32_t s10 = s_base[li + 1] + atomicAdd(s_cnt + li + 1, 1u);
-                                             const uint32_t s01 = s_base[li + ww] + atomicAdd(s_cnt + li + ww, 1u);
-                                             const uint32_t s11 = s_base[li + ww + 1] + atomicAdd(s_cnt + li + ww + 1, 1u);
+                                             const uint32_t s00 = atomicAdd(s_cnt + li, 1u);
+                                             const uint32_t s10 = atomicAdd(s_cnt + li + 1, 1u);
+                                             const uint32_t s01 = atomicAdd(s_cnt + li + ww, 1u);
+                                             const uint32_t s11 = atomicAdd(s_cnt + li + ww + 1, 1u);
                                              store_frag(frags + s00, make_uint4(pid, zb, alpha(dx0, dy0), ei), keep);
                                              store_frag(frags + s10, make_uint4(pid, zb, alpha(dx1, dy0), ei), keep);
                                              store_frag(frags + s01, make_uint4(pid, zb, alpha(dx0, dy1), ei), keep);
                                              store_frag(frags + s11, make_uint4(pid, zb, alpha(dx1, dy1), ei), keep);
                                          });
-                __syncthreads();  // the next bin of this chunk reuses s_cnt / s_base
+                __syncthreads();  // the next bin of this chunk reuses s_cnt
             }
         }
     }
