@@ -49,19 +49,21 @@ struct Geom
     int bins_x, bins_y, n_bins;         // 32x32 screen bins of layer 0
 };
 
-// Per-view constants built on the device from the pose / intrinsics tensors (setup_cams_kernel).
+// Per-view constants built on the device from the pose / intrinsics tensors (setup_cams_kernel).  First what the projection of a
+// point reads.
 struct CamConst
 {
-    float qx, qy, qz, qw, tx, ty, tz;
-    float R[9];
-    float fx, fy, cx, cy, s;
-    float cfx, cfy, ccx, ccy, cs;
+    float qx, qy, qz, qw;
+    float tx, ty, tz, s;
+    float fx, fy, cx, cy;
+    float cfx, cfy, ccx, ccy;
     float r00, r01, r10, r11;
-    float cenx, ceny;
+    float cenx, ceny, cs;
+    int dist;                              // apply the distortion and the cut-off radius
+    float R[9];
     int image_index, camera_index;
     float k1, k2, k3, k4, k5, k6, p1, p2;  // lens distortion (TripsRenderParams.distortion)
     float cut2;                            // dist_cutoff^2
-    int dist;                              // apply the distortion and the cut-off radius
 };
 
 struct LayerPtrs

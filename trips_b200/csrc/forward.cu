@@ -113,9 +113,12 @@ cudaError_t launch_setup_cams(const TripsView* h_views, int B, const double* pos
 // ------------------------------------------------------------------------------------------------------------
 struct Projected
 {
-    float u, v, z, ps, rad;
+    float u, v, z, ps;
     bool ok;
 };
+
+// radius of a point in pixels; read with drop_out_points_by_radius only
+__device__ __forceinline__ float projected_radius(const CamConst& cam, const float4& p, float z) { return cam.fx * cam.cfx * p.w / z; }
 
 // Visibility test of one point in one view (RenderForward.cu:224-340).  `sp` caches softplus(raw) across the views of
 // the point: negative = not computed yet (softplus is never negative); only visible points pay for it.
@@ -125,11 +128,14 @@ __device__ __forceinline__ Projected project_visible(const CamConst& cam, const 
     Projected r;
     const float fxc = cam.fx * cam.cfx;
     project_point(cam, p.x, p.y, p.z, r.u, r.v, r.z);
-    r.rad = fxc * p.w / r.z;
-    r.ps  = 0.f;
+    r.ps = 0.f;
     bool ok = !(r.z <= 0.f || r.u < 0.f || r.u >= (float)(g.W[0] - 1) || r.v < 0.f || r.v >= (float)(g.H[0] - 1));
     // the first pipeline's test takes an int (RenderForward.cu:212-218), the second's the float (RenderForward.cu:1527-1531)
-    if (ok && pr.drop_out_points_by_radius && (second_pipeline(pr) ? r.rad : (float)(int)r.rad) < pr.drop_out_radius_threshold) ok = false;
+    if (ok && pr.drop_out_points_by_radius)
+    {
+        const float rad = projected_radius(cam, p, r.z);
+        if ((second_pipeline(pr) ? rad : (float)(int)rad) < pr.drop_out_radius_threshold) ok = false;
+    }
     if (ok)
     {
         if (sp < 0.f) sp = tm_softplus(raw);
@@ -139,8 +145,16 @@ __device__ __forceinline__ Projected project_visible(const CamConst& cam, const 
     return r;
 }
 
+// A camera as the binning kernels hold it in shared memory: on 16 bytes, so that it is read four words at a time.  (For CamConst itself
+// the alignment costs point_grad_kernel registers: 753 -> 808 us on 20 M points in 2 views.)
+struct alignas(16) BinCam : CamConst
+{
+};
+static_assert(sizeof(BinCam) == sizeof(CamConst), "copied word by word");
+
 constexpr int kBinThreads     = 256;
 constexpr int kBinBlocksPerSM = 8;
+constexpr int kCountMinBlocks = 4;     // 64 registers; 5 blocks of 48: the same, uncapped 74 registers
 constexpr int kScatterMinBlocks = 4, kScatterMinBlocksWide = 3;  // up to 4 channels / more; measured at 3 / 4: 6 M points 1.26 / 1.23 ms (8 views), 0.346 / 0.313 ms (1 view); 8 channels 0.116 / 0.127 ms
 constexpr int kBinChunk       = 8192;  // points per bounding box
 constexpr int kBinTicket      = 1024;  // points per work ticket of the binning kernels; a ticket lies inside one box
@@ -315,34 +329,48 @@ struct PointHead
 
 // ACT: the scene tensors may be raw parameters (fused texture preparation); compiled separately so that the common case
 // carries none of its code.  One launch handles the views [v0, v0 + nv).
+// A thread takes four points at a time, so that a camera is read from shared memory (24 words) once for four projections and four
+// points are on their way from memory at once; the radius of a point is only computed where it is asked for.  Together with the
+// projections that wait in shared memory in the scatter pass and cameras read four words at a time: bin_points 1204 -> 1097 us (6 M
+// points x 8 views), 241 -> 206 (2 M x 4), 1733 -> 1660 (20 M x 2), 64 views of 10 M points 16.5 -> 15.4 ms.  Issue slots bound both
+// passes (57 and 69 % in use before).
 template <bool ACT>
-__global__ __launch_bounds__(kBinThreads) void bin_count_kernel(ScenePtrs sc, const CamConst* __restrict__ cams, const __grid_constant__ Geom g,
+__global__ __launch_bounds__(kBinThreads, kCountMinBlocks) void bin_count_kernel(ScenePtrs sc, const CamConst* __restrict__ cams, const __grid_constant__ Geom g,
                                                                 TripsRenderParams pr, FwdBuffers fb, int v0, int nv, unsigned* ticket)
 {
-    __shared__ CamConst s_cam[kViewGroup];
+    __shared__ BinCam s_cam[kViewGroup];
     __shared__ unsigned s_ticket;
     for (int k = threadIdx.x; k < nv * (int)(sizeof(CamConst) / 4); k += kBinThreads) ((int*)s_cam)[k] = ((const int*)(cams + v0))[k];
     const bool use_dropout = pr.train && sc.dropout;  // the mask applies with and without viewer_only (RenderForward.cu:224-240)
+    constexpr int kPoints = kBinTicket / kBinThreads;  // of a thread: a camera is read from shared memory once for all of them
     int first, last;
     unsigned skip;
     while (next_point_ticket(ticket, sc.N, &s_ticket, fb.block_skip, v0, nv, first, last, skip))
     {
-        PointHead nx;
-        nx.fetch(sc, first + threadIdx.x, last);
-        for (int i = first + threadIdx.x; i < last; i += kBinThreads)
+        float4 p[kPoints];
+        unsigned there = 0;
+#pragma unroll
+        for (int k = 0; k < kPoints; ++k)
         {
-            const PointHead h = nx;
-            nx.fetch(sc, i + kBinThreads, last);
-            if (discarded_for_confidence<ACT>(sc, pr, h.tex)) continue;
-            const float4 p  = h.p;
-            const float raw = h.raw;
-            float sp        = -1.f;
-            for (int v = 0; v < nv; ++v)
+            const int i = first + (int)threadIdx.x + k * kBinThreads;
+            p[k]        = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (i >= last) continue;
+            p[k] = __ldg(sc.position + i);
+            if (!(pr.viewer_only && discarded_for_confidence<ACT>(sc, pr, sc.index ? __ldg(sc.index + i) : i))) there |= 1u << k;
+        }
+        for (int v = 0; v < nv; ++v)
+        {
+            if ((skip >> v) & 1u) continue;  // uniform
+            const BinCam cam = s_cam[v];
+            uint32_t* counters = fb.bin_count + ((size_t)(v0 + v) * g.n_bins << kSubShift);
+#pragma unroll
+            for (int k = 0; k < kPoints; ++k)
             {
-                if ((skip >> v) & 1u) continue;  // uniform
-                if (use_dropout && __ldg(sc.dropout + (size_t)(v0 + v) * sc.N + i) == 1.f) continue;
-                const Projected r = project_visible(s_cam[v], g, pr, p, raw, sp);
-                if (r.ok) atomicAdd(fb.bin_count + ((size_t)(v0 + v) * g.n_bins << kSubShift) + bin_key(g, r.u, r.v), 1u);
+                if (!((there >> k) & 1u)) continue;
+                if (use_dropout && __ldg(sc.dropout + (size_t)(v0 + v) * sc.N + first + threadIdx.x + k * kBinThreads) == 1.f) continue;
+                float sp          = 0.f;  // (the size is not asked for)
+                const Projected r = project_visible(cam, g, pr, p[k], 0.f, sp);
+                if (r.ok) atomicAdd(counters + bin_key(g, r.u, r.v), 1u);
             }
         }
     }
@@ -480,7 +508,7 @@ __device__ __forceinline__ void fetch_point_row(const ScenePtrs& sc, const Trips
 
 // Writes entry `at` (index into the entry arrays) of point i as projected by `r`.
 template <int C>
-__device__ __forceinline__ void write_entry(const FwdBuffers& fb, const Geom& g, const TripsRenderParams& pr, unsigned long long at, int i,
+__device__ __forceinline__ void write_entry(const FwdBuffers& fb, const Geom& g, const TripsRenderParams& pr, const CamConst& cam, unsigned long long at, int i,
                                             const float4& p, float raw, const Projected& r, const PointRow<C>& d)
 {
     constexpr int TS = tail_stride(C);
@@ -500,7 +528,7 @@ __device__ __forceinline__ void write_entry(const FwdBuffers& fb, const Geom& g,
     const bool second = second_pipeline(pr);
     const float sc0   = __int_as_float((127 - first) << 23);  // 2^-first
     int layer = first;
-    float x = r.u * sc0, y = r.v * sc0, rad = r.rad * sc0;
+    float x = r.u * sc0, y = r.v * sc0, rad = pr.drop_out_points_by_radius ? projected_radius(cam, p, r.z) * sc0 : 0.f;
     for (; layer < hi + 1; ++layer, x *= 0.5f, y *= 0.5f, rad *= 0.5f)
     {
         const int px = __float2int_rd(x), py = __float2int_rd(y);
@@ -524,9 +552,10 @@ template <int C, bool ACT>
 __global__ __launch_bounds__(kBinThreads, (C <= 4 ? kScatterMinBlocks : kScatterMinBlocksWide)) void bin_scatter_kernel(ScenePtrs sc, const CamConst* __restrict__ cams, const __grid_constant__ Geom g,
                                                                   TripsRenderParams pr, FwdBuffers fb, int v0, int nv, unsigned* ticket)
 {
-    __shared__ CamConst s_cam[kViewGroup];
+    __shared__ BinCam s_cam[kViewGroup];
     __shared__ unsigned long long s_ebase[kViewGroup + 1];
     __shared__ unsigned s_ticket;
+    __shared__ float4 s_proj[kSweep][kBinThreads];  // u v z ps of the thread's visible views of a sweep
     for (int k = threadIdx.x; k < nv * (int)(sizeof(CamConst) / 4); k += kBinThreads) ((int*)s_cam)[k] = ((const int*)(cams + v0))[k];
     if (threadIdx.x <= nv) s_ebase[threadIdx.x] = fb.entry_base[v0 + threadIdx.x];
     __syncthreads();
@@ -558,9 +587,8 @@ __global__ __launch_bounds__(kBinThreads, (C <= 4 ? kScatterMinBlocks : kScatter
             if (fb.point_state && v0 == 0) fb.point_state[i] = make_float4(p.x, p.y, p.z, raw);
             float sp        = -1.f;
             // Views are handled kSweep at a time in two sweeps: the first projects and takes the entry slots (up to kSweep
-            // returning atomics in flight per thread instead of one), the second projects again (the same arithmetic,
-            // hence the same bits) and writes the entries.  Waiting for each slot before the next projection made the
-            // kernel latency-bound.
+            // returning atomics in flight per thread instead of one), the second writes the entries.  Waiting for each slot before
+            // the next projection made the kernel latency-bound.
             for (int vb = 0; vb < nv; vb += kSweep)
             {
                 uint32_t slot[kSweep];
@@ -575,6 +603,7 @@ __global__ __launch_bounds__(kBinThreads, (C <= 4 ? kScatterMinBlocks : kScatter
                     const Projected r = project_visible(s_cam[v], g, pr, p, raw, sp);
                     if (!r.ok) continue;
                     vis |= 1u << j;
+                    s_proj[j][threadIdx.x] = make_float4(r.u, r.v, r.z, r.ps);
                     slot[j] = atomicAdd(fb.bin_base + ((size_t)(v0 + v) * g.n_bins << kSubShift) + bin_key(g, r.u, r.v), 1u);
                 }
                 if (vis) fetch_point_row<C, ACT>(sc, pr, fb, i, d);  // travels with the slots
@@ -582,9 +611,11 @@ __global__ __launch_bounds__(kBinThreads, (C <= 4 ? kScatterMinBlocks : kScatter
                 for (int j = 0; j < kSweep; ++j)
                 {
                     if (!((vis >> j) & 1u)) continue;
-                    const int v       = vb + j;
-                    const Projected r = project_visible(s_cam[v], g, pr, p, raw, sp);
-                    write_entry<C>(fb, g, pr, s_ebase[v] + slot[j], i, p, raw, r, d);
+                    const int v     = vb + j;
+                    const float4 uv = s_proj[j][threadIdx.x];
+                    Projected r;
+                    r.u = uv.x, r.v = uv.y, r.z = uv.z, r.ps = uv.w, r.ok = true;
+                    write_entry<C>(fb, g, pr, s_cam[v], s_ebase[v] + slot[j], i, p, raw, r, d);
                 }
                 if (fb.note_entry)  // behind the entries: the slots are on their way while the points are projected again
 #pragma unroll
@@ -655,7 +686,7 @@ template <bool ACT>
 __global__ __launch_bounds__(kBinThreads) void bin_count_hot_kernel(ScenePtrs sc, const CamConst* __restrict__ cams, const __grid_constant__ Geom g,
                                                                     TripsRenderParams pr, FwdBuffers fb, int v0, int nv, unsigned* ticket)
 {
-    __shared__ CamConst s_cam[kViewGroup];
+    __shared__ BinCam s_cam[kViewGroup];
     __shared__ uint32_t s_tag[kHotSlots], s_cnt[kHotSlots];
     __shared__ unsigned s_ticket;
     for (int k = threadIdx.x; k < nv * (int)(sizeof(CamConst) / 4); k += kBinThreads) ((int*)s_cam)[k] = ((const int*)(cams + v0))[k];
@@ -697,7 +728,7 @@ template <int C, bool ACT>
 __global__ __launch_bounds__(kBinThreads) void bin_scatter_hot_kernel(ScenePtrs sc, const CamConst* __restrict__ cams, const __grid_constant__ Geom g,
                                                                       TripsRenderParams pr, FwdBuffers fb, int v0, int nv, unsigned* ticket)
 {
-    __shared__ CamConst s_cam[kViewGroup];
+    __shared__ BinCam s_cam[kViewGroup];
     __shared__ unsigned long long s_ebase[kViewGroup + 1];
     __shared__ uint32_t s_tag[kHotSlots], s_cnt[kHotSlots], s_base[kHotSlots];
     __shared__ unsigned s_ticket;
@@ -774,7 +805,7 @@ __global__ __launch_bounds__(kBinThreads) void bin_scatter_hot_kernel(ScenePtrs 
                 }
                 if (fb.note_entry) fb.note_entry[(size_t)(v0 + v) * sc.N + i] = slot;
                 if (slot == kNoEntry) continue;
-                write_entry<C>(fb, g, pr, s_ebase[v] + slot, i, p, raw, r, d);
+                write_entry<C>(fb, g, pr, s_cam[v], s_ebase[v] + slot, i, p, raw, r, d);
             }
         }
     }
