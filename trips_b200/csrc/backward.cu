@@ -60,20 +60,26 @@ constexpr int kBwdWarps   = kBwdThreads / 32;
 // at 16-20 resident warps per SM; DRAM is at 20-30 %.  Hence the care for lines per instruction (entries ordered by
 // tile, paired atomics, coalesced staging) and for instructions per fragment (fragment table, no shuffle searches).
 constexpr int kBwdBlocksPerSM = 12;  // grid size of the persistent kernel, in blocks per SM
-// Resident blocks, 4 / 5 / 6 (register caps 128 / 96 / 80), grid 12 blocks per SM at 5 and as many as are resident otherwise: 6 M points
-// x 8 views 3.66 / 3.11 / 2.97 ms, 20 M x 2 views 0.81 / 0.70 / 0.77, 1.3 M points with long lists x 5 views 0.56 / 0.49 / 0.62.
-constexpr int kBwdMinBlocks = 5;
+// Resident blocks.  Shared memory allows six; with six, 16 KB of L1 are left, with five 52 KB.  Where a tile's entries are few the sixth
+// block hides more latency, where they are many its rows no longer stay in L1 between the fragments of neighbouring pixels.
+// blend_backward, six / five blocks, us, by visible points per pixel of layer 0: 0.8 281 / 322, 1.5 (6 M points x 8 views) 2752 / 2904,
+// 1.65 206 / 209, 1.84 228 / 206, 2.05 499 / 469, 2.6 1094 / 978, 2.8 290 / 257, 3.65 718 / 586.  DENSE is the variant for more than
+// 1.75: the table of fragments is written by an unrolled loop, which takes 87 registers (4 channels) instead of 72 and thereby leaves room for
+// five blocks.
+constexpr int kBwdMinBlocks = 6, kBwdMinBlocksDense = 5;
+inline bool dense_entries(unsigned long long entries, const Geom& g, int B) { return 4 * entries > 7ull * g.W[0] * g.H[0] * B; }
 // SAT: saturated_alpha_accumulation as the reference's backward pass has it (RenderBackward.cu:227-259); a separate
 // instantiation, so that the common case carries none of its code or registers.
-template <int C, bool SAT>
-__global__ __launch_bounds__(kBwdThreads, (C <= 4 ? kBwdMinBlocks : 1)) void blend_backward_kernel(ScenePtrs sc, const CamConst* __restrict__ cams,
+template <int C, bool SAT, bool DENSE>
+__global__ __launch_bounds__(kBwdThreads, (C <= 4 ? (SAT || DENSE ? kBwdMinBlocksDense : kBwdMinBlocks) : 1)) void blend_backward_kernel(ScenePtrs sc, const CamConst* __restrict__ cams,
                                                                      const __grid_constant__ Geom g, TripsRenderParams pr, int B,
                                                                      FwdBuffers fb, BwdBuffers bb,
                                                                      const __grid_constant__ ConstLayerPtrs grad_in)
 {
     constexpr int DS = tail_stride(C);
     constexpr int GS = egrad_stride(C);
-    __shared__ float s_g[kBwdWarps][C][32];
+    constexpr int C4 = (C + 3) & ~3;
+    __shared__ float4 s_g[kBwdWarps][C4 / 4][32];  // image gradients of the tile's pixels, four channels together
     __shared__ float s_d[kBwdWarps][32 * kPad];   // G_j, then dA_j = G_j T_j, finally d_j
     __shared__ float s_sum[SAT ? kBwdWarps : 1][SAT ? 32 * kPad : 1];  // SAT: sum of the descriptor channels of fragment j
     __shared__ uint16_t s_map[kBwdWarps][32 * 16];
@@ -110,9 +116,9 @@ __global__ __launch_bounds__(kBwdThreads, (C <= 4 ? kBwdMinBlocks : 1)) void ble
         tile_pixel(g, (int)tile, lane, layer, gx, gy, p);
         const int gx0 = __shfl_sync(kFull, gx, 0), gy0 = __shfl_sync(kFull, gy, 0);  // tile origin: lane l is pixel (gx0 + (l & 7), gy0 + (l >> 3))
         int m = 0;
-        float gin[C];
+        float gin[C4];
 #pragma unroll
-        for (int c = 0; c < C; ++c) gin[c] = 0.f;
+        for (int c = 0; c < C4; ++c) gin[c] = 0.f;
         if (p >= 0)
         {
             m            = fb.rec_n[(size_t)ticket * 32 + lane];  // tickets run over the tiles of all views
@@ -122,10 +128,8 @@ __global__ __launch_bounds__(kBwdThreads, (C <= 4 ? kBwdMinBlocks : 1)) void ble
             for (int c = 0; c < C; ++c) gin[c] = __ldg(gi + (size_t)c * Hl * Wl);
         }
 #pragma unroll
-        for (int c = 0; c < C; ++c) s_g[warp][c][lane] = gin[c];
-        int m_max = m;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) m_max = max(m_max, __shfl_xor_sync(kFull, m_max, o));
+        for (int c = 0; c < C4; c += 4) s_g[warp][c / 4][lane] = make_float4(gin[c], gin[c + 1], gin[c + 2], gin[c + 3]);
+        const int m_max = (int)__reduce_max_sync(kFull, (unsigned)m);
         // lanes <-> kept fragments of the tile: exclusive prefix of the record counts
         int incl = m;
 #pragma unroll
@@ -152,9 +156,18 @@ __global__ __launch_bounds__(kBwdThreads, (C <= 4 ? kBwdMinBlocks : 1)) void ble
         // pixels' lanes replaces a binary search over warp shuffles in every round of both fragment phases
         {
             uint16_t* mp = s_map[warp] + rel;
+            if constexpr (DENSE)
+            {
 #pragma unroll
-            for (int j = 0; j < 16; ++j)
-                if (j < m) mp[j] = (uint16_t)((lane << 10) | (lane * kPad + j));
+                for (int j = 0; j < 16; ++j)
+                    if (j < m) mp[j] = (uint16_t)((lane << 10) | (lane * kPad + j));
+            }
+            else
+            {
+#pragma unroll 4
+                for (int j = 0; j < m_max; ++j)
+                    if (j < m) mp[j] = (uint16_t)((lane << 10) | (lane * kPad + j));
+            }
         }
         __syncwarp();
         auto locate = [&](int e, int& seg, int& slot) {
@@ -197,11 +210,11 @@ __global__ __launch_bounds__(kBwdThreads, (C <= 4 ? kBwdMinBlocks : 1)) void ble
 #pragma unroll
                     for (int c = 0; c < C; c += 4)
                     {
-                        const float4 v4 = row[c / 4];
-                        G += v4.x * s_g[warp][c][seg];
-                        if (c + 1 < C) G += v4.y * s_g[warp][c + 1][seg];
-                        if (c + 2 < C) G += v4.z * s_g[warp][c + 2][seg];
-                        if (c + 3 < C) G += v4.w * s_g[warp][c + 3][seg];
+                        const float4 v4 = row[c / 4], g4 = s_g[warp][c / 4][seg];
+                        G = fmaf(v4.x, g4.x, G);
+                        if (c + 1 < C) G = fmaf(v4.y, g4.y, G);
+                        if (c + 2 < C) G = fmaf(v4.z, g4.z, G);
+                        if (c + 3 < C) G = fmaf(v4.w, g4.w, G);
                     }
                     s_d[warp][j] = G;
                     if constexpr (SAT)
@@ -311,8 +324,8 @@ __global__ __launch_bounds__(kBwdThreads, (C <= 4 ? kBwdMinBlocks : 1)) void ble
                 const float a   = al[j];
                 const float dA  = my_d[j];
                 const float dem = 1.f / (1.f - a + 1e-9f);
-                my_d[j]         = dA - R * dem;
-                R += dA * a;
+                my_d[j]         = fmaf(-R, dem, dA);
+                R               = fmaf(dA, a, R);
             }
         }
         }
@@ -354,23 +367,27 @@ __global__ __launch_bounds__(kBwdThreads, (C <= 4 ? kBwdMinBlocks : 1)) void ble
                 const float fac = __int_as_float((127 - layer_s) << 23);
                 const float ux = e0v.x * fac, uy = e0v.y * fac;
                 const float ps = e0v.z;
-                const int q    = ((float)gx_s < ux ? 0 : 1) + ((float)gy_s < uy ? 0 : 2);
+                const bool nx = (float)gx_s < ux, ny = (float)gy_s < uy;  // the pixel is the near one of the two columns / rows
                 const float sx = ux - floorf(ux), sy = uy - floorf(uy);
-                float bf = ((q & 1) ? sx : (1.f - sx)) * ((q & 2) ? sy : (1.f - sy));
-                const float J0 = (q & 1) ? ((q & 2) ? sy : (1.f - sy)) : ((q & 2) ? -sy : (sy - 1.f));
-                const float J1 = (q & 2) ? ((q & 1) ? sx : (1.f - sx)) : ((q & 1) ? -sx : (sx - 1.f));
-                if (fabsf(ux - (float)gx_s) > 1.f || fabsf(uy - (float)gy_s) > 1.f) bf *= 0.f;
+                const float wx = nx ? 1.f - sx : sx, wy = ny ? 1.f - sy : sy;
+                float bf       = wx * wy;
+                if (pr.combine_lists && (fabsf(ux - (float)gx_s) > 1.f || fabsf(uy - (float)gy_s) > 1.f)) bf *= 0.f;  // (fragments of other layers only)
                 float lf_grad   = 0.f;
                 // (without use_layer_point_size the forward pass applied no layer factor: none here, and no size gradient)
                 const float lf  = pr.use_layer_point_size ? layer_factor<true>(ps, layer_s, g.L, &lf_grad) : 1.f;
                 const float gbs = conf * lf * ga;  // dLoss / d(bilinear weight) (RenderBackward.cu:385)
                 // image-space sums of the entry: the chain to position / size / pose is linear in them and is applied
                 // once per entry by point_grad_kernel
-                const float4 h0 = make_float4(J0 * gbs, J1 * gbs, bf * conf * lf_grad * ga, bf * lf * ga);
-                float gt[(C + 3) & ~3];
+                const float bg_a = bf * ga;
+                const float4 h0  = make_float4((nx ? -wy : wy) * gbs, (ny ? -wx : wx) * gbs, conf * lf_grad * bg_a, lf * bg_a);
+                float gt[C4];
 #pragma unroll
-                for (int c = 0; c < ((C + 3) & ~3); ++c) gt[c] = (c < C) ? w * s_g[warp][c < C ? c : 0][seg] : 0.f;
-                if constexpr (((C + 3) & ~3) == 4)
+                for (int c = 0; c < C4; c += 4)
+                {
+                    const float4 g4 = s_g[warp][c / 4][seg];
+                    gt[c] = w * g4.x, gt[c + 1] = w * g4.y, gt[c + 2] = w * g4.z, gt[c + 3] = w * g4.w;
+                }
+                if constexpr (C4 == 4)
                 {
                     // The row of an entry is 32 bytes: two 16-byte atomics.  Lanes work in pairs: the even lane adds the
                     // first half and the odd lane the second half of the SAME row (first the even lane's fragment, then
@@ -394,7 +411,7 @@ __global__ __launch_bounds__(kBwdThreads, (C <= 4 ? kBwdMinBlocks : 1)) void ble
                 {
                     float* eg = egrad + (size_t)eidx * GS;
                     atomicAdd(reinterpret_cast<float4*>(eg), h0);
-                    atomic_add_row<((C + 3) & ~3)>(eg + 4, gt);
+                    atomic_add_row<C4>(eg + 4, gt);
                 }
             }
         }
@@ -428,15 +445,17 @@ cudaError_t launch_zero_entry_rows(int C, int B, const FwdBuffers& fb, const Bwd
 
 cudaError_t launch_blend_backward(const ScenePtrs& sc, const CamConst* cams, const Geom& g, const TripsRenderParams& pr,
                                   int B, const FwdBuffers& fb, const BwdBuffers& bb, const ConstLayerPtrs& grad_in,
-                                  bool want_cam_grads, int sm_count, cudaStream_t st)
+                                  unsigned long long entries_hint, int sm_count, cudaStream_t st)
 {
     const int grid = (int)max(1u, min((unsigned)(sm_count * kBwdBlocksPerSM), ((unsigned)g.n_tiles * (unsigned)B + kBwdWarps - 1) / kBwdWarps));
 #define TRIPS_BWD_CASE(CC)                                                                                         \
     case CC:                                                                                                       \
         if (pr.saturated_alpha_accumulation)                                                                       \
-            blend_backward_kernel<CC, true><<<grid, kBwdThreads, 0, st>>>(sc, cams, g, pr, B, fb, bb, grad_in);   \
+            blend_backward_kernel<CC, true, false><<<grid, kBwdThreads, 0, st>>>(sc, cams, g, pr, B, fb, bb, grad_in);           \
+        else if (CC <= 4 && dense_entries(entries_hint, g, B))                                                     \
+            blend_backward_kernel<CC, false, (CC <= 4)><<<grid, kBwdThreads, 0, st>>>(sc, cams, g, pr, B, fb, bb, grad_in);      \
         else                                                                                                       \
-            blend_backward_kernel<CC, false><<<grid, kBwdThreads, 0, st>>>(sc, cams, g, pr, B, fb, bb, grad_in);  \
+            blend_backward_kernel<CC, false, false><<<grid, kBwdThreads, 0, st>>>(sc, cams, g, pr, B, fb, bb, grad_in);          \
         break;
     switch (sc.C)
     {

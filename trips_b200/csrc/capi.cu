@@ -648,7 +648,7 @@ int trips_backward(TripsContext* ctx, const TripsScene* scene, const float* cons
     for (int l = 0; l < g.L; ++l) gin.p[l] = grad_layers[l];
     const bool cam_grads = grads->pose_tangent || grads->intrinsics;
     STAGE(ctx, TRIPS_STAGE_BACKWARD, 1, st,
-          launch_blend_backward(sp, (const CamConst*)ctx->cams.p, g, ctx->params, B, fb, bb, gin, cam_grads, ctx->sm_count, st));
+          launch_blend_backward(sp, (const CamConst*)ctx->cams.p, g, ctx->params, B, fb, bb, gin, ctx->need_entries, ctx->sm_count, st));
     const int n_unpack = (N > 0 ? unpack_launches(B, fb.entry_views) + (cam_grads ? 1 : 0) : 0) + 1;
     STAGE(ctx, TRIPS_STAGE_UNPACK, n_unpack, st,
           launch_unpack_grads(sp, (const CamConst*)ctx->cams.p, B, fb, bb, *grads, ctx->params, ctx->sm_count, st));

@@ -421,7 +421,7 @@ cudaError_t launch_sort_blend(const ScenePtrs& sc, const Geom& g, const TripsRen
 cudaError_t launch_zero_entry_rows(int C, int B, const FwdBuffers& fb, const BwdBuffers& bb, int sm_count, cudaStream_t st);
 cudaError_t launch_blend_backward(const ScenePtrs& sc, const CamConst* cams, const Geom& g, const TripsRenderParams& pr,
                                   int B, const FwdBuffers& fb, const BwdBuffers& bb, const ConstLayerPtrs& grad_in,
-                                  bool want_cam_grads, int sm_count, cudaStream_t st);
+                                  unsigned long long entries_hint, int sm_count, cudaStream_t st);
 int unpack_launches(int B, int entry_views);  // launches of the point gradients
 cudaError_t launch_unpack_grads(const ScenePtrs& sc, const CamConst* cams, int B, const FwdBuffers& fb, const BwdBuffers& bb,
                                 const TripsGrads& out, const TripsRenderParams& pr, int sm_count, cudaStream_t st);
