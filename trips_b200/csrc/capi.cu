@@ -120,7 +120,7 @@ struct TripsContext
     int sm_count = 148;
     std::string error;
     // forward scratch
-    DevBuf heavy, cams, zeroed, bin_base, view_total, bin_cursor, entry_base, entries, offsets, partial, view_base, frags, rec_n, records, stats, point_entry, point_state, resize_scratch, block_box, block_skip;
+    DevBuf heavy, cams, zeroed, bin_base, view_total, bin_cursor, entry_base, entries, offsets, view_base, frags, rec_n, records, stats, point_entry, point_state, resize_scratch, block_skip;
     size_t zero_bins = 0, zero_counts = 0;  // where bin_count and counts start inside `zeroed` (behind the work counters)
     // backward scratch
     DevBuf egrad, g_small;
@@ -141,7 +141,6 @@ struct TripsContext
     Geom geom{};
     TripsRenderParams params{};
     int B = 0, N = 0, n_tex = 0, C = 0;
-    int nchunks = 0;
     size_t entry_cap = 0;                  // entries the two entry arrays (head | tail, in this order) are laid out for
     TripsStats host_stats{};
 };
@@ -237,7 +236,6 @@ static FwdBuffers fwd_buffers(TripsContext* c, int B)
     fb.ent_tail   = (float*)c->entries.p + 8 * c->entry_cap;
     fb.counts     = (uint32_t*)((char*)c->zeroed.p + c->zero_counts);
     fb.offsets    = (uint32_t*)c->offsets.p;
-    fb.partial    = (uint32_t*)c->partial.p;
     fb.view_base  = (unsigned long long*)c->view_base.p;
     fb.frags      = (uint4*)c->frags.p;
     fb.frag_cap   = c->frags.bytes / sizeof(uint4);
@@ -248,11 +246,12 @@ static FwdBuffers fwd_buffers(TripsContext* c, int B)
     fb.ticket_count   = fb.ticket + ticket_groups(B);
     fb.ticket_collect = fb.ticket_count + B;
     fb.ticket_blend   = fb.ticket + blend_ticket_at(B);
+    fb.finished       = fb.ticket_blend + 32;  // on another line than the blend's counter
+    fb.list_cursor    = fb.finished + 2;
     fb.point_entry = c->params.train ? (uint32_t*)c->point_entry.p : nullptr;
     fb.entry_views = entry_views(B, c->N);
     fb.note_entry  = fb.entry_views == B ? fb.point_entry : nullptr;
     fb.point_state = c->params.train ? (float4*)c->point_state.p : nullptr;
-    fb.block_box  = (const float*)c->block_box.p;
     fb.block_skip = (const uint8_t*)c->block_skip.p;
     fb.heavy      = heavy_lists(c->N, c->geom.L, B, c->heavy.p);
     return fb;
@@ -311,8 +310,8 @@ void trips_context_destroy(TripsContext* c)
 {
     if (!c) return;
     DevBuf* all[] = {&c->heavy, &c->cams, &c->zeroed, &c->bin_base, &c->view_total, &c->bin_cursor, &c->entry_base, &c->entries, &c->offsets,
-                     &c->partial, &c->view_base, &c->frags, &c->rec_n, &c->records, &c->stats, &c->egrad,
-                     &c->point_entry, &c->point_state, &c->g_small, &c->adam_tab, &c->resize_scratch, &c->block_box, &c->block_skip};
+                     &c->view_base, &c->frags, &c->rec_n, &c->records, &c->stats, &c->egrad,
+                     &c->point_entry, &c->point_state, &c->g_small, &c->adam_tab, &c->resize_scratch, &c->block_skip};
     for (DevBuf* b : all) free_buf(*b);
     c->timers.destroy();
     if (c->h_pinned) cudaFreeHost(c->h_pinned);
@@ -418,13 +417,12 @@ static int forward_views(TripsContext* ctx, const TripsScene* scene, const Trips
     const size_t N    = (size_t)scene->n_points;
     const size_t P    = (size_t)g.P;
     const int C       = scene->channels;
-    const int nchunks = (int)((P + kScanChunk - 1) / kScanChunk);
     const size_t n_box = (N + 8191) / 8192 + 1;
 
     CU_CHECK(ctx, ensure(ctx->cams, sizeof(CamConst) * B));
     // everything a pass wants zeroed, in one buffer and one clear: work counters | visible points per (bin, 8x4 tile of the bin) | list lengths
     auto aligned      = [](size_t n) { return (n + 255) & ~(size_t)255; };
-    ctx->zero_bins    = aligned(sizeof(unsigned) * (blend_ticket_at(B) + 1));
+    ctx->zero_bins    = aligned(sizeof(unsigned) * (blend_ticket_at(B) + 32 + B + 2));
     ctx->zero_counts  = ctx->zero_bins + aligned(sizeof(uint32_t) * (size_t)g.n_bins * 32 * B);
     const size_t zero_bytes = ctx->zero_counts + sizeof(uint32_t) * P * B;
     CU_CHECK(ctx, ensure(ctx->zeroed, zero_bytes));
@@ -432,11 +430,9 @@ static int forward_views(TripsContext* ctx, const TripsScene* scene, const Trips
     CU_CHECK(ctx, ensure(ctx->view_total, sizeof(uint32_t) * B));
     CU_CHECK(ctx, ensure(ctx->bin_cursor, sizeof(uint32_t) * (size_t)g.n_bins * B));
     CU_CHECK(ctx, ensure(ctx->entry_base, sizeof(unsigned long long) * (B + 1)));
-    CU_CHECK(ctx, ensure(ctx->block_box, sizeof(float) * 6 * n_box));
     CU_CHECK(ctx, ensure(ctx->block_skip, (size_t)B * n_box));
     CU_CHECK(ctx, ensure(ctx->heavy, heavy_bytes(heavy_lists((int)N, g.L, B, nullptr))));
     CU_CHECK(ctx, ensure(ctx->offsets, sizeof(uint32_t) * P * B));
-    CU_CHECK(ctx, ensure(ctx->partial, sizeof(uint32_t) * (size_t)nchunks * B));
     CU_CHECK(ctx, ensure(ctx->view_base, sizeof(unsigned long long) * (B + 1)));
     CU_CHECK(ctx, ensure_stats(ctx, st));
     if (params->train)
@@ -479,7 +475,7 @@ static int forward_views(TripsContext* ctx, const TripsScene* scene, const Trips
     {
         FwdBuffers fscan = fb;
         if (wait_for_sizes) fscan.frag_cap = ~0ull;  // sizing pass: the list buffer is grown below, nothing can overflow yet
-        STAGE(ctx, TRIPS_STAGE_SCAN, 3, st, launch_scan(g, B, params->k_keep, fscan, nchunks, st));
+        STAGE(ctx, TRIPS_STAGE_SCAN, 1, st, launch_list_starts(g, B, params->k_keep, fscan, st));
     }
     CU_CHECK(ctx, cudaMemcpyAsync(h_stats, ctx->stats.p, sizeof(DevStats), cudaMemcpyDeviceToHost, st));
     if (wait_for_sizes)
@@ -514,7 +510,6 @@ static int forward_views(TripsContext* ctx, const TripsScene* scene, const Trips
             return e != cudaSuccess ? e : launch_sort_blend(sp, g, *params, B, fb, out, ctx->sm_count, st);
         }());
     ctx->B       = B;
-    ctx->nchunks = nchunks;
     return TRIPS_OK;
 }
 
@@ -902,17 +897,26 @@ int trips_debug_lists(TripsContext* ctx, int view, int32_t* counts, int64_t* off
     CU_CHECK(ctx, cudaStreamSynchronize(st));
     const unsigned long long nf = vb[1] - vb[0];
     if (n_frags) *n_frags = (int64_t)nf;
+    // the lists lie in the buffer in the order in which their blocks came; here they follow one another in pixel order
+    int64_t next = 0;
     for (size_t i = 0; i < P; ++i)
     {
         if (counts) counts[i] = (int32_t)c[i];
-        if (offsets) offsets[i] = (int64_t)e[i] - (int64_t)c[i];  // the collect pass advanced the offsets to the list ends
+        if (offsets) offsets[i] = next;
+        next += c[i];
     }
     if (frags && nf)
     {
         std::vector<uint4> f(nf);
         CU_CHECK(ctx, cudaMemcpyAsync(f.data(), (uint4*)ctx->frags.p + vb[0], sizeof(uint4) * nf, cudaMemcpyDeviceToHost, st));
         CU_CHECK(ctx, cudaStreamSynchronize(st));
-        for (unsigned long long i = 0; i < nf; ++i) frags[i] = ((uint64_t)f[i].y << 32) | f[i].x;
+        size_t n = 0;
+        for (size_t i = 0; i < P; ++i)
+        {
+            const size_t first = (size_t)e[i] - c[i];  // the collect pass advanced the starts to the list ends
+            for (size_t k = 0; k < c[i] && n < nf; ++k)
+                if (first + k < nf) frags[n++] = ((uint64_t)f[first + k].y << 32) | f[first + k].x;
+        }
     }
     return TRIPS_OK;
 }

@@ -123,8 +123,7 @@ struct FwdBuffers
     float4* ent_head;                 // [sum V_b, 2]
     float* ent_tail;                  // [sum V_b, tail_stride]
     uint32_t* counts;                 // [B,P] list lengths
-    uint32_t* offsets;                // [B,P] list start within the view (list end after the collect pass)
-    uint32_t* partial;                // [B,nchunks] scan partials
+    uint32_t* offsets;                // [B,P] list start within the view, the lists in no particular order (list end after the collect pass)
     unsigned long long* view_base;    // [B+1] first fragment of each view in `frags`
     uint4* frags;                     // [frag_cap] x = point id, y = depth bits (y:x = 64-bit sort key), z = alpha bits, w = entry index within the view
     unsigned long long frag_cap;
@@ -137,12 +136,13 @@ struct FwdBuffers
     unsigned int* ticket_count;       // [B] count pass
     unsigned int* ticket_collect;     // [B] collect pass
     unsigned int* ticket_blend;
+    unsigned int* finished;           // [2] blocks that are done, of the bin scan and of list_starts_kernel
+    uint32_t* list_cursor;            // [B] fragments of the views as list_starts_kernel adds them up
     uint32_t* point_entry;            // training: [entry_views,N] entry (within the view) of every point, kNoEntry where it is not visible
     int entry_views;                  // B, or fewer where the table of all views would be larger than kEntryTableBytes: the backward
                                       // pass then fills it for so many views at a time
     uint32_t* note_entry;             // point_entry where the binning pass notes the entries of all views, else nullptr
     float4* point_state;              // training: [N] position and raw size of the points that were not discarded, as this pass saw them
-    const float* block_box;           // [ceil(N / 8192), 6] bounding boxes (min xyz, max xyz) of blocks of consecutive points
     const uint8_t* block_skip;        // [B, ceil(N / 8192)] 1 = the block cannot hold a point visible in that view
     HeavyLists heavy;
 };
@@ -405,7 +405,7 @@ int bin_scatter_launches(int N, int B);
 size_t resize_scratch_bytes(int64_t n_points);
 cudaError_t launch_resize_points(const int64_t* remove, int64_t n_remove, int64_t n_points, int64_t n_new, const TripsPointTensor* tensors,
                                  int n_tensors, void* scratch, DevStats* stats, int sm_count, cudaStream_t st);
-cudaError_t launch_scan(const Geom& g, int B, int k_keep, const FwdBuffers& fb, int nchunks, cudaStream_t st);
+cudaError_t launch_list_starts(const Geom& g, int B, int k_keep, const FwdBuffers& fb, cudaStream_t st);
 // strict: an entry's layers start at the layer below log2(size) instead of layer 0 (strict_layers above)
 // entries_hint: the number of entries of the call as far as the host knows it (selects the size of the work tickets)
 cudaError_t launch_count(const ScenePtrs& sc, const Geom& g, int B, const FwdBuffers& fb, bool strict, unsigned long long entries_hint, int sm_count,
@@ -443,6 +443,11 @@ struct L1Args
     int L;
 };
 cudaError_t launch_l1_loss(const L1Args& a, int64_t total, double* loss_out, int sm_count, cudaStream_t st);
-constexpr int kScanChunk    = 2048;
+// Pixels whose lists a block of list_starts_kernel places one after another.  Blocks come in any order: the smaller the ranges, the more
+// places of the list buffer the passes behind it work on at a time.  scan / collect / sort_blend, us, of 2048 / 4096 / 8192 / 16384 pixels:
+// 6 M points x 8 views 83 / 52 / 58 / 70, 1227 / 1209 / 1201 / 1191, 2287 / 2305 / 2300 / 2288 (chunk totals scanned in pixel order: 130 for
+// the scan), 64 views of 10 M points 697 / 429 / 484 / 554, - / 14907 / 14770 / 14558, 22617 / 22814 / 22767 / 22590.
+constexpr int kScanThreads = 1024, kScanPerLane = 16;
+constexpr int kScanChunk   = kScanThreads * kScanPerLane;
 constexpr int kAdamPerBlock = 1024 * 4;  // elements handled by one Adam block
 }  // namespace trips

@@ -2,7 +2,7 @@
 //
 // Stage map to the reference (src/lib/rendering/RenderForward.cu):
 //   bin_count / bin_scan / bin_scatter kernels <- CountAndCollectTiled (:168-366)
-//   scan_*_kernel         <- cub::DeviceScan + host glue (:1155-1232), here one device-side scan per view, no host sync
+//   list_starts_kernel    <- cub::DeviceScan + host glue (:1155-1232), no host sync
 //   collect_kernel        <- SplattingPass               (:368-436)
 //   sort_blend_kernel     <- FastSortFusedNew            (:474-1059)
 // All views of a call are processed by one launch per stage (grid.y / ticket space spans the batch).
@@ -161,55 +161,6 @@ constexpr int kBinTicket      = 1024;  // points per work ticket of the binning 
 constexpr int kSweep          = 4;     // views whose entry slots a thread requests before it waits for any of them
 static_assert(kBinChunk % kBinTicket == 0, "a ticket must not straddle two bounding boxes");
 
-// Bounding boxes of blocks of consecutive points and the conservative frustum test on them: the reference computes
-// such boxes per 10 240 points (NeuralPointCloudCuda.cpp:339-384) but never uses them.  Point clouds stored in a
-// spatially coherent order (scans, reconstructions) have compact blocks, and a block whose box lies outside a view
-// is skipped by both binning passes; for a cloud in random order every box spans the scene and nothing is skipped.
-// Boxes are recomputed by every forward pass (points move): one read of the positions.
-__global__ __launch_bounds__(256) void block_box_kernel(const float4* __restrict__ pos, int N, float* __restrict__ boxes)
-{
-    const int first = blockIdx.x * kBinChunk, last = min(N, first + kBinChunk);
-    float lo[3] = {3.0e38f, 3.0e38f, 3.0e38f}, hi[3] = {-3.0e38f, -3.0e38f, -3.0e38f};
-    bool bad = false;
-    for (int i = first + threadIdx.x; i < last; i += 256)
-    {
-        const float4 p = pos[i];
-        const float v[3] = {p.x, p.y, p.z};
-#pragma unroll
-        for (int k = 0; k < 3; ++k)
-        {
-            bad |= !(fabsf(v[k]) < 3.0e38f);  // NaN or infinite: the block is never skipped
-            lo[k] = fminf(lo[k], v[k]);
-            hi[k] = fmaxf(hi[k], v[k]);
-        }
-    }
-    __shared__ float s_lo[8][3], s_hi[8][3];
-    __shared__ int s_bad;
-    if (threadIdx.x == 0) s_bad = 0;
-    __syncthreads();
-    if (bad) s_bad = 1;
-#pragma unroll
-    for (int k = 0; k < 3; ++k)
-    {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-        {
-            lo[k] = fminf(lo[k], __shfl_xor_sync(kFull, lo[k], o));
-            hi[k] = fmaxf(hi[k], __shfl_xor_sync(kFull, hi[k], o));
-        }
-        if ((threadIdx.x & 31) == 0) s_lo[threadIdx.x >> 5][k] = lo[k], s_hi[threadIdx.x >> 5][k] = hi[k];
-    }
-    __syncthreads();
-    if (threadIdx.x < 3)
-    {
-        float a = s_lo[0][threadIdx.x], b = s_hi[0][threadIdx.x];
-        for (int w = 1; w < 8; ++w) a = fminf(a, s_lo[w][threadIdx.x]), b = fmaxf(b, s_hi[w][threadIdx.x]);
-        if (s_bad) a = -3.4e38f, b = 3.4e38f;
-        boxes[(size_t)blockIdx.x * 6 + threadIdx.x]     = a;
-        boxes[(size_t)blockIdx.x * 6 + 3 + threadIdx.x] = b;
-    }
-}
-
 // True when no point inside the box can pass the visibility test of project_visible for this view.  The image position
 // is an affine map of (x/z, y/z); multiplied by z > 0 every image border becomes a plane through the camera centre,
 // i.e. a linear function of the view-space position, and a box lies outside a plane when its 8 corners do.  The borders
@@ -251,19 +202,63 @@ __device__ __forceinline__ bool box_outside_view(const CamConst& c, const Geom& 
     return all_behind || all_left || all_right || all_up || all_down;
 }
 
-// skip[b * n_blocks + k] = 1 when block k of the point cloud cannot hold a point visible in view b.  A kernel of its
-// own: inside the binning kernels the test would cost their loops 30 registers.
-__global__ __launch_bounds__(128) void block_visibility_kernel(const CamConst* __restrict__ cams, const __grid_constant__ Geom g, int B,
-                                                               int n_blocks, const float* __restrict__ boxes, uint8_t* __restrict__ skip,
-                                                               DevStats* stats)
+// Bounding boxes of blocks of consecutive points and the conservative frustum test on them: the reference computes
+// such boxes per 10 240 points (NeuralPointCloudCuda.cpp:339-384) but never uses them.  Point clouds stored in a
+// spatially coherent order (scans, reconstructions) have compact blocks, and a block whose box lies outside a view
+// is skipped by both binning passes; for a cloud in random order every box spans the scene and nothing is skipped.
+// Boxes are recomputed by every forward pass (points move): one read of the positions.  skip[b * n_blocks + k] = 1 when block k of
+// the point cloud cannot hold a point visible in view b (a test inside the binning kernels would cost their loops 30
+// registers).
+__global__ __launch_bounds__(256) void block_visibility_kernel(const float4* __restrict__ pos, int N, const CamConst* __restrict__ cams,
+                                                               const __grid_constant__ Geom g, int B, uint8_t* __restrict__ skip, DevStats* stats)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= B * n_blocks) return;
-    const int b = i / n_blocks, k = i - b * n_blocks;
-    const CamConst cam = cams[b];
-    const bool out = box_outside_view(cam, g, boxes + (size_t)k * 6);
-    skip[i] = out ? 1 : 0;
-    if (out) atomicAdd(&stats->culled_blocks, 1u);
+    const int first = blockIdx.x * kBinChunk, last = min(N, first + kBinChunk);
+    float lo[3] = {3.0e38f, 3.0e38f, 3.0e38f}, hi[3] = {-3.0e38f, -3.0e38f, -3.0e38f};
+    bool bad = false;
+    for (int i = first + threadIdx.x; i < last; i += 256)
+    {
+        const float4 p = pos[i];
+        const float v[3] = {p.x, p.y, p.z};
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+        {
+            bad |= !(fabsf(v[k]) < 3.0e38f);  // NaN or infinite: the block is never skipped
+            lo[k] = fminf(lo[k], v[k]);
+            hi[k] = fmaxf(hi[k], v[k]);
+        }
+    }
+    __shared__ float s_lo[8][3], s_hi[8][3], s_box[6];
+    __shared__ int s_bad;
+    if (threadIdx.x == 0) s_bad = 0;
+    __syncthreads();
+    if (bad) s_bad = 1;
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+    {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+        {
+            lo[k] = fminf(lo[k], __shfl_xor_sync(kFull, lo[k], o));
+            hi[k] = fmaxf(hi[k], __shfl_xor_sync(kFull, hi[k], o));
+        }
+        if ((threadIdx.x & 31) == 0) s_lo[threadIdx.x >> 5][k] = lo[k], s_hi[threadIdx.x >> 5][k] = hi[k];
+    }
+    __syncthreads();
+    if (threadIdx.x < 3)
+    {
+        float a = s_lo[0][threadIdx.x], b = s_hi[0][threadIdx.x];
+        for (int w = 1; w < 8; ++w) a = fminf(a, s_lo[w][threadIdx.x]), b = fmaxf(b, s_hi[w][threadIdx.x]);
+        if (s_bad) a = -3.4e38f, b = 3.4e38f;
+        s_box[threadIdx.x] = a, s_box[3 + threadIdx.x] = b;
+    }
+    __syncthreads();
+    for (int b = threadIdx.x; b < B; b += 256)
+    {
+        const CamConst cam = cams[b];
+        const bool out     = box_outside_view(cam, g, s_box);
+        skip[(size_t)b * gridDim.x + blockIdx.x] = out ? 1 : 0;
+        if (out) atomicAdd(&stats->culled_blocks, 1u);
+    }
 }
 
 // Work distribution of the binning kernels: tickets of kBinTicket consecutive points from one counter, so that every SM
@@ -382,8 +377,42 @@ __global__ __launch_bounds__(kBinThreads, kCountMinBlocks) void bin_count_kernel
 // 64 of them, each two dependent loads and three barriers long.
 // Measured on a 1080p view: 90 us with one key per thread and turn; sixteen take the whole binning stage from 0.326 to 0.270 ms.
 constexpr int kScanKeys = 16;
+
+// One of `n` blocks that end with this call: true in all threads of the last one, which then sees what the others wrote before it.
+__device__ __forceinline__ bool last_block(unsigned* finished, unsigned n)
+{
+    __shared__ unsigned s_last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atomicAdd(finished, 1u) == n - 1 ? 1u : 0u;
+    __syncthreads();
+    if (s_last) __threadfence();
+    return s_last != 0;
+}
+
+// First entry of every view in the entry arrays.  A view whose entries do not fit the arrays (entry_cap entries: the
+// arrays are sized from the previous call's count, not for the worst case) gets none: it renders as background, the
+// status word says so and stats->visible still carries the number that was needed, so that the host grows the arrays.
+__device__ __forceinline__ void first_entries(const uint32_t* view_total, int B, unsigned long long entry_cap, unsigned long long* entry_base, DevStats* stats)
+{
+    unsigned long long base = 0, need = 0;
+    for (int b = 0; b < B; ++b)
+    {
+        const uint32_t n = __ldcg(view_total + b);
+        entry_base[b]    = base;
+        need += n;
+        if (base + n <= entry_cap)
+            base += n;
+        else
+            atomicOr(&stats->status, TRIPS_DEV_ENTRY_OVERFLOW);
+    }
+    entry_base[B]  = base;
+    stats->visible = need;
+}
+
 __global__ __launch_bounds__(1024) void bin_scan_kernel(const uint32_t* __restrict__ counts, uint32_t* __restrict__ key_first,
-                                                        uint32_t* __restrict__ bin_first, int n_keys, uint32_t* __restrict__ view_total, DevStats* stats)
+                                                        uint32_t* __restrict__ bin_first, int n_keys, uint32_t* view_total, unsigned long long entry_cap,
+                                                        unsigned long long* __restrict__ entry_base, unsigned* finished, DevStats* stats)
 {
     __shared__ uint32_t sm[32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -437,27 +466,7 @@ __global__ __launch_bounds__(1024) void bin_scan_kernel(const uint32_t* __restri
         __syncthreads();  // the warp sums are overwritten by the next turn
     }
     if (threadIdx.x == 0) view_total[b] = carry;
-}
-
-// First entry of every view in the entry arrays.  A view whose entries do not fit the arrays (entry_cap entries: the
-// arrays are sized from the previous call's count, not for the worst case) gets none: it renders as background, the
-// status word says so and stats->visible still carries the number that was needed, so that the host grows the arrays.
-__global__ void entry_base_kernel(const uint32_t* __restrict__ view_total, int B, unsigned long long entry_cap,
-                                  unsigned long long* __restrict__ entry_base, DevStats* stats)
-{
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    unsigned long long base = 0, need = 0;
-    for (int b = 0; b < B; ++b)
-    {
-        entry_base[b] = base;
-        need += view_total[b];
-        if (base + view_total[b] <= entry_cap)
-            base += view_total[b];
-        else
-            atomicOr(&stats->status, TRIPS_DEV_ENTRY_OVERFLOW);
-    }
-    entry_base[B]  = base;
-    stats->visible = need;
+    if (last_block(finished, gridDim.x) && threadIdx.x == 0) first_entries(view_total, (int)gridDim.x, entry_cap, entry_base, stats);
 }
 
 // One 32-byte store (sm_100 has 256-bit global stores) for the two float4 halves of a 32-byte-aligned record: half the
@@ -819,12 +828,8 @@ cudaError_t launch_bin_count(const ScenePtrs& sc, const CamConst* cams, const Ge
     const int n_keys   = g.n_bins << kSubShift;
     const int grid     = sm_count * kBinBlocksPerSM;
     const int n_groups = (B + kViewGroup - 1) / kViewGroup;
-    if (sc.N > 0 && fb.block_box && fb.block_skip)
-    {
-        const int nbk = (sc.N + kBinChunk - 1) / kBinChunk;
-        block_box_kernel<<<nbk, 256, 0, st>>>(sc.position, sc.N, const_cast<float*>(fb.block_box));
-        block_visibility_kernel<<<(B * nbk + 127) / 128, 128, 0, st>>>(cams, g, B, nbk, fb.block_box, const_cast<uint8_t*>(fb.block_skip), fb.stats);
-    }
+    if (sc.N > 0 && fb.block_skip)
+        block_visibility_kernel<<<(sc.N + kBinChunk - 1) / kBinChunk, 256, 0, st>>>(sc.position, sc.N, cams, g, B, const_cast<uint8_t*>(fb.block_skip), fb.stats);
     const bool act = pr.confidence_is_raw || pr.texture_abs;
     if (sc.N > 0)
         for (int gi = 0; gi < n_groups; ++gi)
@@ -839,12 +844,11 @@ cudaError_t launch_bin_count(const ScenePtrs& sc, const CamConst* cams, const Ge
             else
                 bin_count_kernel<false><<<grid, kBinThreads, 0, st>>>(sc, cams, g, pr, fb, v0, nv, fb.ticket + gi);
         }
-    bin_scan_kernel<<<B, 1024, 0, st>>>(fb.bin_count, fb.bin_base, fb.bin_cursor, n_keys, fb.view_total, fb.stats);
-    entry_base_kernel<<<1, 32, 0, st>>>(fb.view_total, B, entry_cap, fb.entry_base, fb.stats);
+    bin_scan_kernel<<<B, 1024, 0, st>>>(fb.bin_count, fb.bin_base, fb.bin_cursor, n_keys, fb.view_total, entry_cap, fb.entry_base, fb.finished, fb.stats);
     return cudaGetLastError();
 }
 
-int bin_count_launches(int N, int B) { return 2 + (N > 0 ? 2 + (B + kViewGroup - 1) / kViewGroup : 0); }
+int bin_count_launches(int N, int B) { return 1 + (N > 0 ? 1 + (B + kViewGroup - 1) / kViewGroup : 0); }
 int bin_scatter_launches(int N, int B) { return N > 0 ? (B + kViewGroup - 1) / kViewGroup : 0; }
 
 // Scatter pass of the binning stage: writes the entries (the arrays must hold fb.entry_base[B] entries).
@@ -885,7 +889,9 @@ cudaError_t launch_bin_scatter(const ScenePtrs& sc, const CamConst* cams, const 
 }
 
 // ------------------------------------------------------------------------------------------------------------
-// exclusive scan of the list lengths of every view (three small kernels, no spin-waits)
+// list starts.  The lists of a view need not follow one another in pixel order: a block scans the lengths of kScanChunk consecutive
+// pixels and takes a range of the view's list buffer for them from the view's counter.  One pass over the lengths and one
+// kernel; chunk totals, their scan and a second pass over the lengths, which this replaces, were three.
 // ------------------------------------------------------------------------------------------------------------
 __device__ __forceinline__ uint32_t warp_incl_scan(uint32_t v, int lane)
 {
@@ -898,34 +904,23 @@ __device__ __forceinline__ uint32_t warp_incl_scan(uint32_t v, int lane)
     return v;
 }
 
-// block of 256 threads: exclusive scan of one value per thread, returns the block total through `total`
-__device__ __forceinline__ uint32_t block_excl_scan_256(uint32_t v, uint32_t* smem /*[8]*/, uint32_t& total)
+// A warp takes 32 consecutive lengths at a time, kScanPerLane times: the lists of neighbouring pixels are neighbours.
+// cursor: [B] fragments of the views so far, zero before; finished: blocks that are done, zero before.
+__global__ __launch_bounds__(kScanThreads) void list_starts_kernel(const uint32_t* __restrict__ counts, int P, int k_keep, uint32_t* __restrict__ offsets, uint32_t* cursor,
+                                                                   unsigned* finished, unsigned long long* __restrict__ view_base, unsigned long long frag_cap,
+                                                                   DevStats* stats, HeavyLists heavy)
 {
+    __shared__ uint32_t s_warp[kScanThreads / 32], s_kept[kScanThreads / 32], s_most[kScanThreads / 32], s_base;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint32_t inc   = warp_incl_scan(v, lane);
-    if (lane == 31) smem[warp] = inc;
-    __syncthreads();
-    uint32_t wsum = (lane < 8) ? smem[lane] : 0;
-    uint32_t winc = warp_incl_scan(wsum, lane);
-    total         = __shfl_sync(kFull, winc, 7);
-    uint32_t woff = __shfl_sync(kFull, winc - wsum, warp);
-    __syncthreads();
-    return woff + inc - v;
-}
-
-__global__ __launch_bounds__(256) void scan_reduce_kernel(const uint32_t* __restrict__ counts, int P, int nchunks, int k_keep,
-                                                          uint32_t* __restrict__ partial, DevStats* stats, HeavyLists heavy)
-{
-    __shared__ uint32_t sm[8];
     const int b           = blockIdx.y;
     const uint32_t* c     = counts + (size_t)b * P;
-    const int start       = blockIdx.x * kScanChunk + threadIdx.x;
-    uint32_t v[8], sum = 0, kept = 0, mx = 0;
+    const int start       = blockIdx.x * kScanChunk + warp * 32 * kScanPerLane + lane;
+    uint32_t v[kScanPerLane], sum = 0, kept = 0, mx = 0;
 #pragma unroll
-    for (int k = 0; k < 8; ++k)
+    for (int k = 0; k < kScanPerLane; ++k) v[k] = start + k * 32 < P ? c[start + k * 32] : 0u;
+#pragma unroll
+    for (int k = 0; k < kScanPerLane; ++k)
     {
-        const int i = start + k * 256;  // the order of a sum does not matter: neighbouring threads read neighbouring counts
-        v[k]        = (i < P) ? c[i] : 0u;
         sum += v[k];
         kept += min(v[k], (uint32_t)k_keep);
         mx = max(mx, v[k]);
@@ -934,11 +929,10 @@ __global__ __launch_bounds__(256) void scan_reduce_kernel(const uint32_t* __rest
     // atomic per list queued up where most lists are long: 90 k long lists of 88x88 pixels in 11 views 0.041 -> 0.025 ms)
     if (__any_sync(kFull, mx > (uint32_t)kHeavyList))
     {
-        const int lane = threadIdx.x & 31;
         auto parts_of  = [](uint32_t n) { return n > (uint32_t)kHeavyList ? min((n - 1) / kHeavyPart + 1, (uint32_t)kHeavyParts) : 0u; };
         uint32_t items = 0, shared_items = 0;
 #pragma unroll
-        for (int k = 0; k < 8; ++k)
+        for (int k = 0; k < kScanPerLane; ++k)
         {
             const uint32_t parts = parts_of(v[k]);
             items += parts;
@@ -954,130 +948,65 @@ __global__ __launch_bounds__(256) void scan_reduce_kernel(const uint32_t* __rest
         slot   = __shfl_sync(kFull, slot, 31) + items_incl - items;
         shared = __shfl_sync(kFull, shared, 31) + shared_incl - shared_items;
 #pragma unroll 1
-        for (int k = 0; k < 8; ++k)
+        for (int k = 0; k < kScanPerLane; ++k)
         {
-            const uint32_t n     = c[min(start + k * 256, P - 1)];
-            const uint32_t parts = start + k * 256 < P ? parts_of(n) : 0u;
+            const uint32_t n     = c[min(start + k * 32, P - 1)];
+            const uint32_t parts = start + k * 32 < P ? parts_of(n) : 0u;
             // no room for its parts: one block takes the whole list, the other items stay empty
             const bool whole = parts > 1 && shared + parts > heavy.shared_cap;
             if (parts > 1 && !whole) heavy.finished[shared] = 0;
             for (uint32_t t = 0; t < parts && slot + t < heavy.cap; ++t)
-                heavy.item[slot + t] = make_uint4((unsigned)b, (unsigned)(start + k * 256), whole ? (t == 0 ? 1u << 16 : 0u) : t | parts << 16, shared);
+                heavy.item[slot + t] = make_uint4((unsigned)b, (unsigned)(start + k * 32), whole ? (t == 0 ? 1u << 16 : 0u) : t | parts << 16, shared);
             slot += parts;
             shared += parts > 1 ? parts : 0u;
         }
     }
-    uint32_t total;
-    block_excl_scan_256(sum, sm, total);
-    uint32_t kept_total;
-    block_excl_scan_256(kept, sm, kept_total);
-    for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(kFull, mx, o));
-    if ((threadIdx.x & 31) == 0 && mx) atomicMax(&stats->max_len, mx);
-    if (threadIdx.x == 0)
-    {
-        partial[(size_t)b * nchunks + blockIdx.x] = total;
-        if (kept_total) atomicAdd(&stats->kept, (unsigned long long)kept_total);
-    }
-}
-
-// one block: per view, exclusive scan of the chunk totals in place; view_base = running 64-bit fragment offset
-__global__ __launch_bounds__(1024) void scan_partials_kernel(uint32_t* __restrict__ partial, int nchunks, int B,
-                                                             unsigned long long* __restrict__ view_base,
-                                                             unsigned long long frag_cap, DevStats* stats)
-{
-    __shared__ uint32_t sm[32];
-    __shared__ uint32_t carry_s;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    unsigned long long base = 0, need = 0;
-    for (int b = 0; b < B; ++b)
-    {
-        uint32_t* p = partial + (size_t)b * nchunks;
-        if (threadIdx.x == 0) carry_s = 0;
-        __syncthreads();
-        for (int s = 0; s < nchunks; s += 1024)
-        {
-            int i        = s + threadIdx.x;
-            uint32_t v   = (i < nchunks) ? p[i] : 0u;
-            uint32_t inc = warp_incl_scan(v, lane);
-            if (lane == 31) sm[warp] = inc;
-            __syncthreads();
-            uint32_t wsum = sm[lane];
-            uint32_t winc = warp_incl_scan(wsum, lane);
-            uint32_t tot  = __shfl_sync(kFull, winc, 31);
-            uint32_t woff = __shfl_sync(kFull, winc - wsum, warp);
-            uint32_t carry = carry_s;
-            if (i < nchunks) p[i] = carry + woff + inc - v;
-            __syncthreads();
-            if (threadIdx.x == 0) carry_s = carry + tot;
-            __syncthreads();
-        }
-        if (threadIdx.x == 0)
-        {
-            // a view that does not fit the list buffer (sized from the previous call) gets no fragments at all: the
-            // collect pass skips it and the blend treats its lists as empty
-            view_base[b] = base;
-            need += carry_s;
-            if (base + carry_s <= frag_cap)
-                base += carry_s;
-            else
-                atomicOr(&stats->status, TRIPS_DEV_FRAGMENT_OVERFLOW);
-        }
-        __syncthreads();
-    }
-    if (threadIdx.x == 0)
-    {
-        view_base[B]     = base;
-        stats->frag_need = need;
-    }
-}
-
-__global__ __launch_bounds__(256) void scan_apply_kernel(const uint32_t* __restrict__ counts, int P, int nchunks,
-                                                         const uint32_t* __restrict__ partial, uint32_t* __restrict__ offsets)
-{
-    __shared__ uint32_t sm[8];
-    __shared__ uint32_t s_v[kScanChunk + kScanChunk / 8];  // element e at e + e / 8: a thread's 8 consecutive ones without bank conflicts
-    const int b       = blockIdx.y;
-    const uint32_t* c = counts + (size_t)b * P;
-    uint32_t* o       = offsets + (size_t)b * P;
-    const int start   = blockIdx.x * kScanChunk;
-    // through shared memory: neighbouring threads read and write neighbouring elements, but scan 8 consecutive ones each
-#pragma unroll
-    for (int k = 0; k < 8; ++k)
-    {
-        const int e      = k * 256 + threadIdx.x;
-        s_v[e + (e >> 3)] = start + e < P ? c[start + e] : 0u;
-    }
+    sum  = __reduce_add_sync(kFull, sum);
+    kept = __reduce_add_sync(kFull, kept);
+    mx   = __reduce_max_sync(kFull, mx);
+    if (lane == 0) s_warp[warp] = sum, s_kept[warp] = kept, s_most[warp] = mx;
     __syncthreads();
-    uint32_t v[8];
-    uint32_t sum = 0;
-#pragma unroll
-    for (int k = 0; k < 8; ++k)
+    const uint32_t w = lane < kScanThreads / 32 ? s_warp[lane] : 0u;
+    if (warp == 0)  // one update of the call's counters per block
     {
-        v[k] = s_v[threadIdx.x * 9 + k];
-        sum += v[k];
+        kept = __reduce_add_sync(kFull, lane < kScanThreads / 32 ? s_kept[lane] : 0u);
+        mx   = __reduce_max_sync(kFull, lane < kScanThreads / 32 ? s_most[lane] : 0u);
+        if (lane == 0 && mx) atomicMax(&stats->max_len, mx), atomicAdd(&stats->kept, (unsigned long long)kept);
     }
-    uint32_t total;
-    uint32_t run = block_excl_scan_256(sum, sm, total) + partial[(size_t)b * nchunks + blockIdx.x];
-#pragma unroll
-    for (int k = 0; k < 8; ++k)
-    {
-        s_v[threadIdx.x * 9 + k] = run;
-        run += v[k];
-    }
+    const uint32_t w_incl = warp_incl_scan(w, lane);
+    const uint32_t total  = __shfl_sync(kFull, w_incl, 31);
+    if (threadIdx.x == 0) s_base = total ? atomicAdd(cursor + b, total) : 0u;
     __syncthreads();
+    uint32_t run = s_base + __shfl_sync(kFull, w_incl - w, warp);
 #pragma unroll
-    for (int k = 0; k < 8; ++k)
+    for (int k = 0; k < kScanPerLane; ++k)
     {
-        const int e = k * 256 + threadIdx.x;
-        if (start + e < P) o[start + e] = s_v[e + (e >> 3)];
+        const uint32_t incl = warp_incl_scan(v[k], lane);
+        if (start + k * 32 < P) offsets[(size_t)b * P + start + k * 32] = run + incl - v[k];
+        run += __shfl_sync(kFull, incl, 31);
     }
+    if (!last_block(finished, gridDim.x * gridDim.y) || threadIdx.x != 0) return;
+    // First fragment of every view.  A view that does not fit the list buffer (sized from the previous call) gets no fragments at
+    // all: the collect pass skips it and the blend treats its lists as empty.
+    unsigned long long at = 0, need = 0;
+    for (int w = 0; w < (int)gridDim.y; ++w)
+    {
+        const uint32_t n = __ldcg(cursor + w);
+        view_base[w]     = at;
+        need += n;
+        if (at + n <= frag_cap)
+            at += n;
+        else
+            atomicOr(&stats->status, TRIPS_DEV_FRAGMENT_OVERFLOW);
+    }
+    view_base[gridDim.y] = at;
+    stats->frag_need     = need;
 }
 
-cudaError_t launch_scan(const Geom& g, int B, int k_keep, const FwdBuffers& fb, int nchunks, cudaStream_t st)
+cudaError_t launch_list_starts(const Geom& g, int B, int k_keep, const FwdBuffers& fb, cudaStream_t st)
 {
-    scan_reduce_kernel<<<dim3(nchunks, B), 256, 0, st>>>(fb.counts, g.P, nchunks, k_keep, fb.partial, fb.stats, fb.heavy);
-    scan_partials_kernel<<<1, 1024, 0, st>>>(fb.partial, nchunks, B, fb.view_base, fb.frag_cap, fb.stats);
-    scan_apply_kernel<<<dim3(nchunks, B), 256, 0, st>>>(fb.counts, g.P, nchunks, fb.partial, fb.offsets);
+    list_starts_kernel<<<dim3((g.P + kScanChunk - 1) / kScanChunk, B), kScanThreads, 0, st>>>(fb.counts, g.P, k_keep, fb.offsets, fb.list_cursor, fb.finished + 1,
+                                                                                    fb.view_base, fb.frag_cap, fb.stats, fb.heavy);
     return cudaGetLastError();
 }
 
@@ -1497,8 +1426,8 @@ constexpr int kSbWarps   = kSbThreads / 32;
 // threads takes one such list and moves its 16 nearest fragments to the front, in depth order, by swapping them with the
 // fragments that were there - the list stays the same set of fragments.  The blend kernel then reads only the first 16
 // entries of every list longer than kHeavyList.  A list longer than kHeavyPart is shared by several blocks, each of which
-// selects the 16 nearest of its part; the last one to finish selects from those and swaps.  Lists and parts are found by the
-// scan (scan_reduce_kernel); with more than kHeavyCap of them nothing is done here and the blend kernel, which sees the same
+// selects the 16 nearest of its part; the last one to finish selects from those and swaps.  Lists and parts are found by
+// list_starts_kernel; with more than kHeavyCap of them nothing is done here and the blend kernel, which sees the same
 // counter, walks the lists itself.
 //
 // What bounds it: on long lists the two walks over the keys (8 of 16 bytes used; the second comes from L2), on lists of about
