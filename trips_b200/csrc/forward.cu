@@ -1040,6 +1040,10 @@ constexpr int kWinChunkCollectFew = 512;
 // Threads of a block.  Half as many per barrier suits the counting pass (40 M entries 0.405 -> 0.380 ms, crowded clouds 0.145 ->
 // 0.122 ms); the collecting pass at 1024 entries per chunk wants 256 (1.25 against 1.45 ms with 128).
 constexpr int kWinThreadsCount = 128, kWinThreadsCollect = 256, kWinThreadsCollectFew = 128;
+// List ranges a thread reserves before it waits for any of them: all of a window's 1659 pixels by 256 threads.  One after another
+// they were most of a chunk's time (barriers and waits for atomics 13 of 20 cycles per instruction); with the search of the first bin by
+// 32 lanes: collect 217 -> 201 us (2 M points x 4 views), 66 -> 60 (8 channels), 1227 -> 1196 (6 M x 8), crowded cloud 430 -> 414.
+constexpr int kWinReserve      = 7;
 constexpr int kWinWarpsPerSM   = 64;  // grid size of the window kernels, in warps per SM
 constexpr int kWinMinWarps     = 40;  // resident warps the register allocation leaves room for
 constexpr int kWinMax     = 34 * 34 + 18 * 18 + 10 * 10 + 6 * 6 + 4 * 4 + 3 * 3 * 3;  // 1659 window pixels over 8 layers
@@ -1090,23 +1094,27 @@ __device__ __forceinline__ bool next_chunk(const FwdBuffers& fb, const Geom& g, 
                                            uint32_t& c0, uint32_t& c1, int& first_bin)
 {
     __syncthreads();
-    if (threadIdx.x == 0)
+    if (threadIdx.x < 32)
     {
-        const uint32_t t = atomicAdd(ticket + b, 1u);
-        uint32_t lo      = (uint32_t)min((unsigned long long)t * kWinChunk, (unsigned long long)n_entry);
-        s_tmp[0]         = lo;
-        // last bin whose first entry is <= lo (empty bins share their first entry with the next non-empty one)
+        uint32_t t = 0;
+        if (threadIdx.x == 0) t = atomicAdd(ticket + b, 1u);
+        t                 = __shfl_sync(kFull, t, 0);
+        const uint32_t lo = (uint32_t)min((unsigned long long)t * kWinChunk, (unsigned long long)n_entry);
+        // Last bin whose first entry is <= lo (empty bins share their first entry with the next non-empty one).  The lanes probe 32
+        // bins at a time: three steps for the bins of a 1080p view, where a search by halves is eleven dependent loads that the
+        // whole block waits for.
         const uint32_t* bf = fb.bin_cursor + (size_t)b * g.n_bins;
-        int a = 0, z = g.n_bins;  // invariant: bf[a] <= lo
+        int a = 0, z = lo < n_entry ? g.n_bins : 1;  // invariant: bf[a] <= lo, and bf[z] > lo or z is the end
         while (z - a > 1)
         {
-            const int mid = (a + z) >> 1;
-            if (bf[mid] <= lo)
-                a = mid;
-            else
-                z = mid;
+            const int step   = (z - a + 31) >> 5;
+            const int probe  = a + ((int)threadIdx.x + 1) * step;  // ascending with the lane
+            const bool below = probe < z && bf[probe] <= lo;
+            const int n      = __popc(__ballot_sync(kFull, below));
+            z                = min(z, a + (n + 1) * step);
+            a += n * step;
         }
-        s_tmp[1] = (uint32_t)a;
+        if (threadIdx.x == 0) s_tmp[0] = lo, s_tmp[1] = (uint32_t)a;
     }
     __syncthreads();
     c0        = s_tmp[0];
@@ -1302,16 +1310,32 @@ __global__ __launch_bounds__(THREADS, kWinMinWarps * 32 / THREADS) void window_k
                                       });
             __syncthreads();
             // ---- one global atomic per touched pixel ----
-            for (int i = threadIdx.x; i < n_win; i += THREADS)
+            if constexpr (COLLECT)
             {
-                const uint32_t c = s_cnt[i];
-                if (c)
+                // several of them on their way at a time: their results are the pixels' next free slots
+                for (int i0 = threadIdx.x; i0 < n_win; i0 += THREADS * kWinReserve)
                 {
-                    const int pix = window_pixel(g, w, i);
-                    if (COLLECT)
-                        s_cnt[i] = pix >= 0 ? atomicAdd(pixel_ctr + pix, c) : 0u;  // from here on the pixel's next free slot
-                    else if (pix >= 0)
-                        atomicAdd(pixel_ctr + pix, c);
+                    uint32_t slot[kWinReserve];
+#pragma unroll
+                    for (int k = 0; k < kWinReserve; ++k)
+                    {
+                        const int i      = i0 + k * THREADS;
+                        const uint32_t c = i < n_win ? s_cnt[i] : 0u;
+                        const int pix    = c ? window_pixel(g, w, i) : -1;
+                        slot[k]          = pix >= 0 ? atomicAdd(pixel_ctr + pix, c) : 0u;
+                    }
+#pragma unroll
+                    for (int k = 0; k < kWinReserve; ++k)
+                        if (i0 + k * THREADS < n_win) s_cnt[i0 + k * THREADS] = slot[k];
+                }
+            }
+            else
+            {
+                for (int i = threadIdx.x; i < n_win; i += THREADS)
+                {
+                    const uint32_t c = s_cnt[i];
+                    const int pix    = c ? window_pixel(g, w, i) : -1;
+                    if (pix >= 0) atomicAdd(pixel_ctr + pix, c);
                 }
             }
             __syncthreads();
