@@ -118,6 +118,7 @@ __device__ __forceinline__ void adam_block(const TripsAdamTensor* tensors, const
 __global__ __launch_bounds__(256, kAdamMinBlocks) void adam_kernel(const TripsAdamTensor* __restrict__ tensors,
                                                    const int64_t* __restrict__ block_start, int n_tensors)
 {
+    follow_previous();
     adam_block(tensors, block_start, n_tensors);
 }
 
@@ -129,6 +130,7 @@ struct AdamTable
 };
 __global__ __launch_bounds__(256, kAdamMinBlocks) void adam_by_value_kernel(const __grid_constant__ AdamTable table, int n_tensors)
 {
+    follow_previous();
     adam_block(table.tensors, table.block_start, n_tensors);
 }
 
@@ -139,7 +141,7 @@ cudaError_t launch_adam_by_value(const TripsAdamTensor* h_tensors, const int64_t
     AdamTable t{};
     for (int i = 0; i < n_tensors; ++i) t.tensors[i] = h_tensors[i];
     for (int i = 0; i <= n_tensors; ++i) t.block_start[i] = h_block_start[i];
-    adam_by_value_kernel<<<(unsigned)h_block_start[n_tensors], 256, 0, st>>>(t, n_tensors);
+    launch_following(adam_by_value_kernel, (unsigned)h_block_start[n_tensors], 256, st, t, n_tensors);
     return cudaGetLastError();
 }
 
@@ -147,7 +149,7 @@ cudaError_t launch_adam(const TripsAdamTensor* d_tensors, const int64_t* d_block
                         cudaStream_t st)
 {
     if (total_blocks <= 0) return cudaSuccess;
-    adam_kernel<<<(unsigned)total_blocks, 256, 0, st>>>(d_tensors, d_block_start, n_tensors);
+    launch_following(adam_kernel, (unsigned)total_blocks, 256, st, d_tensors, d_block_start, n_tensors);
     return cudaGetLastError();
 }
 

@@ -76,6 +76,7 @@ __global__ __launch_bounds__(kBwdThreads, (C <= 4 ? (SAT || DENSE ? kBwdMinBlock
                                                                      FwdBuffers fb, BwdBuffers bb,
                                                                      const __grid_constant__ ConstLayerPtrs grad_in)
 {
+    follow_previous();
     constexpr int DS = tail_stride(C);
     constexpr int GS = egrad_stride(C);
     constexpr int C4 = (C + 3) & ~3;
@@ -431,6 +432,7 @@ __global__ __launch_bounds__(kBwdThreads, (C <= 4 ? (SAT || DENSE ? kBwdMinBlock
 __global__ __launch_bounds__(256) void zero_entry_rows_kernel(float4* __restrict__ egrad, const unsigned long long* __restrict__ entry_base, int B,
                                                               int row_f4)
 {
+    follow_previous();
     const unsigned long long n = entry_base[B] * (unsigned long long)row_f4;
     const float4 z             = make_float4(0.f, 0.f, 0.f, 0.f);
     for (unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (unsigned long long)gridDim.x * blockDim.x)
@@ -439,7 +441,7 @@ __global__ __launch_bounds__(256) void zero_entry_rows_kernel(float4* __restrict
 
 cudaError_t launch_zero_entry_rows(int C, int B, const FwdBuffers& fb, const BwdBuffers& bb, int sm_count, cudaStream_t st)
 {
-    zero_entry_rows_kernel<<<sm_count * 8, 256, 0, st>>>(reinterpret_cast<float4*>(bb.egrad), fb.entry_base, B, egrad_stride(C) / 4);
+    launch_following(zero_entry_rows_kernel, sm_count * 8, 256, st, reinterpret_cast<float4*>(bb.egrad), fb.entry_base, B, egrad_stride(C) / 4);
     return cudaGetLastError();
 }
 
@@ -451,11 +453,11 @@ cudaError_t launch_blend_backward(const ScenePtrs& sc, const CamConst* cams, con
 #define TRIPS_BWD_CASE(CC)                                                                                         \
     case CC:                                                                                                       \
         if (pr.saturated_alpha_accumulation)                                                                       \
-            blend_backward_kernel<CC, true, false><<<grid, kBwdThreads, 0, st>>>(sc, cams, g, pr, B, fb, bb, grad_in);           \
+            launch_following(blend_backward_kernel<CC, true, false>, grid, kBwdThreads, st, sc, cams, g, pr, B, fb, bb, grad_in);           \
         else if (CC <= 4 && dense_entries(entries_hint, g, B))                                                     \
-            blend_backward_kernel<CC, false, (CC <= 4)><<<grid, kBwdThreads, 0, st>>>(sc, cams, g, pr, B, fb, bb, grad_in);      \
+            launch_following(blend_backward_kernel<CC, false, (CC <= 4)>, grid, kBwdThreads, st, sc, cams, g, pr, B, fb, bb, grad_in);      \
         else                                                                                                       \
-            blend_backward_kernel<CC, false, false><<<grid, kBwdThreads, 0, st>>>(sc, cams, g, pr, B, fb, bb, grad_in);          \
+            launch_following(blend_backward_kernel<CC, false, false>, grid, kBwdThreads, st, sc, cams, g, pr, B, fb, bb, grad_in);          \
         break;
     switch (sc.C)
     {
@@ -534,6 +536,7 @@ __global__ __launch_bounds__(256, (C <= 4 ? 4 : 1)) void point_grad_kernel(Scene
                                                          TripsGrads out, const float* __restrict__ raw_texture,
                                                          const float* __restrict__ raw_confidence, float confidence_scale)
 {
+    follow_previous();
     constexpr int GS = egrad_stride(C);
     constexpr int C4 = (C + 3) & ~3;
     __shared__ CamConst s_cam[kGradCams];
@@ -643,6 +646,7 @@ __global__ __launch_bounds__(256, (C <= 4 ? 4 : 1)) void point_grad_kernel(Scene
 // Fills the point-to-entry table of a view group from the entries (view v0 + blockIdx.y); it holds kNoEntry before.
 __global__ __launch_bounds__(256) void note_entries_kernel(FwdBuffers fb, int v0, int N)
 {
+    follow_previous();
     const int v = v0 + blockIdx.y;
     const unsigned long long first = fb.entry_base[v], n = fb.entry_base[v + 1] - first;
     uint32_t* table = fb.point_entry + (size_t)blockIdx.y * N;
@@ -659,6 +663,7 @@ __global__ __launch_bounds__(256) void note_entries_kernel(FwdBuffers fb, int v0
 template <int C, bool DIST>
 __global__ __launch_bounds__(256) void entry_cam_grad_kernel(FwdBuffers fb, BwdBuffers bb, const CamConst* __restrict__ cams, int B)
 {
+    follow_previous();
     constexpr int GS = egrad_stride(C);
     constexpr int NA = DIST ? 19 : 11;  // 6 pose + 5 pinhole (+ 8 distortion) sums per view
     __shared__ CamConst cam;
@@ -752,6 +757,7 @@ __global__ __launch_bounds__(64) void unpack_small_kernel(int C, int B, const Ca
                                                           const double* __restrict__ g_pose, const double* __restrict__ g_k,
                                                           const double* __restrict__ g_dis, float* out_bg, double* out_pose, float* out_intr)
 {
+    follow_previous();
     const int t = threadIdx.x;
     if (out_bg && t < C) out_bg[t] = (float)g_bg[t];
     if (out_pose && t < 6)
@@ -775,9 +781,9 @@ cudaError_t launch_unpack_grads(const ScenePtrs& sc, const CamConst* cams, int B
 #define TRIPS_CAM_CASE(CC)                                                              \
     case CC:                                                                            \
         if (pr.distortion)                                                              \
-            entry_cam_grad_kernel<CC, true><<<grid, 256, 0, st>>>(fb, bb, cams, B);     \
+            launch_following(entry_cam_grad_kernel<CC, true>, grid, 256, st, fb, bb, cams, B);     \
         else                                                                            \
-            entry_cam_grad_kernel<CC, false><<<grid, 256, 0, st>>>(fb, bb, cams, B);    \
+            launch_following(entry_cam_grad_kernel<CC, false>, grid, 256, st, fb, bb, cams, B);    \
         break;
         switch (sc.C)
         {
@@ -818,10 +824,10 @@ cudaError_t launch_unpack_grads(const ScenePtrs& sc, const CamConst* cams, int B
             {
                 cudaError_t e = cudaMemsetAsync(fb.point_entry, 0xff, sizeof(uint32_t) * (size_t)sc.N * nv, st);  // kNoEntry
                 if (e != cudaSuccess) return e;
-                note_entries_kernel<<<dim3(max(1, sm_count * 8 / nv), nv), 256, 0, st>>>(fb, v0, sc.N);
+                launch_following(note_entries_kernel, dim3(max(1, sm_count * 8 / nv), nv), 256, st, fb, v0, sc.N);
             }
 #define TRIPS_POINT_LAUNCH(CC, DIST, ACC) \
-    point_grad_kernel<CC, DIST, ACC><<<blocks, 256, 0, st>>>(sc, fbv, bb, cams + v0, nv, out, raw_tex, raw_conf, pr.confidence_scale)
+    launch_following(point_grad_kernel<CC, DIST, ACC>, blocks, 256, st, sc, fbv, bb, cams + v0, nv, out, raw_tex, raw_conf, pr.confidence_scale)
 #define TRIPS_POINT_CASE(CC)                                                                              \
     case CC:                                                                                              \
         if (pr.distortion)                                                                                \
@@ -842,7 +848,7 @@ cudaError_t launch_unpack_grads(const ScenePtrs& sc, const CamConst* cams, int B
 #undef TRIPS_POINT_LAUNCH
         }
     }
-    unpack_small_kernel<<<1, 64, 0, st>>>(sc.C, B, cams, bb.g_bg, bb.g_pose, bb.g_k, bb.g_dis, out.background, out.pose_tangent,
+    launch_following(unpack_small_kernel, 1, 64, st, sc.C, B, cams, bb.g_bg, bb.g_pose, bb.g_k, bb.g_dis, out.background, out.pose_tangent,
                                          out.intrinsics);
     return cudaGetLastError();
 }

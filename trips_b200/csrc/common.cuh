@@ -181,6 +181,31 @@ __host__ __device__ inline bool strict_layers(const TripsRenderParams& pr)
     return pr.use_layer_point_size && !pr.render_points_in_all_lower_resolutions;
 }
 
+// Kernels of a call follow one another on one stream.  A kernel that starts with follow_previous() may be launched by
+// launch_following() while its predecessor drains: its blocks are in place when the last ones of that kernel end, and wait there
+// until all of its memory operations are visible.  Every kernel waits before it does anything, so that the end of one kernel
+// implies the end of all before it.  14 kernels of a step, us, one after another / like this: 800 k points x 2 views 698 / 682, 2 M x 4
+// 1715 / 1691, a 640x480 frame (10 kernels) 228 / 213, a 1080p frame 843 / 825, 6 M x 8 views 8823 / 8800.
+__device__ __forceinline__ void follow_previous()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+template <class... Params, class... Args>
+cudaError_t launch_following(void (*kernel)(Params...), dim3 grid, dim3 block, cudaStream_t st, Args&&... args)
+{
+    cudaLaunchAttribute overlap{};
+    overlap.id                                         = cudaLaunchAttributeProgrammaticStreamSerialization;
+    overlap.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t config{};
+    config.gridDim  = grid;
+    config.blockDim = block;
+    config.stream   = st;
+    config.attrs    = &overlap;
+    config.numAttrs = 1;
+    return cudaLaunchKernelEx(&config, kernel, static_cast<Args&&>(args)...);
+}
+
 // ---- device helpers (op order mirrors the CPU oracle; compiled with -fmad=false) ----
 
 __device__ __forceinline__ void transform_point(const CamConst& V, float px, float py, float pz, float& ox, float& oy,

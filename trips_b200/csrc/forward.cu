@@ -23,6 +23,7 @@ __global__ void setup_cams_kernel(const __grid_constant__ ViewTable views, int b
                                   const float* __restrict__ intrinsics, int n_cameras, int distortion, float dist_cutoff,
                                   CamConst* __restrict__ cams, DevStats* stats)
 {
+    follow_previous();
     const int b = b0 + (int)threadIdx.x;
     if (b == 0)
     {
@@ -94,7 +95,7 @@ cudaError_t launch_setup_cams(const TripsView* h_views, int B, const double* pos
         const int n = min(kViewTable, B - b0);
         for (int k = 0; k < n; ++k) t.v[k] = h_views[b0 + k];
         for (int k = n; k < kViewTable; ++k) t.v[k] = h_views[b0];
-        setup_cams_kernel<<<1, kViewTable, 0, st>>>(t, b0, B, poses, n_images, intrinsics, n_cameras, distortion, dist_cutoff, cams, stats);
+        launch_following(setup_cams_kernel, 1, kViewTable, st, t, b0, B, poses, n_images, intrinsics, n_cameras, distortion, dist_cutoff, cams, stats);
     }
     return cudaGetLastError();
 }
@@ -212,6 +213,7 @@ __device__ __forceinline__ bool box_outside_view(const CamConst& c, const Geom& 
 __global__ __launch_bounds__(256) void block_visibility_kernel(const float4* __restrict__ pos, int N, const CamConst* __restrict__ cams,
                                                                const __grid_constant__ Geom g, int B, uint8_t* __restrict__ skip, DevStats* stats)
 {
+    follow_previous();
     const int first = blockIdx.x * kBinChunk, last = min(N, first + kBinChunk);
     float lo[3] = {3.0e38f, 3.0e38f, 3.0e38f}, hi[3] = {-3.0e38f, -3.0e38f, -3.0e38f};
     bool bad = false;
@@ -333,6 +335,7 @@ template <bool ACT>
 __global__ __launch_bounds__(kBinThreads, kCountMinBlocks) void bin_count_kernel(ScenePtrs sc, const CamConst* __restrict__ cams, const __grid_constant__ Geom g,
                                                                 TripsRenderParams pr, FwdBuffers fb, int v0, int nv, unsigned* ticket)
 {
+    follow_previous();
     __shared__ BinCam s_cam[kViewGroup];
     __shared__ unsigned s_ticket;
     for (int k = threadIdx.x; k < nv * (int)(sizeof(CamConst) / 4); k += kBinThreads) ((int*)s_cam)[k] = ((const int*)(cams + v0))[k];
@@ -414,6 +417,7 @@ __global__ __launch_bounds__(1024) void bin_scan_kernel(const uint32_t* __restri
                                                         uint32_t* __restrict__ bin_first, int n_keys, uint32_t* view_total, unsigned long long entry_cap,
                                                         unsigned long long* __restrict__ entry_base, unsigned* finished, DevStats* stats)
 {
+    follow_previous();
     __shared__ uint32_t sm[32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int b    = blockIdx.x;
@@ -561,6 +565,7 @@ template <int C, bool ACT>
 __global__ __launch_bounds__(kBinThreads, (C <= 4 ? kScatterMinBlocks : kScatterMinBlocksWide)) void bin_scatter_kernel(ScenePtrs sc, const CamConst* __restrict__ cams, const __grid_constant__ Geom g,
                                                                   TripsRenderParams pr, FwdBuffers fb, int v0, int nv, unsigned* ticket)
 {
+    follow_previous();
     __shared__ BinCam s_cam[kViewGroup];
     __shared__ unsigned long long s_ebase[kViewGroup + 1];
     __shared__ unsigned s_ticket;
@@ -695,6 +700,7 @@ template <bool ACT>
 __global__ __launch_bounds__(kBinThreads) void bin_count_hot_kernel(ScenePtrs sc, const CamConst* __restrict__ cams, const __grid_constant__ Geom g,
                                                                     TripsRenderParams pr, FwdBuffers fb, int v0, int nv, unsigned* ticket)
 {
+    follow_previous();
     __shared__ BinCam s_cam[kViewGroup];
     __shared__ uint32_t s_tag[kHotSlots], s_cnt[kHotSlots];
     __shared__ unsigned s_ticket;
@@ -737,6 +743,7 @@ template <int C, bool ACT>
 __global__ __launch_bounds__(kBinThreads) void bin_scatter_hot_kernel(ScenePtrs sc, const CamConst* __restrict__ cams, const __grid_constant__ Geom g,
                                                                       TripsRenderParams pr, FwdBuffers fb, int v0, int nv, unsigned* ticket)
 {
+    follow_previous();
     __shared__ BinCam s_cam[kViewGroup];
     __shared__ unsigned long long s_ebase[kViewGroup + 1];
     __shared__ uint32_t s_tag[kHotSlots], s_cnt[kHotSlots], s_base[kHotSlots];
@@ -829,22 +836,22 @@ cudaError_t launch_bin_count(const ScenePtrs& sc, const CamConst* cams, const Ge
     const int grid     = sm_count * kBinBlocksPerSM;
     const int n_groups = (B + kViewGroup - 1) / kViewGroup;
     if (sc.N > 0 && fb.block_skip)
-        block_visibility_kernel<<<(sc.N + kBinChunk - 1) / kBinChunk, 256, 0, st>>>(sc.position, sc.N, cams, g, B, const_cast<uint8_t*>(fb.block_skip), fb.stats);
+        launch_following(block_visibility_kernel, (sc.N + kBinChunk - 1) / kBinChunk, 256, st, sc.position, sc.N, cams, g, B, const_cast<uint8_t*>(fb.block_skip), fb.stats);
     const bool act = pr.confidence_is_raw || pr.texture_abs;
     if (sc.N > 0)
         for (int gi = 0; gi < n_groups; ++gi)
         {
             const int v0 = gi * kViewGroup, nv = min(kViewGroup, B - v0);
             if (hot && act)
-                bin_count_hot_kernel<true><<<grid, kBinThreads, 0, st>>>(sc, cams, g, pr, fb, v0, nv, fb.ticket + gi);
+                launch_following(bin_count_hot_kernel<true>, grid, kBinThreads, st, sc, cams, g, pr, fb, v0, nv, fb.ticket + gi);
             else if (hot)
-                bin_count_hot_kernel<false><<<grid, kBinThreads, 0, st>>>(sc, cams, g, pr, fb, v0, nv, fb.ticket + gi);
+                launch_following(bin_count_hot_kernel<false>, grid, kBinThreads, st, sc, cams, g, pr, fb, v0, nv, fb.ticket + gi);
             else if (act)
-                bin_count_kernel<true><<<grid, kBinThreads, 0, st>>>(sc, cams, g, pr, fb, v0, nv, fb.ticket + gi);
+                launch_following(bin_count_kernel<true>, grid, kBinThreads, st, sc, cams, g, pr, fb, v0, nv, fb.ticket + gi);
             else
-                bin_count_kernel<false><<<grid, kBinThreads, 0, st>>>(sc, cams, g, pr, fb, v0, nv, fb.ticket + gi);
+                launch_following(bin_count_kernel<false>, grid, kBinThreads, st, sc, cams, g, pr, fb, v0, nv, fb.ticket + gi);
         }
-    bin_scan_kernel<<<B, 1024, 0, st>>>(fb.bin_count, fb.bin_base, fb.bin_cursor, n_keys, fb.view_total, entry_cap, fb.entry_base, fb.finished, fb.stats);
+    launch_following(bin_scan_kernel, B, 1024, st, fb.bin_count, fb.bin_base, fb.bin_cursor, n_keys, fb.view_total, entry_cap, fb.entry_base, fb.finished, fb.stats);
     return cudaGetLastError();
 }
 
@@ -866,13 +873,13 @@ cudaError_t launch_bin_scatter(const ScenePtrs& sc, const CamConst* cams, const 
 #define TRIPS_SCATTER_CASE(CC)                                                                                    \
     case CC:                                                                                                      \
         if (hot && act)                                                                                           \
-            bin_scatter_hot_kernel<CC, true><<<grid, kBinThreads, 0, st>>>(sc, cams, g, pr, fb, v0, nv, tk);     \
+            launch_following(bin_scatter_hot_kernel<CC, true>, grid, kBinThreads, st, sc, cams, g, pr, fb, v0, nv, tk);     \
         else if (hot)                                                                                             \
-            bin_scatter_hot_kernel<CC, false><<<grid, kBinThreads, 0, st>>>(sc, cams, g, pr, fb, v0, nv, tk);    \
+            launch_following(bin_scatter_hot_kernel<CC, false>, grid, kBinThreads, st, sc, cams, g, pr, fb, v0, nv, tk);    \
         else if (act)                                                                                             \
-            bin_scatter_kernel<CC, true><<<grid, kBinThreads, 0, st>>>(sc, cams, g, pr, fb, v0, nv, tk);         \
+            launch_following(bin_scatter_kernel<CC, true>, grid, kBinThreads, st, sc, cams, g, pr, fb, v0, nv, tk);         \
         else                                                                                                      \
-            bin_scatter_kernel<CC, false><<<grid, kBinThreads, 0, st>>>(sc, cams, g, pr, fb, v0, nv, tk);        \
+            launch_following(bin_scatter_kernel<CC, false>, grid, kBinThreads, st, sc, cams, g, pr, fb, v0, nv, tk);        \
         break;
         switch (sc.C)
         {
@@ -910,6 +917,7 @@ __global__ __launch_bounds__(kScanThreads) void list_starts_kernel(const uint32_
                                                                    unsigned* finished, unsigned long long* __restrict__ view_base, unsigned long long frag_cap,
                                                                    DevStats* stats, HeavyLists heavy)
 {
+    follow_previous();
     __shared__ uint32_t s_warp[kScanThreads / 32], s_kept[kScanThreads / 32], s_most[kScanThreads / 32], s_base;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int b           = blockIdx.y;
@@ -1005,7 +1013,7 @@ __global__ __launch_bounds__(kScanThreads) void list_starts_kernel(const uint32_
 
 cudaError_t launch_list_starts(const Geom& g, int B, int k_keep, const FwdBuffers& fb, cudaStream_t st)
 {
-    list_starts_kernel<<<dim3((g.P + kScanChunk - 1) / kScanChunk, B), kScanThreads, 0, st>>>(fb.counts, g.P, k_keep, fb.offsets, fb.list_cursor, fb.finished + 1,
+    launch_following(list_starts_kernel, dim3((g.P + kScanChunk - 1) / kScanChunk, B), kScanThreads, st, fb.counts, g.P, k_keep, fb.offsets, fb.list_cursor, fb.finished + 1,
                                                                                     fb.view_base, fb.frag_cap, fb.stats, fb.heavy);
     return cudaGetLastError();
 }
@@ -1266,6 +1274,7 @@ __device__ __noinline__ void sparse_bin_footprints(const Geom& g, const float4* 
 template <int THREADS, bool COLLECT, bool STRICT>
 __global__ __launch_bounds__(THREADS, kWinMinWarps * 32 / THREADS) void window_kernel(const __grid_constant__ Geom g, FwdBuffers fb, int B, int chunk)
 {
+    follow_previous();
     __shared__ uint32_t s_cnt[kWinMax];
     __shared__ uint32_t s_tmp[2];
     const uint64_t keep = evict_last_policy();
@@ -1394,9 +1403,9 @@ static void run_window(const Geom& g, int B, const FwdBuffers& fb, bool strict, 
     const unsigned long long want = entries_hint / chunk + B;
     const int grid                = (int)min(most, max((unsigned long long)sm_count * 4, want));
     if (strict)
-        window_kernel<THREADS, COLLECT, true><<<grid, THREADS, 0, st>>>(g, fb, B, chunk);
+        launch_following(window_kernel<THREADS, COLLECT, true>, grid, THREADS, st, g, fb, B, chunk);
     else
-        window_kernel<THREADS, COLLECT, false><<<grid, THREADS, 0, st>>>(g, fb, B, chunk);
+        launch_following(window_kernel<THREADS, COLLECT, false>, grid, THREADS, st, g, fb, B, chunk);
 }
 
 cudaError_t launch_count(const ScenePtrs& sc, const Geom& g, int B, const FwdBuffers& fb, bool strict, unsigned long long entries_hint, int sm_count,
@@ -1561,6 +1570,7 @@ __device__ int nearest_16(uint32_t n, KeyAt&& key_at, HeavyShared& sh)
 
 __global__ __launch_bounds__(256, kHeavyBlocks) void heavy_topk_kernel(const __grid_constant__ Geom g, FwdBuffers fb, int B)
 {
+    follow_previous();
     __shared__ HeavyShared sh;
     __shared__ uint32_t s_vac[16];
     __shared__ unsigned s_last;
@@ -1630,7 +1640,7 @@ __global__ __launch_bounds__(256, kHeavyBlocks) void heavy_topk_kernel(const __g
 
 cudaError_t launch_heavy_topk(const Geom& g, int B, const FwdBuffers& fb, int sm_count, cudaStream_t st)
 {
-    heavy_topk_kernel<<<sm_count * kHeavyBlocks, 256, 0, st>>>(g, fb, B);
+    launch_following(heavy_topk_kernel, sm_count * kHeavyBlocks, 256, st, g, fb, B);
     return cudaGetLastError();
 }
 
@@ -1699,6 +1709,7 @@ __global__ __launch_bounds__(kSbThreads, (C <= 4 ? kSbMinBlocks : (C <= 8 ? kSbM
                                                                 int B, FwdBuffers fb, const __grid_constant__ LayerPtrs out,
                                                                 unsigned n_tiles_total)
 {
+    follow_previous();
     constexpr int ES = tail_stride(C);
     __shared__ uint32_t s_key[kSbWarps][32 * kSbPitch];  // depths of a chunk of 16 fragments per pixel; later the sorted list positions, [rank][lane]
     __shared__ uint2 s_az[kSbWarps][32 * kSbPitch];      // (alpha bits, entry index) of the chunk
@@ -2010,11 +2021,11 @@ cudaError_t launch_sort_blend(const ScenePtrs& sc, const Geom& g, const TripsRen
     blocks     = max(blocks, 1);
     switch (sc.C)
     {
-        case 3: sort_blend_kernel<3><<<blocks, kSbThreads, 0, st>>>(sc, g, pr, B, fb, out, n_tiles); break;
-        case 4: sort_blend_kernel<4><<<blocks, kSbThreads, 0, st>>>(sc, g, pr, B, fb, out, n_tiles); break;
-        case 6: sort_blend_kernel<6><<<blocks, kSbThreads, 0, st>>>(sc, g, pr, B, fb, out, n_tiles); break;
-        case 8: sort_blend_kernel<8><<<blocks, kSbThreads, 0, st>>>(sc, g, pr, B, fb, out, n_tiles); break;
-        case 16: sort_blend_kernel<16><<<blocks, kSbThreads, 0, st>>>(sc, g, pr, B, fb, out, n_tiles); break;
+        case 3: launch_following(sort_blend_kernel<3>, blocks, kSbThreads, st, sc, g, pr, B, fb, out, n_tiles); break;
+        case 4: launch_following(sort_blend_kernel<4>, blocks, kSbThreads, st, sc, g, pr, B, fb, out, n_tiles); break;
+        case 6: launch_following(sort_blend_kernel<6>, blocks, kSbThreads, st, sc, g, pr, B, fb, out, n_tiles); break;
+        case 8: launch_following(sort_blend_kernel<8>, blocks, kSbThreads, st, sc, g, pr, B, fb, out, n_tiles); break;
+        case 16: launch_following(sort_blend_kernel<16>, blocks, kSbThreads, st, sc, g, pr, B, fb, out, n_tiles); break;
         default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();
