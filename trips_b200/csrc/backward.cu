@@ -212,10 +212,10 @@ __global__ __launch_bounds__(kBwdThreads, (C <= 4 ? (SAT || DENSE ? kBwdMinBlock
                     for (int c = 0; c < C; c += 4)
                     {
                         const float4 v4 = row[c / 4], g4 = s_g[warp][c / 4][seg];
-                        G = fmaf(v4.x, g4.x, G);
-                        if (c + 1 < C) G = fmaf(v4.y, g4.y, G);
-                        if (c + 2 < C) G = fmaf(v4.z, g4.z, G);
-                        if (c + 3 < C) G = fmaf(v4.w, g4.w, G);
+                        G += v4.x * g4.x;
+                        if (c + 1 < C) G += v4.y * g4.y;
+                        if (c + 2 < C) G += v4.z * g4.z;
+                        if (c + 3 < C) G += v4.w * g4.w;
                     }
                     s_d[warp][j] = G;
                     if constexpr (SAT)
@@ -325,8 +325,8 @@ __global__ __launch_bounds__(kBwdThreads, (C <= 4 ? (SAT || DENSE ? kBwdMinBlock
                 const float a   = al[j];
                 const float dA  = my_d[j];
                 const float dem = 1.f / (1.f - a + 1e-9f);
-                my_d[j]         = fmaf(-R, dem, dA);
-                R               = fmaf(dA, a, R);
+                my_d[j]         = dA - R * dem;
+                R += dA * a;
             }
         }
         }
@@ -379,8 +379,7 @@ __global__ __launch_bounds__(kBwdThreads, (C <= 4 ? (SAT || DENSE ? kBwdMinBlock
                 const float gbs = conf * lf * ga;  // dLoss / d(bilinear weight) (RenderBackward.cu:385)
                 // image-space sums of the entry: the chain to position / size / pose is linear in them and is applied
                 // once per entry by point_grad_kernel
-                const float bg_a = bf * ga;
-                const float4 h0  = make_float4((nx ? -wy : wy) * gbs, (ny ? -wx : wx) * gbs, conf * lf_grad * bg_a, lf * bg_a);
+                const float4 h0 = make_float4((nx ? -wy : wy) * gbs, (ny ? -wx : wx) * gbs, bf * conf * lf_grad * ga, bf * lf * ga);
                 float gt[C4];
 #pragma unroll
                 for (int c = 0; c < C4; c += 4)
