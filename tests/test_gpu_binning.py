@@ -26,3 +26,20 @@ def test_entries_of_ragged_clouds(oracle_lib, cuda_lib, n_points, n_views, radiu
             onrec, opid, oalpha = f.records()
             assert np.array_equal(nrec, onrec) and np.array_equal(pid, opid)
             assert rel_err(alpha, oalpha, floor=1e-6) <= 1e-5
+
+
+@pytest.mark.parametrize("w,h,layers", [(61, 43, 6), (64, 48, 7), (97, 65, 8), (2, 2, 2), (33, 3, 4)])
+def test_layers_at_the_far_border(oracle_lib, cuda_lib, w, h, layers):
+    """Large points around the right and lower border, where the footprint leaves some layer before the last one."""
+    s = scenes.tiny(seed=450 + w, n_points=1500, n_views=2, width=w, height=h, num_layers=layers, size_range=(0.05, 3.0), fx=0.9 * w)
+    s.intrinsics[:, 2] = 0.85 * w
+    s.intrinsics[:, 3] = 0.85 * h
+    _, _, frames = oracle_frames(s, train=True)
+    _, info, blend = gpu_render(s, train=True)
+    blend(info)
+    assert info.cache.last_status() == 0
+    for b, f in enumerate(frames):
+        nrec, pid, alpha = info.cache.debug_records(b, f.P)
+        onrec, opid, oalpha = f.records()
+        assert np.array_equal(nrec, onrec) and np.array_equal(pid, opid)
+        assert rel_err(alpha, oalpha, floor=1e-6) <= 1e-5

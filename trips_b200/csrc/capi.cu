@@ -3,6 +3,7 @@
 // parts of RenderFast16 / BlendBackwardsBilinearFast / MyAdam::step.
 #include <algorithm>
 #include <cfloat>
+#include <cmath>
 #include <cstdio>
 #include <cstring>
 #include <new>
@@ -333,6 +334,17 @@ static bool make_geom(int w, int h, int L, Geom& g)
         base += (long long)lw * lh;
         lw = (lw + 1) / 2;  // ceil halving, PointRenderer.cu:385-389
         lh = (lh + 1) / 2;
+    }
+    double in_x = DBL_MAX, in_y = DBL_MAX;
+    for (int l = 0; l < TRIPS_MAX_LAYERS; ++l)
+    {
+        if (l < g.L)
+        {
+            in_x = std::min(in_x, std::ldexp((double)(g.W[l] - 1), l));
+            in_y = std::min(in_y, std::ldexp((double)(g.H[l] - 1), l));
+        }
+        auto below = [](double v) { return (double)(float)v > v ? std::nextafterf((float)v, 0.f) : (float)v; };
+        g.inside_x[l] = below(in_x), g.inside_y[l] = below(in_y);
     }
     for (int l = g.L; l <= TRIPS_MAX_LAYERS; ++l) g.base[l] = (int)base;
     if (base > (1ll << 30)) return false;

@@ -34,6 +34,8 @@ struct Geom
     int L;
     int W[TRIPS_MAX_LAYERS];            // ceil-halved layer sizes (PointRenderer.cu:385-389)
     int H[TRIPS_MAX_LAYERS];
+    float inside_x[TRIPS_MAX_LAYERS];   // layer-0 positions below these have their footprint inside layers 0..l: min (W_k - 1) 2^k
+    float inside_y[TRIPS_MAX_LAYERS];
     int base[TRIPS_MAX_LAYERS + 1];     // first pixel of every layer in the per-view pixel arrays (row-major)
     int P;                              // pixels per view
     // Tile order of a view: first the 64x64-pixel regions of layer 0 in row-major order, each with its tiles of
