@@ -129,6 +129,7 @@ struct FwdBuffers
     unsigned long long* view_base;    // [B+1] first fragment of each view in `frags`
     uint4* frags;                     // [frag_cap] x = point id, y = depth bits (y:x = 64-bit sort key), z = alpha bits, w = entry index within the view
     unsigned long long frag_cap;
+    bool report_overflow;             // raise a status bit for views that do not fit (off where the host looks and renders again)
     uint8_t* rec_n;                   // [B,n_tiles,32] records kept for backward, by tile and lane (pixel of the tile)
     uint2* records;                   // [B,n_tiles,16,32] (entry index within the view, alpha bits), by tile, rank and lane: a warp's
                                       // access to one rank of its tile is 256 consecutive bytes

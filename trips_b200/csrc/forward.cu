@@ -396,7 +396,7 @@ __device__ __forceinline__ bool last_block(unsigned* finished, unsigned n)
 // First entry of every view in the entry arrays.  A view whose entries do not fit the arrays (entry_cap entries: the
 // arrays are sized from the previous call's count, not for the worst case) gets none: it renders as background, the
 // status word says so and stats->visible still carries the number that was needed, so that the host grows the arrays.
-__device__ __forceinline__ void first_entries(const uint32_t* view_total, int B, unsigned long long entry_cap, unsigned long long* entry_base, DevStats* stats)
+__device__ __forceinline__ void first_entries(const uint32_t* view_total, int B, unsigned long long entry_cap, unsigned long long* entry_base, bool report, DevStats* stats)
 {
     unsigned long long base = 0, need = 0;
     for (int b = 0; b < B; ++b)
@@ -406,7 +406,7 @@ __device__ __forceinline__ void first_entries(const uint32_t* view_total, int B,
         need += n;
         if (base + n <= entry_cap)
             base += n;
-        else
+        else if (report)
             atomicOr(&stats->status, TRIPS_DEV_ENTRY_OVERFLOW);
     }
     entry_base[B]  = base;
@@ -415,7 +415,7 @@ __device__ __forceinline__ void first_entries(const uint32_t* view_total, int B,
 
 __global__ __launch_bounds__(1024) void bin_scan_kernel(const uint32_t* __restrict__ counts, uint32_t* __restrict__ key_first,
                                                         uint32_t* __restrict__ bin_first, int n_keys, uint32_t* view_total, unsigned long long entry_cap,
-                                                        unsigned long long* __restrict__ entry_base, unsigned* finished, DevStats* stats)
+                                                        unsigned long long* __restrict__ entry_base, bool report, unsigned* finished, DevStats* stats)
 {
     follow_previous();
     __shared__ uint32_t sm[32];
@@ -470,7 +470,7 @@ __global__ __launch_bounds__(1024) void bin_scan_kernel(const uint32_t* __restri
         __syncthreads();  // the warp sums are overwritten by the next turn
     }
     if (threadIdx.x == 0) view_total[b] = carry;
-    if (last_block(finished, gridDim.x) && threadIdx.x == 0) first_entries(view_total, (int)gridDim.x, entry_cap, entry_base, stats);
+    if (last_block(finished, gridDim.x) && threadIdx.x == 0) first_entries(view_total, (int)gridDim.x, entry_cap, entry_base, report, stats);
 }
 
 // One 32-byte store (sm_100 has 256-bit global stores) for the two float4 halves of a 32-byte-aligned record: half the
@@ -859,7 +859,7 @@ cudaError_t launch_bin_count(const ScenePtrs& sc, const CamConst* cams, const Ge
             else
                 launch_following(bin_count_kernel<false>, grid, kBinThreads, st, sc, cams, g, pr, fb, v0, nv, fb.ticket + gi);
         }
-    launch_following(bin_scan_kernel, B, 1024, st, fb.bin_count, fb.bin_base, fb.bin_cursor, n_keys, fb.view_total, entry_cap, fb.entry_base, fb.finished, fb.stats);
+    launch_following(bin_scan_kernel, B, 1024, st, fb.bin_count, fb.bin_base, fb.bin_cursor, n_keys, fb.view_total, entry_cap, fb.entry_base, fb.report_overflow, fb.finished, fb.stats);
     return cudaGetLastError();
 }
 
@@ -922,7 +922,7 @@ __device__ __forceinline__ uint32_t warp_incl_scan(uint32_t v, int lane)
 // A warp takes 32 consecutive lengths at a time, kScanPerLane times: the lists of neighbouring pixels are neighbours.
 // cursor: [B] fragments of the views so far, zero before; finished: blocks that are done, zero before.
 __global__ __launch_bounds__(kScanThreads) void list_starts_kernel(const uint32_t* __restrict__ counts, int P, int k_keep, uint32_t* __restrict__ offsets, uint32_t* cursor,
-                                                                   unsigned* finished, unsigned long long* __restrict__ view_base, unsigned long long frag_cap,
+                                                                   unsigned* finished, unsigned long long* __restrict__ view_base, unsigned long long frag_cap, bool report,
                                                                    DevStats* stats, HeavyLists heavy)
 {
     follow_previous();
@@ -1012,7 +1012,7 @@ __global__ __launch_bounds__(kScanThreads) void list_starts_kernel(const uint32_
         need += n;
         if (at + n <= frag_cap)
             at += n;
-        else
+        else if (report)
             atomicOr(&stats->status, TRIPS_DEV_FRAGMENT_OVERFLOW);
     }
     view_base[gridDim.y] = at;
@@ -1022,7 +1022,7 @@ __global__ __launch_bounds__(kScanThreads) void list_starts_kernel(const uint32_
 cudaError_t launch_list_starts(const Geom& g, int B, int k_keep, const FwdBuffers& fb, cudaStream_t st)
 {
     launch_following(list_starts_kernel, dim3((g.P + kScanChunk - 1) / kScanChunk, B), kScanThreads, st, fb.counts, g.P, k_keep, fb.offsets, fb.list_cursor, fb.finished + 1,
-                                                                                    fb.view_base, fb.frag_cap, fb.stats, fb.heavy);
+                                                                                    fb.view_base, fb.frag_cap, fb.report_overflow, fb.stats, fb.heavy);
     return cudaGetLastError();
 }
 
