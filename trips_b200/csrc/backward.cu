@@ -71,7 +71,7 @@ inline bool dense_entries(unsigned long long entries, const Geom& g, int B) { re
 // SAT: saturated_alpha_accumulation as the reference's backward pass has it (RenderBackward.cu:227-259); a separate
 // instantiation, so that the common case carries none of its code or registers.
 template <int C, bool SAT, bool DENSE>
-__global__ __launch_bounds__(kBwdThreads, (C <= 4 ? (SAT || DENSE ? kBwdMinBlocksDense : kBwdMinBlocks) : 1)) void blend_backward_kernel(ScenePtrs sc, const CamConst* __restrict__ cams,
+__global__ __launch_bounds__(kBwdThreads, (C <= 4 ? (SAT || DENSE ? kBwdMinBlocksDense : kBwdMinBlocks) : 1)) void blend_backward_kernel(ScenePtrs sc, const CamConst* cams,
                                                                      const __grid_constant__ Geom g, TripsRenderParams pr, int B,
                                                                      FwdBuffers fb, BwdBuffers bb,
                                                                      const __grid_constant__ ConstLayerPtrs grad_in)
@@ -428,7 +428,7 @@ __global__ __launch_bounds__(kBwdThreads, (C <= 4 ? (SAT || DENSE ? kBwdMinBlock
 
 // The gradient rows of the entries the forward pass wrote start from zero.  Their number is known on the device only
 // (entry_base[B]): the host does not wait for the forward pass's counts.
-__global__ __launch_bounds__(256) void zero_entry_rows_kernel(float4* __restrict__ egrad, const unsigned long long* __restrict__ entry_base, int B,
+__global__ __launch_bounds__(256) void zero_entry_rows_kernel(float4* egrad, const unsigned long long* entry_base, int B,
                                                               int row_f4)
 {
     follow_previous();
@@ -531,7 +531,7 @@ __device__ __forceinline__ ViewGrad view_gradient(const CamConst& cam, float vx,
 constexpr int kGradViews = 4;   // views whose rows a thread requests before it waits for any of them
 constexpr int kGradCams  = 32;  // cameras held in shared memory; further ones are read from global memory (uniform addresses)
 template <int C, bool DIST, bool ACC>
-__global__ __launch_bounds__(256, (C <= 4 ? 4 : 1)) void point_grad_kernel(ScenePtrs sc, FwdBuffers fb, BwdBuffers bb, const CamConst* __restrict__ cams, int B,
+__global__ __launch_bounds__(256, (C <= 4 ? 4 : 1)) void point_grad_kernel(ScenePtrs sc, FwdBuffers fb, BwdBuffers bb, const CamConst* cams, int B,
                                                          TripsGrads out, const float* __restrict__ raw_texture,
                                                          const float* __restrict__ raw_confidence, float confidence_scale)
 {
@@ -543,7 +543,7 @@ __global__ __launch_bounds__(256, (C <= 4 ? 4 : 1)) void point_grad_kernel(Scene
     __syncthreads();
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < (size_t)sc.N; i += (size_t)gridDim.x * blockDim.x)
     {
-        const float4 p = __ldg(fb.point_state + i);  // x y z raw size
+        const float4 p = fb.point_state[i];  // x y z raw size
         float gp0 = 0.f, gp1 = 0.f, gp2 = 0.f, gl = 0.f, gc = 0.f;
         float gt[C4];
 #pragma unroll
@@ -553,7 +553,7 @@ __global__ __launch_bounds__(256, (C <= 4 ? 4 : 1)) void point_grad_kernel(Scene
             uint32_t ent[kGradViews];
             float4 s4[kGradViews], row[kGradViews][C4 / 4];
 #pragma unroll
-            for (int j = 0; j < kGradViews; ++j) ent[j] = vb + j < B ? __ldg(fb.point_entry + (size_t)(vb + j) * sc.N + i) : kNoEntry;
+            for (int j = 0; j < kGradViews; ++j) ent[j] = vb + j < B ? fb.point_entry[(size_t)(vb + j) * sc.N + i] : kNoEntry;
 #pragma unroll
             for (int j = 0; j < kGradViews; ++j)
                 if (ent[j] != kNoEntry)
@@ -660,7 +660,7 @@ __global__ __launch_bounds__(256) void note_entries_kernel(FwdBuffers fb, int v0
 // DIST: the view-space position comes from the entry's world position (the stored projection cannot be undistorted in
 // closed form) and the eight coefficients receive J_dis_dis^T (PointRendererHelper.h:468-491).
 template <int C, bool DIST>
-__global__ __launch_bounds__(256) void entry_cam_grad_kernel(FwdBuffers fb, BwdBuffers bb, const CamConst* __restrict__ cams, int B)
+__global__ __launch_bounds__(256) void entry_cam_grad_kernel(FwdBuffers fb, BwdBuffers bb, const CamConst* cams, int B)
 {
     follow_previous();
     constexpr int GS = egrad_stride(C);
@@ -752,9 +752,9 @@ __global__ __launch_bounds__(256) void entry_cam_grad_kernel(FwdBuffers fb, BwdB
 
 // One block; a thread per component (the views of a call may share an image / camera index, so every component adds its
 // views in order).  One thread for everything took 12 us longer with 4 views: 76 dependent read-modify-writes.
-__global__ __launch_bounds__(64) void unpack_small_kernel(int C, int B, const CamConst* __restrict__ cams, const double* __restrict__ g_bg,
-                                                          const double* __restrict__ g_pose, const double* __restrict__ g_k,
-                                                          const double* __restrict__ g_dis, float* out_bg, double* out_pose, float* out_intr)
+__global__ __launch_bounds__(64) void unpack_small_kernel(int C, int B, const CamConst* cams, const double* g_bg,
+                                                          const double* g_pose, const double* g_k,
+                                                          const double* g_dis, float* out_bg, double* out_pose, float* out_intr)
 {
     follow_previous();
     const int t = threadIdx.x;

@@ -210,8 +210,8 @@ __device__ __forceinline__ bool box_outside_view(const CamConst& c, const Geom& 
 // Boxes are recomputed by every forward pass (points move): one read of the positions.  skip[b * n_blocks + k] = 1 when block k of
 // the point cloud cannot hold a point visible in view b (a test inside the binning kernels would cost their loops 30
 // registers).
-__global__ __launch_bounds__(256) void block_visibility_kernel(const float4* __restrict__ pos, int N, const CamConst* __restrict__ cams,
-                                                               const __grid_constant__ Geom g, int B, uint8_t* __restrict__ skip, DevStats* stats)
+__global__ __launch_bounds__(256) void block_visibility_kernel(const float4* __restrict__ pos, int N, const CamConst* cams,
+                                                               const __grid_constant__ Geom g, int B, uint8_t* skip, DevStats* stats)
 {
     follow_previous();
     const int first = blockIdx.x * kBinChunk, last = min(N, first + kBinChunk);
@@ -269,7 +269,7 @@ __global__ __launch_bounds__(256) void block_visibility_kernel(const float4* __r
 // first would take two each - 130 k points in 11 views 0.23 instead of 0.17 ms - and elsewhere it gains nothing.)
 // Returns false when the cloud is exhausted; `skip` gets one bit per view of the group whose bounding-box test rules the
 // ticket's points out.
-__device__ __forceinline__ bool next_point_ticket(unsigned* ticket, int N, unsigned* s_ticket, const uint8_t* __restrict__ block_skip, int v0,
+__device__ __forceinline__ bool next_point_ticket(unsigned* ticket, int N, unsigned* s_ticket, const uint8_t* block_skip, int v0,
                                                   int nv, int& first, int& last, unsigned& skip)
 {
     __syncthreads();
@@ -332,7 +332,7 @@ struct PointHead
 // points x 8 views), 241 -> 206 (2 M x 4), 1733 -> 1660 (20 M x 2), 64 views of 10 M points 16.5 -> 15.4 ms.  Issue slots bound both
 // passes (57 and 69 % in use before).
 template <bool ACT>
-__global__ __launch_bounds__(kBinThreads, kCountMinBlocks) void bin_count_kernel(ScenePtrs sc, const CamConst* __restrict__ cams, const __grid_constant__ Geom g,
+__global__ __launch_bounds__(kBinThreads, kCountMinBlocks) void bin_count_kernel(ScenePtrs sc, const CamConst* cams, const __grid_constant__ Geom g,
                                                                 TripsRenderParams pr, FwdBuffers fb, int v0, int nv, unsigned* ticket)
 {
     follow_previous();
@@ -413,9 +413,9 @@ __device__ __forceinline__ void first_entries(const uint32_t* view_total, int B,
     stats->visible = need;
 }
 
-__global__ __launch_bounds__(1024) void bin_scan_kernel(const uint32_t* __restrict__ counts, uint32_t* __restrict__ key_first,
-                                                        uint32_t* __restrict__ bin_first, int n_keys, uint32_t* view_total, unsigned long long entry_cap,
-                                                        unsigned long long* __restrict__ entry_base, bool report, unsigned* finished, DevStats* stats)
+__global__ __launch_bounds__(1024) void bin_scan_kernel(const uint32_t* counts, uint32_t* key_first,
+                                                        uint32_t* bin_first, int n_keys, uint32_t* view_total, unsigned long long entry_cap,
+                                                        unsigned long long* entry_base, bool report, unsigned* finished, DevStats* stats)
 {
     follow_previous();
     __shared__ uint32_t sm[32];
@@ -570,7 +570,7 @@ __device__ __forceinline__ void write_entry(const FwdBuffers& fb, const Geom& g,
 }
 
 template <int C, bool ACT>
-__global__ __launch_bounds__(kBinThreads, (C <= 4 ? kScatterMinBlocks : kScatterMinBlocksWide)) void bin_scatter_kernel(ScenePtrs sc, const CamConst* __restrict__ cams, const __grid_constant__ Geom g,
+__global__ __launch_bounds__(kBinThreads, (C <= 4 ? kScatterMinBlocks : kScatterMinBlocksWide)) void bin_scatter_kernel(ScenePtrs sc, const CamConst* cams, const __grid_constant__ Geom g,
                                                                   TripsRenderParams pr, FwdBuffers fb, int v0, int nv, unsigned* ticket)
 {
     follow_previous();
@@ -705,7 +705,7 @@ __device__ __forceinline__ bool next_hot_ticket(unsigned* ticket, int N, unsigne
 }
 
 template <bool ACT>
-__global__ __launch_bounds__(kBinThreads) void bin_count_hot_kernel(ScenePtrs sc, const CamConst* __restrict__ cams, const __grid_constant__ Geom g,
+__global__ __launch_bounds__(kBinThreads) void bin_count_hot_kernel(ScenePtrs sc, const CamConst* cams, const __grid_constant__ Geom g,
                                                                     TripsRenderParams pr, FwdBuffers fb, int v0, int nv, unsigned* ticket)
 {
     follow_previous();
@@ -748,7 +748,7 @@ __global__ __launch_bounds__(kBinThreads) void bin_count_hot_kernel(ScenePtrs sc
 }
 
 template <int C, bool ACT>
-__global__ __launch_bounds__(kBinThreads) void bin_scatter_hot_kernel(ScenePtrs sc, const CamConst* __restrict__ cams, const __grid_constant__ Geom g,
+__global__ __launch_bounds__(kBinThreads) void bin_scatter_hot_kernel(ScenePtrs sc, const CamConst* cams, const __grid_constant__ Geom g,
                                                                       TripsRenderParams pr, FwdBuffers fb, int v0, int nv, unsigned* ticket)
 {
     follow_previous();
@@ -921,8 +921,8 @@ __device__ __forceinline__ uint32_t warp_incl_scan(uint32_t v, int lane)
 
 // A warp takes 32 consecutive lengths at a time, kScanPerLane times: the lists of neighbouring pixels are neighbours.
 // cursor: [B] fragments of the views so far, zero before; finished: blocks that are done, zero before.
-__global__ __launch_bounds__(kScanThreads) void list_starts_kernel(const uint32_t* __restrict__ counts, int P, int k_keep, uint32_t* __restrict__ offsets, uint32_t* cursor,
-                                                                   unsigned* finished, unsigned long long* __restrict__ view_base, unsigned long long frag_cap, bool report,
+__global__ __launch_bounds__(kScanThreads) void list_starts_kernel(const uint32_t* counts, int P, int k_keep, uint32_t* offsets, uint32_t* cursor,
+                                                                   unsigned* finished, unsigned long long* view_base, unsigned long long frag_cap, bool report,
                                                                    DevStats* stats, HeavyLists heavy)
 {
     follow_previous();
@@ -1149,7 +1149,7 @@ __device__ __forceinline__ int strict_first_layer(float ps, int L) { return ps >
 
 // first_warp: the warp of the block that takes the first 32 entries
 template <int THREADS, bool WITH_E1, bool STRICT, class Body>
-__device__ __forceinline__ void for_each_footprint(const float4* __restrict__ head, uint32_t lo, uint32_t hi, uint8_t* queue, int L, Body&& body, unsigned first_warp = 0)
+__device__ __forceinline__ void for_each_footprint(const float4* head, uint32_t lo, uint32_t hi, uint8_t* queue, int L, Body&& body, unsigned first_warp = 0)
 {
     const int lane = threadIdx.x & 31;
     uint32_t base  = lo + ((threadIdx.x + 32 * first_warp) & (THREADS - 32));
@@ -1239,7 +1239,7 @@ __device__ __forceinline__ uint64_t evict_last_policy()
 // chunks (20 M points at 1440p: count 0.29 -> 0.17 ms, collect in chunks of 1024 0.91 -> 0.55; 4 k points in 11 views 0.67 -> 0.35
 // and 1.63 -> 0.50).  Not inlined: the dense path keeps its registers.
 template <int THREADS, bool COLLECT, bool STRICT>
-__device__ __noinline__ void sparse_bin_footprints(const Geom& g, const float4* __restrict__ head, uint32_t lo, uint32_t hi, uint8_t* queue,
+__device__ __noinline__ void sparse_bin_footprints(const Geom& g, const float4* head, uint32_t lo, uint32_t hi, uint8_t* queue,
                                                    uint32_t* pixel_ctr, uint4* frags, uint64_t keep, unsigned first_warp)
 {
     for_each_footprint<THREADS, COLLECT, STRICT>(head, lo, hi, queue, g.L, [&](const float4& e0, const float4& e1, float x, float y, int layer, uint32_t ei) {
