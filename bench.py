@@ -171,13 +171,13 @@ def stage_bytes(stage, N, P, C, B, F, Kf, V=0):
 # gather and Adam from one view of config 3 (rasterizer_kernels_c3_6Mpts_1view_ncu_sections.md: same list density and the
 # same N as the benchmark), the binning kernels, which read every point once for all views of a call, from a quarter of the
 # points with all 8 views (binning_adam_kernels_1.5Mpts_8views_ncu_sections.md).  Traffic grows in proportion to the unit
-# count.  The scan has no capture and is left out of the sums.  Units: F fragments, Kf kept fragments, NB points x views, V
+# count.  The scan (two passes over the list lengths) is left out of the sums.  Units: F fragments, Kf kept fragments, NB points x views, V
 # entries (visible points over all views), N points.
-# unpack_grads: 15.1 bytes per row cleared, 127.2 per row gathered (127 bytes of DRAM for a 32-byte row at a random address),
+# unpack_grads: 15.2 bytes per row cleared, 127.2 per row gathered (127 bytes of DRAM for a 32-byte row at a random address),
 # 4 per entry index, 16 of point state and 35 of gradients per point.
-DRAM_BYTES_PER_UNIT = {"count": [(5.2, "F")], "collect": [(20.2, "F")], "sort_blend": [(34.5, "F")], "blend_backward": [(36.0, "Kf")],
-                       "bin_points": [(48.8, "NB")], "unpack_grads": [(15.1 + 127.2, "V"), (4.0, "NB"), (16.0 + 35.0, "N")],
-                       "adam": [(337.3, "N")]}
+DRAM_BYTES_PER_UNIT = {"count": [(5.2, "F")], "collect": [(20.4, "F")], "sort_blend": [(34.6, "F")], "blend_backward": [(35.9, "Kf")],
+                       "bin_points": [(48.3, "NB")], "unpack_grads": [(15.2 + 127.2, "V"), (4.0, "NB"), (16.0 + 35.0, "N")],
+                       "adam": [(339.8, "N")]}
 
 
 def stage_traffic(stage, N, B, F, Kf, V=0):
