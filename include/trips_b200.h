@@ -291,11 +291,15 @@ int trips_l1_loss_backward(TripsContext* ctx, const float* const* out_layers, co
 /* Per-point results of view `view`: depth [N] (-1 = culled), nlayers [N] int32, record [N,4] (u, v, size_px, texture index bits).
  * HOST output pointers, any may be NULL.  RenderForward.cu:311-363. */
 int trips_debug_points(TripsContext* ctx, int view, float* depth, int32_t* nlayers, float* record, void* stream);
-/* Per-pixel list lengths [P] int32, start offsets [P] int64 (relative to the view's first fragment) and the
- * view's fragments (64-bit keys: depth bits << 32 | point id) in list order.  HOST pointers; pass frags = NULL
- * and read *n_frags first to size the buffer.  RenderForward.cu:387-413. */
+/* Per-pixel list lengths [P] int32, the view's fragments (64-bit keys: depth bits << 32 | point id) list by list in pixel order,
+ * and where each list starts among them, offsets [P] int64.  (On the device the lists are in no particular order:
+ * trips_debug_list_starts.)  HOST pointers; pass frags = NULL and read *n_frags first to size the buffer.  TRIPS_ERR_CUDA
+ * when the lists on the device overlap or leave the view's part of the list buffer.  RenderForward.cu:387-413. */
 int trips_debug_lists(TripsContext* ctx, int view, int32_t* counts, int64_t* offsets, uint64_t* frags, int64_t* n_frags,
                       void* stream);
+/* First slot [P] int64 of every list in the view's part of the device's list buffer.  HOST pointer.  Checks and errors as
+ * trips_debug_lists.  RenderForward.cu:1201-1232 (there in pixel order). */
+int trips_debug_list_starts(TripsContext* ctx, int view, int64_t* starts, void* stream);
 /* Backward records of view `view`: nrec [P] int32, point ids [P,16] int32 (-1 = absent), alphas [P,16] (-1 = absent).
  * RenderForward.cu:957-979. */
 int trips_debug_records(TripsContext* ctx, int view, int32_t* nrec, int32_t* rec_pid, float* rec_alpha, void* stream);

@@ -110,6 +110,7 @@ SYMBOLS = {
                                          C.POINTER(C.c_int64), C.c_int, C.c_void_p, C.c_void_p]),
     "trips_debug_points": (C.c_int, [C.c_void_p, C.c_int, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]),
     "trips_debug_lists": (C.c_int, [C.c_void_p, C.c_int, C.c_void_p, C.c_void_p, C.c_void_p, C.POINTER(C.c_int64), C.c_void_p]),
+    "trips_debug_list_starts": (C.c_int, [C.c_void_p, C.c_int, C.c_void_p, C.c_void_p]),
     "trips_debug_records": (C.c_int, [C.c_void_p, C.c_int, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]),
     "trips_debug_nearest": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int, C.c_void_p, C.POINTER(C.c_int), C.c_void_p]),
 }

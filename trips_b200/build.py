@@ -19,7 +19,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libtrips_b200.so")
 SOURCES = ["forward.cu", "second.cu", "backward.cu", "adam.cu", "resize.cu", "capi.cu", "noalloc.cu"]
-HEADERS = ["common.cuh", "trips_math.h", os.path.join("..", "..", "include", "trips_b200.h")]
+HEADERS = ["common.cuh", "trips_math.h", "list_order.h", os.path.join("..", "..", "include", "trips_b200.h")]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "-lineinfo", "-fmad=false",

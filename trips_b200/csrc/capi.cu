@@ -11,6 +11,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "list_order.h"
 
 using namespace trips;
 
@@ -921,25 +922,39 @@ int trips_debug_points(TripsContext* ctx, int view, float* depth, int32_t* nlaye
     return TRIPS_OK;
 }
 
+// List lengths of a view, its number of fragments and where the lists start in its part of the list buffer.  An error when the lists
+// do not fill that part exactly.
+static int read_lists(TripsContext* ctx, int view, cudaStream_t st, std::vector<uint32_t>& counts, std::vector<uint32_t>& starts, unsigned long long (&vb)[2])
+{
+    if (!ctx->have_forward) return fail(ctx, TRIPS_ERR_NO_FORWARD, "no forward pass");
+    if (view < 0 || view >= ctx->B) return fail(ctx, TRIPS_ERR_INVALID_ARG, "view out of range");
+    const size_t P = (size_t)ctx->geom.P, off = (size_t)view * P;
+    counts.resize(P), starts.resize(P);
+    CU_CHECK(ctx, cudaMemcpyAsync(vb, (unsigned long long*)ctx->view_base.p + view, sizeof(vb), cudaMemcpyDeviceToHost, st));
+    CU_CHECK(ctx, cudaMemcpyAsync(counts.data(), (const uint32_t*)((const char*)ctx->zeroed.p + ctx->zero_counts) + off, sizeof(uint32_t) * P, cudaMemcpyDeviceToHost, st));
+    CU_CHECK(ctx, cudaMemcpyAsync(starts.data(), (uint32_t*)ctx->offsets.p + off, sizeof(uint32_t) * P, cudaMemcpyDeviceToHost, st));
+    CU_CHECK(ctx, cudaStreamSynchronize(st));
+    if (vb[1] == vb[0]) return TRIPS_OK;  // no fragments, or the view did not fit: the collect pass has skipped it
+    for (size_t i = 0; i < P; ++i) starts[i] -= counts[i];  // the collect pass advanced the starts to the list ends
+    if (!lists_cover(starts.data(), counts.data(), P, vb[1] - vb[0]))
+        return fail(ctx, TRIPS_ERR_CUDA, "the lists of the view overlap or leave their part of the list buffer (internal error)");
+    return TRIPS_OK;
+}
+
 int trips_debug_lists(TripsContext* ctx, int view, int32_t* counts, int64_t* offsets, uint64_t* frags, int64_t* n_frags,
                       void* stream)
 {
     if (!ctx) return TRIPS_ERR_INVALID_ARG;
-    if (!ctx->have_forward) return fail(ctx, TRIPS_ERR_NO_FORWARD, "no forward pass");
-    if (view < 0 || view >= ctx->B) return fail(ctx, TRIPS_ERR_INVALID_ARG, "view out of range");
     cudaStream_t st = (cudaStream_t)stream;
-    const size_t P = (size_t)ctx->geom.P, off = (size_t)view * P;
+    std::vector<uint32_t> c, s;
     unsigned long long vb[2];
-    CU_CHECK(ctx, cudaMemcpyAsync(vb, (unsigned long long*)ctx->view_base.p + view, sizeof(vb), cudaMemcpyDeviceToHost, st));
-    std::vector<uint32_t> c(P), e(P);
-    CU_CHECK(ctx, cudaMemcpyAsync(c.data(), (const uint32_t*)((const char*)ctx->zeroed.p + ctx->zero_counts) + off, sizeof(uint32_t) * P, cudaMemcpyDeviceToHost, st));
-    CU_CHECK(ctx, cudaMemcpyAsync(e.data(), (uint32_t*)ctx->offsets.p + off, sizeof(uint32_t) * P, cudaMemcpyDeviceToHost, st));
-    CU_CHECK(ctx, cudaStreamSynchronize(st));
+    const int rc = read_lists(ctx, view, st, c, s, vb);
+    if (rc != TRIPS_OK) return rc;
     const unsigned long long nf = vb[1] - vb[0];
     if (n_frags) *n_frags = (int64_t)nf;
     // the lists lie in the buffer in the order in which their blocks came; here they follow one another in pixel order
     int64_t next = 0;
-    for (size_t i = 0; i < P; ++i)
+    for (size_t i = 0; i < c.size(); ++i)
     {
         if (counts) counts[i] = (int32_t)c[i];
         if (offsets) offsets[i] = next;
@@ -950,14 +965,21 @@ int trips_debug_lists(TripsContext* ctx, int view, int32_t* counts, int64_t* off
         std::vector<uint4> f(nf);
         CU_CHECK(ctx, cudaMemcpyAsync(f.data(), (uint4*)ctx->frags.p + vb[0], sizeof(uint4) * nf, cudaMemcpyDeviceToHost, st));
         CU_CHECK(ctx, cudaStreamSynchronize(st));
-        size_t n = 0;
-        for (size_t i = 0; i < P; ++i)
-        {
-            const size_t first = (size_t)e[i] - c[i];  // the collect pass advanced the starts to the list ends
-            for (size_t k = 0; k < c[i] && n < nf; ++k)
-                if (first + k < nf) frags[n++] = ((uint64_t)f[first + k].y << 32) | f[first + k].x;
-        }
+        for (size_t i = 0; i < c.size(); ++i)
+            for (size_t k = 0; k < c[i]; ++k) *frags++ = ((uint64_t)f[s[i] + k].y << 32) | f[s[i] + k].x;
     }
+    return TRIPS_OK;
+}
+
+int trips_debug_list_starts(TripsContext* ctx, int view, int64_t* starts, void* stream)
+{
+    if (!ctx) return TRIPS_ERR_INVALID_ARG;
+    if (!starts) return fail(ctx, TRIPS_ERR_INVALID_ARG, "null argument");
+    std::vector<uint32_t> c, s;
+    unsigned long long vb[2];
+    const int rc = read_lists(ctx, view, (cudaStream_t)stream, c, s, vb);
+    if (rc != TRIPS_OK) return rc;
+    std::copy(s.begin(), s.end(), starts);
     return TRIPS_OK;
 }
 

@@ -267,6 +267,12 @@ class PointRendererCache:
         _lib.check(_lib.lib().trips_debug_lists(self._h, view, None, None, frags.ctypes.data, C.byref(nf), st), self._h)
         return counts, offsets, frags
 
+    def debug_list_starts(self, view: int, n_pixels: int):
+        import numpy as np
+        starts = np.empty(n_pixels, np.int64)
+        _lib.check(_lib.lib().trips_debug_list_starts(self._h, view, starts.ctypes.data, _stream_ptr(self.device)), self._h)
+        return starts
+
     def debug_records(self, view: int, n_pixels: int):
         import numpy as np
         nrec = np.empty(n_pixels, np.int32)
