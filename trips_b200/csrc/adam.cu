@@ -22,11 +22,12 @@ struct AdamRule
 
 // Bias-corrected learning rate of the last step count seen by this thread, and what follows from it alone: neighbouring
 // elements (the coordinates of a point, the channels of a descriptor) almost always share their step count, and the two powf
-// dominate the update.
+// dominate the update.  No step count stands for an empty cache: all 2^32 are counts.
 struct LrCache
 {
-    int step = -1;
-    float lr = 0.f, keep = 0.f, pull = 0.f;  // relative and absolute weight decay at this rate
+    bool filled = false;
+    int step;
+    float lr, keep, pull;  // keep, pull: relative and absolute weight decay at this rate
 };
 
 __device__ __forceinline__ void adam_element(const AdamRule& t, float& w, float g, float& m, float& v, int& step, LrCache& cache)
@@ -35,10 +36,11 @@ __device__ __forceinline__ void adam_element(const AdamRule& t, float& w, float 
     const float gsq = g * g;
     m               = t.beta1 * m + (1.f - t.beta1) * g;
     v               = t.beta2 * v + (1.f - t.beta2) * gsq;
-    step            = step + 1;
-    if (step != cache.step)
+    step            = (int)((unsigned)step + 1u);
+    if (!cache.filled || step != cache.step)
     {
         const float fs = (float)(unsigned)step;
+        cache.filled   = true;
         cache.step     = step;
         cache.lr       = t.lr * (sqrtf(1.f - powf(t.beta2, fs)) / (1.f - powf(t.beta1, fs)));
         cache.keep     = 1.f - t.relative_weight_decay * cache.lr;
@@ -209,14 +211,14 @@ __global__ __launch_bounds__(256) void fused_reduce_adam_kernel(const __grid_con
 #pragma unroll
         for (int k = 0; k < 4; ++k) mm[k] = m_state[j + k], vv[k] = v_state[j + k], ss[k] = steps[j + k];
         const int s0 = segment_of(i), s3 = segment_of(i + 3);
-        if (s0 != s3 || s0 != cache_seg) cache.step = -1;  // the cached learning rate belongs to one segment
+        if (s0 != s3 || s0 != cache_seg) cache.filled = false;  // the cached learning rate belongs to one segment
         cache_seg = s3;
         adam_element(AdamRule::of(a.seg[s0]), w.x, g.x, mm[0], vv[0], ss[0], cache);
-        if (s0 != s3) cache.step = -1;
+        if (s0 != s3) cache.filled = false;
         adam_element(AdamRule::of(a.seg[s0 == s3 ? s0 : segment_of(i + 1)]), w.y, g.y, mm[1], vv[1], ss[1], cache);
-        if (s0 != s3) cache.step = -1;
+        if (s0 != s3) cache.filled = false;
         adam_element(AdamRule::of(a.seg[s0 == s3 ? s0 : segment_of(i + 2)]), w.z, g.z, mm[2], vv[2], ss[2], cache);
-        if (s0 != s3) cache.step = -1;
+        if (s0 != s3) cache.filled = false;
         adam_element(AdamRule::of(a.seg[s3]), w.w, g.w, mm[3], vv[3], ss[3], cache);
 #pragma unroll
         for (int k = 0; k < 4; ++k) m_state[j + k] = mm[k], v_state[j + k] = vv[k], steps[j + k] = ss[k];
@@ -337,12 +339,12 @@ __global__ __launch_bounds__(256) void fused_multicast_adam_kernel(const __grid_
 #pragma unroll
             for (int k = 0; k < 4; ++k) mm[k] = m_state[j + k], vv[k] = v_state[j + k], ss[k] = steps[j + k];
             const int s0 = segment_of(i), s3 = segment_of(i + 3);
-            if (s0 != s3 || s0 != cache_seg) cache.step = -1;  // the cached learning rate belongs to one segment
+            if (s0 != s3 || s0 != cache_seg) cache.filled = false;  // the cached learning rate belongs to one segment
             cache_seg = s3;
 #pragma unroll
             for (int k = 0; k < 4; ++k)
             {
-                if (k > 0 && s0 != s3) cache.step = -1;
+                if (k > 0 && s0 != s3) cache.filled = false;
                 adam_element(AdamRule::of(a.seg[s0 == s3 ? s0 : segment_of(i + k)]), ww[k], gg[k], mm[k], vv[k], ss[k], cache);
             }
 #pragma unroll
