@@ -418,17 +418,20 @@ constexpr double kGrowth      = 1.25;  // head room of the entry / fragment buff
 constexpr int kEvalSubBatch   = 8;     // views rendered per pass when nothing has to be kept for a backward pass
 }  // namespace
 
+// When a pass learns how many entries and fragments its views have.
+enum class Sizes
+{
+    wait,   // before it writes them: the buffers are sized from the pass's own counts, which costs two host synchronisations (the
+            // reference synchronises 2 * num_layers times per view for the same purpose, RenderForward.cu:1201-1208)
+    later,  // the buffers keep the capacity found by earlier calls (need x 1.25) and nothing is waited for: the totals travel to pinned
+            // host memory behind an event, and the next training call reads them
+    look,   // an inference pass: everything is launched with the buffers as they are, and the totals are looked at while the GPU
+            // renders.  A pass that does not fit is given up on the device (place_views) and taken up from where it stopped
+};
+
 // One pass over `B` views (all views of a training call; up to kEvalSubBatch views of an inference call).
-//   wait_for_sizes = true : the entry and fragment buffers are sized from this pass's own counts, which costs two host
-//                           synchronisations (the reference synchronises 2 * num_layers times per view for the same
-//                           purpose, RenderForward.cu:1201-1208);
-//   wait_for_sizes = false: the buffers keep the capacity found by earlier calls (need x 1.25) and nothing is waited
-//                           for: the totals travel to pinned host memory behind an event.  A training call leaves it to the
-//                           next call to read them; an inference call reads them itself while its blend runs, and renders the
-//                           views again where they did not fit.
 static int forward_views(TripsContext* ctx, const TripsScene* scene, const TripsView* views, int B, const TripsRenderParams* params,
-                         const Geom& g, float* const* out_layers, size_t out_view_offset, const float* dropout, cudaStream_t st,
-                         bool wait_for_sizes)
+                         const Geom& g, float* const* out_layers, size_t out_view_offset, const float* dropout, cudaStream_t st, Sizes sizes)
 {
     const size_t N    = (size_t)scene->n_points;
     const size_t P    = (size_t)g.P;
@@ -475,33 +478,95 @@ static int forward_views(TripsContext* ctx, const TripsScene* scene, const Trips
           launch_setup_cams(views, B, scene->poses, scene->n_images, scene->intrinsics, scene->n_cameras, params->distortion,
                             params->dist_cutoff, (CamConst*)ctx->cams.p, fb.stats, st));
     const CamConst* cams = (const CamConst*)ctx->cams.p;
-    // crowded: the last call that reported back saw more than kHotKey visible points in one (view, bin, tile) group
-    STAGE(ctx, TRIPS_STAGE_BIN_POINTS, bin_count_launches((int)N, B), st,
-          launch_bin_count(sp, cams, g, *params, B, fb, wait_for_sizes ? ~0ull : (unsigned long long)ctx->entry_cap, ctx->crowded, ctx->sm_count, st));
-    if (wait_for_sizes)
-    {
-        CU_CHECK(ctx, cudaMemcpyAsync(h_stats, ctx->stats.p, sizeof(DevStats), cudaMemcpyDeviceToHost, st));
-        CU_CHECK(ctx, cudaStreamSynchronize(st));
-        CU_CHECK(ctx, ensure_entries(ctx, (size_t)h_stats->visible, C, kGrowth));
-        ctx->crowded = h_stats->max_key >= kHotKey;  // this call's own count pass already knows
-        fb           = fwd_buffers(ctx, B);
-    }
-    STAGE(ctx, TRIPS_STAGE_BIN_POINTS, bin_scatter_launches((int)N, B), st, launch_bin_scatter(sp, cams, g, *params, B, fb, ctx->crowded, ctx->sm_count, st));
-    if (N > 0) STAGE(ctx, TRIPS_STAGE_COUNT, 1, st, launch_count(sp, g, B, fb, strict_layers(*params), wait_for_sizes ? (unsigned long long)h_stats->visible : ctx->need_entries, ctx->sm_count, st));
-    {
+    unsigned long long entries = ctx->need_entries;  // as far as the host knows
+
+    // ---- the steps of a pass ----
+    auto write_lists = [&](bool sized) -> int {  // entries, list lengths, list starts; sized: the list buffer is grown behind it
+        STAGE(ctx, TRIPS_STAGE_BIN_POINTS, bin_scatter_launches((int)N, B), st, launch_bin_scatter(sp, cams, g, *params, B, fb, ctx->crowded, ctx->sm_count, st));
+        if (N > 0) STAGE(ctx, TRIPS_STAGE_COUNT, 1, st, launch_count(sp, g, B, fb, strict_layers(*params), entries, ctx->sm_count, st));
         FwdBuffers fscan = fb;
-        if (wait_for_sizes) fscan.frag_cap = ~0ull;  // sizing pass: the list buffer is grown below, nothing can overflow yet
+        if (sized) fscan.frag_cap = ~0ull;
         STAGE(ctx, TRIPS_STAGE_SCAN, 1, st, launch_list_starts(g, B, params->k_keep, fscan, st));
-    }
-    CU_CHECK(ctx, cudaMemcpyAsync(h_stats, ctx->stats.p, sizeof(DevStats), cudaMemcpyDeviceToHost, st));
-    if (wait_for_sizes)
-    {
-        CU_CHECK(ctx, cudaStreamSynchronize(st));
+        CU_CHECK(ctx, cudaMemcpyAsync(h_stats, ctx->stats.p, sizeof(DevStats), cudaMemcpyDeviceToHost, st));
+        return TRIPS_OK;
+    };
+    auto render = [&]() -> int {
+        if (N > 0) STAGE(ctx, TRIPS_STAGE_COLLECT, 1, st, launch_collect(sp, g, B, fb, strict_layers(*params), entries, ctx->sm_count, st));
+        LayerPtrs out{};
+        for (int l = 0; l < g.L; ++l) out.p[l] = out_layers[l] + out_view_offset * (size_t)C * g.W[l] * g.H[l];
+        if (second_pipeline(*params))
+            STAGE(ctx, TRIPS_STAGE_SORT_BLEND, 1, st, launch_second_blend(sp, g, *params, B, fb, out, ctx->sm_count, st));
+        else
+            STAGE(ctx, TRIPS_STAGE_SORT_BLEND, 2, st, [&]() -> cudaError_t {
+                cudaError_t e = launch_heavy_topk(g, B, fb, ctx->sm_count, st);
+                return e != cudaSuccess ? e : launch_sort_blend(sp, g, *params, B, fb, out, ctx->sm_count, st);
+            }());
+        return TRIPS_OK;
+    };
+    auto grow_entries = [&]() -> int {
+        CU_CHECK(ctx, ensure_entries(ctx, (size_t)h_stats->visible, C, kGrowth));
+        ctx->crowded = h_stats->max_key >= kHotKey;  // this pass's own counts already know
+        entries      = h_stats->visible;
+        fb           = fwd_buffers(ctx, B);
+        return TRIPS_OK;
+    };
+    auto grow_lists = [&]() -> int {
         if ((size_t)h_stats->frag_need * sizeof(uint4) > ctx->frags.bytes)
         {
             CU_CHECK(ctx, ensure(ctx->frags, (size_t)h_stats->frag_need * sizeof(uint4), kGrowth));
             fb = fwd_buffers(ctx, B);
         }
+        return TRIPS_OK;
+    };
+#define STEP(expr)                             \
+    do                                         \
+    {                                          \
+        const int _rc = (expr);                \
+        if (_rc != TRIPS_OK) return _rc;       \
+    } while (0)
+
+    // crowded: the last pass that reported back saw more than kHotKey visible points in one (view, bin, tile) group
+    STAGE(ctx, TRIPS_STAGE_BIN_POINTS, bin_count_launches((int)N, B), st,
+          launch_bin_count(sp, cams, g, *params, B, fb, sizes == Sizes::wait ? ~0ull : (unsigned long long)ctx->entry_cap, ctx->crowded, ctx->sm_count, st));
+    if (sizes == Sizes::wait)
+    {
+        CU_CHECK(ctx, cudaMemcpyAsync(h_stats, ctx->stats.p, sizeof(DevStats), cudaMemcpyDeviceToHost, st));
+        CU_CHECK(ctx, cudaStreamSynchronize(st));
+        STEP(grow_entries());
+        STEP(write_lists(true));
+        CU_CHECK(ctx, cudaStreamSynchronize(st));
+        STEP(grow_lists());
+        STEP(render());
+    }
+    else
+    {
+        STEP(write_lists(false));
+        CU_CHECK(ctx, cudaEventRecord(ctx->totals_ev, st));
+        ctx->pending = sizes == Sizes::later;
+        STEP(render());
+    }
+    if (sizes == Sizes::look)
+    {
+        CU_CHECK(ctx, cudaEventSynchronize(ctx->totals_ev));
+        const bool entries_fit = h_stats->visible <= ctx->entry_cap;
+        ctx->crowded           = h_stats->max_key >= kHotKey;
+        if (!entries_fit)
+        {
+            STEP(grow_entries());
+            STAGE(ctx, TRIPS_STAGE_BIN_POINTS, 1, st, launch_place_views(B, fb, true, st));
+            STEP(write_lists(true));
+            CU_CHECK(ctx, cudaStreamSynchronize(st));
+        }
+        if (!entries_fit || (size_t)h_stats->frag_need * sizeof(uint4) > ctx->frags.bytes)
+        {
+            STEP(grow_lists());
+            if (entries_fit) STAGE(ctx, TRIPS_STAGE_SCAN, 1, st, launch_place_views(B, fb, false, st));
+            STEP(render());
+        }
+    }
+#undef STEP
+    if (sizes != Sizes::later)
+    {
         ctx->need_entries = h_stats->visible;
         ctx->need_frags   = h_stats->frag_need;
         ctx->host_stats.visible_points += (int64_t)h_stats->visible;
@@ -510,21 +575,6 @@ static int forward_views(TripsContext* ctx, const TripsScene* scene, const Trips
         ctx->host_stats.max_list_length = std::max<int64_t>(ctx->host_stats.max_list_length, (int64_t)h_stats->max_len);
         ctx->host_stats.culled_point_blocks += (int64_t)h_stats->culled_blocks;
     }
-    else
-    {
-        CU_CHECK(ctx, cudaEventRecord(ctx->totals_ev, st));
-        ctx->pending = true;
-    }
-    if (N > 0) STAGE(ctx, TRIPS_STAGE_COLLECT, 1, st, launch_collect(sp, g, B, fb, strict_layers(*params), wait_for_sizes ? (unsigned long long)h_stats->visible : ctx->need_entries, ctx->sm_count, st));
-    LayerPtrs out{};
-    for (int l = 0; l < g.L; ++l) out.p[l] = out_layers[l] + out_view_offset * (size_t)C * g.W[l] * g.H[l];
-    if (second_pipeline(*params))
-        STAGE(ctx, TRIPS_STAGE_SORT_BLEND, 1, st, launch_second_blend(sp, g, *params, B, fb, out, ctx->sm_count, st));
-    else
-        STAGE(ctx, TRIPS_STAGE_SORT_BLEND, 2, st, [&]() -> cudaError_t {
-            cudaError_t e = launch_heavy_topk(g, B, fb, ctx->sm_count, st);
-            return e != cudaSuccess ? e : launch_sort_blend(sp, g, *params, B, fb, out, ctx->sm_count, st);
-        }());
     ctx->B       = B;
     return TRIPS_OK;
 }
@@ -590,7 +640,7 @@ int trips_forward(TripsContext* ctx, const TripsScene* scene, const TripsView* v
                 steady = ensure(ctx->frags, (size_t)ctx->need_frags * sizeof(uint4), kGrowth) == cudaSuccess;
             (void)cudaGetLastError();
         }
-        const int rc = forward_views(ctx, scene, views, B, params, g, out_layers, 0, scene->dropout, st, !steady);
+        const int rc = forward_views(ctx, scene, views, B, params, g, out_layers, 0, scene->dropout, st, steady ? Sizes::later : Sizes::wait);
         if (rc != TRIPS_OK)
         {
             ctx->have_sizes = false;
@@ -610,31 +660,9 @@ int trips_forward(TripsContext* ctx, const TripsScene* scene, const TripsView* v
             const int nb = std::min(kEvalSubBatch, B - b0);
             // With buffers from an earlier pass at hand everything is launched at once and the sizes are looked at afterwards, while the
             // collect pass and the blend run: waiting for them in between left the GPU idle twice per pass (640x480 frame of 200 k
-            // points 209 -> 185 us, 1080p frame of 6 M 774 -> 758, the latter with the binning pass made faster in between).  If they did
-            // not fit, the views are rendered again with the sizes known.
-            bool rendered = false;
-            if (ctx->frags.p && ctx->entries.p && ctx->entry_C == scene->channels)
-            {
-                int rc = forward_views(ctx, scene, views + b0, nb, params, g, out_layers, (size_t)b0, nullptr, st, false);
-                if (rc != TRIPS_OK) return rc;
-                const TripsStats before = ctx->host_stats;
-                rc = resolve_pending(ctx);
-                if (rc != TRIPS_OK) return rc;
-                const TripsStats now = ctx->host_stats;
-                ctx->host_stats      = before;
-                rendered = ctx->need_entries <= ctx->entry_cap && (size_t)ctx->need_frags * sizeof(uint4) <= ctx->frags.bytes;
-                if (rendered)
-                {
-                    ctx->host_stats.visible_points += now.visible_points;
-                    ctx->host_stats.fragments += now.fragments;
-                    ctx->host_stats.kept_fragments += now.kept_fragments;
-                    ctx->host_stats.max_list_length = std::max(before.max_list_length, now.max_list_length);
-                    ctx->host_stats.culled_point_blocks += now.culled_point_blocks;
-                }
-            }
-            if (rendered) continue;
-            const int rc = forward_views(ctx, scene, views + b0, nb, params, g, out_layers, (size_t)b0,
-                                         nullptr, st, true);
+            // points 209 -> 185 us, 1080p frame of 6 M 774 -> 758, the latter with the binning pass made faster in between).
+            const bool buffers = ctx->frags.p && ctx->entries.p && ctx->entry_C == scene->channels;
+            const int rc = forward_views(ctx, scene, views + b0, nb, params, g, out_layers, (size_t)b0, nullptr, st, buffers ? Sizes::look : Sizes::wait);
             if (rc != TRIPS_OK) return rc;
         }
     }

@@ -88,6 +88,7 @@ struct DevStats
     unsigned int max_key;          // largest number of visible points in one (view, screen bin, tile) group
     unsigned int n_shared;         // parts of shared lists among them
     unsigned int status;
+    unsigned int given_up;       // an inference pass that does not fit the buffers: its blend writes nothing, the host takes it up again
     unsigned int culled_blocks;  // (view, block of consecutive points) pairs skipped by the bounding-box test, counted once per pass
 };
 
@@ -129,7 +130,7 @@ struct FwdBuffers
     unsigned long long* view_base;    // [B+1] first fragment of each view in `frags`
     uint4* frags;                     // [frag_cap] x = point id, y = depth bits (y:x = 64-bit sort key), z = alpha bits, w = entry index within the view
     unsigned long long frag_cap;
-    bool report_overflow;             // raise a status bit for views that do not fit (off where the host looks and renders again)
+    bool report_overflow;             // training: raise a status bit for views that do not fit; off where the host looks (place_views)
     uint8_t* rec_n;                   // [B,n_tiles,32] records kept for backward, by tile and lane (pixel of the tile)
     uint2* records;                   // [B,n_tiles,16,32] (entry index within the view, alpha bits), by tile, rank and lane: a warp's
                                       // access to one rank of its tile is 256 consecutive bytes
@@ -139,7 +140,7 @@ struct FwdBuffers
     unsigned int* ticket_count;       // [B] count pass
     unsigned int* ticket_collect;     // [B] collect pass
     unsigned int* ticket_blend;
-    unsigned int* finished;           // [2] blocks that are done, of the bin scan and of list_starts_kernel
+    unsigned int* finished;           // [2] blocks that are done, of the bin scan and of list_starts_kernel (which clears it again)
     uint32_t* list_cursor;            // [B] fragments of the views as list_starts_kernel adds them up
     uint32_t* point_entry;            // training: [entry_views,N] entry (within the view) of every point, kNoEntry where it is not visible
     int entry_views;                  // B, or fewer where the table of all views would be larger than kEntryTableBytes: the backward
@@ -435,6 +436,7 @@ size_t resize_scratch_bytes(int64_t n_points);
 cudaError_t launch_resize_points(const int64_t* remove, int64_t n_remove, int64_t n_points, int64_t n_new, const TripsPointTensor* tensors,
                                  int n_tensors, void* scratch, DevStats* stats, int sm_count, cudaStream_t st);
 cudaError_t launch_list_starts(const Geom& g, int B, int k_keep, const FwdBuffers& fb, cudaStream_t st);
+cudaError_t launch_place_views(int B, const FwdBuffers& fb, bool entries, cudaStream_t st);  // of the entries, or of the lists
 // strict: an entry's layers start at the layer below log2(size) instead of layer 0 (strict_layers above)
 // entries_hint: the number of entries of the call as far as the host knows it (selects the size of the work tickets)
 cudaError_t launch_count(const ScenePtrs& sc, const Geom& g, int B, const FwdBuffers& fb, bool strict, unsigned long long entries_hint, int sm_count,

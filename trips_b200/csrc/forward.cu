@@ -30,7 +30,7 @@ __global__ void setup_cams_kernel(const __grid_constant__ ViewTable views, int b
         // the counters of the call start from zero; the status word keeps the bits raised by earlier calls until
         // trips_last_status reads them
         stats->visible = stats->kept = stats->frag_need = 0ull;
-        stats->max_len = stats->n_heavy = stats->max_key = stats->n_shared = stats->culled_blocks = 0u;
+        stats->max_len = stats->n_heavy = stats->max_key = stats->n_shared = stats->culled_blocks = stats->given_up = 0u;
     }
     if (b >= B) return;
     const TripsView& v = views.v[threadIdx.x];
@@ -393,24 +393,30 @@ __device__ __forceinline__ bool last_block(unsigned* finished, unsigned n)
     return s_last != 0;
 }
 
-// First entry of every view in the entry arrays.  A view whose entries do not fit the arrays (entry_cap entries: the
-// arrays are sized from the previous call's count, not for the worst case) gets none: it renders as background, the
-// status word says so and stats->visible still carries the number that was needed, so that the host grows the arrays.
-__device__ __forceinline__ void first_entries(const uint32_t* view_total, int B, unsigned long long entry_cap, unsigned long long* entry_base, bool report, DevStats* stats)
+// Where every view starts in a buffer of `cap` places, of which view b needs totals[b]: in the entry arrays and in the list buffer, which
+// are sized from an earlier pass, not for the worst case.  In a training pass (report) a view that does not fit gets no places: it renders
+// as background, the status word says so, and the host grows the buffer behind the number that was needed.  An inference pass that does
+// not fit as a whole is given up: no view gets any places, so that the kernels behind have nothing to do, and the host takes it up again
+// here once the buffer is large enough (launch_place_views).
+__device__ __forceinline__ void place_views(const uint32_t* totals, int B, unsigned long long cap, unsigned long long* base, bool report, unsigned status,
+                                            unsigned long long* need, DevStats* stats)
 {
-    unsigned long long base = 0, need = 0;
+    unsigned long long at = 0, sum = 0;
     for (int b = 0; b < B; ++b)
     {
-        const uint32_t n = __ldcg(view_total + b);
-        entry_base[b]    = base;
-        need += n;
-        if (base + n <= entry_cap)
-            base += n;
+        const uint32_t n = __ldcg(totals + b);
+        base[b]          = at;
+        sum += n;
+        if (at + n <= cap)
+            at += n;
         else if (report)
-            atomicOr(&stats->status, TRIPS_DEV_ENTRY_OVERFLOW);
+            atomicOr(&stats->status, status);
     }
-    entry_base[B]  = base;
-    stats->visible = need;
+    base[B] = at;
+    *need   = sum;
+    if (report || sum <= cap) return;
+    for (int b = 0; b <= B; ++b) base[b] = 0;
+    stats->given_up = 1;
 }
 
 __global__ __launch_bounds__(1024) void bin_scan_kernel(const uint32_t* counts, uint32_t* key_first,
@@ -470,7 +476,7 @@ __global__ __launch_bounds__(1024) void bin_scan_kernel(const uint32_t* counts, 
         __syncthreads();  // the warp sums are overwritten by the next turn
     }
     if (threadIdx.x == 0) view_total[b] = carry;
-    if (last_block(finished, gridDim.x) && threadIdx.x == 0) first_entries(view_total, (int)gridDim.x, entry_cap, entry_base, report, stats);
+    if (last_block(finished, gridDim.x) && threadIdx.x == 0) place_views(view_total, (int)gridDim.x, entry_cap, entry_base, report, TRIPS_DEV_ENTRY_OVERFLOW, &stats->visible, stats);
 }
 
 // One 32-byte store (sm_100 has 256-bit global stores) for the two float4 halves of a 32-byte-aligned record: half the
@@ -583,6 +589,7 @@ __global__ __launch_bounds__(kBinThreads, (C <= 4 ? kScatterMinBlocks : kScatter
     __syncthreads();
     unsigned no_room = 0;  // views without entries: nothing visible, or the view did not fit the entry arrays
     for (int v = 0; v < nv; ++v) no_room |= (s_ebase[v + 1] == s_ebase[v] ? 1u : 0u) << v;
+    if (!fb.point_state && s_ebase[0] == s_ebase[nv]) return;  // nothing to write (a training pass still notes its points)
     const bool use_dropout = pr.train && sc.dropout;
     int first, last;
     unsigned skip;
@@ -761,6 +768,7 @@ __global__ __launch_bounds__(kBinThreads) void bin_scatter_hot_kernel(ScenePtrs 
     __syncthreads();
     unsigned no_room = 0;  // views without entries: nothing visible, or the view did not fit the entry arrays
     for (int v = 0; v < nv; ++v) no_room |= (s_ebase[v + 1] == s_ebase[v] ? 1u : 0u) << v;
+    if (!fb.point_state && s_ebase[0] == s_ebase[nv]) return;  // nothing to write (a training pass still notes its points)
     const bool use_dropout = pr.train && sc.dropout;
     const uint32_t n_keys  = (uint32_t)g.n_bins << kSubShift;
     uint32_t* cursors      = fb.bin_base + (size_t)v0 * n_keys;
@@ -1002,21 +1010,25 @@ __global__ __launch_bounds__(kScanThreads) void list_starts_kernel(const uint32_
         run += __shfl_sync(kFull, incl, 31);
     }
     if (!last_block(finished, gridDim.x * gridDim.y) || threadIdx.x != 0) return;
-    // First fragment of every view.  A view that does not fit the list buffer (sized from the previous call) gets no fragments at
-    // all: the collect pass skips it and the blend treats its lists as empty.
-    unsigned long long at = 0, need = 0;
-    for (int w = 0; w < (int)gridDim.y; ++w)
-    {
-        const uint32_t n = __ldcg(cursor + w);
-        view_base[w]     = at;
-        need += n;
-        if (at + n <= frag_cap)
-            at += n;
-        else if (report)
-            atomicOr(&stats->status, TRIPS_DEV_FRAGMENT_OVERFLOW);
-    }
-    view_base[gridDim.y] = at;
-    stats->frag_need     = need;
+    // First fragment of every view.  A view without places: the collect pass skips it and the blend treats its lists as empty.
+    place_views(cursor, (int)gridDim.y, frag_cap, view_base, report, TRIPS_DEV_FRAGMENT_OVERFLOW, &stats->frag_need, stats);
+    *finished = 0;  // an inference pass that was given up before this kernel runs it again
+}
+
+// Takes up an inference pass that was given up (place_views), the buffer being large enough now.
+__global__ void place_views_kernel(const uint32_t* totals, int B, unsigned long long* base, unsigned long long* need, unsigned* ticket_blend, DevStats* stats)
+{
+    follow_previous();
+    place_views(totals, B, ~0ull, base, false, 0u, need, stats);
+    stats->given_up = 0;
+    *ticket_blend   = 0;  // the blend that gave up had asked for tiles
+}
+
+cudaError_t launch_place_views(int B, const FwdBuffers& fb, bool entries, cudaStream_t st)
+{
+    launch_following(place_views_kernel, 1, 1, st, entries ? fb.view_total : fb.list_cursor, B, entries ? fb.entry_base : fb.view_base,
+                     entries ? &fb.stats->visible : &fb.stats->frag_need, fb.ticket_blend, fb.stats);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_list_starts(const Geom& g, int B, int k_keep, const FwdBuffers& fb, cudaStream_t st)
@@ -1291,10 +1303,11 @@ __global__ __launch_bounds__(THREADS, kWinMinWarps * 32 / THREADS) void window_k
     // where blocks cross over), which keeps the partially written list sectors of a view in L2 until they are complete
     for (int b = 0; b < B; ++b)
     {
-    if (COLLECT && fb.view_base[b + 1] == fb.view_base[b]) continue;  // no fragments, or the view did not fit the list buffer (status bit raised by the scan)
+    if (COLLECT && fb.view_base[b + 1] == fb.view_base[b]) continue;  // no fragments, or the view did not fit the list buffer
     uint32_t* pixel_ctr   = (COLLECT ? fb.offsets : fb.counts) + (size_t)b * g.P;
     uint4* frags          = fb.frags + fb.view_base[COLLECT ? b : 0];
     const uint32_t n_entry = (uint32_t)(fb.entry_base[b + 1] - fb.entry_base[b]);
+    if (!COLLECT && n_entry == 0) continue;  // (no ticket is taken: the pass may be taken up again)
     const float4* head     = fb.ent_head + fb.entry_base[b] * 2;
     const uint32_t* bfirst = fb.bin_cursor + (size_t)b * g.n_bins;
     uint32_t c0, c1;
@@ -1731,6 +1744,7 @@ __global__ __launch_bounds__(kSbThreads, (C <= 4 ? kSbMinBlocks : (C <= 8 ? kSbM
     const bool preselected = fb.stats->n_heavy <= fb.heavy.cap;  // heavy_topk_kernel handled every long list
     unsigned next_ticket = 0;
     if (lane == 0) next_ticket = atomicAdd(fb.ticket_blend, 1u);
+    if (fb.stats->given_up) return;  // (looked at while the first ticket is on its way)
     for (;;)
     {
         // the ticket of the following tile is requested now, a whole tile ahead of its use
