@@ -426,7 +426,8 @@ enum class Sizes
     later,  // the buffers keep the capacity found by earlier calls (need x 1.25) and nothing is waited for: the totals travel to pinned
             // host memory behind an event, and the next training call reads them
     look,   // an inference pass: everything is launched with the buffers as they are, and the totals are looked at while the GPU
-            // renders.  A pass that does not fit is given up on the device (place_views) and taken up from where it stopped
+            // renders.  A pass that does not fit them, or calls for other kernels, is given up on the device (place_views) and taken up
+            // from where it stopped
 };
 
 // One pass over `B` views (all views of a training call; up to kEvalSubBatch views of an inference call).
@@ -527,7 +528,8 @@ static int forward_views(TripsContext* ctx, const TripsScene* scene, const Trips
 
     // crowded: the last pass that reported back saw more than kHotKey visible points in one (view, bin, tile) group
     STAGE(ctx, TRIPS_STAGE_BIN_POINTS, bin_count_launches((int)N, B), st,
-          launch_bin_count(sp, cams, g, *params, B, fb, sizes == Sizes::wait ? ~0ull : (unsigned long long)ctx->entry_cap, ctx->crowded, ctx->sm_count, st));
+          launch_bin_count(sp, cams, g, *params, B, fb, sizes == Sizes::wait ? ~0ull : (unsigned long long)ctx->entry_cap,
+                           PassGuess{sizes == Sizes::look, ctx->crowded, entries}, ctx->sm_count, st));
     if (sizes == Sizes::wait)
     {
         CU_CHECK(ctx, cudaMemcpyAsync(h_stats, ctx->stats.p, sizeof(DevStats), cudaMemcpyDeviceToHost, st));
@@ -548,19 +550,19 @@ static int forward_views(TripsContext* ctx, const TripsScene* scene, const Trips
     if (sizes == Sizes::look)
     {
         CU_CHECK(ctx, cudaEventSynchronize(ctx->totals_ev));
-        const bool entries_fit = h_stats->visible <= ctx->entry_cap;
+        const GivenUp given_up = h_stats->given_up;
         ctx->crowded           = h_stats->max_key >= kHotKey;
-        if (!entries_fit)
+        if (given_up == kGivenUpEntries)
         {
             STEP(grow_entries());
             STAGE(ctx, TRIPS_STAGE_BIN_POINTS, 1, st, launch_place_views(B, fb, true, st));
             STEP(write_lists(true));
             CU_CHECK(ctx, cudaStreamSynchronize(st));
         }
-        if (!entries_fit || (size_t)h_stats->frag_need * sizeof(uint4) > ctx->frags.bytes)
+        if (given_up != kNotGivenUp)
         {
             STEP(grow_lists());
-            if (entries_fit) STAGE(ctx, TRIPS_STAGE_SCAN, 1, st, launch_place_views(B, fb, false, st));
+            if (given_up == kGivenUpLists) STAGE(ctx, TRIPS_STAGE_SCAN, 1, st, launch_place_views(B, fb, false, st));
             STEP(render());
         }
     }
@@ -962,7 +964,11 @@ static int read_lists(TripsContext* ctx, int view, cudaStream_t st, std::vector<
     CU_CHECK(ctx, cudaMemcpyAsync(counts.data(), (const uint32_t*)((const char*)ctx->zeroed.p + ctx->zero_counts) + off, sizeof(uint32_t) * P, cudaMemcpyDeviceToHost, st));
     CU_CHECK(ctx, cudaMemcpyAsync(starts.data(), (uint32_t*)ctx->offsets.p + off, sizeof(uint32_t) * P, cudaMemcpyDeviceToHost, st));
     CU_CHECK(ctx, cudaStreamSynchronize(st));
-    if (vb[1] == vb[0]) return TRIPS_OK;  // no fragments, or the view did not fit: the collect pass has skipped it
+    if (vb[1] == vb[0])  // no fragments, or the view did not fit: the collect pass has skipped it
+    {
+        starts.assign(P, 0);
+        return TRIPS_OK;
+    }
     for (size_t i = 0; i < P; ++i) starts[i] -= counts[i];  // the collect pass advanced the starts to the list ends
     if (!lists_cover(starts.data(), counts.data(), P, vb[1] - vb[0]))
         return fail(ctx, TRIPS_ERR_CUDA, "the lists of the view overlap or leave their part of the list buffer (internal error)");

@@ -77,6 +77,14 @@ struct ConstLayerPtrs
     const float* p[TRIPS_MAX_LAYERS];
 };
 
+// Where an inference pass was given up because it does not suit what it was launched with (place_views in forward.cu).
+enum GivenUp : unsigned int
+{
+    kNotGivenUp,
+    kGivenUpEntries,  // before its entries were written: they do not fit, or PassGuess was wrong
+    kGivenUpLists,    // before its lists were written: they do not fit
+};
+
 // Device-side counters of one forward call.
 struct DevStats
 {
@@ -88,7 +96,7 @@ struct DevStats
     unsigned int max_key;          // largest number of visible points in one (view, screen bin, tile) group
     unsigned int n_shared;         // parts of shared lists among them
     unsigned int status;
-    unsigned int given_up;       // an inference pass that does not fit the buffers: its blend writes nothing, the host takes it up again
+    GivenUp given_up;            // an inference pass: its remaining kernels write nothing, the host takes it up again
     unsigned int culled_blocks;  // (view, block of consecutive points) pairs skipped by the bounding-box test, counted once per pass
 };
 
@@ -140,7 +148,7 @@ struct FwdBuffers
     unsigned int* ticket_count;       // [B] count pass
     unsigned int* ticket_collect;     // [B] collect pass
     unsigned int* ticket_blend;
-    unsigned int* finished;           // [2] blocks that are done, of the bin scan and of list_starts_kernel (which clears it again)
+    unsigned int* finished;           // [2] blocks that are done, of the bin scan and of list_starts_kernel
     uint32_t* list_cursor;            // [B] fragments of the views as list_starts_kernel adds them up
     uint32_t* point_entry;            // training: [entry_views,N] entry (within the view) of every point, kNoEntry where it is not visible
     int entry_views;                  // B, or fewer where the table of all views would be larger than kEntryTableBytes: the backward
@@ -425,8 +433,19 @@ struct TileTickets
 cudaError_t launch_setup_cams(const TripsView* h_views, int B, const double* poses, int n_images, const float* intrinsics,
                               int n_cameras, int distortion, float dist_cutoff, CamConst* cams, DevStats* stats, cudaStream_t st);
 constexpr int kViewTable = 32;  // views passed to one launch of setup_cams_kernel as an argument;
+// What the kernels of a pass are launched with before its counts are known.
+struct PassGuess
+{
+    bool look;                   // the host looks at the counts while the pass runs: one that the guess does not suit is given up
+    bool hot;                    // binning kernels that aggregate in shared memory (kHotKey)
+    unsigned long long entries;  // the size of the window passes' tickets and grids
+};
+// More entries than kGuessFactor times the guess, and at least kGuessEntries: too few blocks for them.  One 1080p view taken in turn with
+// one that sees less, us, with the guess of that one / its own: 7.0 M entries (6 times the guess) 1370 / 1361, (28 times) 1502 / 1361,
+// 13.9 M (33 times) 2609 / 2415, 1.4 M (6 to 1000 times) 562 / 523; a pass that is given up takes 50 longer.
+constexpr unsigned long long kGuessFactor = 8, kGuessEntries = 2ull << 20;
 cudaError_t launch_bin_count(const ScenePtrs& sc, const CamConst* cams, const Geom& g, const TripsRenderParams& pr, int B,
-                             const FwdBuffers& fb, unsigned long long entry_cap, bool hot, int sm_count, cudaStream_t st);
+                             const FwdBuffers& fb, unsigned long long entry_cap, PassGuess guess, int sm_count, cudaStream_t st);
 cudaError_t launch_bin_scatter(const ScenePtrs& sc, const CamConst* cams, const Geom& g, const TripsRenderParams& pr, int B,
                                const FwdBuffers& fb, bool hot, int sm_count, cudaStream_t st);
 constexpr unsigned kHotKey = 4096;  // visible points in one (view, bin, tile) group beyond which the binning passes aggregate in shared memory

@@ -30,7 +30,8 @@ __global__ void setup_cams_kernel(const __grid_constant__ ViewTable views, int b
         // the counters of the call start from zero; the status word keeps the bits raised by earlier calls until
         // trips_last_status reads them
         stats->visible = stats->kept = stats->frag_need = 0ull;
-        stats->max_len = stats->n_heavy = stats->max_key = stats->n_shared = stats->culled_blocks = stats->given_up = 0u;
+        stats->max_len = stats->n_heavy = stats->max_key = stats->n_shared = stats->culled_blocks = 0u;
+        stats->given_up = kNotGivenUp;
     }
     if (b >= B) return;
     const TripsView& v = views.v[threadIdx.x];
@@ -394,12 +395,12 @@ __device__ __forceinline__ bool last_block(unsigned* finished, unsigned n)
 }
 
 // Where every view starts in a buffer of `cap` places, of which view b needs totals[b]: in the entry arrays and in the list buffer, which
-// are sized from an earlier pass, not for the worst case.  In a training pass (report) a view that does not fit gets no places: it renders
-// as background, the status word says so, and the host grows the buffer behind the number that was needed.  An inference pass that does
-// not fit as a whole is given up: no view gets any places, so that the kernels behind have nothing to do, and the host takes it up again
-// here once the buffer is large enough (launch_place_views).
-__device__ __forceinline__ void place_views(const uint32_t* totals, int B, unsigned long long cap, unsigned long long* base, bool report, unsigned status,
-                                            unsigned long long* need, DevStats* stats)
+// are sized from an earlier pass, not for the worst case.  In a training pass a view that does not fit gets no places: it renders
+// as background, the status word says so (status_bit), and the host grows the buffer behind the number that was needed.  An inference pass
+// (status_bit 0) that needs more than `most` is given up: no view gets any places, so that the kernels behind have nothing to do, and the
+// host takes it up again here (launch_place_views).
+__device__ __forceinline__ void place_views(const uint32_t* totals, int B, unsigned long long cap, unsigned long long most, unsigned long long* base,
+                                            unsigned status_bit, GivenUp where, unsigned long long* need, DevStats* stats)
 {
     unsigned long long at = 0, sum = 0;
     for (int b = 0; b < B; ++b)
@@ -409,19 +410,19 @@ __device__ __forceinline__ void place_views(const uint32_t* totals, int B, unsig
         sum += n;
         if (at + n <= cap)
             at += n;
-        else if (report)
-            atomicOr(&stats->status, status);
+        else if (status_bit)
+            atomicOr(&stats->status, status_bit);
     }
     base[B] = at;
     *need   = sum;
-    if (report || sum <= cap) return;
+    if (status_bit || sum <= most) return;
     for (int b = 0; b <= B; ++b) base[b] = 0;
-    stats->given_up = 1;
+    stats->given_up = where;
 }
 
 __global__ __launch_bounds__(1024) void bin_scan_kernel(const uint32_t* counts, uint32_t* key_first,
                                                         uint32_t* bin_first, int n_keys, uint32_t* view_total, unsigned long long entry_cap,
-                                                        unsigned long long* entry_base, bool report, unsigned* finished, DevStats* stats)
+                                                        unsigned long long* entry_base, bool report, PassGuess guess, unsigned* finished, DevStats* stats)
 {
     follow_previous();
     __shared__ uint32_t sm[32];
@@ -476,7 +477,18 @@ __global__ __launch_bounds__(1024) void bin_scan_kernel(const uint32_t* counts, 
         __syncthreads();  // the warp sums are overwritten by the next turn
     }
     if (threadIdx.x == 0) view_total[b] = carry;
-    if (last_block(finished, gridDim.x) && threadIdx.x == 0) place_views(view_total, (int)gridDim.x, entry_cap, entry_base, report, TRIPS_DEV_ENTRY_OVERFLOW, &stats->visible, stats);
+    if (!last_block(finished, gridDim.x) || threadIdx.x != 0) return;
+    // An inference pass was launched with the kernels that suit the pass before.  One that calls for the other scatter kernel or has many
+    // more entries is given up as well: the host now knows better.  Two views of a cloud in turn, us, with the kernels of the view before /
+    // given up: 3 M points in 100x100 pixels and near by 1788 / 1615 for the pair, 20 M points after a view that sees 0.4 M of them
+    // 2609 / 2450.  In passes of 8 views the scatter kernel matters less than the time it takes to give up: 13.59 / 13.73 ms for 32 views.
+    unsigned long long most = entry_cap;
+    if (guess.look)
+    {
+        most = min(most, max(kGuessFactor * guess.entries, kGuessEntries));
+        if ((__ldcg(&stats->max_key) >= kHotKey) != guess.hot) most = 0;
+    }
+    place_views(view_total, (int)gridDim.x, entry_cap, most, entry_base, report ? TRIPS_DEV_ENTRY_OVERFLOW : 0u, kGivenUpEntries, &stats->visible, stats);
 }
 
 // One 32-byte store (sm_100 has 256-bit global stores) for the two float4 halves of a 32-byte-aligned record: half the
@@ -663,8 +675,8 @@ __global__ __launch_bounds__(kBinThreads, (C <= 4 ? kScatterMinBlocks : kScatter
 // table (linear probing, at most four probes; a key that finds no slot simply uses the global counter directly), and
 // touches the global counter of every key it met once per ticket.  In the scatter pass that one returning atomic
 // reserves a range of the key's entries for the whole ticket, and the slots inside the range come from the table.
-// The host selects these variants when the previous call (or, in a sized call, this call's own count pass) saw more
-// than kHotKey visible points in one (view, bin, tile) group; ordinary scenes never do and run the kernels above.
+// They run when the previous pass saw more than kHotKey visible points in one (view, bin, tile) group; the scatter pass of an inference or
+// a sized call goes by its own counts (bin_scan_kernel); ordinary scenes never do and run the kernels above.
 // ------------------------------------------------------------------------------------------------------------
 constexpr int kHotTicket        = 2048;
 constexpr int kHotSlots         = 2048;
@@ -846,8 +858,9 @@ __global__ __launch_bounds__(kBinThreads) void bin_scatter_hot_kernel(ScenePtrs 
 // Count pass of the binning stage: bounding boxes, visible points per (view, bin, tile), their exclusive scan and the
 // first entry of every view.  After it fb.view_total / stats->visible say how many entries the scatter pass will write.
 cudaError_t launch_bin_count(const ScenePtrs& sc, const CamConst* cams, const Geom& g, const TripsRenderParams& pr, int B,
-                             const FwdBuffers& fb, unsigned long long entry_cap, bool hot, int sm_count, cudaStream_t st)
+                             const FwdBuffers& fb, unsigned long long entry_cap, PassGuess guess, int sm_count, cudaStream_t st)
 {
+    const bool hot     = guess.hot;
     const int n_keys   = g.n_bins << kSubShift;
     const int grid     = sm_count * kBinBlocksPerSM;
     const int n_groups = (B + kViewGroup - 1) / kViewGroup;
@@ -867,7 +880,7 @@ cudaError_t launch_bin_count(const ScenePtrs& sc, const CamConst* cams, const Ge
             else
                 launch_following(bin_count_kernel<false>, grid, kBinThreads, st, sc, cams, g, pr, fb, v0, nv, fb.ticket + gi);
         }
-    launch_following(bin_scan_kernel, B, 1024, st, fb.bin_count, fb.bin_base, fb.bin_cursor, n_keys, fb.view_total, entry_cap, fb.entry_base, fb.report_overflow, fb.finished, fb.stats);
+    launch_following(bin_scan_kernel, B, 1024, st, fb.bin_count, fb.bin_base, fb.bin_cursor, n_keys, fb.view_total, entry_cap, fb.entry_base, fb.report_overflow, guess, fb.finished, fb.stats);
     return cudaGetLastError();
 }
 
@@ -929,7 +942,7 @@ __device__ __forceinline__ uint32_t warp_incl_scan(uint32_t v, int lane)
 
 // A warp takes 32 consecutive lengths at a time, kScanPerLane times: the lists of neighbouring pixels are neighbours.
 // cursor: [B] fragments of the views so far, zero before; finished: blocks that are done, zero before.
-__global__ __launch_bounds__(kScanThreads) void list_starts_kernel(const uint32_t* counts, int P, int k_keep, uint32_t* offsets, uint32_t* cursor,
+__global__ __launch_bounds__(kScanThreads) void list_starts_kernel(const unsigned long long* entry_base, const uint32_t* counts, int P, int k_keep, uint32_t* offsets, uint32_t* cursor,
                                                                    unsigned* finished, unsigned long long* view_base, unsigned long long frag_cap, bool report,
                                                                    DevStats* stats, HeavyLists heavy)
 {
@@ -942,6 +955,14 @@ __global__ __launch_bounds__(kScanThreads) void list_starts_kernel(const uint32_
     uint32_t v[kScanPerLane], sum = 0, kept = 0, mx = 0;
 #pragma unroll
     for (int k = 0; k < kScanPerLane; ++k) v[k] = start + k * 32 < P ? c[start + k * 32] : 0u;
+    // No view has an entry, in a pass that was given up above all: no lists.  The collect pass must not meet the starts of an earlier
+    // pass.  (Looked at while the lengths are on their way; `stats` lies on a line that all blocks update.)
+    if (entry_base[gridDim.y] == 0)
+    {
+        if (blockIdx.x == 0 && blockIdx.y == 0)
+            for (int w = threadIdx.x; w <= (int)gridDim.y; w += kScanThreads) view_base[w] = 0;
+        return;
+    }
 #pragma unroll
     for (int k = 0; k < kScanPerLane; ++k)
     {
@@ -1011,16 +1032,15 @@ __global__ __launch_bounds__(kScanThreads) void list_starts_kernel(const uint32_
     }
     if (!last_block(finished, gridDim.x * gridDim.y) || threadIdx.x != 0) return;
     // First fragment of every view.  A view without places: the collect pass skips it and the blend treats its lists as empty.
-    place_views(cursor, (int)gridDim.y, frag_cap, view_base, report, TRIPS_DEV_FRAGMENT_OVERFLOW, &stats->frag_need, stats);
-    *finished = 0;  // an inference pass that was given up before this kernel runs it again
+    place_views(cursor, (int)gridDim.y, frag_cap, frag_cap, view_base, report ? TRIPS_DEV_FRAGMENT_OVERFLOW : 0u, kGivenUpLists, &stats->frag_need, stats);
 }
 
-// Takes up an inference pass that was given up (place_views), the buffer being large enough now.
+// Takes up an inference pass that was given up (place_views); the buffer is large enough now.
 __global__ void place_views_kernel(const uint32_t* totals, int B, unsigned long long* base, unsigned long long* need, unsigned* ticket_blend, DevStats* stats)
 {
     follow_previous();
-    place_views(totals, B, ~0ull, base, false, 0u, need, stats);
-    stats->given_up = 0;
+    place_views(totals, B, ~0ull, ~0ull, base, 0u, kNotGivenUp, need, stats);
+    stats->given_up = kNotGivenUp;
     *ticket_blend   = 0;  // the blend that gave up had asked for tiles
 }
 
@@ -1033,7 +1053,7 @@ cudaError_t launch_place_views(int B, const FwdBuffers& fb, bool entries, cudaSt
 
 cudaError_t launch_list_starts(const Geom& g, int B, int k_keep, const FwdBuffers& fb, cudaStream_t st)
 {
-    launch_following(list_starts_kernel, dim3((g.P + kScanChunk - 1) / kScanChunk, B), kScanThreads, st, fb.counts, g.P, k_keep, fb.offsets, fb.list_cursor, fb.finished + 1,
+    launch_following(list_starts_kernel, dim3((g.P + kScanChunk - 1) / kScanChunk, B), kScanThreads, st, fb.entry_base, fb.counts, g.P, k_keep, fb.offsets, fb.list_cursor, fb.finished + 1,
                                                                                     fb.view_base, fb.frag_cap, fb.report_overflow, fb.stats, fb.heavy);
     return cudaGetLastError();
 }
@@ -1744,7 +1764,7 @@ __global__ __launch_bounds__(kSbThreads, (C <= 4 ? kSbMinBlocks : (C <= 8 ? kSbM
     const bool preselected = fb.stats->n_heavy <= fb.heavy.cap;  // heavy_topk_kernel handled every long list
     unsigned next_ticket = 0;
     if (lane == 0) next_ticket = atomicAdd(fb.ticket_blend, 1u);
-    if (fb.stats->given_up) return;  // (looked at while the first ticket is on its way)
+    if (fb.stats->given_up != kNotGivenUp) return;  // (looked at while the first ticket is on its way)
     for (;;)
     {
         // the ticket of the following tile is requested now, a whole tile ahead of its use

@@ -26,7 +26,7 @@ __global__ __launch_bounds__(128) void second_blend_kernel(ScenePtrs sc, const _
 {
     constexpr int ES = tail_stride(C);
     const int K      = pr.k_keep;
-    if (fb.stats->given_up) return;
+    if (fb.stats->given_up != kNotGivenUp) return;
     const size_t total = (size_t)B * (size_t)g.P;
     float bg[C];
 #pragma unroll
