@@ -56,16 +56,18 @@ constexpr int kBwdWarps   = kBwdThreads / 32;
 //   phase 2 (lane = kept fragment): descriptor gradient and the image-space sums of the fragment's entry
 //     (RenderBackward.cu:335-393), accumulated with two vector atomics into the per-entry gradient rows, which are
 //     in screen-bin order like the entries and therefore stay hot in L2 while a region of the image is processed.
-// What bounds the kernel (ncu): about 50 % of the issue slots and 48 % of the load/store unit's line rate are in use
-// at 16-20 resident warps per SM; DRAM is at 20-30 %.  Hence the care for lines per instruction (entries ordered by
+// What bounds the kernel (ncu, one 1080p view of 6 M points): 48 % of the issue slots and 66 % of the load/store
+// unit's wavefront rate are in use at 26 active warps per SM; DRAM is at 20 %.  Hence the care for lines per instruction (entries ordered by
 // tile, paired atomics, coalesced staging) and for instructions per fragment (fragment table, no shuffle searches).
 constexpr int kBwdBlocksPerSM = 12;  // grid size of the persistent kernel, in blocks per SM
-// Resident blocks.  Shared memory allows six; with six, 16 KB of L1 are left, with five 52 KB.  Where a tile's entries are few the sixth
-// block hides more latency, where they are many its rows no longer stay in L1 between the fragments of neighbouring pixels.
-// blend_backward, six / five blocks, us, by visible points per pixel of layer 0: 0.8 281 / 322, 1.5 (6 M points x 8 views) 2752 / 2904,
-// 1.65 206 / 209, 1.84 228 / 206, 2.05 499 / 469, 2.6 1094 / 978, 2.8 290 / 257, 3.65 718 / 586.  DENSE is the variant for more than
-// 1.75: the table of fragments is written by an unrolled loop, which takes 87 registers (4 channels) instead of 72 and thereby leaves room for
-// five blocks.
+// Resident blocks: seven, and five of the variant DENSE, with 3 and 4 channels.  Seven is what 72 registers (70 with 3 channels) and 32.5 KB
+// of shared memory per block allow; the bound of six below is a minimum, and six have not been measured.  The L1 that is left holds next to
+// nothing then (1.7 % of the sectors of that view hit; 20.7 % in an earlier build with five blocks).  Where a tile's entries are few the
+// further blocks hide more latency, where they are many its rows should stay in L1 between the fragments of neighbouring pixels.
+// blend_backward, seven / five blocks, us, by visible points per pixel of layer 0: 0.8 281 / 322, 1.5 (6 M points x 8 views) 2752 / 2904,
+// 1.65 206 / 209, 1.84 228 / 206, 2.05 499 / 469, 2.6 1094 / 978, 2.8 290 / 257, 3.65 718 / 586 (4 channels).  DENSE is the variant for more
+// than 1.75: the table of fragments is written by an unrolled loop, and its 87 registers (84 with 3 channels) leave room for five blocks.
+// That is the compiler's doing (-Xptxas -v): to be looked at again when the kernel or the compiler changes.
 constexpr int kBwdMinBlocks = 6, kBwdMinBlocksDense = 5;
 inline bool dense_entries(unsigned long long entries, const Geom& g, int B) { return 4 * entries > 7ull * g.W[0] * g.H[0] * B; }
 // SAT: saturated_alpha_accumulation as the reference's backward pass has it (RenderBackward.cu:227-259); a separate

@@ -132,10 +132,10 @@ struct TripsContext
     void* h_pinned        = nullptr;
     cudaEvent_t totals_ev = nullptr;
     bool pending          = false;  // the totals of the last forward call have not been read yet
-    // sizes the last training call needed, and the shapes they belong to
+    // shapes of the last training call, while it may be followed by one of the same shapes that does not wait for its counts
     SizeKey size_key{};
     bool have_sizes                 = false;
-    unsigned long long need_entries = 0, need_frags = 0;
+    unsigned long long need_entries = 0, need_frags = 0;  // of the last pass whose totals were read (training and inference)
     int entry_C                     = 0;  // channel count the entry arrays are laid out for
     bool crowded                    = false;  // the point cloud crowds into few screen tiles: use the aggregating binning kernels
     // state of the last forward call

@@ -310,7 +310,7 @@ __device__ __forceinline__ bool discarded_for_confidence(const ScenePtrs& sc, co
     return c < pr.stability_cutoff_value;
 }
 
-// What both binning passes read of a point; requested one point ahead.
+// What the scatter pass reads of a point; requested one point ahead.
 struct PointHead
 {
     float4 p;
@@ -658,7 +658,7 @@ __global__ __launch_bounds__(kBinThreads, (C <= 4 ? kScatterMinBlocks : kScatter
                     r.u = uv.x, r.v = uv.y, r.z = uv.z, r.ps = uv.w, r.ok = true;
                     write_entry<C>(fb, g, pr, s_cam[v], s_ebase[v] + slot[j], i, p, raw, r, d);
                 }
-                if (fb.note_entry)  // behind the entries: the slots are on their way while the points are projected again
+                if (fb.note_entry)  // behind the entries
 #pragma unroll
                     for (int j = 0; j < kSweep; ++j)
                         if (vb + j < nv) fb.note_entry[(size_t)(v0 + vb + j) * sc.N + i] = slot[j];
