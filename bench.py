@@ -171,19 +171,19 @@ def stage_bytes(stage, N, P, C, B, F, Kf, V=0):
 # gather and Adam from one view of config 3 (rasterizer_kernels_c3_6Mpts_1view_ncu_sections.md: same list density and the
 # same N as the benchmark), the binning kernels, which read every point once for all views of a call, from a quarter of the
 # points with all 8 views (binning_adam_kernels_1.5Mpts_8views_ncu_sections.md).  Traffic grows in proportion to the unit
-# count.  The scan (two passes over the list lengths) is left out of the sums.  Units: F fragments, Kf kept fragments, NB points x views, V
-# entries (visible points over all views), N points.
-# unpack_grads: 15.2 bytes per row cleared, 127.2 per row gathered (127 bytes of DRAM for a 32-byte row at a random address),
+# count.  Units: F fragments, Kf kept fragments, NB points x views, PB pixels x views, V entries (visible points over all views), N points.
+# The scan's figure is that of 8 views (list lengths read, starts written; the starts of one view stay in L2).
+# unpack_grads: 15.1 bytes per row cleared, 127.2 per row gathered (127 bytes of DRAM for a 32-byte row at a random address),
 # 4 per entry index, 16 of point state and 35 of gradients per point.
-DRAM_BYTES_PER_UNIT = {"count": [(5.2, "F")], "collect": [(20.4, "F")], "sort_blend": [(34.6, "F")], "blend_backward": [(35.9, "Kf")],
-                       "bin_points": [(48.3, "NB")], "unpack_grads": [(15.2 + 127.2, "V"), (4.0, "NB"), (16.0 + 35.0, "N")],
-                       "adam": [(339.8, "N")]}
+DRAM_BYTES_PER_UNIT = {"count": [(5.2, "F")], "scan": [(5.8, "PB")], "collect": [(20.5, "F")], "sort_blend": [(34.7, "F")], "blend_backward": [(35.9, "Kf")],
+                       "bin_points": [(48.4, "NB")], "unpack_grads": [(15.1 + 127.2, "V"), (4.0, "NB"), (16.0 + 35.0, "N")],
+                       "adam": [(338.9, "N")]}
 
 
-def stage_traffic(stage, N, B, F, Kf, V=0):
+def stage_traffic(stage, N, P, B, F, Kf, V=0):
     if stage not in DRAM_BYTES_PER_UNIT:
         return None
-    units = {"F": F, "Kf": Kf, "NB": N * B, "N": N, "V": V}
+    units = {"F": F, "Kf": Kf, "NB": N * B, "PB": P * B, "N": N, "V": V}
     return sum(per * units[unit] for per, unit in DRAM_BYTES_PER_UNIT[stage])
 
 
@@ -580,10 +580,10 @@ def run_ours(args, rank, world, local_rank):
         v["gbs"] = (b_ / (v["ms_per_launch"] * 1e-3) / 1e9) if b_ else None
     total_alg = sum(bytes_of(k) for k in step_stages)
     V = stats["visible_points"]
-    dom_traffic = stage_traffic(dom, N, B, F, Kf, V)
-    total_traffic = sum(stage_traffic(k, N, B, F, Kf, V) or 0 for k in per_stage if k in step_stages)
+    dom_traffic = stage_traffic(dom, N, P, B, F, Kf, V)
+    total_traffic = sum(stage_traffic(k, N, P, B, F, Kf, V) or 0 for k in per_stage if k in step_stages)
     for k, v in per_stage.items():
-        t_ = stage_traffic(k, N, B, F, Kf, V)
+        t_ = stage_traffic(k, N, P, B, F, Kf, V)
         v["dram_gb"] = t_ / 1e9 if t_ else None
         v["traffic_over_alg"] = (t_ / bytes_of(k)) if (t_ and bytes_of(k)) else None
     roofline = {"bound": "hbm", "kernel": dom, "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
@@ -593,7 +593,7 @@ def run_ours(args, rank, world, local_rank):
                 # the whole step against the HBM roofline: algorithmic bytes of all stages / step time, and the same on measured DRAM bytes
                 "step_frac": total_alg / (ms_step * 1e-3) / 1e9 / peak,
                 "step_frac_dram": (total_traffic / (ms_step * 1e-3) / 1e9 / peak) if total_traffic else None,
-                "step_frac_dram_without": [k for k in per_stage if k in step_stages and stage_traffic(k, N, B, F, Kf, V) is None],
+                "step_frac_dram_without": [k for k in per_stage if k in step_stages and stage_traffic(k, N, P, B, F, Kf, V) is None],
                 "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum per unit of work (profiles/rasterizer_kernels_c3_6Mpts_1view_ncu_sections.md, binning_adam_kernels_1.5Mpts_8views_ncu_sections.md) x units of this run",
                 "alg_bytes_per_launch": dom_bytes,
                 "step_alg_bytes": total_alg, "step_gbs": total_alg / (ms_step * 1e-3) / 1e9, "stages": per_stage}
