@@ -61,7 +61,7 @@ constexpr int kBwdWarps   = kBwdThreads / 32;
 // tile, paired atomics, coalesced staging) and for instructions per fragment (fragment table, no shuffle searches).
 constexpr int kBwdBlocksPerSM = 12;  // grid size of the persistent kernel, in blocks per SM
 // Resident blocks: seven, and five of the variant DENSE, with 3 and 4 channels.  Seven is what 72 registers (70 with 3 channels) and 32.5 KB
-// of shared memory per block allow; the bound of six below is a minimum, and six have not been measured.  The L1 that is left holds next to
+// of shared memory per block allow; the bound of six below is a minimum, and six have not been measured with this body.  The L1 that is left holds next to
 // nothing then (1.7 % of the sectors of that view hit; 20.7 % in an earlier build with five blocks).  Where a tile's entries are few the
 // further blocks hide more latency, where they are many its rows should stay in L1 between the fragments of neighbouring pixels.
 // blend_backward, seven / five blocks, us, by visible points per pixel of layer 0: 0.8 281 / 322, 1.5 (6 M points x 8 views) 2752 / 2904,
